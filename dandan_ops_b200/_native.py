@@ -40,6 +40,8 @@ _SIGNATURES = {
     "b2_w4a16_repack": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp]),
     "b2_w4a16_unrepack": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "b2_w4a16_pack": (_int, [_vp, _i64, _i64, _vp, _vp]),
+    "b2_w4a16_quantize": (_int, [_vp, _int, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "b2_w4a16_dequantize_state": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _i64, _vp]),
     "b2_w4a16_dequantize": (_int, [_vp, _i64, _i64, _vp, _i64, _vp]),
     "b2_w4a16_dequantize_fp16": (_int, [_vp, _i64, _i64, _vp, _i64, _vp]),
     "b2_w4a16_workspace_bytes": (_i64, [_i64, _i64, _i64]),
@@ -91,6 +93,10 @@ def load():
 def _check(rc):
     if rc != OK:
         raise RuntimeError("b2_w4a16: " + _lib.b2_w4a16_last_error().decode())
+
+
+def _ptr(t):
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
@@ -228,6 +234,43 @@ def pack(codes):
     with torch.cuda.device(codes.device):
         out = torch.empty((n, (k + 7) // 8), dtype=torch.int32, device=codes.device)
         _check(lib.b2_w4a16_pack(codes.data_ptr(), n, k, out.data_ptr(), _stream()))
+    return out
+
+
+QUANT_NONFINITE, QUANT_STEP_NOT_FP16 = 1, 2
+
+
+def quantize(weight, want_codes=False, want_layer=True):
+    """One pass over a contiguous CUDA FP16/FP32 [N, K] weight with group size 64: (codes or None, packed or None,
+    scales, zeros, image or None, flags); `want_layer` asks for the packed words and the native image.  `flags` is a
+    one-element tensor of QUANT_* bits that the caller reads."""
+    lib = load()
+    n, k = weight.shape
+    dev = weight.device
+    size = lib.b2_w4a16_native_bytes(n, k)
+    if size <= 0:
+        raise RuntimeError("b2_w4a16: W4A16 dimensions exceed the kernel index range")
+    words, groups = (k + 7) // 8, (k + 63) // 64
+    with torch.cuda.device(dev):
+        codes = torch.empty((n, k), dtype=torch.uint8, device=dev) if want_codes else None
+        packed = torch.empty((n, words), dtype=torch.int32, device=dev) if want_layer else None
+        image = torch.empty(size, dtype=torch.uint8, device=dev) if want_layer else None
+        scales = torch.empty((n, groups), dtype=torch.float32, device=dev)
+        zeros = torch.empty((n, groups), dtype=torch.int32, device=dev)
+        flags = torch.zeros(1, dtype=torch.int32, device=dev)
+        _check(lib.b2_w4a16_quantize(weight.data_ptr(), weight.element_size() * 8, n, k, _ptr(codes), _ptr(packed),
+                                     scales.data_ptr(), zeros.data_ptr(), _ptr(image), flags.data_ptr(), _stream()))
+        return codes, packed, scales, zeros, image, flags
+
+
+def dequantize_state(packed, scales, zeros, k):
+    """Reference-layout CUDA tensors (group size 64) -> FP32 [N, K] weights."""
+    lib = load()
+    n = packed.shape[0]
+    with torch.cuda.device(packed.device):
+        out = torch.empty((n, k), dtype=torch.float32, device=packed.device)
+        _check(lib.b2_w4a16_dequantize_state(packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(), n, k,
+                                             out.data_ptr(), k, _stream()))
     return out
 
 
@@ -405,10 +448,6 @@ def silu_mul_pairs(y_pairs):
         _check(lib.b2_w4a16_silu_mul_pairs(y_pairs.data_ptr(), y_pairs.stride(0), out.data_ptr(), out.stride(0),
                                            m, n, _stream()))
     return out
-
-
-def _ptr(t):
-    return t.data_ptr() if t is not None else None
 
 
 def residual_rms_norm(x, residual, weight, eps, want_sum=True):

@@ -1,12 +1,14 @@
 """Compile the CUDA sources of this package into lib/libb2w4a16.so for sm_100a.
 
-The library is a plain C-ABI shared object (no torch headers), so one nvcc call
-builds it in a few seconds, with or without a GPU in the machine.
+The library is a plain C-ABI shared object (no torch headers); its translation units
+compile side by side, with or without a GPU in the machine.
 """
 import hashlib
 import os
 import shutil
 import subprocess
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -22,7 +24,7 @@ SHIM_STAMP = LIB_DIR / "dandan_ops_b200_C.stamp"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
 ]
 
 
@@ -54,14 +56,19 @@ def build(force=False, verbose=False):
     if not force and is_current():
         return LIB_PATH
     LIB_DIR.mkdir(exist_ok=True)
-    units = sorted(str(p) for p in CSRC.glob("*.cu"))
-    cmd = [nvcc_path(), *NVCC_FLAGS, *(["-Xptxas", "-v"] if verbose else []),
-           "-I", str(INCLUDE), "-o", str(LIB_PATH), *units]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
-    if verbose:
-        print(proc.stdout + proc.stderr)
+    def nvcc(*args):
+        proc = subprocess.run([nvcc_path(), *NVCC_FLAGS, *args], capture_output=True, text=True)
+        if proc.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
+        if verbose:
+            print(proc.stdout + proc.stderr)
+
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor(4) as pool:      # the units side by side, then one link
+        units = sorted(CSRC.glob("*.cu"))
+        objects = [os.path.join(tmp, u.stem + ".o") for u in units]
+        list(pool.map(lambda u, o: nvcc(*(["-Xptxas", "-v"] if verbose else []), "-I", str(INCLUDE), "-c", "-o", o, str(u)),
+                      units, objects))
+        nvcc("-shared", "-o", str(LIB_PATH), *objects)
     STAMP.write_text(source_digest() + "\n")
     return LIB_PATH
 

@@ -10,8 +10,8 @@
 #include <string>
 
 #include "../../include/b2_w4a16.h"
+#include "host_common.cuh"
 #include "layout.cuh"
-#include "layout_kernels.cuh"
 #include "stream_kernel.cuh"
 #include "stream2_kernel.cuh"
 #include "stream2d_kernel.cuh"
@@ -26,20 +26,39 @@ namespace {
 thread_local std::string g_error;
 std::atomic<int64_t> g_launches{0};
 
+}  // namespace
+
+namespace b2host {
+
 int fail(int code, const std::string& msg) {
     g_error = msg;
     return code;
 }
 
-int cuda_fail(const char* what, cudaError_t e) {
-    return fail(B2_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
-}
-
 int after_launch(const char* what) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
     const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(what, e);
+    if (e != cudaSuccess) return fail(B2_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
     return B2_OK;
+}
+
+int check_dims(int64_t n, int64_t k) {
+    if (n <= 0 || k <= 0) return fail(B2_ERR_ARGUMENT, "n and k must be positive");
+    if (k > INT_MAX - 256 || n > INT_MAX - 64 || n * k > INT_MAX)
+        return fail(B2_ERR_RANGE, "W4A16 dimensions exceed the kernel index range");
+    return B2_OK;
+}
+
+}  // namespace b2host
+
+namespace {
+
+using b2host::after_launch;
+using b2host::check_dims;
+using b2host::fail;
+
+int cuda_fail(const char* what, cudaError_t e) {
+    return fail(B2_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 struct DeviceInfo {
@@ -65,13 +84,6 @@ int device_info(DeviceInfo& out) {
         ready[dev].store(true, std::memory_order_release);
     }
     out = cache[dev];
-    return B2_OK;
-}
-
-int check_dims(int64_t n, int64_t k) {
-    if (n <= 0 || k <= 0) return fail(B2_ERR_ARGUMENT, "n and k must be positive");
-    if (k > INT_MAX - 256 || n > INT_MAX - 64 || n * k > INT_MAX)
-        return fail(B2_ERR_RANGE, "W4A16 dimensions exceed the kernel index range");
     return B2_OK;
 }
 
@@ -806,65 +818,6 @@ int b2_w4a16_set_gemm_shape(int shape, int k_splits) {
     g_forced_shape.store(shape, std::memory_order_relaxed);
     g_forced_splits.store(k_splits, std::memory_order_relaxed);
     return B2_OK;
-}
-
-int64_t b2_w4a16_native_bytes(int64_t n, int64_t k) {
-    if (check_dims(n, k) != B2_OK) return 0;
-    return b2::native_bytes(b2::make_dims(n, k));
-}
-
-int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* zeros, int64_t n,
-                    int64_t k, void* native, void* stream) {
-    if (!packed || !scales || !zeros || !native) return fail(B2_ERR_ARGUMENT, "null pointer");
-    if (int rc = check_dims(n, k)) return rc;
-    if (reinterpret_cast<uintptr_t>(native) % 256) return fail(B2_ERR_ARGUMENT, "native image must be 256-byte aligned");
-    const b2::Dims d = b2::make_dims(n, k);
-    const int64_t blocks = int64_t(d.n16) * d.kb;
-    b2::repack_kernel<<<unsigned(blocks), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        packed, scales, zeros, d, static_cast<uint8_t*>(native));
-    return after_launch("repack_kernel");
-}
-
-int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed, float* scales,
-                      int32_t* zeros, void* stream) {
-    if (!packed || !scales || !zeros || !native) return fail(B2_ERR_ARGUMENT, "null pointer");
-    if (int rc = check_dims(n, k)) return rc;
-    const b2::Dims d = b2::make_dims(n, k);
-    const int64_t total = int64_t(d.n) * d.words;
-    b2::unrepack_kernel<<<unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(native), d, packed, scales, zeros);
-    return after_launch("unrepack_kernel");
-}
-
-int b2_w4a16_pack(const uint8_t* codes, int64_t n, int64_t k, int32_t* packed, void* stream) {
-    if (!codes || !packed) return fail(B2_ERR_ARGUMENT, "null pointer");
-    if (int rc = check_dims(n, k)) return rc;
-    const b2::Dims d = b2::make_dims(n, k);
-    const int64_t total = int64_t(d.n) * d.words;
-    b2::pack_kernel<<<unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(codes, d, packed);
-    return after_launch("pack_kernel");
-}
-
-int b2_w4a16_dequantize(const void* native, int64_t n, int64_t k, float* out, int64_t ldo, void* stream) {
-    if (!native || !out) return fail(B2_ERR_ARGUMENT, "null pointer");
-    if (int rc = check_dims(n, k)) return rc;
-    if (ldo < k) return fail(B2_ERR_ARGUMENT, "ldo must be at least k");
-    const b2::Dims d = b2::make_dims(n, k);
-    const int64_t total = int64_t(d.n) * d.words;
-    b2::dequantize_kernel<float><<<unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(native), d, out, ldo);
-    return after_launch("dequantize_kernel");
-}
-
-int b2_w4a16_dequantize_fp16(const void* native, int64_t n, int64_t k, void* out, int64_t ldo, void* stream) {
-    if (!native || !out) return fail(B2_ERR_ARGUMENT, "null pointer");
-    if (int rc = check_dims(n, k)) return rc;
-    if (ldo < k) return fail(B2_ERR_ARGUMENT, "ldo must be at least k");
-    const b2::Dims d = b2::make_dims(n, k);
-    const int64_t total = int64_t(d.n) * d.words;
-    b2::dequantize_kernel<__half><<<unsigned((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(native), d, static_cast<__half*>(out), ldo);
-    return after_launch("dequantize_kernel");
 }
 
 int b2_w4a16_plan(int64_t m, int64_t n, int64_t k, int* route, int* k_splits, int* grid, int* rows_per_launch) {

@@ -1,6 +1,6 @@
-// Load-time kernels: packing, relayout between the reference tensors and the native
-// image, and the exact dequantizers.  All are plain gather/scatter kernels bound by HBM
-// traffic; none is on the per-token path.
+// Load-time kernels: packing and relayout between the reference tensors and the native
+// image.  All are plain gather/scatter kernels bound by HBM traffic; none is on the
+// per-token path.
 #pragma once
 #include "layout.cuh"
 
@@ -83,29 +83,6 @@ pack_kernel(const uint8_t* __restrict__ codes, Dims d, int32_t* __restrict__ pac
     uint32_t out = 0;
     for (int c = 0; c < valid; ++c) out |= (uint32_t(src[c]) & 15u) << (4 * c);
     packed[idx] = int32_t(out);
-}
-
-// One thread per (row, eight columns): w = fp32(code - zero) * step, one FP32 rounding,
-// optionally followed by the FP16 rounding of the linear path.
-template <typename Out>
-__global__ void __launch_bounds__(256)
-dequantize_kernel(const uint8_t* __restrict__ native, Dims d, Out* __restrict__ out, int64_t ldo) {
-    const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= int64_t(d.n) * d.words) return;
-    const int row = int(idx / d.words), cw = int(idx - int64_t(row) * d.words);
-    const WordRef w = locate(d, row, cw);
-    const uint8_t* base = native + w.block;
-    const uint32_t nat = reinterpret_cast<const uint32_t*>(base)[w.word];
-    const float step = reinterpret_cast<const float*>(base + kStepOffset)[w.meta];
-    const int zero = (base[kZeroOffset + (w.meta >> 1)] >> (4 * (w.meta & 1))) & 15;
-    const int valid = min(8, d.k - cw * 8);
-    Out* dst = out + int64_t(row) * ldo + cw * 8;
-    for (int c = 0; c < valid; ++c) {
-        const int q = int((nat >> (4 * nibble_slot(c))) & 15u);
-        const float v = __fmul_rn(float(q - zero), step);
-        if constexpr (sizeof(Out) == 2) dst[c] = __float2half_rn(v);
-        else dst[c] = v;
-    }
 }
 
 }  // namespace b2

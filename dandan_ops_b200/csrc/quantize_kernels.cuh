@@ -1,0 +1,312 @@
+// Conversion kernels between floating-point weights, the checkpoint tensors and the native image.
+//
+// quantize_kernel is bound by HBM: every weight is read once (2 or 4 bytes) and everything a layer keeps of it -
+// packed codes, FP32 step, zero point, native image - is written in the same pass.  The same steps as separate
+// elementwise and reduction passes over an FP32 copy move about forty bytes per weight.  Measured on 4096 x 12288
+// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 50 us here
+// (2.0 TB/s of input and everything written; the instructions of the range and rounding, not memory, are the rest).
+#pragma once
+#include <cfloat>
+#include <type_traits>
+#include "layout.cuh"
+
+namespace b2 {
+
+constexpr unsigned kQuantNonFinite = 1u;     // a weight is NaN or infinite
+constexpr unsigned kQuantStepNotFp16 = 2u;   // some step is not exactly representable in FP16
+
+struct QuantizeArgs {
+    const void* weight;      // [N, K] contiguous
+    uint8_t* codes;          // [N, K], may be null
+    int32_t* packed;         // [N, ceil(K/8)], may be null
+    float* scales;           // [N, ceil(K/64)]
+    int32_t* zeros;          // [N, ceil(K/64)]
+    uint8_t* native;         // native image, may be null
+    unsigned* flags;         // OR of kQuant*; zero before the launch
+    Dims d;
+};
+
+// Eight consecutive weights of a row, held as they are stored; columns >= valid are zero (they take part in the
+// range, as the zero padding of the reference's last group does).
+template <typename T> struct Eight;
+template <> struct Eight<float> {
+    float v[8];
+    template <bool VEC> __device__ __forceinline__ void load(const float* src, int valid) {
+        if (VEC && valid > 0) {            // K % 8 == 0: a word is whole or absent
+            const float4 a = __ldcs(reinterpret_cast<const float4*>(src)), b = __ldcs(reinterpret_cast<const float4*>(src) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = c < valid ? __ldg(src + c) : 0.0f;
+        }
+    }
+    __device__ __forceinline__ void range(float& lo, float& hi, bool& finite) const {
+        float poison = 0.0f;                                 // NaN as soon as one weight is not finite
+        lo = hi = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            lo = fminf(lo, v[c]);
+            hi = fmaxf(hi, v[c]);
+            poison = fmaf(v[c], 0.0f, poison);
+        }
+        finite = finite && poison == 0.0f;
+    }
+    __device__ __forceinline__ void widen(float (&f)[8]) const {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) f[c] = v[c];
+    }
+};
+template <> struct Eight<__half> {
+    uint32_t p[4];
+    template <bool VEC> __device__ __forceinline__ void load(const __half* src, int valid) {
+        if (VEC && valid > 0) {
+            const uint4 a = __ldcs(reinterpret_cast<const uint4*>(src));
+            p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t lo = 2 * c < valid ? __half_as_ushort(__ldg(src + 2 * c)) : 0u;
+                const uint32_t hi = 2 * c + 1 < valid ? __half_as_ushort(__ldg(src + 2 * c + 1)) : 0u;
+                p[c] = lo | hi << 16;
+            }
+        }
+    }
+    __device__ __forceinline__ __half2 pair(int c) const { return *reinterpret_cast<const __half2*>(&p[c]); }
+    __device__ __forceinline__ void range(float& lo, float& hi, bool& finite) const {      // two weights per instruction
+        const __half2 zero = __half2half2(__ushort_as_half(0));
+        __half2 l = zero, h = zero, poison = zero;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            l = __hmin2(l, pair(c));
+            h = __hmax2(h, pair(c));
+            poison = __hfma2(pair(c), zero, poison);
+        }
+        const float2 lf = __half22float2(l), hf = __half22float2(h);
+        lo = fminf(lf.x, lf.y);
+        hi = fmaxf(hf.x, hf.y);
+        finite = finite && __hbeq2(poison, zero);
+    }
+    __device__ __forceinline__ void widen(float (&f)[8]) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float2 w = __half22float2(pair(c));
+            f[2 * c] = w.x; f[2 * c + 1] = w.y;
+        }
+    }
+};
+
+// Reference word (nibble c = column c) -> native word of a whole word: even columns to the low half, odd ones to the high.
+__device__ __forceinline__ uint32_t split_nibbles(uint32_t ref) {
+    const uint32_t even = ref & 0x0F0F0F0Fu, odd = (ref >> 4) & 0x0F0F0F0Fu;
+    return __byte_perm(even | (even >> 4), odd | (odd >> 4), 0x6420);
+}
+
+__device__ __forceinline__ float reciprocal(float v) {       // to one unit in the last place
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Packed codes of eight weights: code = clamp(round_half_even(fl(fl(w / step) + zero)), 0, 15).
+//
+// The sum is first taken as w * (1 / step) + zero with the approximate reciprocal: |w / step| is at most 15 plus
+// rounding, so it is off by less than 2^-17 together with the two roundings of the definition.  Only a sum that close
+// to a half-integer can round to another code; where one of the eight is (one word in ~10^4), or where the
+// reciprocal of the step is not a normal number, the eight weights are divided.
+//
+// Rounding is an addition of 1.5 * 2^23, whose ulp is 1: exact half-to-even for sums this small, and the code is then
+// in the low mantissa bits (rintf and the float-to-int conversion run at an eighth of the rate of an addition).
+constexpr float kRoundMagic = 12582912.0f;
+__device__ __forceinline__ int code_of(float u) { return __float_as_int(u) - 0x4B400000; }
+// Appends two codes, clamped to 0..15, in front of those that `words` already holds.
+__device__ __forceinline__ uint32_t push_codes(int high, int low, uint32_t words) {
+    uint32_t r;
+    asm("cvt.pack.sat.u4.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(high), "r"(low), "r"(words));
+    return r;
+}
+__device__ __forceinline__ uint32_t quantize_word(const float (&v)[8], float step, float zero) {
+    const float inverse = reciprocal(step);
+    float off = step < 0x1p100f ? 0.0f : 1.0f;              // largest distance of a sum from the integer it rounds to
+    int q[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float t = fmaf(v[c], inverse, zero), u = __fadd_rn(t, kRoundMagic);
+        off = fmaxf(off, fabsf(__fsub_rn(t, __fsub_rn(u, kRoundMagic))));
+        q[c] = code_of(u);
+    }
+    if (off > 0.5f - 0x1p-16f) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) q[c] = code_of(__fadd_rn(__fadd_rn(__fdiv_rn(v[c], step), zero), kRoundMagic));
+    }
+    uint32_t word = 0;
+#pragma unroll
+    for (int c = 6; c >= 0; c -= 2) word = push_codes(q[c + 1], q[c], word);
+    return word;
+}
+
+// One CTA of four warps per 16 x 256 block; warp w takes the rows w, w + 4, w + 8 and w + 12, lane 8t + i word i of
+// group t.  The eight lanes of a group reduce the ranges of the four rows together: each exchange halves the number
+// of rows a lane carries, so that lane i ends with the range of row i % 4 and computes that row's step and zero
+// point (IEEE divisions are what this kernel could least afford to repeat in every lane), which the others fetch.
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(128, 8)
+quantize_kernel(const QuantizeArgs a) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const Dims& d = a.d;
+    const int nt = int(blockIdx.x) / d.kb, kb = int(blockIdx.x) - nt * d.kb;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane >> 3, wi = lane & 7;
+    const int k0 = kb * kBlockCols + lane * 8, grp = kb * 4 + t;
+    const int valid = min(8, d.k - k0);
+    Eight<T> v[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int row = nt * 16 + w + 4 * p;
+        v[p].template load<VEC>(static_cast<const T*>(a.weight) + int64_t(row) * d.k + k0, row < d.n ? valid : 0);
+    }
+    float lo[4], hi[4];
+    bool finite = true;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) v[p].range(lo[p], hi[p], finite);
+    unsigned found = finite ? 0u : kQuantNonFinite;
+    const bool b0 = wi & 1, b1 = wi & 2;
+    auto exchange = [&](float& keep, float mine, float give, int mask, bool low) {
+        const float got = __shfl_xor_sync(kAll, give, mask);
+        keep = low ? fminf(mine, got) : fmaxf(mine, got);
+    };
+#pragma unroll
+    for (int p = 0; p < 4; p += 2) {                         // rows p and p + 1 -> row p + b0
+        exchange(lo[p], b0 ? lo[p + 1] : lo[p], b0 ? lo[p] : lo[p + 1], 1, true);
+        exchange(hi[p], b0 ? hi[p + 1] : hi[p], b0 ? hi[p] : hi[p + 1], 1, false);
+    }
+    exchange(lo[0], b1 ? lo[2] : lo[0], b1 ? lo[0] : lo[2], 2, true);
+    exchange(hi[0], b1 ? hi[2] : hi[0], b1 ? hi[0] : hi[2], 2, false);
+    exchange(lo[0], lo[0], lo[0], 4, true);                  // lanes i and i + 4 hold the same row
+    exchange(hi[0], hi[0], hi[0], 4, false);
+    // two quotients and a difference, each rounded; never below the smallest normal FP32; 1 for an all-zero group
+    float my_step = fmaxf(__fsub_rn(__fdiv_rn(hi[0], 15.0f), __fdiv_rn(lo[0], 15.0f)), FLT_MIN);
+    if (hi[0] == 0.0f && lo[0] == 0.0f) my_step = 1.0f;
+    const float my_zero = fminf(fmaxf(rintf(__fdiv_rn(-lo[0], my_step)), 0.0f), 15.0f);
+    uint8_t* block = a.native ? a.native + (int64_t(kb) * d.n16 + nt) * kBlockBytes : nullptr;
+    {   // lane i < 4 of a group keeps the books of row w + 4i
+        const int r = w + 4 * (wi & 3), row = nt * 16 + r;
+        const bool real = row < d.n && grp < d.groups;
+        if (wi < 4) {
+            if (real) {
+                if (__half2float(__float2half_rn(my_step)) != my_step) found |= kQuantStepNotFp16;
+                a.scales[int64_t(row) * d.groups + grp] = my_step;
+                a.zeros[int64_t(row) * d.groups + grp] = int32_t(my_zero);
+            }
+            if (block) reinterpret_cast<float*>(block + kStepOffset)[(4 * (r & 7) + t) * 2 + (r >> 3)] = real ? my_step : 1.0f;
+        }
+        // zero points of rows r and r + 8 share a byte
+        const unsigned z = real ? unsigned(int(my_zero)) : 0u, z8 = __shfl_xor_sync(kAll, z, 2);
+        if (block && wi < 2) block[kZeroOffset + 4 * (r & 7) + t] = uint8_t(z | z8 << 4);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int r = w + 4 * p, row = nt * 16 + r;
+        const float step = __shfl_sync(kAll, my_step, (lane & 24) | p), zero = __shfl_sync(kAll, my_zero, (lane & 24) | p);
+        const bool real = row < d.n && grp < d.groups;
+        float f[8];
+        v[p].widen(f);
+        uint32_t ref = quantize_word(f, step, zero);
+        if (!VEC && valid < 8) ref &= valid > 0 ? 0xffffffffu >> (32 - 4 * valid) : 0u;
+        if (real && valid > 0) {
+            if (a.packed) a.packed[int64_t(row) * d.words + (k0 >> 3)] = int32_t(ref);
+            if (a.codes) {
+                uint8_t* dst = a.codes + int64_t(row) * d.k + k0;
+                if constexpr (VEC) {
+                    const uint32_t even = ref & 0x0F0F0F0Fu, odd = (ref >> 4) & 0x0F0F0F0Fu;
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(even, odd, 0x5140), __byte_perm(even, odd, 0x7362));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        if (c < valid) dst[c] = uint8_t((ref >> (4 * c)) & 15u);
+                }
+            }
+        }
+        if (block) {                   // rows and groups that do not exist: code 0; columns beyond K: the zero point
+            const uint32_t fill = uint32_t(int(zero));
+            const uint32_t nat = !real ? 0u : valid >= 8 ? split_nibbles(ref) : permute_word(ref, max(valid, 0), fill);
+            reinterpret_cast<uint32_t*>(block)[(2 * (r >> 3) + (wi >> 2)) * 128 + (4 * (r & 7) + t) * 4 + (wi & 3)] = nat;
+        }
+    }
+    // nearly every warp of a layer finds a step that FP16 cannot hold: only the first ones write the word
+    found = __reduce_or_sync(kAll, found);
+    if (lane == 0 && (found & ~*static_cast<volatile unsigned*>(a.flags))) atomicOr(a.flags, found);
+}
+
+__device__ __forceinline__ float dequantize_one(uint32_t code, int zero, float step) {
+    return __fmul_rn(float(int(code) - zero), step);
+}
+
+template <typename Out, int V>
+__device__ __forceinline__ void store_unit(Out* dst, const float (&v)[V]) {
+    if constexpr (V == 1) {
+        if constexpr (sizeof(Out) == 2) *dst = __float2half_rn(v[0]);
+        else *dst = v[0];
+    } else if constexpr (sizeof(Out) == 2) {           // V = 8
+        uint32_t p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            p[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        __stcs(reinterpret_cast<uint4*>(dst), make_uint4(p[0], p[1], p[2], p[3]));
+    } else {                                            // V = 4
+        __stcs(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
+    }
+}
+
+// Unit = V consecutive columns of a row, one 16-byte store (V = 1: one element, for rows that are not whole
+// units); the lanes of a warp write consecutive units.  Bound by the FP32 (FP16) stores: 6144 x 4096 to FP32, through
+// the image and with a thread per eight columns 96 us, straight from the checkpoint tensors 27 us (4.3 TB/s).  A thread takes
+// kDequantUnits units a CTA apart so that their loads are in flight together.
+// IMAGE: from the native image, else from the checkpoint tensors.
+constexpr int kDequantUnits = 4;
+template <typename Out, int V, bool IMAGE>
+__global__ void __launch_bounds__(256)
+dequantize_kernel(const uint8_t* __restrict__ native, const int32_t* __restrict__ packed, const float* __restrict__ scales,
+                  const int32_t* __restrict__ zeros, Dims d, Out* __restrict__ out, int64_t ldo) {
+    const unsigned per_row = unsigned(d.k) / V;
+    const int64_t total = int64_t(d.n) * per_row;
+    const int64_t u0 = int64_t(blockIdx.x) * (256 * kDequantUnits) + threadIdx.x;
+    uint32_t word[kDequantUnits];
+    float step[kDequantUnits];
+    int zero[kDequantUnits];
+#pragma unroll
+    for (int i = 0; i < kDequantUnits; ++i) {
+        const int64_t u = u0 + i * 256;
+        word[i] = 0; step[i] = 0.0f; zero[i] = 0;
+        if (u < total) {
+            const int row = int(unsigned(u) / per_row), col = int(unsigned(u) - unsigned(row) * per_row) * V;
+            if constexpr (IMAGE) {
+                const WordRef w = locate(d, row, col >> 3);
+                const uint8_t* base = native + w.block;
+                word[i] = __ldg(reinterpret_cast<const uint32_t*>(base) + w.word);
+                step[i] = __ldg(reinterpret_cast<const float*>(base + kStepOffset) + w.meta);
+                zero[i] = (__ldg(base + kZeroOffset + (w.meta >> 1)) >> (4 * (w.meta & 1))) & 15;
+            } else {
+                const int64_t at = int64_t(row) * d.groups + (col >> 6);
+                word[i] = uint32_t(__ldg(packed + int64_t(row) * d.words + (col >> 3)));
+                step[i] = __ldg(scales + at);
+                zero[i] = __ldg(zeros + at) & 15;          // as the image holds it
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kDequantUnits; ++i) {
+        const int64_t u = u0 + i * 256;
+        if (u >= total) break;
+        const int row = int(unsigned(u) / per_row), col = int(unsigned(u) - unsigned(row) * per_row) * V;
+        float v[V];
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            const int cc = (col & 7) + c;
+            v[c] = dequantize_one((word[i] >> (4 * (IMAGE ? nibble_slot(cc) : cc))) & 15u, zero[i], step[i]);
+        }
+        store_unit<Out, V>(out + int64_t(row) * ldo + col, v);
+    }
+}
+
+}  // namespace b2

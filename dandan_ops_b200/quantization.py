@@ -6,10 +6,11 @@ format (unsigned 4-bit codes, eight per int32 with code j in bits 4j..4j+3, one 
 step and one int32 zero point per output row and group of inputs).
 
 What differs is where the work runs.  Format conversions that touch every weight on
-a CUDA tensor go through the native library (`pack_int4`, `dequantize_int4`); the
-quantizer itself stays a sequence of individually rounded FP32 torch operations on the
-weight's own device, because its result has to match the reference bit for bit.  There
-is no CPU dequantizer: the package computes on the GPU only.
+a CUDA tensor go through the native library: the quantizer is one pass over the weight
+(`b2_w4a16_quantize`, each FP32 operation rounded as the reference rounds it), as are
+`pack_int4` and `dequantize_int4`.  CPU weights and other group sizes are quantized by a
+sequence of individually rounded FP32 torch operations.  There is no CPU dequantizer: the
+package computes on the GPU only.
 """
 import torch
 
@@ -58,6 +59,32 @@ def validate_int4_state(packed, scales, zeros, in_features, group_size=64, *, va
             raise ValueError("zero points must be in [0,15]")
 
 
+def check_weight(weight):
+    """Metadata checks of the quantizer, in the reference's order up to the one that reads values."""
+    if not isinstance(weight, torch.Tensor):
+        raise TypeError("weight must be a Tensor")
+    if weight.ndim != 2 or 0 in weight.shape:
+        raise ValueError("weight must be a non-empty [N, K] tensor")
+    if weight.dtype not in (torch.float16, torch.float32):
+        raise TypeError("weight must be float16 or float32")
+    if weight.device.type not in ("cpu", "cuda"):
+        raise ValueError("weight must be on CPU or CUDA")
+
+
+def native_quantizer(weight, group_size):
+    """Whether the one-pass CUDA quantizer takes this (checked) weight: a CUDA tensor, the kernels' group size and an
+    index range the C ABI admits."""
+    return weight.is_cuda and _positive_int(group_size) and group_size == 64 and weight.numel() < 2**31
+
+
+def read_quantizer_flags(flags):
+    """Flags of `_native.quantize` on the host (synchronizes), with the quantizer's finiteness check."""
+    found = flags.item()
+    if found & _native.QUANT_NONFINITE:
+        raise ValueError("weight must contain only finite values")
+    return found
+
+
 def quantize_int4(weight, group_size=64):
     """Asymmetric min/max uint4 quantization of a [N, K] FP16/FP32 weight.
 
@@ -67,14 +94,11 @@ def quantize_int4(weight, group_size=64):
     `hi/15 - lo/15` (dividing first keeps finite inputs finite), clamped to the smallest
     normal FP32, an all-zero group uses step 1, and rounding is half-to-even.
     """
-    if not isinstance(weight, torch.Tensor):
-        raise TypeError("weight must be a Tensor")
-    if weight.ndim != 2 or 0 in weight.shape:
-        raise ValueError("weight must be a non-empty [N, K] tensor")
-    if weight.dtype not in (torch.float16, torch.float32):
-        raise TypeError("weight must be float16 or float32")
-    if weight.device.type not in ("cpu", "cuda"):
-        raise ValueError("weight must be on CPU or CUDA")
+    check_weight(weight)
+    if native_quantizer(weight, group_size):
+        codes, _, steps, zero_points, _, flags = _native.quantize(weight.detach().contiguous(), want_codes=True, want_layer=False)
+        read_quantizer_flags(flags)
+        return codes, steps, zero_points
     if not bool(torch.isfinite(weight).all()):
         raise ValueError("weight must contain only finite values")
     _require_group_size(group_size)
@@ -145,5 +169,4 @@ def dequantize_int4(packed, scales, zeros, original_k, group_size=64):
     validate_int4_state(packed, scales, zeros, original_k, group_size)
     if not packed.is_cuda or group_size != 64:
         raise ValueError("dequantize_int4 " + CUDA_ONLY.replace(" FP16", ""))
-    image = _native.repack(packed.contiguous(), scales.contiguous(), zeros.contiguous(), original_k)
-    return _native.dequantize(image, packed.shape[0], original_k)
+    return _native.dequantize_state(packed.contiguous(), scales.contiguous(), zeros.contiguous(), original_k)

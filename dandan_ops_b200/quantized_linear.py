@@ -25,7 +25,8 @@ import torch
 
 from . import _native
 from . import ops as _ops_module
-from .quantization import CUDA_ONLY, pack_int4, quantize_int4, validate_int4_state
+from .quantization import (CUDA_ONLY, check_weight, native_quantizer, pack_int4, quantize_int4,
+                           read_quantizer_flags, validate_int4_state)
 
 BACKENDS = ("auto", "cuda", "gemv", "small", "tensorcore", "naive", "reference")
 FORMAT_VERSION = 2
@@ -126,25 +127,21 @@ class QuantizedLinear(torch.nn.Module):
         if backend not in BACKENDS:
             raise ValueError("invalid quantized backend")
         validate_int4_state(packed_weight, scales, zeros, in_features, group_size, values=True)
+        self._set_state(packed_weight, scales, zeros, in_features, group_size, bias, backend)
+        if self.packed_weight.is_cuda and group_size == 64 and not defer_image:
+            self._native_image()
+
+    def _set_state(self, packed_weight, scales, zeros, in_features, group_size, bias, backend):
+        """Attributes and buffers of a layer whose quantized state is known to be valid."""
         _check_bias(bias, packed_weight.shape[0], packed_weight.device)
-        self.in_features = in_features
-        self.out_features = packed_weight.shape[0]
-        self.group_size = group_size
-        self.backend = backend
+        # plain attributes go straight into the instance (Module.__setattr__ looks for parameters and submodules)
+        self.__dict__.update(in_features=in_features, out_features=packed_weight.shape[0], group_size=group_size,
+                             backend=backend, _image=None, _image_key=None, _image_flags=0, _bias16=None,
+                             _bias16_key=None, _checked_key=None, _checked_device=None, training=False)
         self.register_buffer("packed_weight", packed_weight.detach().contiguous())
         self.register_buffer("scales", scales.detach().contiguous())
         self.register_buffer("zeros", zeros.detach().contiguous())
         self.register_buffer("bias", None if bias is None else bias.detach().clone().contiguous())
-        self._image = None
-        self._image_key = None
-        self._image_flags = 0
-        self._bias16 = None
-        self._bias16_key = None
-        self._checked_key = None
-        self._checked_device = None
-        self.eval()
-        if self.packed_weight.is_cuda and group_size == 64 and not defer_image:
-            self._native_image()
 
     # -- construction ----------------------------------------------------------------------
     @classmethod
@@ -152,6 +149,17 @@ class QuantizedLinear(torch.nn.Module):
         """Quantize a floating-point [N, K] weight (dandan_ops/quantized_linear.py:158-165)."""
         if not isinstance(bits, int) or isinstance(bits, bool) or bits != 4:
             raise ValueError("only bits=4 is supported")
+        check_weight(weight)
+        if (native_quantizer(weight, group_size) and backend in BACKENDS and cls.__init__ is QuantizedLinear.__init__):
+            # One pass gives the state and the image of it.  Its steps are positive normal FP32 numbers and its zero
+            # points 0..15 by construction, so nothing is read back to check them.
+            with torch.no_grad():
+                _, packed, steps, zero_points, image, flags = _native.quantize(weight.detach().contiguous())
+                layer = cls.__new__(cls)                      # (built while the kernel runs)
+                torch.nn.Module.__init__(layer)
+                layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
+                layer._set_image(image, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
+            return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)
         return cls(pack_int4(codes), steps, zero_points, in_features=weight.shape[1],
@@ -215,9 +223,18 @@ class QuantizedLinear(torch.nn.Module):
         return self
 
     # -- native image ----------------------------------------------------------------------
+    def _state_key(self):
+        return (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
+                self.packed_weight._version, self.scales._version, self.zeros._version)
+
+    def _set_image(self, image, fp16_steps):
+        """Adopt an image of the current state that is complete in memory (its stream has been synchronized)."""
+        self._image, self._image_key = image, self._state_key()
+        self._image_flags = ((_native.FLAG_FP16_STEPS if fp16_steps else 0)
+                             | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0))
+
     def _native_image(self):
-        key = (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
-               self.packed_weight._version, self.scales._version, self.zeros._version)
+        key = self._state_key()
         if self._image is None or self._image_key != key:
             self._image = _native.repack(self.packed_weight, self.scales, self.zeros, self.in_features)
             self._image_key = key
@@ -243,8 +260,7 @@ class QuantizedLinear(torch.nn.Module):
                 image.numel() != _native.native_bytes(self.out_features, self.in_features):
             raise ValueError("not a native image of this layer")
         self._image = image
-        self._image_key = (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
-                           self.packed_weight._version, self.scales._version, self.zeros._version)
+        self._image_key = self._state_key()
         self._image_flags = self._layer_flags()
 
     def _bias_fp16(self):

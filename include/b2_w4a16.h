@@ -82,6 +82,19 @@ int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed,
  * Replaces pack_int4 (dandan_ops/quantization.py:85-103). */
 int b2_w4a16_pack(const uint8_t* codes, int64_t n, int64_t k, int32_t* packed, void* stream);
 
+/* Quantizes a contiguous [N,K] weight (weight_bits 16: FP16, 32: FP32) with group size 64 in one pass: packed codes
+ * (may be NULL), uint8 codes (may be NULL), FP32 steps, zero points and the native image (256-byte aligned, may be NULL).
+ * Replaces quantize_int4 and pack_int4 (dandan_ops/quantization.py:62-103), bit for bit.  *flags must be zero before the
+ * call and receives bit 0 = a weight is not finite (the results are then undefined), bit 1 = some step is not
+ * representable in FP16 (B2_FLAG_FP16_STEPS does not apply). */
+int b2_w4a16_quantize(const void* weight, int weight_bits, int64_t n, int64_t k, uint8_t* codes, int32_t* packed,
+                      float* scales, int32_t* zeros, void* native, unsigned* flags, void* stream);
+
+/* Checkpoint tensors -> FP32 weights [N,K] (row stride ldo), bit-identical to dequantize_int4
+ * (dandan_ops/quantization.py:124-143), without a native image. */
+int b2_w4a16_dequantize_state(const int32_t* packed, const float* scales, const int32_t* zeros, int64_t n, int64_t k,
+                              float* out, int64_t ldo, void* stream);
+
 /* Native image -> FP32 weights [N,K] (row stride ldo), bit-identical to
  * dequantize_int4 (dandan_ops/quantization.py:124-143). */
 int b2_w4a16_dequantize(const void* native, int64_t n, int64_t k, float* out, int64_t ldo,
