@@ -12,8 +12,9 @@ import torch
 from . import build as _build
 
 OK = 0
-ROUTE_AUTO, ROUTE_STREAM, ROUTE_TCGEN05, ROUTE_TILE = 0, 1, 2, 3
-ROUTE_NAMES = {ROUTE_STREAM: "b200_stream", ROUTE_TCGEN05: "b200_tcgen05", ROUTE_TILE: "b200_tile"}
+ROUTE_AUTO, ROUTE_STREAM, ROUTE_TCGEN05, ROUTE_TILE, ROUTE_BATCH = 0, 1, 2, 3, 4
+ROUTE_NAMES = {ROUTE_STREAM: "b200_stream", ROUTE_TCGEN05: "b200_tcgen05", ROUTE_TILE: "b200_tile",
+               ROUTE_BATCH: "b200_batch"}
 GEMM_SHAPES = {"auto": 0, "128x128": 1, "256x128": 2, "256x192": 3, "pair256": 4, "pair192": 5}
 STREAM_MAX_M = 64
 TICKET_BYTES = 32768

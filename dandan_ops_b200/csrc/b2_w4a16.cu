@@ -20,6 +20,7 @@
 #include "tile_kernel.cuh"
 #include "gather_kernel.cuh"
 #include "rmsnorm.cuh"
+#include "batch.cuh"
 
 namespace {
 
@@ -581,13 +582,31 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// B2_ROUTE_AUTO hands a batch to the tensor-memory GEMM above 64 rows, and already above 32 rows on
-// layers of at least 4096 native blocks (~10 MB): measured on the 8B/70B projections the pair
-// kernel takes 50 / 87 / 160 us for any M in 33..192 where the streaming kernel needs 63 / 126 /
-// 224 us at M = 48 (its cost grows with every 8 rows of x); at M = 32 the streaming kernel is
-// still ahead (43 / 80 / 141 us), and on small layers the two are within 15 % of each other.
+// The GEMM's share of B2_ROUTE_AUTO where the batch kernel does not apply: above 64 rows, and already above 32 rows on
+// layers of at least 4096 native blocks (~10 MB), where the pair kernel takes 50 / 87 / 160 us on the 8B/70B projections for any M
+// in 33..192 and the streaming kernel 63 / 126 / 224 us at M = 48.
 bool gemm_preferred(int64_t m, const b2::Dims& d) {
     return m > B2_STREAM_MAX_M || (m > 32 && int64_t(d.n16) * d.kb >= 4096);
+}
+
+// The batch kernel reads x by TMA; its step numbers stay far inside 32 bits.
+constexpr int64_t kBatchMaxM = 128;
+bool batch_applicable(int64_t m, const b2::Dims& d) {
+    return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 <= (int64_t(1) << 24);
+}
+
+// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of whatever ran before (us, old -> batch):
+//   9..16 rows   above 4096 native blocks, where the tile kernel stops (6144 x 4096 14.2 -> 11.4 at M = 16, 24576 x 4096
+//                28.8 -> 24.4, 57344 x 8192 94 -> 80; on 4096 x 4096 level with the tile kernel)
+//   17..32       from 4096 blocks on (4096 x 4096 12.4 -> 10.5 at M = 32, 24576 x 4096 35.8 -> 25.4; on 2048 x 4096 the streaming
+//                kernel's shorter start wins, 9.1 against 10.2)
+//   33..64       always (1024 x 2048 12.2 -> 9.3, 4096 x 4096 20.4 -> 12.6, 57344 x 8192 154 -> 91)
+//   65..128      above 4096 blocks (6144 x 4096 23.0 -> 18.2, 57344 x 8192 158 -> 119; 2048 x 4096 level with the GEMM's K-split)
+// Up to 8 rows the tile and streaming kernels are level or ahead (57344 x 8192 at M = 8: 77.7 against 79.4).
+bool batch_preferred(int64_t m, const b2::Dims& d) {
+    const int64_t blocks = int64_t(d.n16) * d.kb;
+    if (!batch_applicable(m, d)) return false;
+    return m <= 8 ? false : m <= 16 ? blocks > 4096 : m <= 32 ? blocks >= 4096 : m <= 64 ? true : blocks > 4096;
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
@@ -788,6 +807,37 @@ int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
     return vec ? launch_gemm_one<2, 192, true>(map, a, grid, s) : launch_gemm_one<2, 192, false>(map, a, grid, s);
 }
 
+// x [M <= 128, K] through the batch kernel.
+int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t m, const b2::Dims& d, void* workspace,
+              int64_t workspace_bytes, cudaStream_t s, int sms, const void* bias, int act, bool h16, bool overlap) {
+    EncodeTiledFn encode = encode_tiled();
+    if (!encode) return fail(B2_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available from the driver");
+    const b2host::BatchPlan p = b2host::plan_batch(m, d, sms);
+    if (workspace == nullptr || workspace_bytes < B2_W4A16_TICKET_BYTES + p.partial_bytes)
+        return fail(B2_ERR_WORKSPACE, "workspace smaller than b2_w4a16_workspace_bytes()");
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {cuuint64_t(d.k), cuuint64_t(m)};
+    const cuuint64_t strides[1] = {cuuint64_t(ldx) * 2};
+    const cuuint32_t box[2] = {cuuint32_t(b2::kGemmBK), cuuint32_t(p.nx)};
+    const cuuint32_t elem[2] = {1, 1};
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return fail(B2_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    b2::BatchArgs a;
+    a.native = static_cast<const uint8_t*>(native);
+    a.y = static_cast<__half*>(y);
+    a.bias = static_cast<const __half*>(bias);
+    a.tickets = static_cast<unsigned*>(workspace);
+    a.partial = reinterpret_cast<float4*>(static_cast<char*>(workspace) + B2_W4A16_TICKET_BYTES);
+    a.status = a.tickets + (B2_W4A16_TICKET_BYTES / 4 - 1);
+    a.ldy = ldy;
+    a.m = int(m); a.n = d.n; a.n16 = d.n16; a.kb = d.kb;
+    a.steps = p.steps;
+    a.act = act;
+    a.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
+    return b2host::launch_batch(p, map, a, h16, overlap, s);
+}
+
 }  // namespace
 
 extern "C" {
@@ -827,7 +877,15 @@ int b2_w4a16_plan(int64_t m, int64_t n, int64_t k, int* route, int* k_splits, in
     if (device_info(dev) != B2_OK) dev.sm_count = 148;   // planning also works without a device
     const b2::Dims d = b2::make_dims(n, k);
     const StreamPlan p = plan_stream(m > 0 ? m : 1, d, dev.sm_count);
-    if (gemm_preferred(m, d) && d.k % 8 == 0) {    // assuming an aligned x, as execution_info cannot see the pointer
+    if (m > 0 && batch_preferred(m, d)) {          // assuming an aligned x, as execution_info cannot see the pointer
+        const b2host::BatchPlan bp = b2host::plan_batch(m, d, dev.sm_count);
+        if (route) *route = gemm_preferred(m, d) ? B2_ROUTE_TCGEN05 : B2_ROUTE_STREAM;     // it stands in for either family
+        if (k_splits) *k_splits = bp.max_parts;
+        if (grid) *grid = bp.grid;
+        if (rows_per_launch) *rows_per_launch = int(m);
+        return B2_OK;
+    }
+    if (gemm_preferred(m, d) && d.k % 8 == 0) {
         const GemmShape shape = gemm_shape(m, d.n, d.kb, dev.sm_count > 0 ? dev.sm_count : 148);
         if (route) *route = B2_ROUTE_TCGEN05;
         if (k_splits) *k_splits = shape.splits;
@@ -873,6 +931,8 @@ int64_t b2_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) {
     int64_t need = stream_workspace_bytes(m > 0 ? m : 1, d, dev.sm_count);
     if (gemm_preferred(m, d))     // room for the partial tiles of a K-split tensor-memory GEMM
         need = std::max(need, B2_W4A16_TICKET_BYTES + gemm_shape(m, d.n, d.kb, dev.sm_count > 0 ? dev.sm_count : 148).partial_bytes(m, d.n));
+    if (m > 0 && batch_applicable(m, d))           // partial tiles of the batch kernel (also when its route is asked for)
+        need = std::max(need, B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes);
     return need;
 }
 
@@ -974,6 +1034,9 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
+    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d) && gemm_applicable(x, ldx, d) &&
+        workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes)
+        route = B2_ROUTE_BATCH;
     if (route == B2_ROUTE_AUTO)
         route = tile_applicable(m, d, tile_split) ? B2_ROUTE_TILE
               : (gemm_preferred(m, d) && gemm_applicable(x, ldx, d)) ? B2_ROUTE_TCGEN05 : B2_ROUTE_STREAM;
@@ -1000,6 +1063,12 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
         if (workspace_bytes < B2_W4A16_TICKET_BYTES)
             return fail(B2_ERR_WORKSPACE, "workspace smaller than b2_w4a16_workspace_bytes()");
         return run_gemm(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count, bias, act, h16);
+    }
+    if (route == B2_ROUTE_BATCH) {
+        if (!batch_applicable(m, d) || !gemm_applicable(x, ldx, d))
+            return fail(B2_ERR_UNSUPPORTED, "the batch route needs M <= 128, K % 8 == 0 and a 16-byte aligned x");
+        return run_batch(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count,
+                         bias, act, h16, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
     }
     return fail(B2_ERR_UNSUPPORTED, "unknown route");
 }
@@ -1096,7 +1165,7 @@ int b2_w4a16_silu_mul_is_fused(int64_t m, int64_t n, int64_t k) {
     DeviceInfo dev;
     if (device_info(dev) != B2_OK) dev.sm_count = 148;
     const b2::Dims d = b2::make_dims(n, k);
-    if (d.k % 8 != 0) return 1;                            // the streaming kernel in chunks of 64 rows
+    if (d.k % 8 != 0 || batch_preferred(m, d)) return 1;   // the streaming kernel in chunks of 64 rows, or the batch kernel
     return gemm_shape_for_call(m, d, dev.sm_count > 0 ? dev.sm_count : 148, INT64_MAX).pair_mt != 0 ? 1 : 0;
 }
 

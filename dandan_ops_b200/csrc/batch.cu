@@ -1,0 +1,69 @@
+// Launch plan and launch of the batch kernel (batch_kernel.cuh).
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
+
+#include "../../include/b2_w4a16.h"
+#include "batch.cuh"
+#include "host_common.cuh"
+
+namespace {
+
+// A CTA's share of a small layer: below this many steps the hand-over of partial tiles costs more than the shorter range gives.
+constexpr int kMinSteps = 6;
+
+template <int NX, bool H16>
+int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
+    auto kernel = b2::w4a16_batch_kernel<NX, H16>;
+    constexpr int smem = b2::batch_smem_bytes(NX);
+    static std::atomic<uint64_t> configured{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return b2host::fail(B2_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(b2::kBatchThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xmap, a);
+    if (e != cudaSuccess) return b2host::fail(B2_ERR_CUDA, std::string("w4a16_batch_kernel: ") + cudaGetErrorString(e));
+    return b2host::after_launch("w4a16_batch_kernel");
+}
+
+}  // namespace
+
+namespace b2host {
+
+BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
+    BatchPlan p;
+    p.nx = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows, tsteps = d.kb * 4;
+    const int64_t steps = int64_t(tiles) * tsteps;
+    p.steps = int(steps);
+    p.grid = int(std::max<int64_t>(1, std::min<int64_t>(sm_count > 0 ? sm_count : 148, std::max<int64_t>(tiles, steps / kMinSteps))));
+    const int64_t per_cta = std::max<int64_t>(1, steps / p.grid);
+    p.max_parts = int(std::min<int64_t>(p.grid, (tsteps + per_cta - 1) / per_cta + 1));
+    p.partial_bytes = b2::batch_partial_bytes(p.nx, p.grid);
+    return p;
+}
+
+int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool h16, bool overlap, cudaStream_t s) {
+    switch (p.nx) {
+        case 16: return h16 ? launch_one<16, true>(xmap, a, p.grid, overlap, s) : launch_one<16, false>(xmap, a, p.grid, overlap, s);
+        case 32: return h16 ? launch_one<32, true>(xmap, a, p.grid, overlap, s) : launch_one<32, false>(xmap, a, p.grid, overlap, s);
+        case 64: return h16 ? launch_one<64, true>(xmap, a, p.grid, overlap, s) : launch_one<64, false>(xmap, a, p.grid, overlap, s);
+        default: return h16 ? launch_one<128, true>(xmap, a, p.grid, overlap, s) : launch_one<128, false>(xmap, a, p.grid, overlap, s);
+    }
+}
+
+}  // namespace b2host

@@ -1,0 +1,399 @@
+// Batch kernel: a weight-streaming projection on the 5th-generation tensor cores for up to 128 rows of x.
+//
+// At these batch sizes every weight is used once per launch, so the work is to fetch the image and to decode it; the
+// streaming kernel does that too, but its mma.sync products cost as much again as the decoding from 17 rows of x on
+// (eight per fragment at 64 rows).  Here the decoded weights go to tensor memory as the A operand of one
+// tcgen05.mma per 16 columns of K, issued by a single thread and the same instruction whatever the number of rows:
+//
+//   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x)
+//     += A[n][k] (weights, FP16, tensor memory, written by the converter warps) * B[m][k] (x, shared memory, TMA)
+//
+// Work split ("stream-K"): the layer is cut into steps = (tile of 128 weight rows) x (64 columns of K), numbered
+// tile by tile and dealt out in equal contiguous ranges to one persistent CTA per SM (a block of 256 columns that two
+// CTAs share is fetched and decoded by both, each multiplying its own steps).  A tile that several CTAs share is added up
+// by the last of them to arrive (a ticket per tile and warp, nobody waits), in CTA order, so the result does not depend
+// on which that is.
+//
+// Roles (20 warps):
+//   warp 0      bulk copies of the raw blocks: one copy per 256 columns of K (8 native blocks, contiguous)
+//   warp 1      issues the MMAs, one wait and one commit per block (256 columns)
+//   warp 2      TMA loads of x, one tile of NX rows x 64 columns per step
+//   warp 3      allocates and frees tensor memory
+//   warps 4..19 converters: of the four warps of a tensor-memory lane quadrant two take the even blocks and two the odd
+//               ones, two quantization groups (64 columns) each; then the same warps read the accumulators back,
+//               NX / 4 columns each.  The accumulator is double-buffered and a tile's epilogue runs after the warp's
+//               first block of a later tile, so the tensor cores are through with the tile by then and have work
+//               while it is read.
+//
+// Lane l of quadrant q holds weight row 32q + 16 (l & 1) + 8 hi8 + g of the tile: neighbouring lanes read from two blocks
+// and two row pairs, which makes the 16-byte reads of the codes two-way bank conflicts (four-way in row order).
+//
+// Barriers (bounded waits; a role that gives up raises the CTA's abort flag and the others leave):
+//   raw_full/raw_free[r]  bulk copy of a block landed / its converter warps have read it
+//   full[b % R]           the x tiles (bytes) and the eight converter warps' weights of block b are in place
+//   done[b % R]           tcgen05.commit: the MMAs of block b have completed
+//   acc_full/acc_free[b]  accumulator b complete (commit) / read by all converter warps
+#pragma once
+#include "gemm_kernel.cuh"
+
+namespace b2 {
+
+constexpr int kBatchRows = 128;                     // weight rows per tile
+constexpr int kBatchBlocks = kBatchRows / 16;       // native blocks per 256 columns
+constexpr int kBatchRawBytes = kBatchBlocks * kBlockBytes;
+constexpr int kBatchWarps = 16;                     // converters
+constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
+constexpr uint32_t kBatchWCols = 32;                // tensor-memory columns of a step's weights
+constexpr int kBatchTickets = kBatchWarps;          // per split tile
+// Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside two accumulators.
+__host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; }
+__host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
+__host__ __device__ constexpr int batch_raw_stages(int nx) {
+    const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx) * batch_x_bytes(nx)) / kBatchRawBytes;
+    return fit < 8 ? fit : 8;
+}
+__host__ __device__ constexpr int batch_smem_bytes(int nx) {
+    return 1024 + 4 * batch_ring(nx) * batch_x_bytes(nx) + batch_raw_stages(nx) * kBatchRawBytes + 512;
+}
+// Bytes of all partial tiles of a launch: a CTA has at most two tiles that it shares.
+__host__ __device__ constexpr int64_t batch_partial_bytes(int nx, int grid) { return int64_t(grid) * 2 * nx * kBatchRows * 4; }
+
+struct BatchArgs {
+    const uint8_t* native;
+    __half* y;
+    const __half* bias;     // optional [N] FP16 (may be null)
+    float4* partial;        // [CTA][first or last tile][NX / 4][128 weight rows] x 4 columns
+    unsigned* tickets;      // [CTA][warp], zero on entry and on exit
+    unsigned* status;
+    int64_t ldy;
+    int m, n;
+    int n16, kb;
+    int steps;              // tiles * kb * 4
+    int act;                // as StreamArgs::act
+    int wait_limit;
+};
+
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// CW accumulator columns of this thread's lane (4, 8 or 16).
+template <int CW>
+__device__ __forceinline__ void batch_ld(uint32_t taddr, float (&f)[CW]) {
+    uint32_t v[CW];
+    if constexpr (CW == 4) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
+    } else if constexpr (CW == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(taddr) : "memory");
+    } else {
+        static_assert(CW == 16, "4, 8 or 16 columns");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                       "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                     : "r"(taddr) : "memory");
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < CW; ++i) f[i] = __uint_as_float(v[i]);
+}
+
+// First step of CTA c's range, and the CTA whose range contains step s.
+__host__ __device__ inline int batch_begin(int steps, int ctas, int c) { return int((int64_t(steps) * c) / ctas); }
+__device__ __forceinline__ int batch_owner(int s, int steps, int ctas) { return int((int64_t(s + 1) * ctas - 1) / steps); }
+
+template <int NX, bool H16>
+__global__ void __launch_bounds__(kBatchThreads, 1)
+w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
+    constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
+    constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
+    static_assert(2 * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* x_base = smem;                                                // [R][4][kXBytes]
+    uint8_t* raw_base = x_base + R * kXStage;                              // [RS][18688]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes);
+    constexpr int RAW_FULL = 0, RAW_FREE = RAW_FULL + RS, FULL = RAW_FREE + RS, DONE = FULL + R, ACC_FULL = DONE + R,
+                  ACC_FREE = ACC_FULL + 2, NBARS = ACC_FREE + 2;
+    static_assert(NBARS * 8 + 8 <= 512, "barrier area");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t bar0 = smem_u32(bars);
+    auto bar = [&](int i) { return bar0 + i * 8; };
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ctas = gridDim.x;
+    const int b0 = batch_begin(a.steps, ctas, blockIdx.x), nsteps = batch_begin(a.steps, ctas, blockIdx.x + 1) - b0;
+    const int tsteps = a.kb * 4;                                           // steps of a tile
+    const int gb0 = b0 >> 2, nblocks = ((b0 + nsteps - 1) >> 2) - gb0 + 1; // blocks of 8 x 256 columns, tile by tile
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < RS; ++i) { mbar_init(bar(RAW_FULL + i), 1); mbar_init(bar(RAW_FREE + i), kBatchWarps / 2); }
+        for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + kBatchWarps / 2); mbar_init(bar(DONE + i), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 3) tmem_alloc(smem_u32(tmem_slot), 512);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // Bounded; the lanes of a warp go on or leave together.
+    auto wait = [&](int idx, uint32_t parity) -> bool {
+        const uint32_t at = bar(idx);
+        if (__all_sync(0xffffffffu, mbar_try_wait(at, parity))) return true;
+        for (int i = 1; i < a.wait_limit; ++i) {
+            if (__all_sync(0xffffffffu, mbar_try_wait_long(at, parity))) return true;
+            if ((i & 63) == 63 && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        }
+        if (lane == 0) {
+            *abort_flag = 1;
+            atomicOr(a.status, kStatusGemmTimeout);
+        }
+        return false;
+    };
+
+    if (warp == 0) {
+        // ------------------------------ raw blocks ---------------------------------------
+        int tile = gb0 / a.kb, kb = gb0 - tile * a.kb, issued = 0;
+        for (; issued < nblocks; ++issued) {
+            const int r = issued % RS;
+            if (issued >= RS && !wait(RAW_FREE + r, ((issued / RS) - 1) & 1)) break;
+            if (elect_one()) {
+                const uint32_t bytes = uint32_t(min(kBatchBlocks, a.n16 - tile * kBatchBlocks)) * kBlockBytes;
+                mbar_expect_tx(bar(RAW_FULL + r), bytes);
+                bulk_copy_g2s(smem_u32(raw_base + r * kBatchRawBytes),
+                              a.native + (int64_t(kb) * a.n16 + tile * kBatchBlocks) * kBlockBytes, bytes, bar(RAW_FULL + r));
+            }
+            __syncwarp();
+            if (++kb == a.kb) { kb = 0; ++tile; }
+        }
+        // after an abort: the last copies land before the shared memory is released
+        for (int i = max(0, issued - RS); i < issued; ++i)
+            for (int p = 0; p < 4096 && !mbar_try_wait(bar(RAW_FULL + i % RS), (i / RS) & 1); ++p) {}
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer ---------------------------------------
+        // D = F32, A = B = F16, both K-major, M = 128 weight rows, N = NX rows of x
+        const uint32_t idesc = (1u << 4) | (uint32_t(NX >> 3) << 17) | (uint32_t(kBatchRows >> 4) << 24);
+        const uint64_t desc0 = umma_desc_sw128(smem_u32(x_base));
+        int left = a.kb - gb0 % a.kb;                 // blocks to the end of the tile
+        int seg = 0;
+        bool fresh = true;                            // the accumulator starts with this block
+        for (int b = 0; b < nblocks; ++b) {
+            const int slot = b % R;
+            if (fresh && seg >= 2 && !wait(ACC_FREE + (seg & 1), ((seg >> 1) - 1) & 1)) break;
+            if (!wait(FULL + slot, (b / R) & 1)) break;
+            tcgen05_fence_after();
+            const bool end = --left == 0 || b == nblocks - 1;
+            if (elect_one()) {
+                const uint32_t w = tmem_base + kWBase + slot * kWStage, d = tmem_base + (seg & 1) * NX;
+                const uint64_t desc = desc0 + uint64_t((slot * kXStage) >> 4);
+                uint32_t accumulate = fresh ? 0u : 1u;
+                auto step = [&](int t) {
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        umma_f16_ts(d, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc, accumulate);
+                        accumulate = 1;
+                    }
+                };
+                const int t0 = b == 0 ? b0 & 3 : 0, t1 = b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;     // steps of the range in this block
+                if (t0 == 0 && t1 == 3) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) step(t);
+                } else {
+#pragma unroll 1
+                    for (int t = t0; t <= t1; ++t) step(t);
+                }
+                umma_commit(bar(DONE + slot));
+                if (end) umma_commit(bar(ACC_FULL + (seg & 1)));
+            }
+            __syncwarp();
+            fresh = end;
+            if (end) {
+                ++seg;
+                left = a.kb;
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------ x tiles ------------------------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int kb = gb0 % a.kb;
+        for (int b = 0; b < nblocks; ++b) {
+            const int slot = b % R;
+            if (b >= R && !wait(DONE + slot, ((b / R) - 1) & 1)) break;
+            if (elect_one()) {
+                const int t0 = b == 0 ? b0 & 3 : 0, t1 = b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
+                mbar_expect_tx(bar(FULL + slot), uint32_t(t1 - t0 + 1) * kXBytes);
+                for (int t = t0; t <= t1; ++t)
+                    tma_load_2d(smem_u32(x_base + slot * kXStage + t * kXBytes), &xmap, (kb * 4 + t) * kGemmBK, 0, bar(FULL + slot));
+            }
+            __syncwarp();
+            if (++kb == a.kb) kb = 0;
+        }
+        for (int p = 0; p < 64 && *abort_flag; ++p) __nanosleep(2000);      // after an abort: loads in flight land first
+    } else if (warp >= 4) {
+        // ------------------------------ converters ---------------------------------------
+        const int quad = warp & 3, u = (warp - 4) >> 2, v = u & 1, set = u >> 1;
+        const int blk = lane & 1, hi8 = (lane >> 2) & 1, g = ((lane >> 1) & 1) | ((lane >> 3) << 1);
+        const int row = quad * 32 + blk * 16 + hi8 * 8 + g;                // weight row of the tile
+        const uint32_t lane_addr = uint32_t(quad * 32) << 16;
+        const int code_at = (quad * 2 + blk) * kBlockBytes + (2 * hi8) * 512 + (4 * g + 2 * v) * 16;
+        const int step_at = (quad * 2 + blk) * kBlockBytes + kStepOffset + (4 * g + 2 * v) * 8 + hi8 * 4;
+        const int zero_at = (quad * 2 + blk) * kBlockBytes + kZeroOffset + 4 * g + 2 * v;
+        const int tile0 = b0 / tsteps;
+        constexpr int CW = NX >= 64 ? 16 : NX / 4;                         // accumulator columns per read
+        bool ok = true;
+        int read = 0;                                                      // tiles of the range that this warp has read
+
+        auto epilogue = [&](int seg) {
+            const int tile = tile0 + seg;
+            if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // bias, tickets, partial tiles, y
+            ok = ok && wait(ACC_FULL + (seg & 1), (seg >> 1) & 1);
+            if (!ok) return;
+            tcgen05_fence_after();
+            const int t0 = tile * tsteps, t1 = t0 + tsteps;
+            const bool whole = b0 <= t0 && t1 <= b0 + nsteps;
+            const int first = whole ? 0 : batch_owner(t0, a.steps, ctas), last = whole ? 0 : batch_owner(t1 - 1, a.steps, ctas);
+            const uint32_t acc = tmem_base + lane_addr + (seg & 1) * NX + u * (NX / 4);
+            auto slot_of = [&](int c) {                                    // partial tile of CTA c, this warp's columns and lanes
+                return a.partial + ((int64_t(c) * 2 + (c == first ? 1 : 0)) * (NX / 4) + u * (NX / 16)) * kBatchRows + quad * 32 + lane;
+            };
+            bool mine = whole;
+            if (!whole) {
+                float4* dst = slot_of(int(blockIdx.x));
+#pragma unroll
+                for (int c0 = 0; c0 < NX / 4; c0 += CW) {
+                    float f[CW];
+                    batch_ld<CW>(acc + c0, f);
+#pragma unroll
+                    for (int q = 0; q < CW / 4; ++q)
+                        if (u * (NX / 4) + c0 + 4 * q < a.m)
+                            __stcg(dst + (c0 / 4 + q) * kBatchRows, make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]));
+                }
+                tcgen05_fence_before();
+                __threadfence();
+                __syncwarp();
+                unsigned prior = 0;
+                unsigned* ticket = a.tickets + first * kBatchTickets + (warp - 4);
+                if (lane == 0) {
+                    mbar_arrive(bar(ACC_FREE + (seg & 1)));
+                    prior = atomicAdd(ticket, 1u);
+                    if (prior == unsigned(last - first)) *ticket = 0u;
+                }
+                mine = __shfl_sync(0xffffffffu, prior, 0) == unsigned(last - first);
+                if (mine) __threadfence();
+            }
+            if (mine) {
+                const int n = tile * kBatchRows + row;
+#pragma unroll
+                for (int c0 = 0; c0 < NX / 4; c0 += CW) {
+                    const int m0 = u * (NX / 4) + c0;
+                    if (m0 < a.m) {
+                        float f[CW];
+                        if (whole) {
+                            batch_ld<CW>(acc + c0, f);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < CW; ++i) f[i] = 0.0f;
+#pragma unroll 2
+                            for (int c = first; c <= last; ++c) {
+                                const float4* src = slot_of(c) + (c0 / 4) * kBatchRows;
+#pragma unroll
+                                for (int q = 0; q < CW / 4; ++q) {
+                                    if (m0 + 4 * q < a.m) {
+                                        const float4 p = __ldcg(src + q * kBatchRows);
+                                        f[4 * q] += p.x; f[4 * q + 1] += p.y; f[4 * q + 2] += p.z; f[4 * q + 3] += p.w;
+                                    }
+                                }
+                            }
+                        }
+                        if (a.act) {
+                            // lanes l and l ^ 4 hold the gate and the up sum of one output column: the gate lane
+                            // finishes the even rows of x, the up lane the odd ones
+                            const int out = (n >> 4) * 8 + g;
+#pragma unroll
+                            for (int i = 0; i < CW; i += 2) {
+                                const float theirs = __shfl_xor_sync(0xffffffffu, hi8 ? f[i] : f[i + 1], 4);
+                                const float gate = hi8 ? theirs : f[i], up = hi8 ? f[i + 1] : theirs;
+                                const int m = m0 + i + hi8;
+                                if (m < a.m && (n | 8) < a.n)
+                                    a.y[int64_t(m) * a.ldy + out] = silu_mul(finish_output(gate, a.bias, n & ~8), finish_output(up, a.bias, n | 8));
+                            }
+                        } else if (n < a.n) {
+#pragma unroll
+                            for (int i = 0; i < CW; ++i)
+                                if (m0 + i < a.m) a.y[int64_t(m0 + i) * a.ldy + n] = finish_output(f[i], a.bias, n);
+                        }
+                    }
+                }
+            }
+            if (whole) {
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(ACC_FREE + (seg & 1)));
+            }
+        };
+
+        int slot = set, r = set, seg = 0, left = a.kb - gb0 % a.kb - set;  // rings and tile of the warp's block
+        uint32_t free_parity = 1, raw_parity = 0;                          // (the first round of the stages is free)
+        for (int b = set; b < nblocks; b += 2) {
+            while (left <= 0) {
+                left += a.kb;
+                ++seg;
+            }
+            if (!(ok = wait(RAW_FULL + r, raw_parity))) break;
+            const uint8_t* raw = raw_base + r * kBatchRawBytes;
+            const uint4 code[4] = {*reinterpret_cast<const uint4*>(raw + code_at), *reinterpret_cast<const uint4*>(raw + code_at + 512),
+                                   *reinterpret_cast<const uint4*>(raw + code_at + 16), *reinterpret_cast<const uint4*>(raw + code_at + 528)};
+            const float steps[2] = {*reinterpret_cast<const float*>(raw + step_at), *reinterpret_cast<const float*>(raw + step_at + 8)};
+            const uint32_t zeros = *reinterpret_cast<const uint16_t*>(raw + zero_at) >> (4 * hi8);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const GroupConst<H16> gc = make_group<H16>((zeros >> (8 * h)) & 15u, steps[h]);
+                const uint32_t words[8] = {code[2 * h].x, code[2 * h].y, code[2 * h].z, code[2 * h].w,
+                                           code[2 * h + 1].x, code[2 * h + 1].y, code[2 * h + 1].z, code[2 * h + 1].w};
+                const uint32_t to = tmem_base + lane_addr + kWBase + slot * kWStage + (2 * v + h) * kBatchWCols;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 p = dequant_word<H16>(words[2 * i], gc), q = dequant_word<H16>(words[2 * i + 1], gc);
+                    if (h == 0 && i == 0) {
+                        if (!(ok = wait(DONE + slot, free_parity))) break;
+                        tcgen05_fence_after();
+                    }
+                    tmem_st8(to + 8 * i, p, q);
+                }
+                if (!ok) break;
+            }
+            if (!ok) break;
+            tmem_st_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bar(FULL + slot));
+                if (b + RS < nblocks) mbar_arrive(bar(RAW_FREE + r));      // the last copies are not waited for
+            }
+            while (read < seg && ok) epilogue(read++);
+            if (!ok) break;
+            left -= 2;
+            if ((slot += 2) >= R) { slot -= R; free_parity ^= 1; }
+            if ((r += 2) >= RS) { r -= RS; raw_parity ^= 1; }
+        }
+        const int segs = (b0 + nsteps - 1) / tsteps - tile0 + 1;
+        while (read < segs && ok) epilogue(read++);
+    }
+    __syncwarp();
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 3) {
+        tcgen05_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+}  // namespace b2

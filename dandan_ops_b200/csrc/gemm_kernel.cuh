@@ -73,6 +73,13 @@ struct GemmArgs {
 };
 
 // ---- tcgen05 / TMA helpers ----------------------------------------------------------------
+// True in one lane of a converged warp.  (With a test of the lane number instead the compiler cannot tell that a single
+// thread executes the tensor-core instructions and their uniform operands are rebuilt around every one of them.)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
@@ -94,6 +101,13 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// 8 registers -> 8 columns of this thread's tensor-memory lane (complete after tmem_st_wait).  Small stores on purpose: with
+// the 32 registers of one 32-column store the compiler moves most of the decoded pairs once more to make them adjacent.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& p, const uint4& q) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(p.x), "r"(p.y), "r"(p.z), "r"(p.w), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                  "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"

@@ -74,7 +74,7 @@ __host__ __device__ constexpr int stream_smem_bytes(int w) {
     return stream_bar_bytes(w) + stream_ring_bytes(w) + stream_x_bytes(w) + kStreamZeroBytes;
 }
 constexpr unsigned kStatusCopyTimeout = 1u;
-constexpr int kWaitLimit = 1 << 20;          // mbarrier polls before a warp gives up
+constexpr int kWaitLimit = 1 << 16;          // mbarrier polls (of kWaitHint ns at most) before a warp gives up
 
 struct StreamArgs {
     const __half* x;        // [M, K], row stride ldx
@@ -332,11 +332,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
-// Bounded wait: false if the phase did not complete within kWaitLimit polls.
+// The same, suspended for up to kWaitHint ns until the phase completes: without the hint a waiting warp is back after a few
+// dozen cycles, and the polls of three waiting role warps were a quarter of all instructions of the batch kernel.
+constexpr uint32_t kWaitHint = 20000;
+__device__ __forceinline__ bool mbar_try_wait_long(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity), "r"(kWaitHint) : "memory");
+    return done != 0;
+}
+// Bounded wait: false if the phase did not complete within `limit` polls.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int limit = kWaitLimit) {
     if (mbar_try_wait(bar, parity)) return true;           // the common case costs no loop bookkeeping
     for (int i = 1; i < limit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait_long(bar, parity)) return true;
     return false;
 }
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {

@@ -37,12 +37,13 @@ extern "C" {
 #define B2_ERR_UNSUPPORTED 5 /* device is not sm_100 or the requested route does not apply */
 
 /* Kernel families selectable through b2_w4a16_linear_route(). */
-#define B2_ROUTE_AUTO 0      /* by size: tile kernel for M <= 16 on layers up to ~10 MB, streaming kernel up to
-                                B2_STREAM_MAX_M rows (32 rows on layers above ~10 MB), tensor-memory GEMM above */
+#define B2_ROUTE_AUTO 0      /* by size: tile and streaming kernel up to 8 rows (32 on layers below ~10 MB), batch kernel up to 64
+                                rows (128 on layers above ~10 MB), tensor-memory GEMM above */
 #define B2_ROUTE_STREAM 1    /* persistent weight-streaming kernel (any M, re-reads the weights every 64 rows) */
 #define B2_ROUTE_TCGEN05 2   /* TMA + tcgen05 GEMM with in-kernel INT4->FP16 converter */
 #define B2_ROUTE_TILE 3      /* one CTA (or a cluster of 2 or 4 CTAs that split K) per 16-row tile, the whole K range
                                 in flight at once (M <= 16; K as far as it fits in shared memory) */
+#define B2_ROUTE_BATCH 4     /* persistent weight-streaming kernel with tcgen05 products (M <= 128, K % 8 == 0, aligned x) */
 
 /* Largest M the weight-streaming kernel takes in one launch; B2_ROUTE_AUTO hands larger
  * batches to the tensor-memory GEMM. */
@@ -237,7 +238,8 @@ int b2_w4a16_residual_rms_norm(const void* x, int64_t ldx, const void* residual,
 int b2_w4a16_silu_mul_pairs(const void* y_pairs, int64_t ld_in, void* out, int64_t ld_out, int64_t m, int64_t n,
                             void* stream);
 
-/* Which kernel family B2_ROUTE_AUTO picks for this problem (a B2_ROUTE_* value) and,
+/* Which kernel family B2_ROUTE_AUTO picks for this problem (a B2_ROUTE_* value; the batch kernel counts to the
+ * family whose batches it takes: streaming, or tensor-memory GEMM above 32 rows of a layer above ~10 MB) and,
  * through the optional out-parameters, the launch plan: K-splits, grid size, rows of x
  * handled per launch.  Pure host arithmetic; used by execution_info(). */
 int b2_w4a16_plan(int64_t m, int64_t n, int64_t k, int* route, int* k_splits, int* grid,

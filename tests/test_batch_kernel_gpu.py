@@ -1,0 +1,95 @@
+"""w4a16_batch_kernel (up to 128 rows of x, products on tcgen05): against the CPU oracle and, on its other forms, against
+the routes it stands in for, at the sizes where tiles, ranges and rings end."""
+import pytest
+import torch
+
+import dandan_ops_b200 as ops
+from dandan_ops_b200 import _native
+from oracle import w4a16_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+BATCH = _native.ROUTE_BATCH
+
+
+def _layer(n, k, seed, fp16_steps=False):
+    g = torch.Generator().manual_seed(seed)
+    layer = ops.QuantizedLinear.from_float((torch.randn(n, k, generator=g) * 0.02).half().cuda())
+    if fp16_steps:
+        layer = ops.QuantizedLinear(layer.packed_weight, layer.scales.half().float(), layer.zeros, in_features=k)
+    return layer, g
+
+
+@pytest.mark.parametrize("m,n,k,fp16_steps", [
+    (1, 8, 8, False),            # one partial tile, one partial step
+    (16, 128, 256, False),       # one whole tile in one block, fewer steps than CTAs
+    (17, 136, 1032, True),       # a second tile of one row tile, ragged K
+    (32, 1000, 520, False),
+    (33, 129, 64, False),        # one row in the last tile, one group of the block
+    (64, 2048, 1024, True),      # tiles shared by several CTAs
+    (65, 384, 8192, False),      # K much longer than a CTA's range
+    (100, 1536, 2056, False),
+    (128, 20000, 128, False),    # several one-block tiles per CTA
+])
+def test_against_the_oracle(m, n, k, fp16_steps):
+    layer, g = _layer(n, k, m + n + k, fp16_steps)
+    x = torch.randn(m, k, generator=g).half()
+    bias = torch.randn(n, generator=g).half().cuda()
+    image, flags = layer._native_image(), layer._image_flags
+    assert bool(flags & _native.FLAG_FP16_STEPS) == fp16_steps
+    y = _native.linear(x.cuda(), image, n, k, route=BATCH, flags=flags)
+    assert torch.equal(y, _native.linear(x.cuda(), image, n, k, route=BATCH, flags=flags & ~_native.FLAG_OVERLAP_LAUNCH))
+    assert torch.equal(y + bias, _native.linear(x.cuda(), image, n, k, route=BATCH, bias=bias, flags=flags))
+    words, step, zero = (t.cpu().numpy() for t in (layer.packed_weight, layer.scales, layer.zeros))
+    rows = sorted({0, m // 2, m - 1})                                    # (the oracle is slow)
+    assert oracle.within_tolerance(y[rows].cpu().numpy(), oracle.linear(x[rows].numpy(), words, step, zero, k))
+    # every row and column: FP64 product of the same FP16 weights, one FP16 rounding apart at most where sums round differently
+    exact = x.double() @ layer.dequantize().half().double().cpu().t()
+    assert ((y.cpu().double() - exact).abs() <= 2e-3 + 2e-3 * exact.abs()).all()
+    assert _native.status() == 0
+
+
+def test_row_strides_of_x_and_y():
+    layer, g = _layer(1000, 520, 5)
+    wide = torch.randn(48, 536, generator=g).half().cuda()
+    out = torch.full((48, 1010), 7.0, dtype=torch.float16, device="cuda")
+    want = _native.linear(wide[:, 8:528].contiguous(), layer._native_image(), 1000, 520, route=BATCH)
+    _native.linear(wide[:, 8:528], layer._native_image(), 1000, 520, route=BATCH, out=out[:, 3:1003])
+    assert torch.equal(out[:, 3:1003], want) and bool((out[:, :3] == 7).all()) and bool((out[:, 1003:] == 7).all())
+
+
+@pytest.mark.parametrize("m,rows,k", [(33, 72, 264), (64, 1536, 1024), (12, 32768, 256), (128, 32768, 512)])
+def test_gate_up_epilogue_matches_the_separate_kernel(m, rows, k):
+    """The automatic route takes the batch kernel on these; the activation sees the same sums in the same order."""
+    gate, g = _layer(rows, k, 1)
+    up, _ = _layer(rows, k, 2)
+    fused = ops.GateUpSilu(gate, up)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    pairs = _native.linear(x, fused.op._native_image(), 2 * rows, k, route=BATCH)
+    assert torch.equal(fused(x), _native.silu_mul_pairs(pairs))
+
+
+def test_dependent_launches_on_shared_scratch():
+    """Programmatic dependents: every call reads the previous one's output and shares its tickets and partial tiles."""
+    layers = [_layer(2048, 2048, s)[0] for s in range(5)]
+    x = torch.randn(40, 2048, generator=torch.Generator().manual_seed(9)).half().cuda()
+
+    def chain(flags):
+        cur = x
+        for layer in layers:
+            cur = _native.linear(cur, layer._native_image(), 2048, 2048, route=BATCH, flags=flags)
+        return cur
+
+    want = chain(0)
+    for _ in range(10):
+        assert torch.equal(chain(_native.FLAG_OVERLAP_LAUNCH), want)
+
+
+def test_what_the_route_refuses():
+    layer, _ = _layer(64, 520, 3)
+    x = torch.zeros(129, 520, dtype=torch.float16, device="cuda")
+    with pytest.raises(RuntimeError, match="batch route"):
+        _native.linear(x, layer._native_image(), 64, 520, route=BATCH)
+    odd = torch.zeros(40 * 520 + 1, dtype=torch.float16, device="cuda")[1:].view(40, 520)      # not 16-byte aligned
+    with pytest.raises(RuntimeError, match="batch route"):
+        _native.linear(odd, layer._native_image(), 64, 520, route=BATCH)
+    assert torch.equal(_native.linear(odd, layer._native_image(), 64, 520), torch.zeros(40, 64, dtype=torch.float16, device="cuda"))
