@@ -589,24 +589,27 @@ bool gemm_preferred(int64_t m, const b2::Dims& d) {
     return m > B2_STREAM_MAX_M || (m > 32 && int64_t(d.n16) * d.kb >= 4096);
 }
 
-// The batch kernel reads x by TMA; its step numbers stay far inside 32 bits.
+// The batch kernel reads x by TMA; the product of its steps and CTAs stays inside 32 bits.
 constexpr int64_t kBatchMaxM = 128;
 bool batch_applicable(int64_t m, const b2::Dims& d) {
-    return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 <= (int64_t(1) << 24);
+    return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 < (int64_t(1) << 23);
 }
 
-// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of whatever ran before (us, old -> batch):
-//   9..16 rows   above 4096 native blocks, where the tile kernel stops (6144 x 4096 14.2 -> 11.4 at M = 16, 24576 x 4096
-//                28.8 -> 24.4, 57344 x 8192 94 -> 80; on 4096 x 4096 level with the tile kernel)
-//   17..32       from 4096 blocks on (4096 x 4096 12.4 -> 10.5 at M = 32, 24576 x 4096 35.8 -> 25.4; on 2048 x 4096 the streaming
-//                kernel's shorter start wins, 9.1 against 10.2)
-//   33..64       always (1024 x 2048 12.2 -> 9.3, 4096 x 4096 20.4 -> 12.6, 57344 x 8192 154 -> 91)
-//   65..128      above 4096 blocks (6144 x 4096 23.0 -> 18.2, 57344 x 8192 158 -> 119; 2048 x 4096 level with the GEMM's K-split)
-// Up to 8 rows the tile and streaming kernels are level or ahead (57344 x 8192 at M = 8: 77.7 against 79.4).
-bool batch_preferred(int64_t m, const b2::Dims& d) {
+// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of what ran before (us, tile / streaming / GEMM -> batch):
+//   up to 8 rows above 4096 native blocks (~10 MB), where the tile kernel runs out (6144 x 4096 at M = 1 / 8 10.0 / 10.2 -> 8.9 / 9.0,
+//                4096 x 12288 14.6 -> 13.1, 12289 x 3072 12.0 / 13.1 -> 10.8; 4096 x 4096 6.0 / 6.5 against 7.3) up to 65536
+//                (8192 x 28672 45.0 / 45.6 -> 44.2 / 44.9; 57344 x 8192 at M = 1 75.9 against 77.9), with FP16 steps up to
+//                16384 (12289 x 3072 10.9 -> 9.0; 24576 x 4096 19.0 against 19.9).  Below 4096 output
+//                columns the kernels that carry the all-gather stay, so that a column slice has the same bits in both forms.
+//   9..16        above 4096 blocks (6144 x 4096 at M = 16 14.2 -> 9.2, 24576 x 4096 28.8 -> 23.4, 57344 x 8192 94 -> 80;
+//                2048 x 4096 5.4 against 6.0)
+//   17..128      always (1024 x 1024 at M = 17 / 64 / 128 5.1 / 12.2 / 12.5 -> 3.9 / 4.9 / 7.3, 4096 x 4096 at M = 64 20.4 -> 10.9,
+//                57344 x 8192 at M = 64 / 128 154 / 158 -> 94 / 120)
+bool batch_preferred(int64_t m, const b2::Dims& d, bool h16 = false) {
     const int64_t blocks = int64_t(d.n16) * d.kb;
     if (!batch_applicable(m, d)) return false;
-    return m <= 8 ? false : m <= 16 ? blocks > 4096 : m <= 32 ? blocks >= 4096 : m <= 64 ? true : blocks > 4096;
+    if (m > 16) return true;
+    return blocks > 4096 && (m > 8 || (d.n >= 4096 && blocks <= (h16 ? 16384 : 65536)));
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
@@ -1034,7 +1037,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
-    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d) && gemm_applicable(x, ldx, d) &&
+    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d, h16) && gemm_applicable(x, ldx, d) &&
         workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes)
         route = B2_ROUTE_BATCH;
     if (route == B2_ROUTE_AUTO)

@@ -19,9 +19,8 @@
 //   warp 1      issues the MMAs, one wait and one commit per block (256 columns)
 //   warp 2      TMA loads of x, one tile of NX rows x 64 columns per step
 //   warp 3      allocates and frees tensor memory
-//   warps 4..19 converters: of the four warps of a tensor-memory lane quadrant two take the even blocks and two the odd
-//               ones, two quantization groups (64 columns) each; then the same warps read the accumulators back,
-//               NX / 4 columns each.  The accumulator is double-buffered and a tile's epilogue runs after the warp's
+//   warps 4..19 converters: two sets of eight warps (two per tensor-memory lane quadrant, two quantization groups each)
+//               that take the blocks in turn; they also read the accumulators back, NX / 4 columns each.  The accumulator is double-buffered and a tile's epilogue runs after the warp's
 //               first block of a later tile, so the tensor cores are through with the tile by then and have work
 //               while it is read.
 //
@@ -41,10 +40,11 @@ namespace b2 {
 constexpr int kBatchRows = 128;                     // weight rows per tile
 constexpr int kBatchBlocks = kBatchRows / 16;       // native blocks per 256 columns
 constexpr int kBatchRawBytes = kBatchBlocks * kBlockBytes;
-constexpr int kBatchWarps = 16;                     // converters
-constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
+constexpr int kBatchEarly = 2;                      // blocks requested ahead of everything else
 constexpr uint32_t kBatchWCols = 32;                // tensor-memory columns of a step's weights
-constexpr int kBatchTickets = kBatchWarps;          // per split tile
+constexpr int kBatchSets = 2;                       // sets of eight converter warps (three sets, 72 registers: 3-4 % slower)
+constexpr int kBatchWarps = 8 * kBatchSets;
+constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
 // Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside two accumulators.
 __host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; }
 __host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
@@ -102,8 +102,9 @@ __device__ __forceinline__ void batch_ld(uint32_t taddr, float (&f)[CW]) {
 }
 
 // First step of CTA c's range, and the CTA whose range contains step s.
-__host__ __device__ inline int batch_begin(int steps, int ctas, int c) { return int((int64_t(steps) * c) / ctas); }
-__device__ __forceinline__ int batch_owner(int s, int steps, int ctas) { return int((int64_t(s + 1) * ctas - 1) / steps); }
+// (32-bit: steps * ctas stays below 2^32, see batch_applicable; 64-bit divisions took 0.4 us of a launch.)
+__device__ __forceinline__ int batch_begin(int steps, int ctas, int c) { return int(unsigned(steps) * unsigned(c) / unsigned(ctas)); }
+__device__ __forceinline__ int batch_owner(int s, int steps, int ctas) { return int((unsigned(s + 1) * unsigned(ctas) - 1u) / unsigned(steps)); }
 
 template <int NX, bool H16>
 __global__ void __launch_bounds__(kBatchThreads, 1)
@@ -130,12 +131,33 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     const int tsteps = a.kb * 4;                                           // steps of a tile
     const int gb0 = b0 >> 2, nblocks = ((b0 + nsteps - 1) >> 2) - gb0 + 1; // blocks of 8 x 256 columns, tile by tile
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < RS; ++i) { mbar_init(bar(RAW_FULL + i), 1); mbar_init(bar(RAW_FREE + i), kBatchWarps / 2); }
-        for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + kBatchWarps / 2); mbar_init(bar(DONE + i), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    auto request = [&](int tile, int kb, int r) {
+        const uint32_t bytes = uint32_t(min(kBatchBlocks, a.n16 - tile * kBatchBlocks)) * kBlockBytes;
+        mbar_expect_tx(bar(RAW_FULL + r), bytes);
+        bulk_copy_g2s(smem_u32(raw_base + r * kBatchRawBytes),
+                      a.native + (int64_t(kb) * a.n16 + tile * kBatchBlocks) * kBlockBytes, bytes, bar(RAW_FULL + r));
+    };
+    // The first blocks are on their way before anything else happens: their trip is the longest part of the start.  (Not a
+    // whole ring of them: x would queue up behind all CTAs' rings.)
+    int tile = gb0 / a.kb, kb = gb0 - tile * a.kb, issued = 0;             // (warp 0: next block to request)
+    if (warp == 0) {
+        if (elect_one()) {
+            for (int i = 0; i < RS; ++i) mbar_init(bar(RAW_FULL + i), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        for (; issued < min(kBatchEarly, nblocks); ++issued) {
+            if (elect_one()) request(tile, kb, issued);
+            __syncwarp();
+            if (++kb == a.kb) { kb = 0; ++tile; }
+        }
+        if (elect_one()) {
+            for (int i = 0; i < RS; ++i) mbar_init(bar(RAW_FREE + i), 8);
+            for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + 8); mbar_init(bar(DONE + i), 1); }
+            for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
+            *abort_flag = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
     }
     if (warp == 3) tmem_alloc(smem_u32(tmem_slot), 512);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -161,16 +183,10 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 
     if (warp == 0) {
         // ------------------------------ raw blocks ---------------------------------------
-        int tile = gb0 / a.kb, kb = gb0 - tile * a.kb, issued = 0;
         for (; issued < nblocks; ++issued) {
             const int r = issued % RS;
             if (issued >= RS && !wait(RAW_FREE + r, ((issued / RS) - 1) & 1)) break;
-            if (elect_one()) {
-                const uint32_t bytes = uint32_t(min(kBatchBlocks, a.n16 - tile * kBatchBlocks)) * kBlockBytes;
-                mbar_expect_tx(bar(RAW_FULL + r), bytes);
-                bulk_copy_g2s(smem_u32(raw_base + r * kBatchRawBytes),
-                              a.native + (int64_t(kb) * a.n16 + tile * kBatchBlocks) * kBlockBytes, bytes, bar(RAW_FULL + r));
-            }
+            if (elect_one()) request(tile, kb, r);
             __syncwarp();
             if (++kb == a.kb) { kb = 0; ++tile; }
         }
@@ -223,7 +239,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     } else if (warp == 2) {
         // ------------------------------ x tiles ------------------------------------------
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        int kb = gb0 % a.kb;
+        kb = gb0 % a.kb;
         for (int b = 0; b < nblocks; ++b) {
             const int slot = b % R;
             if (b >= R && !wait(DONE + slot, ((b / R) - 1) & 1)) break;
@@ -252,7 +268,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         int read = 0;                                                      // tiles of the range that this warp has read
 
         auto epilogue = [&](int seg) {
-            const int tile = tile0 + seg;
+            const int tile = tile0 + seg;                                  // (of the accumulator read here)
             if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // bias, tickets, partial tiles, y
             ok = ok && wait(ACC_FULL + (seg & 1), (seg >> 1) & 1);
             if (!ok) return;
@@ -280,7 +296,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 __threadfence();
                 __syncwarp();
                 unsigned prior = 0;
-                unsigned* ticket = a.tickets + first * kBatchTickets + (warp - 4);
+                unsigned* ticket = a.tickets + first * kBatchWarps + (warp - 4);
                 if (lane == 0) {
                     mbar_arrive(bar(ACC_FREE + (seg & 1)));
                     prior = atomicAdd(ticket, 1u);
@@ -301,16 +317,21 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                         } else {
 #pragma unroll
                             for (int i = 0; i < CW; ++i) f[i] = 0.0f;
-#pragma unroll 2
-                            for (int c = first; c <= last; ++c) {
-                                const float4* src = slot_of(c) + (c0 / 4) * kBatchRows;
+                            constexpr int PARTS = 32 / CW;                 // partial tiles requested together, added in CTA order
+                            for (int c = first; c <= last; c += PARTS) {
+                                float4 p[PARTS][CW / 4];
 #pragma unroll
-                                for (int q = 0; q < CW / 4; ++q) {
-                                    if (m0 + 4 * q < a.m) {
-                                        const float4 p = __ldcg(src + q * kBatchRows);
-                                        f[4 * q] += p.x; f[4 * q + 1] += p.y; f[4 * q + 2] += p.z; f[4 * q + 3] += p.w;
+                                for (int j = 0; j < PARTS; ++j)
+#pragma unroll
+                                    for (int q = 0; q < CW / 4; ++q)
+                                        if (c + j <= last && m0 + 4 * q < a.m) p[j][q] = __ldcg(slot_of(c + j) + (c0 / 4 + q) * kBatchRows);
+                                        else p[j][q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                                for (int j = 0; j < PARTS; ++j)
+#pragma unroll
+                                    for (int q = 0; q < CW / 4; ++q) {
+                                        f[4 * q] += p[j][q].x; f[4 * q + 1] += p[j][q].y; f[4 * q + 2] += p[j][q].z; f[4 * q + 3] += p[j][q].w;
                                     }
-                                }
                             }
                         }
                         if (a.act) {
@@ -342,7 +363,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 
         int slot = set, r = set, seg = 0, left = a.kb - gb0 % a.kb - set;  // rings and tile of the warp's block
         uint32_t free_parity = 1, raw_parity = 0;                          // (the first round of the stages is free)
-        for (int b = set; b < nblocks; b += 2) {
+        for (int b = set; b < nblocks; b += kBatchSets) {
             while (left <= 0) {
                 left += a.kb;
                 ++seg;
@@ -380,9 +401,9 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             }
             while (read < seg && ok) epilogue(read++);
             if (!ok) break;
-            left -= 2;
-            if ((slot += 2) >= R) { slot -= R; free_parity ^= 1; }
-            if ((r += 2) >= RS) { r -= RS; raw_parity ^= 1; }
+            left -= kBatchSets;
+            if ((slot += kBatchSets) >= R) { slot -= R; free_parity ^= 1; }
+            if ((r += kBatchSets) >= RS) { r -= RS; raw_parity ^= 1; }
         }
         const int segs = (b0 + nsteps - 1) / tsteps - tile0 + 1;
         while (read < segs && ok) epilogue(read++);

@@ -37,8 +37,8 @@ extern "C" {
 #define B2_ERR_UNSUPPORTED 5 /* device is not sm_100 or the requested route does not apply */
 
 /* Kernel families selectable through b2_w4a16_linear_route(). */
-#define B2_ROUTE_AUTO 0      /* by size: tile and streaming kernel up to 8 rows (32 on layers below ~10 MB), batch kernel up to 64
-                                rows (128 on layers above ~10 MB), tensor-memory GEMM above */
+#define B2_ROUTE_AUTO 0      /* by size: tile kernel up to 16 rows on layers up to ~10 MB, batch kernel on larger layers and up to
+                                128 rows (streaming kernel where it does not apply), tensor-memory GEMM above */
 #define B2_ROUTE_STREAM 1    /* persistent weight-streaming kernel (any M, re-reads the weights every 64 rows) */
 #define B2_ROUTE_TCGEN05 2   /* TMA + tcgen05 GEMM with in-kernel INT4->FP16 converter */
 #define B2_ROUTE_TILE 3      /* one CTA (or a cluster of 2 or 4 CTAs that split K) per 16-row tile, the whole K range
