@@ -597,19 +597,20 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 
 // B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of what ran before (us, tile / streaming / GEMM -> batch):
 //   up to 8 rows above 4096 native blocks (~10 MB), where the tile kernel runs out (6144 x 4096 at M = 1 / 8 10.0 / 10.2 -> 8.9 / 9.0,
-//                4096 x 12288 14.6 -> 13.1, 12289 x 3072 12.0 / 13.1 -> 10.8; 4096 x 4096 6.0 / 6.5 against 7.3) up to 65536
-//                (8192 x 28672 45.0 / 45.6 -> 44.2 / 44.9; 57344 x 8192 at M = 1 75.9 against 77.9), with FP16 steps up to
-//                16384 (12289 x 3072 10.9 -> 9.0; 24576 x 4096 19.0 against 19.9).  Below 4096 output
-//                columns the kernels that carry the all-gather stay, so that a column slice has the same bits in both forms.
+//                4096 x 12288 14.6 -> 13.1, 12289 x 3072 12.0 / 13.1 -> 10.8; 4096 x 4096 6.0 / 6.5 against 7.3) up to 16384
+//                (24576 x 4096 at M = 1 / 8 23.1 / 24.2 against 23.3 / 23.3 and, with FP16 steps, 19.0 / 20.1 against 19.9 / 20.1;
+//                57344 x 8192 at M = 1 75.9 against 77.9).  One line for both kinds of steps: the flag must not change a
+//                bit.  Below 4096 output columns the kernels that carry the all-gather stay, so that a column slice has the
+//                same bits in both forms.
 //   9..16        above 4096 blocks (6144 x 4096 at M = 16 14.2 -> 9.2, 24576 x 4096 28.8 -> 23.4, 57344 x 8192 94 -> 80;
 //                2048 x 4096 5.4 against 6.0)
 //   17..128      always (1024 x 1024 at M = 17 / 64 / 128 5.1 / 12.2 / 12.5 -> 3.9 / 4.9 / 7.3, 4096 x 4096 at M = 64 20.4 -> 10.9,
 //                57344 x 8192 at M = 64 / 128 154 / 158 -> 94 / 120)
-bool batch_preferred(int64_t m, const b2::Dims& d, bool h16 = false) {
+bool batch_preferred(int64_t m, const b2::Dims& d) {
     const int64_t blocks = int64_t(d.n16) * d.kb;
     if (!batch_applicable(m, d)) return false;
     if (m > 16) return true;
-    return blocks > 4096 && (m > 8 || (d.n >= 4096 && blocks <= (h16 ? 16384 : 65536)));
+    return blocks > 4096 && (m > 8 || (d.n >= 4096 && blocks <= 16384));
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
@@ -1037,7 +1038,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
-    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d, h16) && gemm_applicable(x, ldx, d) &&
+    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d) && gemm_applicable(x, ldx, d) &&
         workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes)
         route = B2_ROUTE_BATCH;
     if (route == B2_ROUTE_AUTO)
