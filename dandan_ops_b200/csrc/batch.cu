@@ -11,13 +11,16 @@ namespace {
 
 // Estimated time of a launch beyond its fixed start, in ns: the longest range of steps, the shared tiles in it (store, fence and
 // ticket of each), and the reading of a tile's partial sums by the last CTA (measured on per-CTA time stamps).
-int64_t launch_cost(int nx, int64_t steps, int tsteps, int64_t grid) {
-    const int64_t range = (steps + grid - 1) / grid;
-    const bool aligned = grid % (steps / tsteps) == 0;                     // every CTA inside one tile
-    const int64_t parts = aligned ? grid / (steps / tsteps) : (tsteps + range - 1) / range + 1;
-    const int64_t step_ns = nx <= 32 ? 220 : nx == 64 ? 250 : 310;
+int launch_cost(int nx, int steps, int tsteps, int grid) {
+    const int range = (steps + grid - 1) / grid;
+    const int tiles = steps / tsteps;
+    const bool aligned = grid % tiles == 0;                     // every CTA inside one tile
+    const int parts = aligned ? grid / tiles : (tsteps + range - 1) / range + 1;
+    const int step_ns = nx <= 32 ? 220 : nx == 64 ? 250 : 310;
     return range * step_ns + (parts == 1 ? 0 : (aligned ? 1 : 2) * 1300 + parts * (200 + 7 * nx));
 }
+
+constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
 template <int NX, bool H16>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
@@ -59,11 +62,13 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     p.steps = int(steps);
     // Either equal ranges over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle):
     // 4096 x 4096 at M = 16 / 64: 148 CTAs 9.1 / 13.0 us, 4 per tile 7.3 / 10.9; 1024 x 2048 at M = 32: 85 CTAs 7.9 us, 24 CTAs 5.8.
-    const int64_t sms = std::min<int64_t>(sm_count > 0 ? sm_count : 148, steps);
-    int64_t best = sms;
-    for (int64_t g = tiles; g <= sms; g += tiles)
-        if (launch_cost(p.nx, steps, tsteps, g) <= launch_cost(p.nx, steps, tsteps, best)) best = g;
-    p.grid = int(best);
+    const int sms = int(std::min<int64_t>(sm_count > 0 ? sm_count : 148, steps));
+    int best_cost = launch_cost(p.nx, p.steps, tsteps, sms);
+    p.grid = sms;
+    for (int g = tiles; g <= std::min(sms, kMaxPerTile * tiles); g += tiles) {
+        const int cost = launch_cost(p.nx, p.steps, tsteps, g);
+        if (cost <= best_cost) { best_cost = cost; p.grid = g; }
+    }
     const int64_t range = (steps + p.grid - 1) / p.grid;
     p.max_parts = p.grid % tiles == 0 ? p.grid / tiles : int(std::min<int64_t>(p.grid, (tsteps + range - 1) / range + 1));
     p.partial_bytes = b2::batch_partial_bytes(p.nx, p.grid);

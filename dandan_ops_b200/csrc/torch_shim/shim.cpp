@@ -142,10 +142,7 @@ at::Tensor legacy_op(const at::Tensor& x, const at::Tensor& packed, const at::Te
     return run_image(x, image_for(packed, scales, zeros, x.size(1)), packed.size(0), x.size(1), c10::nullopt, B2_ROUTE_AUTO);
 }
 
-// x [M, K] FP16 with unit inner stride, image = device-native weight image, bias = FP16 [N] or None,
-// flags = layer flags of the C ABI (B2_FLAG_FP16_STEPS).
-at::Tensor linear_image(const at::Tensor& x, const at::Tensor& image, int64_t n, int64_t k, const c10::optional<at::Tensor>& bias,
-                        int64_t route, int64_t flags) {
+void check_image(const at::Tensor& x, const at::Tensor& image, int64_t n, int64_t k, const c10::optional<at::Tensor>& bias) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kHalf && x.dim() == 2 && x.size(1) == k && x.stride(1) == 1 &&
                     (x.size(0) <= 1 || x.stride(0) >= k), "x must be a CUDA FP16 [M, K] tensor with unit inner stride");
     TORCH_CHECK(image.is_cuda() && image.scalar_type() == at::kByte && image.device() == x.device() &&
@@ -153,7 +150,61 @@ at::Tensor linear_image(const at::Tensor& x, const at::Tensor& image, int64_t n,
     if (bias.has_value() && bias->defined())
         TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == at::kHalf && bias->numel() == n && bias->is_contiguous(),
                     "bias must be a contiguous CUDA FP16 [N] tensor");
+}
+
+// x [M, K] FP16 with unit inner stride, image = device-native weight image, bias = FP16 [N] or None,
+// flags = layer flags of the C ABI (B2_FLAG_FP16_STEPS).
+at::Tensor linear_image(const at::Tensor& x, const at::Tensor& image, int64_t n, int64_t k, const c10::optional<at::Tensor>& bias,
+                        int64_t route, int64_t flags) {
+    check_image(x, image, n, k, bias);
     return run_image(x, image, n, k, bias, route, flags);
+}
+
+const void* data_or_null(const c10::optional<at::Tensor>& t) { return t.has_value() && t->defined() ? t->data_ptr() : nullptr; }
+
+// Gate/up projection with SiLU on a pair-ordered image: [M, K] -> [M, N/2] (as _native.linear_silu_mul).
+at::Tensor silu_mul_image(const at::Tensor& x, const at::Tensor& image, int64_t n, int64_t k, const c10::optional<at::Tensor>& bias,
+                          int64_t flags) {
+    check_image(x, image, n, k, bias);
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t m = x.size(0);
+    at::Tensor y = at::empty({m, n / 2}, x.options());
+    if (m == 0) return y;
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    const bool aligned = reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && (m == 1 || x.stride(0) % 8 == 0);
+    if (!b2_w4a16_silu_mul_is_fused(m, n, k) || (m > B2_STREAM_MAX_M && !aligned && k % 8 == 0)) {
+        at::Tensor full = run_image(x, image, n, k, bias, B2_ROUTE_AUTO, flags);
+        check_rc(b2_w4a16_silu_mul_pairs(full.data_ptr(), n, y.data_ptr(), n / 2, m, n, stream));
+        return y;
+    }
+    at::Tensor ws = workspace_for(x.device(), stream, b2_w4a16_workspace_bytes(m, n, k));
+    check_rc(b2_w4a16_linear_silu_mul_flags(x.data_ptr(), m > 1 ? x.stride(0) : k, image.data_ptr(), data_or_null(bias), y.data_ptr(),
+                                            n / 2, m, n, k, ws.data_ptr(), ws.numel(), stream, int(flags)));
+    return y;
+}
+
+// Residual add + RMSNorm + projection: (y, x + residual) (as _native.rmsnorm_linear).
+std::tuple<at::Tensor, at::Tensor> rmsnorm_image(const at::Tensor& x, const c10::optional<at::Tensor>& residual, const at::Tensor& weight,
+                                                 double eps, const at::Tensor& image, int64_t n, int64_t k,
+                                                 const c10::optional<at::Tensor>& bias) {
+    check_image(x, image, n, k, bias);
+    const bool with_residual = residual.has_value() && residual->defined();
+    if (with_residual)
+        TORCH_CHECK(residual->device() == x.device() && residual->scalar_type() == at::kHalf && residual->sizes() == x.sizes() &&
+                        residual->is_contiguous(), "residual must be a contiguous FP16 tensor of x's shape");
+    TORCH_CHECK(weight.device() == x.device() && weight.scalar_type() == at::kHalf && weight.numel() == k && weight.is_contiguous(),
+                "norm weight must be a contiguous FP16 [K] tensor on x's device");
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t m = x.size(0);
+    at::Tensor y = at::empty({m, n}, x.options()), summed = at::empty({m, k}, x.options());
+    if (m == 0) return {y, summed};
+    at::Tensor scratch = at::empty({m, k}, x.options());
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    at::Tensor ws = workspace_for(x.device(), stream, b2_w4a16_workspace_bytes(m, n, k));
+    check_rc(b2_w4a16_rmsnorm_linear(x.data_ptr(), x.stride(0), data_or_null(residual), with_residual ? residual->stride(0) : 0,
+                                     weight.data_ptr(), float(eps), summed.data_ptr(), k, scratch.data_ptr(), image.data_ptr(),
+                                     data_or_null(bias), y.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), stream));
+    return {y, summed};
 }
 
 int64_t status_all() {
@@ -182,6 +233,8 @@ TORCH_LIBRARY_FRAGMENT(dandan_ops, m) {
     m.def("w4a16_tensorcore(Tensor x, Tensor packed_w, Tensor scales, Tensor zeros, int group_size) -> Tensor");
     m.def("w4a16_small(Tensor x, Tensor packed_w, Tensor scales, Tensor zeros, int group_size) -> Tensor");
     m.def("w4a16_linear_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int route, int flags) -> Tensor");
+    m.def("w4a16_silu_mul_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int flags) -> Tensor");
+    m.def("w4a16_rmsnorm_image(Tensor x, Tensor? residual, Tensor weight, float eps, Tensor image, int n, int k, Tensor? bias) -> (Tensor, Tensor)");
     m.def("w4a16_workspace_status() -> int", &status_all);
 }
 
@@ -191,4 +244,6 @@ TORCH_LIBRARY_IMPL(dandan_ops, CUDA, m) {
     m.impl("w4a16_tensorcore", &legacy_op<Rule::Any>);
     m.impl("w4a16_small", &legacy_op<Rule::Small>);
     m.impl("w4a16_linear_image", &linear_image);
+    m.impl("w4a16_silu_mul_image", &silu_mul_image);
+    m.impl("w4a16_rmsnorm_image", &rmsnorm_image);
 }

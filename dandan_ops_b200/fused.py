@@ -11,7 +11,15 @@ import torch
 from torch import nn
 
 from . import _native
+from . import ops as _ops
 from .quantized_linear import QuantizedLinear
+
+
+def _plain(x):
+    """Whether the C++ operator library runs this call: an ordinary tensor outside autograd, and no private workspace
+    asked for (the operator library keeps its own, one per stream)."""
+    return (_ops.SHIM_LOADED and type(x) is torch.Tensor and not _native._private
+            and not (x.requires_grad and torch.is_grad_enabled()))
 
 
 def concat_layers(layers, backend=None):
@@ -123,6 +131,9 @@ class GateUpSilu(nn.Module):
         if x.stride(1) != 1:
             x = x.contiguous()
         image = self.op._native_image()
+        if _plain(x) and (x.shape[0] <= 1 or x.stride(0) >= self.in_features):
+            return torch.ops.dandan_ops.w4a16_silu_mul_image(x, image, self.op.out_features, self.in_features, self.op._bias_fp16(),
+                                                             self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
         return _native.linear_silu_mul(x, image, self.op.out_features, self.in_features, bias=self.op._bias_fp16(),
                                        flags=self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
 
@@ -176,6 +187,9 @@ class RmsNormLinear(nn.Module):
             raise ValueError("x and residual must have the same shape")
         x = x.contiguous()
         residual = None if residual is None else residual.contiguous()
+        if _plain(x) and (residual is None or _plain(residual)):
+            return torch.ops.dandan_ops.w4a16_rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
+                                                            self.out_features, self.in_features, self.op._bias_fp16())
         return _native.rmsnorm_linear(x, residual, self.norm_weight, self.eps, self.op._native_image(),
                                       self.out_features, self.in_features, bias=self.op._bias_fp16())
 
