@@ -44,6 +44,7 @@ constexpr int kGemmBK = 64;                     // K per step = one quantization
 constexpr int kGemmStages = 3;                  // ring of 64-column FP16 operand stages
 constexpr int kGemmABytes = 128 * kGemmBK * 2;                     // 16384 per 128 rows of x
 constexpr unsigned kStatusGemmTimeout = 2u;
+constexpr int kGemmWaitLimit = 1 << 20;         // polls without a suspend-time hint before a role gives up
 __host__ __device__ constexpr int gemm_raw_stages(int bn) { return bn == 128 ? 3 : 2; }   // 256-column raw blocks
 __host__ __device__ constexpr int gemm_raw_bytes(int bn) { return (bn / 16) * kBlockBytes; }
 __host__ __device__ constexpr int gemm_b_bytes(int bn) { return bn * kGemmBK * 2; }
@@ -198,7 +199,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
     };
     // Bounded wait that also leaves when another role has given up.
     auto wait = [&](int idx, uint32_t parity) -> bool {
-        for (int i = 0; i < kWaitLimit; ++i) {
+        for (int i = 0; i < kGemmWaitLimit; ++i) {
             if (mbar_try_wait(bar(idx), parity)) return true;
             if ((i & 63) == 63 && *abort_flag) return false;
         }

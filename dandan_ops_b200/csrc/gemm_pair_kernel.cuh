@@ -191,7 +191,7 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
         atomicOr(a.status, kStatusGemmTimeout);
     };
     auto wait = [&](int idx, uint32_t parity) -> bool {
-        for (int i = 0; i < kWaitLimit; ++i) {
+        for (int i = 0; i < kGemmWaitLimit; ++i) {
             if (mbar_try_wait(bar(idx), parity)) return true;
             if ((i & 63) == 63 && *abort_flag) return false;
         }
