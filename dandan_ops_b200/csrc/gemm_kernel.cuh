@@ -206,24 +206,29 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
         give_up();
         return false;
     };
+    // the lanes of a role warp go on or leave together
+    auto wait_warp = [&](int idx, uint32_t parity) -> bool { return __all_sync(0xffffffffu, wait(idx, parity)); };
 
     if (warp == 0) {
         // ------------------------------ copy producer ------------------------------------
-        if (lane == 0) {
-            const uint8_t* src = a.native + (int64_t(tile_n) * n_tiles16) * kBlockBytes;
-            const int64_t stride = int64_t(a.n16) * kBlockBytes;
-            // the last row tile group may be short: copy only blocks that exist in the image
-            const int blocks_here = min(n_tiles16, a.n16 - tile_n * n_tiles16);
-            const uint32_t raw_bytes = uint32_t(blocks_here) * kBlockBytes;
-            for (int s = 0; s < ksteps; ++s) {
-                if ((s & 3) == 0) {
-                    const int kb = s >> 2, r = kb % kGemmRawStages;
-                    if (kb >= kGemmRawStages && !wait(RAW_FREE + r, ((kb / kGemmRawStages) - 1) & 1)) break;
+        const uint8_t* src = a.native + (int64_t(tile_n) * n_tiles16) * kBlockBytes;
+        const int64_t stride = int64_t(a.n16) * kBlockBytes;
+        // the last row tile group may be short: copy only blocks that exist in the image
+        const int blocks_here = min(n_tiles16, a.n16 - tile_n * n_tiles16);
+        const uint32_t raw_bytes = uint32_t(blocks_here) * kBlockBytes;
+        for (int s = 0; s < ksteps; ++s) {
+            if ((s & 3) == 0) {
+                const int kb = s >> 2, r = kb % kGemmRawStages;
+                if (kb >= kGemmRawStages && !wait_warp(RAW_FREE + r, ((kb / kGemmRawStages) - 1) & 1)) break;
+                if (elect_one()) {
                     mbar_expect_tx(bar(RAW_FULL + r), raw_bytes);
                     bulk_copy_g2s(smem_u32(raw_base + r * kGemmRawBytes), src + kb * stride, raw_bytes, bar(RAW_FULL + r));
                 }
-                const int st = s % kGemmStages;
-                if (s >= kGemmStages && !wait(AB_FREE + st, ((s / kGemmStages) - 1) & 1)) break;
+                __syncwarp();
+            }
+            const int st = s % kGemmStages;
+            if (s >= kGemmStages && !wait_warp(AB_FREE + st, ((s / kGemmStages) - 1) & 1)) break;
+            if (elect_one()) {
                 mbar_expect_tx(bar(A_FULL + st), MA * kGemmABytes);
                 uint8_t* adst = stage_base + st * kStageBytes + kGemmBBytes;
 #pragma unroll
@@ -231,6 +236,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
                     tma_load_2d(smem_u32(adst + i * kGemmABytes), &xmap, s * kGemmBK, tile_m * (MA * 128) + i * 128,
                                 bar(A_FULL + st));
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ---------------------------------------
@@ -239,9 +245,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
         for (int s = 0; s < ksteps; ++s) {
             const int st = s % kGemmStages;
             const uint32_t par = (s / kGemmStages) & 1;
-            if (!wait(A_FULL + st, par) || !wait(B_FULL + st, par)) break;
+            if (!wait_warp(A_FULL + st, par) || !wait_warp(B_FULL + st, par)) break;
             tcgen05_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t b_addr = smem_u32(stage_base + st * kStageBytes);
 #pragma unroll
                 for (int i = 0; i < MA; ++i) {

@@ -20,7 +20,8 @@
 //               TMA loads of this CTA's x rows; the loads of BOTH CTAs complete the leader's
 //               full barrier (cp.async.bulk.tensor with .cta_group::2)
 //   warp 1      allocates/frees tensor memory (cta_group::2, both CTAs); in the leader CTA
-//               (cluster rank 0) one lane issues the MMAs and one commit per step to both CTAs
+//               (cluster rank 0) one elected lane issues the MMAs and one commit per step to both CTAs
+//               (24576 x 4096 at M = 2048 346 -> 328 us against a branch on the lane number, see elect_one)
 //   warps 2..9  converters: thread = weight row (tensor-memory lane); the two warps of a lane
 //               quadrant take alternate 64-column steps (one 32-column tcgen05.st per step and
 //               quadrant); afterwards the epilogue: tcgen05.ld gives a thread 32 rows of y for
@@ -198,20 +199,22 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
         give_up();
         return false;
     };
+    // the lanes of a role warp go on or leave together
+    auto wait_warp = [&](int idx, uint32_t parity) -> bool { return __all_sync(0xffffffffu, wait(idx, parity)); };
 
     if (warp == 0) {
         // ------------------------------ copy producer ------------------------------------
-        if (lane == 0) {
-            const int nt0 = n0 >> 4;
-            const int blocks_here = max(0, min(kPairRows / 16, a.n16 - nt0));
-            const uint32_t raw_bytes = uint32_t(blocks_here) * kBlockBytes;
-            const uint8_t* src = a.native + int64_t(nt0) * kBlockBytes;
-            const int64_t stride = int64_t(a.n16) * kBlockBytes;
-            const uint32_t full_leader = map_to_cta(bar(FULL), 0);
-            for (int s = 0; s < ksteps; ++s) {
-                if ((s & 3) == 0) {
-                    const int kb = s >> 2, r = kb % RS;
-                    if (kb >= RS && !wait(RAW_FREE + r, ((kb / RS) - 1) & 1)) break;
+        const int nt0 = n0 >> 4;
+        const int blocks_here = max(0, min(kPairRows / 16, a.n16 - nt0));
+        const uint32_t raw_bytes = uint32_t(blocks_here) * kBlockBytes;
+        const uint8_t* src = a.native + int64_t(nt0) * kBlockBytes;
+        const int64_t stride = int64_t(a.n16) * kBlockBytes;
+        const uint32_t full_leader = map_to_cta(bar(FULL), 0);
+        for (int s = 0; s < ksteps; ++s) {
+            if ((s & 3) == 0) {
+                const int kb = s >> 2, r = kb % RS;
+                if (kb >= RS && !wait_warp(RAW_FREE + r, ((kb / RS) - 1) & 1)) break;
+                if (elect_one()) {
                     if (raw_bytes) {
                         mbar_expect_tx(bar(RAW_FULL + r), raw_bytes);
                         bulk_copy_g2s(smem_u32(raw_base + r * kPairRawBytes), src + (kb0 + kb) * stride, raw_bytes, bar(RAW_FULL + r));
@@ -219,37 +222,38 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
                         mbar_arrive(bar(RAW_FULL + r));       // no weight rows here: columns beyond N, masked in the epilogue
                     }
                 }
-                const int st = s % XS;
-                if (s >= XS && !wait(DONE + st, ((s / XS) - 1) & 1)) break;
+                __syncwarp();
+            }
+            const int st = s % XS;
+            if (s >= XS && !wait_warp(DONE + st, ((s / XS) - 1) & 1)) break;
+            if (elect_one()) {
                 if (leader) mbar_expect_tx(bar(FULL + st), 2 * kXBytes);
                 tma_load_2d_pair(smem_u32(x_base + st * kXBytes), &xmap, (s0 + s) * kGemmBK, m0 + int(rank) * (MT / 2), full_leader + st * 8);
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer (one lane of the leader CTA) -----------
-        if (leader && lane == 0) {
+        if (leader) {
             // D = F32, A = B = F16, both K-major, M = 256 weight rows, N = MT rows of x
             const uint32_t idesc = (1u << 4) | (uint32_t(MT >> 3) << 17) | (uint32_t(256 >> 4) << 24);
             const uint64_t desc0 = umma_desc_sw128(smem_u32(x_base));
-            bool have = false;                  // the coming step's barrier was already seen complete
             int xs = 0, ws = 0;
             uint32_t par = 0;
             for (int s = 0; s < ksteps; ++s) {
-                if (!have && !wait(FULL + xs, par)) break;
+                if (!wait_warp(FULL + xs, par)) break;      // (the MMAs of the step before are still queued meanwhile)
                 tcgen05_fence_after();
-                const uint64_t desc = desc0 + uint64_t((xs * kXBytes) >> 4);
-                const uint32_t w_addr = tmem_w + ws * kPairWCols;
-                const int xn = xs + 1 == XS ? 0 : xs + 1;
-                const uint32_t parn = xs + 1 == XS ? par ^ 1 : par;
+                if (elect_one()) {
+                    const uint64_t desc = desc0 + uint64_t((xs * kXBytes) >> 4);
+                    const uint32_t w_addr = tmem_w + ws * kPairWCols;
 #pragma unroll
-                for (int kk = 0; kk < kGemmBK / 16; ++kk) {
-                    // look at the next step's barrier while the tensor cores still have work queued
-                    if (kk == kGemmBK / 16 - 1) have = s + 1 < ksteps && mbar_try_wait(bar(FULL + xn), parn);
-                    umma_f16_pair_ts(tmem_base, w_addr + kk * 8, desc + uint64_t(kk * 2), idesc, (s > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < kGemmBK / 16; ++kk)
+                        umma_f16_pair_ts(tmem_base, w_addr + kk * 8, desc + uint64_t(kk * 2), idesc, (s > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit_pair(bar(DONE + xs));
+                    if (s == ksteps - 1) umma_commit_pair(bar(ACC_FULL));
                 }
-                umma_commit_pair(bar(DONE + xs));
-                if (s == ksteps - 1) umma_commit_pair(bar(ACC_FULL));
-                xs = xn; par = parn;
+                __syncwarp();
+                if (++xs == XS) { xs = 0; par ^= 1; }
                 ws = ws + 1 == WS ? 0 : ws + 1;
             }
         }
