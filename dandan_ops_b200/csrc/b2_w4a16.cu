@@ -839,6 +839,7 @@ int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t l
     a.steps = p.steps;
     a.act = act;
     a.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
+    a.fault_block = g_fault_step.exchange(-1, std::memory_order_relaxed);
     return b2host::launch_batch(p, map, a, h16, overlap, s);
 }
 

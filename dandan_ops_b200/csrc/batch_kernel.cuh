@@ -71,6 +71,7 @@ struct BatchArgs {
     int steps;              // tiles * kb * 4
     int act;                // as StreamArgs::act
     int wait_limit;
+    int fault_block;        // -1; a test passes b >= 0: CTA 0 arms the barrier of its b-th block but skips the copy
 };
 
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -118,7 +119,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     uint8_t* raw_base = x_base + R * kXStage;                              // [RS][18688]
     uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes);
     constexpr int RAW_FULL = 0, RAW_FREE = RAW_FULL + RS, FULL = RAW_FREE + RS, DONE = FULL + R, ACC_FULL = DONE + R,
-                  ACC_FREE = ACC_FULL + 2, NBARS = ACC_FREE + 2;
+                  ACC_FREE = ACC_FULL + 2, DRAIN = ACC_FREE + 2, NBARS = DRAIN + 1;
     static_assert(NBARS * 8 + 8 <= 512, "barrier area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -131,11 +132,13 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     const int tsteps = a.kb * 4;                                           // steps of a tile
     const int gb0 = b0 >> 2, nblocks = ((b0 + nsteps - 1) >> 2) - gb0 + 1; // blocks of 8 x 256 columns, tile by tile
 
-    auto request = [&](int tile, int kb, int r) {
+    auto request = [&](int b, int tile, int kb) {                           // block b of the range
+        const int r = b % RS;
         const uint32_t bytes = uint32_t(min(kBatchBlocks, a.n16 - tile * kBatchBlocks)) * kBlockBytes;
         mbar_expect_tx(bar(RAW_FULL + r), bytes);
-        bulk_copy_g2s(smem_u32(raw_base + r * kBatchRawBytes),
-                      a.native + (int64_t(kb) * a.n16 + tile * kBatchBlocks) * kBlockBytes, bytes, bar(RAW_FULL + r));
+        if (!(blockIdx.x == 0 && b == a.fault_block))
+            bulk_copy_g2s(smem_u32(raw_base + r * kBatchRawBytes),
+                          a.native + (int64_t(kb) * a.n16 + tile * kBatchBlocks) * kBlockBytes, bytes, bar(RAW_FULL + r));
     };
     // The first blocks are on their way before anything else happens: their trip is the longest part of the start.  (Not a
     // whole ring of them: x would queue up behind all CTAs' rings.)
@@ -146,7 +149,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         for (; issued < min(kBatchEarly, nblocks); ++issued) {
-            if (elect_one()) request(tile, kb, issued);
+            if (elect_one()) request(issued, tile, kb);
             __syncwarp();
             if (++kb == a.kb) { kb = 0; ++tile; }
         }
@@ -154,6 +157,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             for (int i = 0; i < RS; ++i) mbar_init(bar(RAW_FREE + i), 8);
             for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + 8); mbar_init(bar(DONE + i), 1); }
             for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
+            mbar_init(bar(DRAIN), 1);
             *abort_flag = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -186,7 +190,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         for (; issued < nblocks; ++issued) {
             const int r = issued % RS;
             if (issued >= RS && !wait(RAW_FREE + r, ((issued / RS) - 1) & 1)) break;
-            if (elect_one()) request(tile, kb, r);
+            if (elect_one()) request(issued, tile, kb);
             __syncwarp();
             if (++kb == a.kb) { kb = 0; ++tile; }
         }
@@ -201,10 +205,11 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         int left = a.kb - gb0 % a.kb;                 // blocks to the end of the tile
         int seg = 0;
         bool fresh = true;                            // the accumulator starts with this block
+        bool ok = true;
         for (int b = 0; b < nblocks; ++b) {
             const int slot = b % R;
-            if (fresh && seg >= 2 && !wait(ACC_FREE + (seg & 1), ((seg >> 1) - 1) & 1)) break;
-            if (!wait(FULL + slot, (b / R) & 1)) break;
+            if (fresh && seg >= 2 && !(ok = wait(ACC_FREE + (seg & 1), ((seg >> 1) - 1) & 1))) break;
+            if (!(ok = wait(FULL + slot, (b / R) & 1))) break;
             tcgen05_fence_after();
             const bool end = --left == 0 || b == nblocks - 1;
             if (elect_one()) {
@@ -236,6 +241,11 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 left = a.kb;
             }
         }
+        if (!ok) {                                    // after an abort: MMAs in flight end before their operands are released
+            if (elect_one()) umma_commit(bar(DRAIN));
+            __syncwarp();
+            for (int p = 0; p < 4096 && !mbar_try_wait(bar(DRAIN), 0); ++p) {}
+        }
     } else if (warp == 2) {
         // ------------------------------ x tiles ------------------------------------------
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -252,7 +262,6 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             __syncwarp();
             if (++kb == a.kb) kb = 0;
         }
-        for (int p = 0; p < 64 && *abort_flag; ++p) __nanosleep(2000);      // after an abort: loads in flight land first
     } else if (warp >= 4) {
         // ------------------------------ converters ---------------------------------------
         const int quad = warp & 3, u = (warp - 4) >> 2, v = u & 1, set = u >> 1;
@@ -411,6 +420,9 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     __syncwarp();
     tcgen05_fence_before();
     __syncthreads();
+    // After an abort x tiles may be on their way to stages whose barrier the converters never completed, which nothing
+    // can wait for: whoever gave up, all roles have stopped requesting, and the last loads get 0.1 ms to land.
+    for (int p = 0; p < 64 && *abort_flag; ++p) __nanosleep(2000);
     if (warp == 3) {
         tcgen05_fence_after();
         tmem_dealloc(tmem_base, 512);

@@ -115,8 +115,9 @@ int b2_w4a16_dequantize_fp16(const void* native, int64_t n, int64_t k, void* out
 int64_t b2_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k);
 
 /* Reads the workspace's sticky status word into *status_host (0 = every kernel that used
- * the workspace ran to completion; bit 0 = a warp gave up waiting for a weight copy and
- * the outputs of that call are undefined).  workspace == NULL reads the word of the scratch built
+ * the workspace ran to completion; bit 0 = a warp of the tile or streaming kernel gave up a
+ * bounded wait, bit 1 = a role of the batch kernel or of a GEMM did; the outputs of that call
+ * are undefined and the tickets of the workspace have to be zeroed again).  workspace == NULL reads the word of the scratch built
  * into the library (b2_w4a16_linear_static).  SYNCHRONIZES the stream; diagnostics only. */
 int b2_w4a16_status(const void* workspace, void* stream, unsigned* status_host);
 
@@ -319,11 +320,11 @@ int b2_w4a16_linear_gather_launches(int64_t m, int64_t n_total, int64_t slice_co
 /* Launches an empty kernel on `stream`: the floor of one graph node, for benchmarks. */
 int b2_w4a16_noop(void* stream);
 
-/* Test hooks, no counterpart in the reference.  wait_limit: polls after which a kernel's bounded
- * wait for a weight copy gives up (<= 0 restores the default, about a million).  skip_copy >= 0: the
- * NEXT decode-kernel launch (tile or streaming) arms the barrier of that copy of its first CTA but does
- * not issue the copy, so the wait runs out, the warp records bit 0 in the status word, drains its other
- * copies and the kernel returns - nothing hangs; -1 = off.  stream_variant: 0 or 1 = the shipped
+/* Test hooks, no counterpart in the reference.  wait_limit: polls after which a bounded wait of the tile, streaming
+ * and batch kernels gives up (<= 0 restores the default, 65536 polls of up to 20 us each).  skip_copy >= 0: the
+ * NEXT launch of one of them arms the barrier of that weight copy of its first CTA but does not issue the copy,
+ * so the wait runs out, bit 0 (batch kernel: bit 1) of the status word is set, the other copies in flight land
+ * and the kernel returns - nothing hangs; -1 = off.  stream_variant: 0 or 1 = the shipped
  * streaming kernel; 2 / 3 = the double-buffered form with 32 / 16 warps per CTA, 4 = the chunk-major
  * two-dimensional split (all M <= 16), kept for measurements. */
 int b2_w4a16_test_hooks(int wait_limit, int skip_copy, int stream_variant);

@@ -1,5 +1,7 @@
 """w4a16_batch_kernel (up to 128 rows of x, products on tcgen05): against the CPU oracle and, on its other forms, against
 the routes it stands in for, at the sizes where tiles, ranges and rings end."""
+import ctypes
+
 import pytest
 import torch
 
@@ -93,3 +95,33 @@ def test_what_the_route_refuses():
     with pytest.raises(RuntimeError, match="batch route"):
         _native.linear(odd, layer._native_image(), 64, 520, route=BATCH)
     assert torch.equal(_native.linear(odd, layer._native_image(), 64, 520), torch.zeros(40, 64, dtype=torch.float16, device="cuda"))
+
+
+@pytest.mark.parametrize("m,skipped", [(9, 0), (9, 5), (40, 1), (128, 3)])
+def test_a_wait_that_runs_out_sets_the_status_word_and_returns(m, skipped):
+    """One weight copy of the first CTA is left out: all roles give up, every copy and product in flight ends, and tensor
+    memory is freed (the next call needs all of it)."""
+    n, k = 4096, 8192
+    layer, g = _layer(n, k, 77)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    lib, image = _native.load(), layer._native_image()
+    ws = torch.zeros(int(lib.b2_w4a16_workspace_bytes(m, n, k)), dtype=torch.uint8, device="cuda")
+    word = ctypes.c_uint(7)
+
+    def call():
+        y = torch.zeros(m, n, dtype=torch.float16, device="cuda")
+        assert lib.b2_w4a16_linear_route(x.data_ptr(), k, image.data_ptr(), y.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(),
+                                         torch.cuda.current_stream().cuda_stream, BATCH) == 0
+        assert lib.b2_w4a16_status(ws.data_ptr(), None, ctypes.byref(word)) == 0
+        return y
+
+    good = call()
+    assert word.value == 0
+    _native.test_hooks(wait_limit=64, skip_copy=skipped)
+    try:
+        call()
+        assert word.value == 2
+    finally:
+        _native.test_hooks()
+    ws.zero_()
+    assert torch.equal(call(), good) and word.value == 0
