@@ -170,13 +170,18 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // Bounded; the lanes of a warp go on or leave together.
+    // Bounded; the lanes of a warp go on or leave together.  As a programmatic dependent the kernel may have been held up by
+    // the one before it, which can last longer than the limit (a gather that waits for its peers): a limit that has run
+    // out counts once more from that kernel's end.  (The same wait up front in every role cost 1 % of small launches.)
     auto wait = [&](int idx, uint32_t parity) -> bool {
         const uint32_t at = bar(idx);
         if (__all_sync(0xffffffffu, mbar_try_wait(at, parity))) return true;
-        for (int i = 1; i < a.wait_limit; ++i) {
-            if (__all_sync(0xffffffffu, mbar_try_wait_long(at, parity))) return true;
-            if ((i & 63) == 63 && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        for (int turn = 0; turn < 2; ++turn) {
+            for (int i = 1; i < a.wait_limit; ++i) {
+                if (__all_sync(0xffffffffu, mbar_try_wait_long(at, parity))) return true;
+                if ((i & 63) == 63 && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            }
+            if (turn == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
         }
         if (lane == 0) {
             *abort_flag = 1;

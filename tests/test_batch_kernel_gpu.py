@@ -125,3 +125,31 @@ def test_a_wait_that_runs_out_sets_the_status_word_and_returns(m, skipped):
         _native.test_hooks()
     ws.zero_()
     assert torch.equal(call(), good) and word.value == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(16, 4096, 8192), (128, 2048, 2048), (40, 256, 256)])
+def test_the_wait_limit_does_not_count_the_kernel_before(m, n, k):
+    """A dependent launch beside a predecessor that lasts longer than the poll limit: a one-launch gather of a small slice,
+    most SMs left free, that waits 0.2 s for packets that never arrive."""
+    layer, g = _layer(n, k, 5)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    image = layer._native_image()
+    want = _native.linear(x, image, n, k, route=BATCH, flags=layer._image_flags)
+    piece, _ = _layer(32, 1032, 6)
+    bufs = [torch.zeros(1, 64, dtype=torch.float16, device="cuda") for _ in range(2)]
+    boxes = [torch.zeros(_native.gather_block_bytes(2, 4096), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    one = torch.randn(1, 1032, generator=g).half().cuda()
+    assert _native.linear_gather_launches(1, 64, 32, 1032, 0, 2, 4096) == 1
+    torch.cuda.synchronize()
+    _native.gather_wait_limit(200000)
+    _native.test_hooks(wait_limit=64)                                    # about a millisecond
+    try:
+        _native.linear_gather(one, piece._native_image(), 1032, [t.data_ptr() for t in bufs], [t.data_ptr() for t in boxes], 4096, 0,
+                              64, 64, 32)
+        y = _native.linear(x, image, n, k, route=BATCH, flags=_native.FLAG_OVERLAP_LAUNCH)
+        torch.cuda.synchronize()
+    finally:
+        _native.gather_wait_limit(0)
+        _native.test_hooks()
+    assert _native.gather_status(boxes[0].data_ptr()) & 4                # the predecessor did wait until its own limit
+    assert torch.equal(y, want) and _native.status() == 0
