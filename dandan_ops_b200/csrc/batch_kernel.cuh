@@ -5,7 +5,7 @@
 // (eight per fragment at 64 rows).  Here the decoded weights go to tensor memory as the A operand of one
 // tcgen05.mma per 16 columns of K, issued by a single thread and the same instruction whatever the number of rows:
 //
-//   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x)
+//   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x; batch_chains(NX) of them, added on reading)
 //     += A[n][k] (weights, FP16, tensor memory, written by the converter warps) * B[m][k] (x, shared memory, TMA)
 //
 // Work split ("stream-K"): the layer is cut into steps = (tile of 128 weight rows) x (64 columns of K), numbered
@@ -20,9 +20,8 @@
 //   warp 2      TMA loads of x, one tile of NX rows x 64 columns per step
 //   warp 3      allocates and frees tensor memory
 //   warps 4..19 converters: two sets of eight warps (two per tensor-memory lane quadrant, two quantization groups each)
-//               that take the blocks in turn; they also read the accumulators back, NX / 4 columns each.  The accumulator is double-buffered and a tile's epilogue runs after the warp's
-//               first block of a later tile, so the tensor cores are through with the tile by then and have work
-//               while it is read.
+//               that take the blocks in turn; they also read the accumulators back, NX / 4 columns each.  A tile's
+//               epilogue runs after the warp's first block of a later tile: the tensor cores are through with it by then.
 //
 // Lane l of quadrant q holds weight row 32q + 16 (l & 1) + 8 hi8 + g of the tile: neighbouring lanes read from two blocks
 // and two row pairs, which makes the 16-byte reads of the codes two-way bank conflicts (four-way in row order).
@@ -45,8 +44,16 @@ constexpr uint32_t kBatchWCols = 32;                // tensor-memory columns of 
 constexpr int kBatchSets = 2;                       // sets of eight converter warps (three sets, 72 registers: 3-4 % slower)
 constexpr int kBatchWarps = 8 * kBatchSets;
 constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
-// Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside two accumulators.
+// Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside the accumulators.
 __host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; }
+// The FP32 sums of a tile run as C chains (the products of 16 columns of K go to chain kk % C), added in order when they
+// are read: a tensor core drops the bits of a product below the running sum, so the error grows with the length of a
+// chain.  Share of FP16 outputs that are not the nearest to the 64-bit sum, one chain -> C (streaming kernel / K-split GEMM):
+// 4096 x 12288 at M = 16 1.4 % -> 0.4 % (0.6 %), M = 24 1.4 -> 0.5 (0.7), M = 64 1.4 -> 0.8 (0.75); 6144 x 4096 at M = 16
+// 0.7 -> 0.2 (0.4).  Reading the chains takes 0.1 us of a launch.  As many as fit beside the weight ring: the accumulator is
+// double-buffered only where that leaves four chains (one buffer is level: a tile's products wait for one read).
+__host__ __device__ constexpr int batch_chains(int nx) { return nx <= 32 ? 4 : 2; }
+__host__ __device__ constexpr int batch_accs(int nx) { return nx == 16 ? 2 : 1; }
 __host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
 __host__ __device__ constexpr int batch_raw_stages(int nx) {
     const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx) * batch_x_bytes(nx)) / kBatchRawBytes;
@@ -79,27 +86,36 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
-// CW accumulator columns of this thread's lane (4, 8 or 16).
+// CW columns of this thread's lane (4 or 8), complete after tcgen05.wait::ld.
 template <int CW>
-__device__ __forceinline__ void batch_ld(uint32_t taddr, float (&f)[CW]) {
-    uint32_t v[CW];
-    if constexpr (CW == 4) {
+__device__ __forceinline__ void batch_ld(uint32_t taddr, uint32_t (&v)[CW]) {
+    static_assert(CW == 4 || CW == 8, "4 or 8 columns");
+    if constexpr (CW == 4)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
-    } else if constexpr (CW == 8) {
+    else
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                      : "r"(taddr) : "memory");
-    } else {
-        static_assert(CW == 16, "4, 8 or 16 columns");
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                       "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                     : "r"(taddr) : "memory");
-    }
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// The sums of CW accumulator columns: the chains (NX columns apart) added in a fixed order.
+template <int NX, int CW>
+__device__ __forceinline__ void batch_sums(uint32_t taddr, float (&f)[CW]) {
+    constexpr int C = batch_chains(NX), W = CW < 8 ? CW : 8;
 #pragma unroll
-    for (int i = 0; i < CW; ++i) f[i] = __uint_as_float(v[i]);
+    for (int at = 0; at < CW; at += W) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            uint32_t v[W];
+            batch_ld<W>(taddr + c * NX + at, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                asm volatile("" : "+r"(v[i]));                                 // (not used before the wait)
+                f[at + i] = c == 0 ? __uint_as_float(v[i]) : __fadd_rn(f[at + i], __uint_as_float(v[i]));
+            }
+        }
+    }
 }
 
 // First step of CTA c's range, and the CTA whose range contains step s.
@@ -112,7 +128,8 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
     constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
     constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
-    static_assert(2 * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
+    constexpr int C = batch_chains(NX), ACCS = batch_accs(NX);
+    static_assert(ACCS * C * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_base = smem;                                                // [R][4][kXBytes]
@@ -213,20 +230,20 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         bool ok = true;
         for (int b = 0; b < nblocks; ++b) {
             const int slot = b % R;
-            if (fresh && seg >= 2 && !(ok = wait(ACC_FREE + (seg & 1), ((seg >> 1) - 1) & 1))) break;
+            if (fresh && seg >= ACCS && !(ok = wait(ACC_FREE + seg % ACCS, (seg / ACCS - 1) & 1))) break;
             if (!(ok = wait(FULL + slot, (b / R) & 1))) break;
             tcgen05_fence_after();
             const bool end = --left == 0 || b == nblocks - 1;
             if (elect_one()) {
-                const uint32_t w = tmem_base + kWBase + slot * kWStage, d = tmem_base + (seg & 1) * NX;
+                const uint32_t w = tmem_base + kWBase + slot * kWStage, d = tmem_base + seg % ACCS * (C * NX);
                 const uint64_t desc = desc0 + uint64_t((slot * kXStage) >> 4);
                 uint32_t accumulate = fresh ? 0u : 1u;
                 auto step = [&](int t) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        umma_f16_ts(d, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc, accumulate);
-                        accumulate = 1;
-                    }
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16_ts(d + kk % C * NX, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc,
+                                    kk < C ? accumulate : 1u);
+                    accumulate = 1;
                 };
                 const int t0 = b == 0 ? b0 & 3 : 0, t1 = b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;     // steps of the range in this block
                 if (t0 == 0 && t1 == 3) {
@@ -237,7 +254,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     for (int t = t0; t <= t1; ++t) step(t);
                 }
                 umma_commit(bar(DONE + slot));
-                if (end) umma_commit(bar(ACC_FULL + (seg & 1)));
+                if (end) umma_commit(bar(ACC_FULL + seg % ACCS));
             }
             __syncwarp();
             fresh = end;
@@ -284,13 +301,13 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         auto epilogue = [&](int seg) {
             const int tile = tile0 + seg;                                  // (of the accumulator read here)
             if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // bias, tickets, partial tiles, y
-            ok = ok && wait(ACC_FULL + (seg & 1), (seg >> 1) & 1);
+            ok = ok && wait(ACC_FULL + seg % ACCS, (seg / ACCS) & 1);
             if (!ok) return;
             tcgen05_fence_after();
             const int t0 = tile * tsteps, t1 = t0 + tsteps;
             const bool whole = b0 <= t0 && t1 <= b0 + nsteps;
             const int first = whole ? 0 : batch_owner(t0, a.steps, ctas), last = whole ? 0 : batch_owner(t1 - 1, a.steps, ctas);
-            const uint32_t acc = tmem_base + lane_addr + (seg & 1) * NX + u * (NX / 4);
+            const uint32_t acc = tmem_base + lane_addr + seg % ACCS * (C * NX) + u * (NX / 4);
             auto slot_of = [&](int c) {                                    // partial tile of CTA c, this warp's columns and lanes
                 return a.partial + ((int64_t(c) * 2 + (c == first ? 1 : 0)) * (NX / 4) + u * (NX / 16)) * kBatchRows + quad * 32 + lane;
             };
@@ -300,7 +317,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
                     float f[CW];
-                    batch_ld<CW>(acc + c0, f);
+                    batch_sums<NX, CW>(acc + c0, f);
 #pragma unroll
                     for (int q = 0; q < CW / 4; ++q)
                         if (u * (NX / 4) + c0 + 4 * q < a.m)
@@ -312,7 +329,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 unsigned prior = 0;
                 unsigned* ticket = a.tickets + first * kBatchWarps + (warp - 4);
                 if (lane == 0) {
-                    mbar_arrive(bar(ACC_FREE + (seg & 1)));
+                    mbar_arrive(bar(ACC_FREE + seg % ACCS));
                     prior = atomicAdd(ticket, 1u);
                     if (prior == unsigned(last - first)) *ticket = 0u;
                 }
@@ -327,7 +344,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     if (m0 < a.m) {
                         float f[CW];
                         if (whole) {
-                            batch_ld<CW>(acc + c0, f);
+                            batch_sums<NX, CW>(acc + c0, f);
                         } else {
 #pragma unroll
                             for (int i = 0; i < CW; ++i) f[i] = 0.0f;
@@ -371,7 +388,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             if (whole) {
                 tcgen05_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar(ACC_FREE + (seg & 1)));
+                if (lane == 0) mbar_arrive(bar(ACC_FREE + seg % ACCS));
             }
         };
 

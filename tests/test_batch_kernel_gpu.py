@@ -153,3 +153,26 @@ def test_the_wait_limit_does_not_count_the_kernel_before(m, n, k):
         _native.test_hooks()
     assert _native.gather_status(boxes[0].data_ptr()) & 4                # the predecessor did wait until its own limit
     assert torch.equal(y, want) and _native.status() == 0
+
+
+def _not_nearest(y, exact):
+    """Share of FP16 outputs that are not the nearest to the 64-bit sum: proportional to the error of the FP32 sums."""
+    return float((y != exact.to(torch.float16)).double().mean())
+
+
+@pytest.mark.parametrize("m,n,k,replaced", [
+    (9, 6144, 4096, _native.ROUTE_STREAM),
+    (16, 4096, 12288, _native.ROUTE_STREAM),
+    (24, 6144, 4096, _native.ROUTE_STREAM),
+    (32, 4096, 12288, _native.ROUTE_STREAM),
+    (64, 4096, 12288, _native.ROUTE_TCGEN05),
+    (128, 8192, 4096, _native.ROUTE_TCGEN05),
+])
+def test_sums_are_no_further_off_than_those_of_the_kernel_it_replaces(m, n, k, replaced):
+    """Against 64-bit sums, over every output.  The bound allows a tenth more, and four standard deviations of the count."""
+    layer, g = _layer(n, k, 3)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    image = layer._native_image()
+    exact = x.double() @ layer.dequantize().half().double().t()
+    mine, theirs = (_not_nearest(_native.linear(x, image, n, k, route=r), exact) for r in (BATCH, replaced))
+    assert mine <= 1.1 * theirs + 4 * (theirs / (m * n)) ** 0.5
