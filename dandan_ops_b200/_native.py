@@ -384,6 +384,7 @@ def linear_static(x, image, n, k, out):
 
 
 FLAG_FP16_STEPS = 1
+FLAG_COLUMN_SLICE = 16       # up to 16 rows the kernels that carry the all-gather (see include/b2_w4a16.h)
 FLAG_OVERLAP_LAUNCH = 2      # the streaming kernel may start under the previous kernel's tail (see include/b2_w4a16.h)
 OVERLAP_LAUNCH = os.environ.get("B2_W4A16_OVERLAP", "1") != "0"
 

@@ -591,6 +591,7 @@ bool gemm_preferred(int64_t m, const b2::Dims& d) {
 
 // The batch kernel reads x by TMA; the product of its steps and CTAs stays inside 32 bits.
 constexpr int64_t kBatchMaxM = 128;
+constexpr int64_t kGatherMaxM = 16;      // rows of x up to which projection and all-gather run as one launch
 bool batch_applicable(int64_t m, const b2::Dims& d) {
     return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 < (int64_t(1) << 23);
 }
@@ -600,13 +601,15 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 //                4096 x 12288 14.6 -> 13.1, 12289 x 3072 12.0 / 13.1 -> 10.8; 4096 x 4096 6.0 / 6.5 against 7.3) up to 16384
 //                (24576 x 4096 at M = 1 / 8 23.1 / 24.2 against 23.3 / 23.3 and, with FP16 steps, 19.0 / 20.1 against 19.9 / 20.1;
 //                57344 x 8192 at M = 1 75.9 against 77.9).  One line for both kinds of steps: the flag must not change a
-//                bit.  Below 4096 output columns the kernels that carry the all-gather stay, so that a column slice has the
-//                same bits in both forms.
+//                bit.  Not below 4096 output columns, the usual width of a slice: there a plain layer, too, has the bits
+//                of the kernels that carry the all-gather.
 //   9..16        above 4096 blocks (6144 x 4096 at M = 16 14.2 -> 9.2, 24576 x 4096 28.8 -> 23.4, 57344 x 8192 94 -> 80;
 //                2048 x 4096 5.4 against 6.0)
 //   17..128      always (1024 x 1024 at M = 17 / 64 / 128 5.1 / 12.2 / 12.5 -> 3.9 / 4.9 / 7.3, 4096 x 4096 at M = 64 20.4 -> 10.9,
 //                57344 x 8192 at M = 64 / 128 154 / 158 -> 94 / 120)
-bool batch_preferred(int64_t m, const b2::Dims& d) {
+// A column slice (B2_FLAG_COLUMN_SLICE) keeps the kernels that carry the all-gather wherever that runs in the same launch.
+bool batch_preferred(int64_t m, const b2::Dims& d, bool slice = false) {
+    if (slice && m <= kGatherMaxM) return false;
     const int64_t blocks = int64_t(d.n16) * d.kb;
     if (!batch_applicable(m, d)) return false;
     if (m > 16) return true;
@@ -1013,6 +1016,8 @@ int make_gather_call(void* const* y_ranks, void* const* flag_blocks, int64_t mai
     return B2_OK;
 }
 
+constexpr int kLayerFlags = B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH | B2_FLAG_COLUMN_SLICE;
+
 // act = 1: rows g / g+8 of every 16-row tile are a gate/up pair and y gets n/2 columns.
 int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,
                 int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
@@ -1039,7 +1044,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
-    if (route == B2_ROUTE_AUTO && !ga && batch_preferred(m, d) && gemm_applicable(x, ldx, d) &&
+    if (route == B2_ROUTE_AUTO && batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0) && gemm_applicable(x, ldx, d) &&
         workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes)
         route = B2_ROUTE_BATCH;
     if (route == B2_ROUTE_AUTO)
@@ -1091,7 +1096,7 @@ int b2_w4a16_linear_bias(const void* x, int64_t ldx, const void* native, const v
 int b2_w4a16_linear_flags(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,
                           int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
                           int64_t workspace_bytes, void* stream, int route, int flags) {
-    if (flags & ~(B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH)) return fail(B2_ERR_ARGUMENT, "unknown flag");
+    if (flags & ~kLayerFlags) return fail(B2_ERR_ARGUMENT, "unknown flag");
     return linear_impl(x, ldx, native, bias_fp16, y, ldy, m, n, k, workspace, workspace_bytes, stream, route, 0, flags);
 }
 
@@ -1104,7 +1109,7 @@ int b2_w4a16_linear_silu_mul(const void* x, int64_t ldx, const void* native, con
 int b2_w4a16_linear_silu_mul_flags(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,
                                    int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
                                    int64_t workspace_bytes, void* stream, int flags) {
-    if (flags & ~(B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH)) return fail(B2_ERR_ARGUMENT, "unknown flag");
+    if (flags & ~kLayerFlags) return fail(B2_ERR_ARGUMENT, "unknown flag");
     return linear_impl(x, ldx, native, bias_fp16, y, ldy, m, n, k, workspace, workspace_bytes, stream, B2_ROUTE_AUTO, 1, flags);
 }
 
@@ -1252,7 +1257,8 @@ int b2_w4a16_linear_gather(const void* x, int64_t ldx, const void* native, const
                            void* const* flag_blocks, int64_t mailbox_slice_bytes, int rank, int world, int64_t m,
                            int64_t ld, int64_t n_total, int64_t slice_cols, int64_t k, void* workspace,
                            int64_t workspace_bytes, void* stream, int flags) {
-    if (flags & ~(B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH)) return fail(B2_ERR_ARGUMENT, "unknown flag");
+    if (flags & ~kLayerFlags) return fail(B2_ERR_ARGUMENT, "unknown flag");
+    flags |= B2_FLAG_COLUMN_SLICE;
     GatherCall c;
     if (int rc = make_gather_call(y_ranks, flag_blocks, mailbox_slice_bytes, rank, world, m, ld, n_total, slice_cols, c)) return rc;
     if (m == 0) return B2_OK;
@@ -1260,7 +1266,7 @@ int b2_w4a16_linear_gather(const void* x, int64_t ldx, const void* native, const
     if (cols > 0) {
         void* y_local = static_cast<__half*>(y_ranks[rank]) + c.a.col0;
         int rc = kNotFused;
-        if (c.mailbox && m <= 16) rc = linear_impl(x, ldx, native, bias_fp16, y_local, ld, m, cols, k, workspace, workspace_bytes,
+        if (c.mailbox && m <= kGatherMaxM) rc = linear_impl(x, ldx, native, bias_fp16, y_local, ld, m, cols, k, workspace, workspace_bytes,
                                                    stream, B2_ROUTE_AUTO, 0, flags, &c.a);
         if (rc != kNotFused) return rc;
         rc = linear_impl(x, ldx, native, bias_fp16, y_local, ld, m, cols, k, workspace, workspace_bytes, stream,
@@ -1278,7 +1284,7 @@ int b2_w4a16_linear_gather_launches(int64_t m, int64_t n_total, int64_t slice_co
     if (cols <= 0) return 1;                                   // nothing to compute: the gather alone
     if (check_dims(cols, k) != B2_OK) return 0;
     const bool mailbox = slice_cols % 2 == 0 && n_total % 2 == 0 && world > 1 && m * slice_cols * 2 <= mailbox_slice_bytes;
-    if (!mailbox || m > 16 || k % 8 != 0) return 2;
+    if (!mailbox || m > kGatherMaxM || k % 8 != 0) return 2;
     DeviceInfo dev;
     if (device_info(dev) != B2_OK) dev.sm_count = 148;
     const b2::Dims d = b2::make_dims(cols, k);

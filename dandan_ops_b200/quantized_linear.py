@@ -227,18 +227,26 @@ class QuantizedLinear(torch.nn.Module):
         return (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
                 self.packed_weight._version, self.scales._version, self.zeros._version)
 
+    _slice_flag = 0
+
+    def serve_as_column_slice(self):
+        """This layer is one rank's slice of a column-sharded layer: up to 16 rows of x every call runs the kernels that
+        carry the all-gather, so that the slice has the same bits in every form of the gather (FLAG_COLUMN_SLICE)."""
+        self._slice_flag = _native.FLAG_COLUMN_SLICE
+        self._image_flags |= self._slice_flag
+
     def _set_image(self, image, fp16_steps):
         """Adopt an image of the current state that is complete in memory (its stream has been synchronized)."""
         self._image, self._image_key = image, self._state_key()
         self._image_flags = ((_native.FLAG_FP16_STEPS if fp16_steps else 0)
-                             | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0))
+                             | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0) | self._slice_flag)
 
     def _native_image(self):
         key = self._state_key()
         if self._image is None or self._image_key != key:
             self._image = _native.repack(self.packed_weight, self.scales, self.zeros, self.in_features)
             self._image_key = key
-            self._image_flags = self._layer_flags()
+            self._image_flags = self._layer_flags() | self._slice_flag
         return self._image
 
     def _layer_flags(self):
@@ -261,7 +269,7 @@ class QuantizedLinear(torch.nn.Module):
             raise ValueError("not a native image of this layer")
         self._image = image
         self._image_key = self._state_key()
-        self._image_flags = self._layer_flags()
+        self._image_flags = self._layer_flags() | self._slice_flag
 
     def _bias_fp16(self):
         """FP16 copy of the bias for the fused epilogue (derived, rebuilt when the bias changes)."""

@@ -113,6 +113,8 @@ class ColumnShardedLinear(torch.nn.Module):
         start, stop = shard_rows(out_features, world_size, rank)
         if local is not None and local.out_features != stop - start:
             raise ValueError("local layer does not match this rank's row range")
+        if isinstance(local, QuantizedLinear):
+            local.serve_as_column_slice()
         self.local = local
         self.out_features = out_features
         self.rank, self.world_size = rank, world_size

@@ -190,6 +190,10 @@ int b2_w4a16_linear_bias(const void* x, int64_t ldx, const void* native, const v
  * the first trip of the weights behind the previous kernel's tail; results are unchanged.  The tensor-core
  * GEMM ignores the flag. */
 #define B2_FLAG_OVERLAP_LAUNCH 2
+/* B2_FLAG_COLUMN_SLICE: the image is one rank's column slice of a sharded layer.  Up to 16 rows B2_ROUTE_AUTO then keeps to
+ * the kernels that carry the all-gather (tile and streaming), which b2_w4a16_linear_gather always does: the slice has the
+ * same bits whether it is gathered in the same launch, by b2_w4a16_gather after it, or by NCCL. */
+#define B2_FLAG_COLUMN_SLICE 16
 int b2_w4a16_linear_flags(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,
                           int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
                           int64_t workspace_bytes, void* stream, int route, int flags);
@@ -307,8 +311,8 @@ int b2_w4a16_gather_wait_limit(int64_t microseconds);      /* <= 0 restores the 
  * Layers of the tile kernel, w4a16_tile_gather_kernel: every CTA sends its tile, and the last CTA to finish
  * collects the peers' packets - taken while that is a single round of four packets per thread.
  * The transfer overlaps the math tile by tile and the launch, fence and flag round trip of a separate gather
- * disappear.  Everything else runs the projection (b2_w4a16_linear_flags into the local slice) followed by
- * b2_w4a16_gather - same result, two launches; b2_w4a16_linear_gather_launches() says which (0 = bad arguments).
+ * disappear.  Everything else runs the projection (b2_w4a16_linear_flags with B2_FLAG_COLUMN_SLICE into the local slice)
+ * followed by b2_w4a16_gather - same bits, two launches; b2_w4a16_linear_gather_launches() says which (0 = bad arguments).
  * All ranks must make the same sequence of calls; waits are bounded as in b2_w4a16_gather. */
 int b2_w4a16_linear_gather(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* const* y_ranks,
                            void* const* flag_blocks, int64_t mailbox_slice_bytes, int rank, int world, int64_t m,

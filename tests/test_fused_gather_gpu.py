@@ -13,6 +13,7 @@ import torch
 
 from dandan_ops_b200 import _native
 from dandan_ops_b200.quantized_linear import QuantizedLinear
+from dandan_ops_b200.sharded import ColumnShardedLinear
 from oracle import w4a16_oracle as oracle
 
 pytestmark = pytest.mark.gpu
@@ -210,3 +211,32 @@ def test_argument_checks_of_the_fused_call():
         _native.linear_gather(x, layer._native_image(), 64, ys, fs, MAILBOX, 0, 64, 64, 16)
     with pytest.raises(RuntimeError, match="unknown flag"):
         _native.linear_gather(x, layer._native_image(), 64, ys, fs, MAILBOX, 0, 64, 64, 32, flags=8)
+
+
+@pytest.mark.parametrize("world,m,cols,k,launches", [
+    (2, 9, 1024, 28672, 1),       # above 10 MB of image: a plain layer takes the batch kernel from 9 rows on,
+    (2, 16, 1024, 28672, 1),
+    (2, 4, 7168, 8192, 1),        # and from 4096 columns on for fewer rows
+    (4, 1, 12288, 4096, 1),
+    (2, 5, 6144, 4096, 2),        # (too much for the tile kernel's one collecting CTA)
+    (2, 24, 1024, 28672, 2),      # the one-launch form ends at 16 rows
+])
+def test_all_forms_of_a_slice_have_the_same_bits(world, m, cols, k, launches):
+    """One launch, projection + gather kernel, and the local forward whose result NCCL gathers."""
+    layer = _layer(cols, k, cols + m, True)
+    sharded = ColumnShardedLinear(layer, out_features=world * cols, rank=0, world_size=world)
+    peers = Peers(world, 0, m, world * cols, cols)
+    assert _native.linear_gather_launches(m, world * cols, cols, k, 0, world, MAILBOX) == launches
+    g = torch.Generator().manual_seed(m)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    theirs = peers.play_peers(1, g)
+    _run(peers, layer, x, k)
+    torch.cuda.synchronize()
+    local = sharded(x)
+    out = torch.empty(m, cols, dtype=torch.float16, device="cuda")
+    assert torch.equal(peers.bufs[0][:, :cols], local) and torch.equal(layer.forward_into(x, out), local)
+    for q, data in theirs.items():
+        assert torch.equal(peers.bufs[0][:, q * cols:(q + 1) * cols], data)
+    layer.scales.mul_(1.0)                                     # a new image of the state keeps the rule
+    assert torch.equal(sharded(x), local)
+    assert _native.gather_status(peers.flags[0].data_ptr()) == 0 and _native.status() == 0
