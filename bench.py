@@ -87,6 +87,25 @@ def measured_peak(key, fallback):
     return fallback, "fallback"
 
 
+ROUTE_KERNELS = {"b200_tile": "w4a16_tile_kernel", "b200_stream": "w4a16_stream_kernel", "b200_batch": "w4a16_batch_kernel",
+                 "b200_tcgen05": "w4a16_gemm_pair_kernel"}
+
+
+def step_kernel(calls):
+    """The kernel that streams most of a rank's weight bytes per step, and the step's DRAM bytes per weight byte (None when
+    one of its kernels has no measured factor)."""
+    from dandan_ops_b200 import _native
+    share = {}
+    for c in calls:
+        flags = _native.FLAG_COLUMN_SLICE if c["sharded"] is not None else 0
+        kernel = ROUTE_KERNELS[_native.plan(c["m"], c["n"], c["k"], flags)["route"]] if c["n"] else None
+        share[kernel] = share.get(kernel, 0.0) + weight_bytes(c["n"], c["k"])
+    factors = {kernel: dram_traffic_factor(kernel) for kernel in share if kernel}
+    total = sum(share.values())
+    factor = None if None in factors.values() else sum(factors[kernel] * share[kernel] for kernel in factors) / max(total, 1.0)
+    return max(share, key=share.get), factor
+
+
 def dram_traffic_factor(kernel):
     """DRAM bytes (read + written) per algorithmic weight byte of a launch, as ncu measured it for
     `kernel`: the table lives in profiles/dram_traffic_per_kernel.md (| kernel | factor | capture |)."""
@@ -495,11 +514,10 @@ def run_gpu(args, rank, world, local_rank):
 
     if rank == 0:
         peak, peak_kind = measured_peak("hbm_gbs", FALLBACK_HBM_GBS)
-        kernel = "w4a16_tile_kernel" if args.workload == "qwen3-0.6b-decode" else "w4a16_stream_kernel"
+        kernel, factor = step_kernel(calls)
         # one rank's projection launches: algorithmic bytes per launch / average launch time (CUDA events over
         # the replayed graph of the projections; at N = 1 that graph is the timed step itself)
         achieved = (step_alg_bytes / proj_launches) / (proj_ms_per_step * 1e-3 / proj_launches) / 1e9
-        factor = dram_traffic_factor(kernel)
         result = {
             "metric": "w4a16_decode_weight_hbm_GBps", "value": round(weight_total / (ms_per_step * 1e-3) / 1e9, 2),
             "unit": "GB/s", "n_gpus": world, "steps": args.steps, "warmup": warm,

@@ -59,6 +59,8 @@ _SIGNATURES = {
     "b2_w4a16_rmsnorm_linear": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.c_float, _vp, _i64, _vp, _vp, _vp, _vp, _i64,
                                        _i64, _i64, _i64, _vp, _i64, _vp]),
     "b2_w4a16_residual_rms_norm": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.c_float, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
+    "b2_w4a16_plan_flags": (_int, [_i64, _i64, _i64, _int, ctypes.POINTER(_int), ctypes.POINTER(_int),
+                                   ctypes.POINTER(_int), ctypes.POINTER(_int)]),
     "b2_w4a16_plan": (_int, [_i64, _i64, _i64, ctypes.POINTER(_int), ctypes.POINTER(_int),
                              ctypes.POINTER(_int), ctypes.POINTER(_int)]),
 }
@@ -284,11 +286,11 @@ def dequantize(image, n, k, dtype=torch.float32):
     return out
 
 
-def plan(m, n, k):
+def plan(m, n, k, flags=0):
     lib = load()
     route, splits, grid, rows = _int(), _int(), _int(), _int()
-    _check(lib.b2_w4a16_plan(m, n, k, ctypes.byref(route), ctypes.byref(splits), ctypes.byref(grid),
-                             ctypes.byref(rows)))
+    _check(lib.b2_w4a16_plan_flags(m, n, k, flags, ctypes.byref(route), ctypes.byref(splits), ctypes.byref(grid),
+                                   ctypes.byref(rows)))
     return {"route": ROUTE_NAMES.get(route.value, str(route.value)), "k_splits": splits.value,
             "grid": grid.value, "rows_per_launch": rows.value}
 

@@ -590,6 +590,7 @@ bool gemm_preferred(int64_t m, const b2::Dims& d) {
 }
 
 // The batch kernel reads x by TMA; the product of its steps and CTAs stays inside 32 bits.
+constexpr int kLayerFlags = B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH | B2_FLAG_COLUMN_SLICE;
 constexpr int64_t kBatchMaxM = 128;
 constexpr int64_t kGatherMaxM = 16;      // rows of x up to which projection and all-gather run as one launch
 bool batch_applicable(int64_t m, const b2::Dims& d) {
@@ -879,15 +880,20 @@ int b2_w4a16_set_gemm_shape(int shape, int k_splits) {
 }
 
 int b2_w4a16_plan(int64_t m, int64_t n, int64_t k, int* route, int* k_splits, int* grid, int* rows_per_launch) {
+    return b2_w4a16_plan_flags(m, n, k, 0, route, k_splits, grid, rows_per_launch);
+}
+
+int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, int* k_splits, int* grid, int* rows_per_launch) {
+    if (flags & ~kLayerFlags) return fail(B2_ERR_ARGUMENT, "unknown flag");
     if (int rc = check_dims(n, k)) return rc;
     if (m < 0) return fail(B2_ERR_ARGUMENT, "m must be non-negative");
     DeviceInfo dev;
     if (device_info(dev) != B2_OK) dev.sm_count = 148;   // planning also works without a device
     const b2::Dims d = b2::make_dims(n, k);
     const StreamPlan p = plan_stream(m > 0 ? m : 1, d, dev.sm_count);
-    if (m > 0 && batch_preferred(m, d)) {          // assuming an aligned x, as execution_info cannot see the pointer
+    if (m > 0 && batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0)) {   // (an aligned x: the pointer is not known here)
         const b2host::BatchPlan bp = b2host::plan_batch(m, d, dev.sm_count);
-        if (route) *route = gemm_preferred(m, d) ? B2_ROUTE_TCGEN05 : B2_ROUTE_STREAM;     // it stands in for either family
+        if (route) *route = B2_ROUTE_BATCH;
         if (k_splits) *k_splits = bp.max_parts;
         if (grid) *grid = bp.grid;
         if (rows_per_launch) *rows_per_launch = int(m);
@@ -1015,8 +1021,6 @@ int make_gather_call(void* const* y_ranks, void* const* flag_blocks, int64_t mai
     c.mailbox = words && world > 1 && m * slice_cols * 2 <= mailbox_slice_bytes && m * slice_cols > 0;
     return B2_OK;
 }
-
-constexpr int kLayerFlags = B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH | B2_FLAG_COLUMN_SLICE;
 
 // act = 1: rows g / g+8 of every 16-row tile are a gate/up pair and y gets n/2 columns.
 int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,

@@ -292,7 +292,7 @@ class QuantizedLinear(torch.nn.Module):
                     "fallback_reason": str(exc), "reason": str(exc), "input_copies": [],
                     "format_version": FORMAT_VERSION, "activation_dtype": str(x.dtype),
                     "group_size": self.group_size, "kernel_plan": None}
-        plan = _native.plan(x.shape[0], self.out_features, self.in_features)
+        plan = _native.plan(x.shape[0], self.out_features, self.in_features, self._slice_flag)
         return {"requested_backend": self.backend, "implementation": plan["route"],
                 "fallback_reason": None, "reason": "selected packed inference backend",
                 "input_copies": [i for i, t in enumerate((x, self.packed_weight, self.scales, self.zeros))

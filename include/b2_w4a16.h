@@ -243,12 +243,14 @@ int b2_w4a16_residual_rms_norm(const void* x, int64_t ldx, const void* residual,
 int b2_w4a16_silu_mul_pairs(const void* y_pairs, int64_t ld_in, void* out, int64_t ld_out, int64_t m, int64_t n,
                             void* stream);
 
-/* Which kernel family B2_ROUTE_AUTO picks for this problem (a B2_ROUTE_* value; the batch kernel counts to the
- * family whose batches it takes: streaming, or tensor-memory GEMM above 32 rows of a layer above ~10 MB) and,
- * through the optional out-parameters, the launch plan: K-splits, grid size, rows of x
- * handled per launch.  Pure host arithmetic; used by execution_info(). */
+/* Which kernel family B2_ROUTE_AUTO picks for this problem (a B2_ROUTE_* value) with a 16-byte aligned x and the
+ * workspace that b2_w4a16_workspace_bytes() asks for and, through the optional out-parameters, the launch plan:
+ * K-splits (batch kernel: most CTAs that share a tile), grid size, rows of x handled per launch.  Pure host
+ * arithmetic; used by execution_info().  `flags`: layer flags of the call. */
 int b2_w4a16_plan(int64_t m, int64_t n, int64_t k, int* route, int* k_splits, int* grid,
                   int* rows_per_launch);
+int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, int* k_splits, int* grid,
+                        int* rows_per_launch);
 
 /* Tile shape of the tensor-memory GEMM (B2_ROUTE_TCGEN05).  B2_GEMM_SHAPE_AUTO picks per call
  * by a cost model (waves x cost per tile); the others force one shape for every later call of

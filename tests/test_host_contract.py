@@ -43,7 +43,8 @@ def test_library_builds_loads_and_exports_every_declared_symbol():
     assert _native.plan(8, 512, 8192) == {"route": "b200_tile", "k_splits": 4, "grid": 128, "rows_per_launch": 8}
     assert _native.plan(16, 1024, 1024)["k_splits"] == 1 and _native.plan(16, 4096, 4096)["k_splits"] == 1
     assert _native.plan(8, 57344, 8192)["route"] == "b200_stream"
-    assert _native.plan(32, 2048, 1024)["route"] == "b200_stream"
+    assert _native.plan(32, 2048, 1024)["route"] == "b200_batch"
+    assert _native.plan(32, 2048, 1025)["route"] == "b200_stream"        # K % 8 != 0
     assert _native.plan(512, 4096, 4096)["route"] == "b200_tcgen05"
     assert _native.plan(512, 4096, 4097)["route"] == "b200_stream"       # K % 8 != 0
     lib2 = _native.load()
@@ -218,13 +219,29 @@ def test_gemm_cost_model_picks_pair_kernels():
     assert _native.plan(512, 12288, 4096)["grid"] == 2 * 48 * 3         # pair, 192 rows of x per pair
     assert _native.plan(2048, 4096, 4096)["grid"] == 2 * 16 * 8         # pair, 256 rows of x per pair
     assert _native.plan(256, 24576, 4096)["grid"] == 128                # single CTA, 256 x 192
-    small = _native.plan(100, 4096, 4096)                               # 16 tiles of one row: K split four ways
+    small = _native.plan(192, 4096, 4096)                               # 16 tiles of one row: K split four ways
     assert small["route"] == "b200_tcgen05" and small["k_splits"] == 4 and small["grid"] == 2 * 16 * 4
-    assert _native.plan(48, 57344, 8192)["route"] == "b200_tcgen05"     # large layer: the GEMM from 33 rows on
-    assert _native.plan(32, 57344, 8192)["route"] == "b200_stream"
-    assert _native.plan(48, 6144, 1024)["route"] == "b200_stream"       # small layer: streaming kernel up to 64 rows
+    assert _native.plan(129, 57344, 8192)["route"] == "b200_tcgen05"    # the GEMM above 128 rows
     split = _native.plan(256, 4096, 28672)                              # 16 tiles, 112 blocks of K: four CTAs per tile
     assert split["k_splits"] == 4 and split["grid"] == 2 * 16 * 4
+
+
+def test_plan_names_the_kernel_that_runs():
+    def route(m, n, k, flags=0):
+        return _native.plan(m, n, k, flags)["route"]
+
+    for m, n, k in ((1, 4096, 12288), (8, 6144, 4096), (16, 24576, 4096), (17, 12289, 3072), (48, 57344, 8192), (64, 6144, 1024),
+                    (100, 4096, 4096), (128, 4096, 4096)):
+        plan = _native.plan(m, n, k)
+        assert plan["route"] == "b200_batch" and plan["rows_per_launch"] == m and 1 <= plan["grid"] <= 148
+    assert route(8, 57344, 8192) == "b200_stream" and route(16, 4096, 4096) == "b200_tile" and route(129, 4096, 4096) == "b200_tcgen05"
+    # one rank's slice keeps the kernels that carry the all-gather as far as that goes
+    piece = _native.FLAG_COLUMN_SLICE
+    assert route(16, 1024, 28672) == "b200_batch" and route(16, 1024, 28672, piece) == "b200_stream"
+    assert route(4, 6144, 4096) == "b200_batch" and route(4, 6144, 4096, piece) == "b200_tile"
+    assert route(17, 1024, 28672, piece) == "b200_batch"
+    with pytest.raises(RuntimeError, match="unknown flag"):
+        _native.plan(1, 64, 64, 4)
 
 
 def test_operator_library_registers_the_reference_op_names():

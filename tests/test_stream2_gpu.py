@@ -1,6 +1,6 @@
 """The other forms of the streaming kernel (large layers, M <= 16) and the give-up path of the bounded waits.
 
-Variant 0 / 1 is the shipped kernel (what B2_ROUTE_AUTO runs); 2 / 3 are the 32- / 16-warp double-buffered
+Variant 0 / 1 is the shipped kernel; 2 / 3 are the 32- / 16-warp double-buffered
 forms, 4 the chunk-major two-dimensional split (w4a16_stream2d_kernel) wherever K exceeds the x buffer - all
 measured slower or level, kept behind the hook.
 
@@ -42,7 +42,7 @@ def test_forced_32_warp_kernel_on_ragged_shapes(hooks, variant, m, n, k):
     x = torch.randn(m, k, generator=g).half().cuda()
     image = layer._native_image()
     hooks(stream_variant=variant)
-    assert _native.plan(m, n, k)["route"] in ("b200_stream", "b200_tile")
+    assert _native.plan(m, n, k)["route"] in ("b200_stream", "b200_tile", "b200_batch")     # what the automatic route takes
     y2 = guarded_linear(x, image, n, k, route=_native.ROUTE_STREAM)
     again = guarded_linear(x, image, n, k, route=_native.ROUTE_STREAM)
     assert torch.equal(y2, again)                                    # split-K sums do not depend on timing

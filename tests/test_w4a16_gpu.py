@@ -270,10 +270,11 @@ def test_tcgen05_route_against_oracle_formula(m, n, k):
     g = torch.Generator().manual_seed(m + n + k)
     layer = ops.QuantizedLinear.from_float((torch.randn(n, k, generator=g) * 0.05).half().cuda())
     x = torch.randn(m, k, generator=g).half().cuda()
-    assert layer.execution_info(x)["implementation"] == "b200_tcgen05"
+    # the automatic route is the batch kernel up to 128 rows, which adds in another order
+    route = _native.ROUTE_BATCH if m <= 128 else _native.ROUTE_TCGEN05
+    assert layer.execution_info(x)["implementation"] == _native.ROUTE_NAMES[route]
     y = layer(x)
-    # up to 128 rows the automatic route is the batch kernel, which adds in another order
-    forced = _native.linear(x, layer._native_image(), n, k, route=_native.ROUTE_BATCH if m <= 128 else _native.ROUTE_TCGEN05)
+    forced = _native.linear(x, layer._native_image(), n, k, route=route)
     assert torch.equal(y, forced)
     assert _native.status() == 0
     expected = (x.double() @ layer.dequantize().half().double().t())
