@@ -945,8 +945,8 @@ int64_t b2_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) {
     int64_t need = stream_workspace_bytes(m > 0 ? m : 1, d, dev.sm_count);
     if (gemm_preferred(m, d))     // room for the partial tiles of a K-split tensor-memory GEMM
         need = std::max(need, B2_W4A16_TICKET_BYTES + gemm_shape(m, d.n, d.kb, dev.sm_count > 0 ? dev.sm_count : 148).partial_bytes(m, d.n));
-    if (m > 0 && batch_applicable(m, d))           // partial tiles of the batch kernel (also when its route is asked for)
-        need = std::max(need, B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes);
+    if (batch_applicable(std::min(m, kBatchMaxM), d))    // room for the batch kernel at this and every smaller batch
+        need = std::max(need, B2_W4A16_TICKET_BYTES + b2host::batch_workspace(m, d, dev.sm_count));
     return need;
 }
 
@@ -1048,15 +1048,17 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
-    if (route == B2_ROUTE_AUTO && batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0) && gemm_applicable(x, ldx, d) &&
-        workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::plan_batch(m, d, dev.sm_count).partial_bytes)
+    const bool batch = batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0);
+    if (route == B2_ROUTE_AUTO && batch && gemm_applicable(x, ldx, d) &&
+        workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::batch_workspace(m, d, dev.sm_count))
         route = B2_ROUTE_BATCH;
     if (route == B2_ROUTE_AUTO)
         route = tile_applicable(m, d, tile_split) ? B2_ROUTE_TILE
               : (gemm_preferred(m, d) && gemm_applicable(x, ldx, d)) ? B2_ROUTE_TCGEN05 : B2_ROUTE_STREAM;
     if (act && route == B2_ROUTE_TCGEN05 && !gemm_shape_for_call(m, d, dev.sm_count, workspace_bytes).pair_mt) {
-        // the single-CTA GEMM has no such epilogue: small batches stream, larger ones take two launches
-        if (m > B2_STREAM_MAX_M)
+        // the single-CTA GEMM has no such epilogue: small batches stream, larger ones take two launches (unless the batch
+        // kernel would have taken them with a larger workspace: b2_w4a16_silu_mul_is_fused() says one launch)
+        if (m > B2_STREAM_MAX_M && !batch)
             return fail(B2_ERR_UNSUPPORTED, "no fused gate/up epilogue for this problem: run b2_w4a16_linear, then b2_w4a16_silu_mul_pairs");
         route = B2_ROUTE_STREAM;
     }

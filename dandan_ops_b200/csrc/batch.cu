@@ -56,7 +56,7 @@ namespace b2host {
 
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     BatchPlan p;
-    p.nx = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    p.nx = b2::batch_nx(m);
     const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows, tsteps = d.kb * 4;
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);

@@ -16,6 +16,13 @@ struct BatchPlan {
     int64_t partial_bytes;
 };
 
+// Partial tiles of any batch of up to m rows (more than 128 count as 128): grows with m, so a workspace that was sized for
+// one batch holds the plan of every smaller one.  At most 19.4 MB.
+inline int64_t batch_workspace(int64_t m, const b2::Dims& d, int sm_count) {
+    const int64_t steps = int64_t((d.n + b2::kBatchRows - 1) / b2::kBatchRows) * d.kb * 4, sms = sm_count > 0 ? sm_count : 148;
+    return b2::batch_partial_bytes(b2::batch_nx(m), int(steps < sms ? steps : sms));
+}
+
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count);
 int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool h16, bool overlap, cudaStream_t s);
 

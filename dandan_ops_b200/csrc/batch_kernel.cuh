@@ -44,6 +44,7 @@ constexpr uint32_t kBatchWCols = 32;                // tensor-memory columns of 
 constexpr int kBatchSets = 2;                       // sets of eight converter warps (three sets, 72 registers: 3-4 % slower)
 constexpr int kBatchWarps = 8 * kBatchSets;
 constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
+__host__ __device__ constexpr int batch_nx(int64_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }    // rows of x of an MMA
 // Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside the accumulators.
 __host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; }
 // The FP32 sums of a tile run as C chains (the products of 16 columns of K go to chain kk % C), added in order when they

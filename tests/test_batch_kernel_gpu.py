@@ -176,3 +176,40 @@ def test_sums_are_no_further_off_than_those_of_the_kernel_it_replaces(m, n, k, r
     exact = x.double() @ layer.dequantize().half().double().t()
     mine, theirs = (_not_nearest(_native.linear(x, image, n, k, route=r), exact) for r in (BATCH, replaced))
     assert mine <= 1.1 * theirs + 4 * (theirs / (m * n)) ** 0.5
+
+
+def _raw(x, layer, ws_bytes, act=False):
+    lib, (m, k), n = _native.load(), x.shape, layer.out_features
+    ws = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda")
+    y = torch.zeros(m, n // 2 if act else n, dtype=torch.float16, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    args = (x.data_ptr(), k, layer._native_image().data_ptr(), None, y.data_ptr(), y.stride(0), m, n, k, ws.data_ptr(), ws_bytes, stream)
+    rc = lib.b2_w4a16_linear_silu_mul(*args) if act else lib.b2_w4a16_linear_bias(*args, _native.ROUTE_AUTO)
+    assert rc == 0, lib.b2_w4a16_last_error()
+    return y
+
+
+@pytest.mark.parametrize("m,n,k", [(100, 6144, 4096), (128, 4096, 12288), (65, 1024, 8192)])
+def test_one_workspace_for_all_batches(m, n, k):
+    layer, g = _layer(n, k, 8)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    size = _native.load().b2_w4a16_workspace_bytes
+    want = _native.linear(x, layer._native_image(), n, k, route=BATCH)
+    for larger in (m, 129, 256, 2048):
+        assert torch.equal(_raw(x, layer, int(size(larger, n, k))), want)
+
+
+def test_a_fused_call_runs_in_less_workspace_too():
+    """What b2_w4a16_silu_mul_is_fused() promises does not depend on the workspace, nor on the GEMM's tile shape (the
+    single-CTA ones, which a device without two-CTA clusters takes, have no such epilogue)."""
+    m, n, k = 100, 512, 256
+    layer, g = _layer(n, k, 8)
+    x = torch.randn(m, k, generator=g).half().cuda()
+    _native.set_gemm_shape("128x128")
+    try:
+        lib = _native.load()
+        assert lib.b2_w4a16_silu_mul_is_fused(m, n, k)
+        need = int(lib.b2_w4a16_workspace_bytes(m, n, k))
+        torch.testing.assert_close(_raw(x, layer, need - 4096, act=True), _raw(x, layer, need, act=True), atol=2e-3, rtol=2e-3)
+    finally:
+        _native.set_gemm_shape()

@@ -284,6 +284,18 @@ def test_stream_plan_keeps_tickets_inside_the_ticket_area():
             assert plan["k_splits"] >= 1 and plan["grid"] >= 1
 
 
+@pytest.mark.parametrize("n,k", [(6144, 4096), (4096, 12288), (128, 64), (12289, 3072), (57344, 8192), (1024, 28672)])
+def test_a_workspace_sized_for_a_large_batch_holds_the_batch_kernel_of_every_smaller_one(n, k):
+    """Otherwise the kernel, and with it the order of the sums, would depend on what else the buffer was sized for."""
+    lib = _native.load()
+    steps = -(-n // 128) * -(-k // 256) * 4
+    for m, nx in ((1, 16), (16, 16), (17, 32), (33, 64), (65, 128), (128, 128)):
+        need = _native.TICKET_BYTES + min(148, steps) * 2 * nx * 128 * 4          # two partial tiles of 128 rows per CTA
+        for larger in (m, 64, 128, 129, 192, 256, 300, 1000, 2048, 4096):
+            if larger >= m:
+                assert lib.b2_w4a16_workspace_bytes(larger, n, k) >= need, (m, larger)
+
+
 def test_gather_form_query_is_a_pure_function_of_the_problem():
     """`b2_w4a16_linear_gather_launches`: which calls run projection and gather as one kernel.  Needs no GPU
     (an unknown device counts as 148 SMs); every rank must get the same answer for equal slices."""
