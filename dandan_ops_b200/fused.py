@@ -16,9 +16,11 @@ from .quantized_linear import QuantizedLinear
 
 
 def _plain(x):
-    """Whether the C++ operator library runs this call: an ordinary tensor outside autograd, and no private workspace
-    asked for (the operator library keeps its own, one per stream)."""
+    """Whether the C++ operator library runs this call: an ordinary tensor outside autograd and functorch transforms
+    (vmap, jvp: the operators have no rules for them, and the ctypes path refuses their wrappers, which have no storage),
+    and no private workspace asked for (the operator library keeps its own, one per stream)."""
     return (_ops.SHIM_LOADED and type(x) is torch.Tensor and not _native._private
+            and not torch._C._functorch.is_functorch_wrapped_tensor(x)
             and not (x.requires_grad and torch.is_grad_enabled()))
 
 

@@ -251,3 +251,21 @@ def test_rmsnorm_linear_matches_norm_then_projection(m, n, k, with_residual):
     if layer.bias is not None:
         expected = (expected.float().half() + layer.bias.half().cpu()).double()
     torch.testing.assert_close(y.cpu().double(), expected, atol=4e-3, rtol=4e-3)
+
+
+def test_functorch_transforms_do_not_reach_the_operator_library(monkeypatch):
+    """The operators have no batching or forward-mode rule (a tangent would be dropped); the other path refuses the wrappers."""
+    from dandan_ops_b200 import fused
+    monkeypatch.setattr(fused._ops, "SHIM_LOADED", True)
+    seen = []
+
+    def f(x):
+        seen.append(fused._plain(x))
+        return x * 2
+
+    x = torch.ones(2, 3)
+    torch.func.vmap(f)(x)
+    torch.func.jvp(f, (x,), (x,))
+    torch.func.grad(lambda t: f(t).sum())(x)
+    f(x)
+    assert seen == [False, False, False, True]
