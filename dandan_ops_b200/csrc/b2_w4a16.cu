@@ -597,24 +597,38 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
     return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 < (int64_t(1) << 23);
 }
 
-// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of what ran before (us, tile / streaming / GEMM -> batch):
-//   up to 8 rows above 4096 native blocks (~10 MB), where the tile kernel runs out (6144 x 4096 at M = 1 / 8 10.0 / 10.2 -> 8.9 / 9.0,
-//                4096 x 12288 14.6 -> 13.1, 12289 x 3072 12.0 / 13.1 -> 10.8; 4096 x 4096 6.0 / 6.5 against 7.3) up to 16384
-//                (24576 x 4096 at M = 1 / 8 23.1 / 24.2 against 23.3 / 23.3 and, with FP16 steps, 19.0 / 20.1 against 19.9 / 20.1;
-//                57344 x 8192 at M = 1 75.9 against 77.9).  One line for both kinds of steps: the flag must not change a
-//                bit.  Not below 4096 output columns, the usual width of a slice: there a plain layer, too, has the bits
-//                of the kernels that carry the all-gather.
-//   9..16        above 4096 blocks (6144 x 4096 at M = 16 14.2 -> 9.2, 24576 x 4096 28.8 -> 23.4, 57344 x 8192 94 -> 80;
-//                2048 x 4096 5.4 against 6.0)
-//   17..128      always (1024 x 1024 at M = 17 / 64 / 128 5.1 / 12.2 / 12.5 -> 3.9 / 4.9 / 7.3, 4096 x 4096 at M = 64 20.4 -> 10.9,
-//                57344 x 8192 at M = 64 / 128 154 / 158 -> 94 / 120)
+// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of what ran before (us in a chain of dependent launches,
+// tile / streaming / GEMM -> batch).  A wide layer has more tiles of 128 columns than SMs: its CTAs pay for reading more than
+// one tile's sums back, which a short K does not carry.
+//   up to 8 rows above 4096 native blocks (~10 MB), where the tile kernel runs out, up to 16384, not on wide layers: 6144 x 4096
+//                at M = 1 / 8 10.1 / 10.4 -> 9.2 / 9.5, 4096 x 12288 14.1 / 14.2 -> 12.7 / 12.9, 14336 x 2048 at M = 8
+//                11.5 -> 8.5; 4096 x 4096 6.2 / 6.7 against 7.3, 24576 x 4096 21.7 / 22.4 against 21.9 / 22.2, 28672 x 1024
+//                11.3 against 11.8.  One line for both kinds of steps: the flag must not change a bit.  Not below 4096
+//                output columns, the usual width of a slice: there a plain layer, too, has the bits of the kernels that
+//                carry the all-gather.
+//   9..16        above 4096 blocks, wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7, 24576 x 4096 26.8 -> 22.5,
+//                57344 x 8192 90 -> 75; 57344 x 512 11.3 against 12.8
+//   17..32       from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
+//                1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 8.4 / 8.7, 57344 x 8192 121 / 125 -> 78
+//                / 80; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4, 256 x 4096 6.2 / 6.2
+//                against 6.8 / 7.2.  (Behind a kernel that does not let it start early the batch kernel's own start shows:
+//                up to 1024 blocks 0.5 to 2.4 us more than the streaming kernel, 1024 x 1024 at M = 17 7.3 against 5.5.  The
+//                two cannot be told apart here, and of a decoder layer's four projections most are in the first position.)
+//   33..64       always: 1024 x 1024 at M = 64 12.4 -> 5.2, 4096 x 4096 19.9 -> 11.1, 57344 x 8192 147 -> 93, 28672 x 1024 16.4
+//                -> 15.5
+//   65..128      wide layers from 13 blocks of 256 columns per SM on: 57344 x 8192 at M = 128 184 -> 125, 40960 x 2048 40.0 ->
+//                33.6, 28672 x 3072 33.2 -> 32.7; 28672 x 2048 25.8 against 27.3, 28672 x 1024 17.2 against 21.6; others
+//                always (4096 x 4096 20.2 -> 15.7, 1024 x 1024 11.2 -> 7.6, 18944 x 1024 13.3 -> 10.1)
 // A column slice (B2_FLAG_COLUMN_SLICE) keeps the kernels that carry the all-gather wherever that runs in the same launch.
-bool batch_preferred(int64_t m, const b2::Dims& d, bool slice = false) {
-    if (slice && m <= kGatherMaxM) return false;
-    const int64_t blocks = int64_t(d.n16) * d.kb;
-    if (!batch_applicable(m, d)) return false;
-    if (m > 16) return true;
-    return blocks > 4096 && (m > 8 || (d.n >= 4096 && blocks <= 16384));
+bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = false) {
+    if ((slice && m <= kGatherMaxM) || !batch_applicable(m, d)) return false;
+    const int64_t blocks = int64_t(d.n16) * d.kb, tiles = (int64_t(d.n) + 127) / 128, sms = sm_count > 0 ? sm_count : 148;
+    const bool wide = tiles > sms;
+    if (m > 64) return !wide || tiles * d.kb >= 13 * sms;
+    if (m > 32) return true;
+    if (m > 16) return d.kb > 1 && (d.n > 512 || d.kb < 8 || d.kb >= 32);
+    if (m > 8) return blocks > 4096 && (!wide || d.kb > 2);
+    return blocks > 4096 && blocks <= 16384 && d.n >= 4096 && !wide;
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
@@ -891,7 +905,7 @@ int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, 
     if (device_info(dev) != B2_OK) dev.sm_count = 148;   // planning also works without a device
     const b2::Dims d = b2::make_dims(n, k);
     const StreamPlan p = plan_stream(m > 0 ? m : 1, d, dev.sm_count);
-    if (m > 0 && batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0)) {   // (an aligned x: the pointer is not known here)
+    if (m > 0 && batch_preferred(m, d, dev.sm_count, (flags & B2_FLAG_COLUMN_SLICE) != 0)) {   // (an aligned x: the pointer is not known here)
         const b2host::BatchPlan bp = b2host::plan_batch(m, d, dev.sm_count);
         if (route) *route = B2_ROUTE_BATCH;
         if (k_splits) *k_splits = bp.max_parts;
@@ -1048,7 +1062,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (dev.cc_major != 10) return fail(B2_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     const b2::Dims d = b2::make_dims(n, k);
     const int tile_split = tile_ksplit(d, dev.sm_count, pair_available());
-    const bool batch = batch_preferred(m, d, (flags & B2_FLAG_COLUMN_SLICE) != 0);
+    const bool batch = batch_preferred(m, d, dev.sm_count, (flags & B2_FLAG_COLUMN_SLICE) != 0);
     if (route == B2_ROUTE_AUTO && batch && gemm_applicable(x, ldx, d) &&
         workspace_bytes >= B2_W4A16_TICKET_BYTES + b2host::batch_workspace(m, d, dev.sm_count))
         route = B2_ROUTE_BATCH;
@@ -1181,7 +1195,7 @@ int b2_w4a16_silu_mul_is_fused(int64_t m, int64_t n, int64_t k) {
     DeviceInfo dev;
     if (device_info(dev) != B2_OK) dev.sm_count = 148;
     const b2::Dims d = b2::make_dims(n, k);
-    if (d.k % 8 != 0 || batch_preferred(m, d)) return 1;   // the streaming kernel in chunks of 64 rows, or the batch kernel
+    if (d.k % 8 != 0 || batch_preferred(m, d, dev.sm_count)) return 1;   // the streaming kernel in chunks of 64 rows, or the batch kernel
     return gemm_shape_for_call(m, d, dev.sm_count > 0 ? dev.sm_count : 148, INT64_MAX).pair_mt != 0 ? 1 : 0;
 }
 

@@ -59,7 +59,7 @@ def test_row_strides_of_x_and_y():
     assert torch.equal(out[:, 3:1003], want) and bool((out[:, :3] == 7).all()) and bool((out[:, 1003:] == 7).all())
 
 
-@pytest.mark.parametrize("m,rows,k", [(33, 72, 264), (64, 1536, 1024), (1, 4096, 2304), (12, 32768, 264), (128, 32768, 512)])
+@pytest.mark.parametrize("m,rows,k", [(33, 72, 264), (64, 1536, 1024), (1, 4096, 2304), (12, 32768, 520), (128, 32768, 1032)])
 def test_gate_up_epilogue_matches_the_separate_kernel(m, rows, k):
     """The automatic route takes the batch kernel on these; the activation sees the same sums in the same order."""
     gate, g = _layer(rows, k, 1)

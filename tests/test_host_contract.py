@@ -244,6 +244,19 @@ def test_plan_names_the_kernel_that_runs():
         _native.plan(1, 64, 64, 4)
 
 
+def test_batch_kernel_only_where_it_is_ahead():
+    """Both sides of every line of the rule; where it was taken beyond, calls were up to a third slower than before."""
+    def batch(m, n, k):
+        return _native.plan(m, n, k)["route"] == "b200_batch"
+
+    assert batch(8, 14336, 2048) and not batch(8, 28672, 1024) and not batch(1, 24576, 1024)       # more tiles than SMs
+    assert batch(16, 28672, 1024) and not batch(16, 57344, 512)
+    assert batch(64, 28672, 1024) and batch(33, 64, 64)
+    assert batch(128, 18944, 512) and not batch(128, 19072, 512) and not batch(65, 28672, 2048) and batch(65, 28672, 3072)
+    assert batch(17, 1024, 1024) and batch(32, 64, 1024) and not batch(32, 2048, 256) and not batch(17, 40960, 256)
+    assert batch(24, 256, 8192) and not batch(24, 256, 4096) and not batch(17, 512, 2048) and batch(17, 576, 2048)
+
+
 def test_operator_library_registers_the_reference_op_names():
     """The C++ operator library (TORCH_LIBRARY over the C ABI) builds without a GPU, loads with
     torch.ops.load_library and defines the reference's native op surface
