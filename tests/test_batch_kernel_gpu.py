@@ -213,3 +213,24 @@ def test_a_fused_call_runs_in_less_workspace_too():
         torch.testing.assert_close(_raw(x, layer, need - 4096, act=True), _raw(x, layer, need, act=True), atol=2e-3, rtol=2e-3)
     finally:
         _native.set_gemm_shape()
+
+
+@pytest.mark.parametrize("m,n,k,bad", [(9, 1000, 520, 4), (33, 384, 1032, 32), (70, 136, 264, 69)])
+def test_a_row_that_is_not_finite_touches_no_other(m, n, k, bad):
+    """Rows of x beyond M and weight rows beyond N are multiplied too: a NaN or an infinity stays in its row, and there is
+    what an exact sum gives."""
+    layer, g = _layer(n, k, 12)
+    x = torch.randn(m, k, generator=g).half()
+    image = layer._native_image()
+    clean = _native.linear(x.cuda(), image, n, k, route=BATCH)
+    x[bad, k - 1] = float("inf")
+    x[bad, 3] = -float("inf")
+    exact = x.double() @ layer.dequantize().half().double().cpu().t()
+    y = _native.linear(x.cuda(), image, n, k, route=BATCH).cpu()
+    others = [r for r in range(m) if r != bad]
+    assert torch.equal(y[others], clean.cpu()[others])
+    assert torch.equal(y[bad].isnan(), exact[bad].isnan()) and torch.equal(y[bad].isposinf(), exact[bad].isposinf())
+    assert bool((y[bad].isnan() | y[bad].isinf()).all()) and bool(y[bad].isnan().any()) and bool(y[bad].isinf().any())
+    x[bad, 5] = float("nan")
+    y = _native.linear(x.cuda(), image, n, k, route=BATCH).cpu()
+    assert torch.equal(y[others], clean.cpu()[others]) and bool(y[bad].isnan().all())

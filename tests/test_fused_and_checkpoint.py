@@ -2,6 +2,8 @@
 
 CPU tests cover the state handling; the GPU tests compare with the separate layers and with a
 fresh repack."""
+import contextlib
+
 import numpy as np
 import pytest
 import torch
@@ -269,3 +271,31 @@ def test_functorch_transforms_do_not_reach_the_operator_library(monkeypatch):
     torch.func.grad(lambda t: f(t).sum())(x)
     f(x)
     assert seen == [False, False, False, True]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [0, 1, 9, 40, 65, 128, 129, 300])
+def test_operator_library_and_ctypes_give_the_same(m):
+    """The fused modules' two ways into the library, over strides of x, with and without a bias, and on a private workspace
+    (which only the second one takes)."""
+    from dandan_ops_b200 import fused, ops as b2ops
+    if not b2ops.SHIM_LOADED:
+        pytest.skip("operator library not built")
+    g = torch.Generator().manual_seed(m)
+    k, rows = 1032, 200
+    gate_up = GateUpSilu(_layer(rows, k, 1, bias=True, device="cuda"), _layer(rows, k, 2, device="cuda"))
+    norm = RmsNormLinear(torch.randn(k, generator=g).half().cuda(), _layer(rows, k, 3, bias=True, device="cuda"), eps=1e-6)
+    wide = torch.randn(m, k + 24, generator=g).half().cuda()
+    residual = torch.randn(m, k, generator=g).half().cuda()
+    inputs = [wide[:, :k].contiguous(), wide[:, 8:k + 8], wide[:, 1:k + 1], wide[:, :k + 24:1][:, 3:k + 3].t().contiguous().t()]
+    for x in inputs:
+        aligned = x if x.data_ptr() % 16 == 0 else x.clone()       # (both ways refuse a misaligned row in front of the norm)
+        ways = []
+        for private in (False, True):
+            with _native.private_workspace() if private else contextlib.nullcontext():
+                assert fused._plain(x) != private
+                ways.append((gate_up(x), *norm(aligned, residual), *norm(aligned)))
+        assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(*ways))
+    with pytest.raises(ValueError, match="in_features"):
+        gate_up(wide)
+    assert _native.status() == 0
