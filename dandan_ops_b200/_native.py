@@ -387,7 +387,7 @@ def linear_static(x, image, n, k, out):
 
 FLAG_FP16_STEPS = 1
 FLAG_COLUMN_SLICE = 16       # up to 16 rows the kernels that carry the all-gather (see include/b2_w4a16.h)
-FLAG_OVERLAP_LAUNCH = 2      # the streaming kernel may start under the previous kernel's tail (see include/b2_w4a16.h)
+FLAG_OVERLAP_LAUNCH = 2      # tile, streaming and batch kernel may start under the previous kernel's tail
 OVERLAP_LAUNCH = os.environ.get("B2_W4A16_OVERLAP", "1") != "0"
 
 
@@ -421,7 +421,7 @@ def linear(x, image, n, k, route=ROUTE_AUTO, out=None, bias=None, flags=0):
 
 def linear_silu_mul(x, image, n, k, bias=None, out=None, flags=0):
     """Fused gate/up projection on a pair-ordered image: [M, K] -> [M, N/2] (see include/b2_w4a16.h).
-    The epilogue runs inside the decode kernels and the pair GEMM; the few problems that take a
+    The epilogue runs inside the tile, streaming and batch kernels and the pair GEMM; the few problems that take a
     single-CTA GEMM tile run the projection and then the elementwise pair kernel."""
     lib = load()
     m = x.shape[0]

@@ -1,10 +1,10 @@
 // Conversion kernels between floating-point weights, the checkpoint tensors and the native image.
 //
-// quantize_kernel is bound by HBM: every weight is read once (2 or 4 bytes) and everything a layer keeps of it -
-// packed codes, FP32 step, zero point, native image - is written in the same pass.  The same steps as separate
+// quantize_kernel reads every weight once (2 or 4 bytes) and writes everything a layer keeps of it - packed codes, FP32
+// step, zero point, native image - in the same pass.  The same steps as separate
 // elementwise and reduction passes over an FP32 copy move about forty bytes per weight.  Measured on 4096 x 12288
-// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 50 us here
-// (2.0 TB/s of input and everything written; the instructions of the range and rounding, not memory, are the rest).
+// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 51 us here
+// (2.0 TB/s of input, 3.2 TB/s with everything written): bound by the instructions of range and rounding.
 #pragma once
 #include <cfloat>
 #include <type_traits>

@@ -103,9 +103,10 @@ class GateUpSilu(nn.Module):
 
     The reference runs the fused `gate_up` projection and then a separate `silu_and_mul` kernel
     (dandan_ops/elementwise.py:168-173).  Here the rows of the two layers are interleaved in
-    groups of eight so that a thread of the decode kernels ends up with the gate and the up sum
+    groups of eight so that a thread (or two lanes of a warp) ends up with the gate and the up sum
     of the same output column, and the activation is applied before anything is written: the
-    [M, 2I] intermediate never exists for M <= 64.  Rounding follows the reference: both sums to
+    [M, 2I] intermediate never exists up to 128 rows of a 16-byte aligned x, nor beyond wherever
+    the GEMM's tile shape has the epilogue.  Rounding follows the reference: both sums to
     FP16 (plus FP16 bias), SiLU rounded to FP16, product rounded to FP16."""
 
     def __init__(self, gate, up):

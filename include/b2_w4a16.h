@@ -45,8 +45,8 @@ extern "C" {
                                 in flight at once (M <= 16; K as far as it fits in shared memory) */
 #define B2_ROUTE_BATCH 4     /* persistent weight-streaming kernel with tcgen05 products (M <= 128, K % 8 == 0, aligned x) */
 
-/* Largest M the weight-streaming kernel takes in one launch; B2_ROUTE_AUTO hands larger
- * batches to the tensor-memory GEMM. */
+/* Largest M the weight-streaming kernel takes in one launch (B2_ROUTE_STREAM runs larger batches in
+ * chunks of as many rows). */
 #define B2_STREAM_MAX_M 64
 
 /* Every workspace starts with this many bytes of arrival counters (one per 16-row tile;
@@ -174,21 +174,22 @@ int b2_w4a16_linear_bias(const void* x, int64_t ldx, const void* native, const v
                          int64_t workspace_bytes, void* stream, int route);
 
 /* Same with layer flags.  B2_FLAG_FP16_STEPS: the caller asserts that EVERY step (scale) of the layer is
- * exactly representable in FP16 - true for checkpoints that store FP16 scales.  The decode kernels (M <= 16,
- * 16-byte aligned x) and the converters of the pair GEMM (16-byte aligned y) then dequantize with two FP16 instructions per weight pair instead of the mixed-precision
+ * exactly representable in FP16 - true for checkpoints that store FP16 scales.  The tile and streaming
+ * kernels (M <= 16, 16-byte aligned x), the batch kernel and the converters of the pair GEMM (16-byte aligned y) then dequantize with two FP16 instructions per weight pair instead of the mixed-precision
  * chain: (code - zero) * step has at most 15 significant bits, so fp16_rn(fp32(code - zero) * step) ==
  * hmul2(code - zero, step) and the weights are bit-identical to the general path.  The flag changes speed only;
  * set on a layer with other steps it gives wrong weights.  No counterpart in the reference (its kernels
  * multiply in FP32 throughout, kernels/w4a16_small.cuh:39). */
 #define B2_FLAG_FP16_STEPS 1
-/* B2_FLAG_OVERLAP_LAUNCH: the decode kernels (tile and streaming) may start before the previous kernel of the
+/* B2_FLAG_OVERLAP_LAUNCH: the tile, streaming and batch kernels may start before the previous kernel of the
  * stream has finished (programmatic dependent launch).  As that kernel drains, CTAs of this one move in, set
- * up their barriers and request their weight blocks (the tile kernel all of them, the streaming kernel the
- * first ring); they touch x, bias, y and the workspace only after the previous kernel has completed and its
+ * up their barriers, request their weight blocks (the tile kernel all of them, the others the first ring) and
+ * the batch kernel decodes them; they touch x, bias, y and the workspace only after the previous kernel has completed and its
  * writes are visible (griddepcontrol.wait).  The caller asserts that the weight IMAGE is not being written by
  * work still in flight on the stream (it is constant after the layer was built).  Hides the launch latency and
  * the first trip of the weights behind the previous kernel's tail; results are unchanged.  The tensor-core
- * GEMM ignores the flag. */
+ * GEMM, which takes the batches above 128 rows, ignores the flag; which kernel takes a batch is not part of this
+ * contract, so the assertion about the image has to hold whatever M is. */
 #define B2_FLAG_OVERLAP_LAUNCH 2
 /* B2_FLAG_COLUMN_SLICE: the image is one rank's column slice of a sharded layer.  Up to 16 rows B2_ROUTE_AUTO then keeps to
  * the kernels that carry the all-gather (tile and streaming), which b2_w4a16_linear_gather always does: the slice has the
@@ -204,10 +205,10 @@ int b2_w4a16_linear_flags(const void* x, int64_t ldx, const void* native, const 
  * dandan_ops/csrc/elementwise.cu:70-73).  The image must be built from rows in PAIR ORDER: every
  * 16-row tile holds 8 gate rows followed by the 8 up rows of the same output columns
  * (N % 16 == 0), and `bias_fp16` follows the same order.  The product and the activation never
- * leave the SM: the decode kernels hold a gate/up pair in one thread, the pair GEMM exchanges
- * the two sums between lanes l and l ^ 8 of its epilogue warps.  b2_w4a16_silu_mul_is_fused() tells
- * whether a problem runs this way (everything except batches above 64 rows whose GEMM tile shape is a
- * single-CTA one); the others call b2_w4a16_linear on the same image and then
+ * leave the SM: the tile and streaming kernels hold a gate/up pair in one thread, the batch kernel
+ * and the pair GEMM exchange the two sums between lanes (l and l ^ 4, l and l ^ 8).  b2_w4a16_silu_mul_is_fused()
+ * tells whether a problem runs this way with a 16-byte aligned x (everything except batches that take the GEMM in a
+ * single-CTA tile shape); the others call b2_w4a16_linear on the same image and then
  * b2_w4a16_silu_mul_pairs, and this function returns B2_ERR_UNSUPPORTED for them. */
 int b2_w4a16_linear_silu_mul(const void* x, int64_t ldx, const void* native, const void* bias_fp16, void* y,
                              int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
