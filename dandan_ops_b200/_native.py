@@ -39,6 +39,7 @@ _SIGNATURES = {
     "b2_w4a16_noop": (_int, [_vp]),
     "b2_w4a16_native_bytes": (_i64, [_i64, _i64]),
     "b2_w4a16_repack": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp]),
+    "b2_w4a16_factor_steps": (_int, [_vp, _i64, _i64, _vp]),
     "b2_w4a16_unrepack": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "b2_w4a16_pack": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "b2_w4a16_quantize": (_int, [_vp, _int, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
@@ -209,6 +210,12 @@ def repack(packed, scales, zeros, k):
         _check(lib.b2_w4a16_repack(packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                                    n, k, image.data_ptr(), _stream()))
     return image
+
+
+def factor_steps(image, n, k):
+    """Steps of a native image to the form that decodes fastest, in place (`b2_w4a16_factor_steps`)."""
+    with torch.cuda.device(image.device):
+        _check(load().b2_w4a16_factor_steps(image.data_ptr(), n, k, _stream()))
 
 
 def image_from_host(host_bytes, device):

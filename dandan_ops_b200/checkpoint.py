@@ -65,14 +65,16 @@ def export_int4_layers(layers):
 # native image cache
 # ---------------------------------------------------------------------------------------------
 IMAGE_MAGIC = b"B2W4IMG1"
-IMAGE_LAYOUT = 1            # 16 x 256 blocks of 2336 bytes: codes, FP32 steps, 4-bit zero points
+IMAGE_LAYOUT = 2            # 16 x 256 blocks of 2336 bytes: codes, step fields, 4-bit zero points
+READABLE_LAYOUTS = (1, 2)   # 1: every step field is a plain FP32 step, which the kernels read as well
 _HEADER = struct.Struct("<8sIIqqqI20x")       # magic, layout, format version, N, K, image bytes, CRC-32 of the image; 64 bytes
 
 
 def state_digest(packed_weight, scales, zeros, in_features):
     """Hex SHA-256 over the layer's checkpoint-format state and shape (the cache key)."""
     h = hashlib.sha256()
-    h.update(struct.pack("<IIqq", IMAGE_LAYOUT, FORMAT_VERSION, packed_weight.shape[0], in_features))
+    # (1: files of both layouts have one name)
+    h.update(struct.pack("<IIqq", 1, FORMAT_VERSION, packed_weight.shape[0], in_features))
     for t in (packed_weight, scales, zeros):
         h.update(np.ascontiguousarray(t.detach().cpu().numpy()).tobytes())
     return h.hexdigest()
@@ -96,8 +98,8 @@ def read_image_file(path, n, k, expected_bytes):
             if len(head) != _HEADER.size:
                 return None
             magic, layout, version, fn, fk, nbytes, crc = _HEADER.unpack(head)
-            if (magic, layout, version, fn, fk, nbytes) != (IMAGE_MAGIC, IMAGE_LAYOUT, FORMAT_VERSION, n, k,
-                                                            expected_bytes):
+            if layout not in READABLE_LAYOUTS or (magic, version, fn, fk, nbytes) != (IMAGE_MAGIC, FORMAT_VERSION, n, k,
+                                                                                      expected_bytes):
                 return None
             data = np.fromfile(f, dtype=np.uint8, count=nbytes)
     except OSError:

@@ -404,23 +404,27 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             const uint8_t* raw = raw_base + r * kBatchRawBytes;
             const uint4 code[4] = {*reinterpret_cast<const uint4*>(raw + code_at), *reinterpret_cast<const uint4*>(raw + code_at + 512),
                                    *reinterpret_cast<const uint4*>(raw + code_at + 16), *reinterpret_cast<const uint4*>(raw + code_at + 528)};
-            const float steps[2] = {*reinterpret_cast<const float*>(raw + step_at), *reinterpret_cast<const float*>(raw + step_at + 8)};
+            const uint32_t fields[2] = {*reinterpret_cast<const uint32_t*>(raw + step_at), *reinterpret_cast<const uint32_t*>(raw + step_at + 8)};
             const uint32_t zeros = *reinterpret_cast<const uint16_t*>(raw + zero_at) >> (4 * hi8);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const GroupConst<H16> gc = make_group<H16>((zeros >> (8 * h)) & 15u, steps[h]);
+            auto convert = [&](int h, auto chain) {
+                const auto gc = make_group<decltype(chain)::value>((zeros >> (8 * h)) & 15u, fields[h]);
                 const uint32_t words[8] = {code[2 * h].x, code[2 * h].y, code[2 * h].z, code[2 * h].w,
                                            code[2 * h + 1].x, code[2 * h + 1].y, code[2 * h + 1].z, code[2 * h + 1].w};
                 const uint32_t to = tmem_base + lane_addr + kWBase + slot * kWStage + (2 * v + h) * kBatchWCols;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint4 p = dequant_word<H16>(words[2 * i], gc), q = dequant_word<H16>(words[2 * i + 1], gc);
+                    const uint4 p = dequant_word(words[2 * i], gc), q = dequant_word(words[2 * i + 1], gc);
                     if (h == 0 && i == 0) {
-                        if (!(ok = wait(DONE + slot, free_parity))) break;
+                        if (!(ok = wait(DONE + slot, free_parity))) return;
                         tcgen05_fence_after();
                     }
                     tmem_st8(to + 8 * i, p, q);
                 }
+            };
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
+                else convert(h, Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
                 if (!ok) break;
             }
             if (!ok) break;

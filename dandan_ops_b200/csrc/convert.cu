@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/b2_w4a16.h"
+#include "factor_steps.cuh"
 #include "host_common.cuh"
 #include "layout.cuh"
 #include "layout_kernels.cuh"
@@ -59,7 +60,18 @@ int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* z
     const int64_t blocks = int64_t(d.n16) * d.kb;
     b2::repack_kernel<<<unsigned(blocks), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         packed, scales, zeros, d, static_cast<uint8_t*>(native));
-    return after_launch("repack_kernel");
+    if (int rc = after_launch("repack_kernel")) return rc;
+    return b2_w4a16_factor_steps(native, n, k, stream);
+}
+
+int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream) {
+    if (!native) return fail(B2_ERR_ARGUMENT, "null pointer");
+    if (int rc = check_dims(n, k)) return rc;
+    if (reinterpret_cast<uintptr_t>(native) % 4) return fail(B2_ERR_ARGUMENT, "misaligned native image");
+    const b2::Dims d = b2::make_dims(n, k);
+    const int64_t blocks = int64_t(d.n16) * d.kb;
+    b2::factor_steps_kernel<<<unsigned((blocks + 3) / 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint8_t*>(native), blocks);
+    return after_launch("factor_steps_kernel");
 }
 
 int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed, float* scales,

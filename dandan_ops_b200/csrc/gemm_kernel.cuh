@@ -134,19 +134,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 }
 
 // Eight weights of one native word -> eight FP16 values in column order (16 bytes).
-// s2 = twice(step), c_even = -(1024 + zero), c_odd = -(64 + zero).
-template <bool H16>
-__device__ __forceinline__ uint4 dequant_word(uint32_t w, const GroupConst<H16>& g) {
+template <int CH>
+__device__ __forceinline__ uint4 dequant_word(uint32_t w, const GroupConst<CH>& g) {
     const uint32_t u = w >> 8;
-    return make_uint4(dq_even<H16>(and_or(w, 0x000F000Fu, 0x64006400u), g), dq_odd<H16>(and_or(w, 0x00F000F0u, 0x64006400u), g),
-                      dq_even<H16>(and_or(u, 0x000F000Fu, 0x64006400u), g), dq_odd<H16>(and_or(u, 0x00F000F0u, 0x64006400u), g));
-}
-__device__ __forceinline__ uint4 dequant_word(uint32_t w, float c_even, float c_odd, uint64_t s2) {
-    const uint32_t u = w >> 8;
-    return make_uint4(dequant_pair_even(and_or(w, 0x000F000Fu, 0x64006400u), c_even, s2),
-                      dequant_pair_odd(and_or(w, 0x00F000F0u, 0x64006400u), c_odd, s2),
-                      dequant_pair_even(and_or(u, 0x000F000Fu, 0x64006400u), c_even, s2),
-                      dequant_pair_odd(and_or(u, 0x00F000F0u, 0x64006400u), c_odd, s2));
+    return make_uint4(dq_even(w, g), dq_odd(w, g), dq_even(u, g), dq_odd(u, g));
 }
 
 // MA = accumulators of 128 rows of x each (1 or 2).  VEC: y rows may be written with
@@ -276,16 +267,17 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
             const uint8_t* nb = raw_base + rs * kGemmRawBytes + blk * kBlockBytes;
             const int lane_idx = 4 * g + t;
             const uint4 code = *reinterpret_cast<const uint4*>(nb + (2 * hi8 + h) * 512 + lane_idx * 16);
-            const float step = *reinterpret_cast<const float*>(nb + kStepOffset + (lane_idx * 2 + hi8) * 4);
-            const float z = float((nb[kZeroOffset + lane_idx] >> (4 * hi8)) & 15);
-            const float c_even = -(1024.0f + z), c_odd = -(64.0f + z);
+            const uint32_t field = *reinterpret_cast<const uint32_t*>(nb + kStepOffset + (lane_idx * 2 + hi8) * 4);
+            const uint32_t z = (nb[kZeroOffset + lane_idx] >> (4 * hi8)) & 15u;
             uint8_t* brow = stage_base + st * kStageBytes + r * 128;
             const uint32_t words[4] = {code.x, code.y, code.z, code.w};
+            auto convert = [&](auto chain) {
+                const auto gc = make_group<decltype(chain)::value>(z, field);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int chunk = 4 * h + i;
-                *reinterpret_cast<uint4*>(brow + ((chunk ^ (r & 7)) << 4)) = dequant_word(words[i], c_even, c_odd, twice(step));
-            }
+                for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(brow + (((4 * h + i) ^ (r & 7)) << 4)) = dequant_word(words[i], gc);
+            };
+            if (all_factored(field)) convert(Chain<kChainFactored>{});
+            else convert(Chain<kChainGeneral>{});
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // generic-proxy stores -> MMA (async proxy)
             __syncwarp();
             if (lane == 0) {

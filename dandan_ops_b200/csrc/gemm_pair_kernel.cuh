@@ -277,15 +277,20 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
             const int lane_idx = 4 * g + t;
             const uint4 code0 = *reinterpret_cast<const uint4*>(nb + (2 * hi8) * 512 + lane_idx * 16);
             const uint4 code1 = *reinterpret_cast<const uint4*>(nb + (2 * hi8 + 1) * 512 + lane_idx * 16);
-            const float step = *reinterpret_cast<const float*>(nb + kStepOffset + (lane_idx * 2 + hi8) * 4);
-            const GroupConst<H16> gc = make_group<H16>((nb[kZeroOffset + lane_idx] >> (4 * hi8)) & 15u, step);
+            const uint32_t field = *reinterpret_cast<const uint32_t*>(nb + kStepOffset + (lane_idx * 2 + hi8) * 4);
+            const uint32_t z = (nb[kZeroOffset + lane_idx] >> (4 * hi8)) & 15u;
             const uint32_t words[8] = {code0.x, code0.y, code0.z, code0.w, code1.x, code1.y, code1.z, code1.w};
             uint32_t o[32];
+            auto convert = [&](auto chain) {
+                const auto gc = make_group<decltype(chain)::value>(z, field);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint4 q = dequant_word<H16>(words[i], gc);
-                o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
-            }
+                for (int i = 0; i < 8; ++i) {
+                    const uint4 q = dequant_word(words[i], gc);
+                    o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
+                }
+            };
+            if (all_factored(field)) convert(Chain<kChainFactored>{});
+            else convert(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
             // the conversion happens in registers before the wait for the free tensor-memory stage
             if (s >= WS) ok = wait(DONE + (s - WS) % XS, ((s - WS) / XS) & 1);
             if (!ok) break;

@@ -16,14 +16,28 @@
 //                 Inside a word, column c of the eight sits in nibble (c>>1) + 4*(c&1):
 //                 nibbles p and p+4 hold an (even, odd) column pair, which makes
 //                 `(word >> 8e) & 0x000F000F` a pair of FP16 mantissas.
-//   [2048, 2304)  64 FP32 steps: index lane*2 + h = step of (row g + 8h, group t).
+//   [2048, 2304)  64 step fields: index lane*2 + h = step of (row g + 8h, group t), see below.
 //   [2304, 2336)  32 bytes of zero points: byte lane = zero(row g, group t) | zero(row g+8, group t) << 4.
 //
 // This is exactly what one lane of an m16n8k16 tensor-core fragment needs: lane (g, t)
 // owns rows g and g+8 of the tile and, for the sixteen MMAs of a block, the columns
 // 64t + 4i .. 64t + 4i + 3 (i = 0..15), i.e. one whole quantization group per row.
 //
-// Padding: rows >= N and groups >= ceil(K/64) get code 0, zero point 0, step 1; columns
+// A step field holds the FP32 step s of a group exactly, in one of two forms.
+//   plain (bit 31 clear): the bits of s.  (A negative step, which no valid state has, is stored as -s with the codes and
+//       the zero point of its group subtracted from 15: the same weights.)
+//   factored (bit 31 set): s as the product of two FP16 numbers and a remainder,
+//       bits 3-9 a1 = 1 + i / 128, bits 16-29 the low bits of a2 in FP16 (2 <= a2, so bit 14 is set), and the distance of
+//       s from a1 * a2 * 2^-14 in units in the last place of FP32, plus 512, in bits 0-2, 10-15 and 30.
+//       A group is stored like this only if for each of the sixteen codes
+//           fp16_rn(fp16_rn(code * a1 - zero * a1) * 2^-14 * a2) == fp16_rn(fp32_rn((code - zero) * s)),
+//       so the kernels may decode it with one FP16 fma and one FP16 multiplication for two weights.  (code - zero) * a1 has
+//       at most eleven significant bits, so only the second operation rounds, and of 128 candidates for a1 nearly always one
+//       leaves a1 * a2 so close to s that no code rounds differently: all but 0 to 5 groups in 10^4 of weights with zero
+//       points in the middle of the range, all but 0.7 % of groups of one sign.  A step that FP16 can hold and that lies
+//       in the range of factored steps (2^-12 to 3.99) always has a1 = 1 and no remainder.
+//
+// Padding: rows >= N and groups >= ceil(K/64) get code 0, zero point 0 and the factored field of step 0.25; columns
 // >= K inside a real group get code == zero point.  Either way the padded weight is
 // exactly 0.0.
 #pragma once
@@ -83,6 +97,21 @@ __host__ __device__ inline uint32_t unpermute_word(uint32_t nat, int valid) {
     for (int c = 0; c < 8; ++c)
         if (c < valid) out |= ((nat >> (4 * nibble_slot(c))) & 15u) << (4 * c);
     return out;
+}
+
+constexpr uint32_t kFactored = 0x80000000u;
+__host__ __device__ constexpr uint32_t factored_field(uint32_t i, uint32_t a2_bits, int remainder) {
+    const uint32_t r = uint32_t(remainder + 512);
+    return kFactored | (r >> 9) << 30 | (a2_bits & 0x3FFFu) << 16 | ((r >> 3) & 63u) << 10 | i << 3 | (r & 7u);
+}
+constexpr uint32_t kPaddingField = factored_field(0, 0x6C00u, 0);        // 2^12 * 2^-14
+// The FP32 step of a field.
+__device__ __forceinline__ float field_step(uint32_t f) {
+    if (int32_t(f) >= 0) return __uint_as_float(f);
+    const float a1 = __uint_as_float(0x3F800000u | (f & 0x3F8u) << 13);
+    const float a2 = __half2float(__ushort_as_half(uint16_t(((f >> 16) & 0x3FFFu) | 0x4000u)));
+    const int remainder = int((f >> 30 & 1u) << 9 | ((f >> 10) & 63u) << 3 | (f & 7u)) - 512;
+    return __int_as_float(__float_as_int(a1 * a2 * 0x1p-14f) + remainder);
 }
 
 // Location of (row, column-word) inside the image.

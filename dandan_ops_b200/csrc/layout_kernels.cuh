@@ -26,26 +26,24 @@ repack_kernel(const int32_t* __restrict__ packed, const float* __restrict__ scal
             const int valid = d.k - k0;   // columns of this word that exist (may be <= 0 or >= 8)
             const uint32_t ref = valid > 0 ? uint32_t(packed[int64_t(row) * d.words + (k0 >> 3)]) : 0u;
             out = permute_word(ref, valid < 0 ? 0 : (valid > 8 ? 8 : valid), z);
+            if (signbit(scales[int64_t(row) * d.groups + grp])) out = ~out;
         }
         code[idx] = out;
     }
-    if (threadIdx.x < 64) {
-        const int lane = threadIdx.x >> 1, h = threadIdx.x & 1;
+    for (int f = threadIdx.x; f < 64; f += 128) {
+        const int lane = f >> 1, h = f & 1;
         const int row = nt * 16 + (lane >> 2) + 8 * h, grp = kb * 4 + (lane & 3);
+        const bool real = row < d.n && grp < d.groups;
         float s = 1.0f;
-        if (row < d.n && grp < d.groups) s = scales[int64_t(row) * d.groups + grp];
-        reinterpret_cast<float*>(base + kStepOffset)[threadIdx.x] = s;
-    } else if (threadIdx.x < 96) {
-        const int lane = threadIdx.x - 64;
-        const int grp = kb * 4 + (lane & 3);
         uint32_t z = 0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = nt * 16 + (lane >> 2) + 8 * h;
-            if (row < d.n && grp < d.groups)
-                z |= (uint32_t(zeros[int64_t(row) * d.groups + grp]) & 15u) << (4 * h);
+        if (real) {
+            s = scales[int64_t(row) * d.groups + grp];
+            z = uint32_t(zeros[int64_t(row) * d.groups + grp]) & 15u;
+            if (signbit(s)) { s = -s; z ^= 15u; }
         }
-        base[kZeroOffset + lane] = uint8_t(z);
+        const uint32_t z8 = __shfl_down_sync(0xffffffffu, z, 1);          // row g + 8 of the same group
+        reinterpret_cast<uint32_t*>(base + kStepOffset)[f] = real ? __float_as_uint(s) : kPaddingField;
+        if (h == 0) base[kZeroOffset + lane] = uint8_t(z | z8 << 4);
     }
 }
 
@@ -67,7 +65,7 @@ unrepack_kernel(const uint8_t* __restrict__ native, Dims d, int32_t* __restrict_
         const int row = int(idx / d.groups), grp = int(idx - int64_t(row) * d.groups);
         const WordRef w = locate(d, row, grp * 8);
         const uint8_t* base = native + w.block;
-        scales[idx] = reinterpret_cast<const float*>(base + kStepOffset)[w.meta];
+        scales[idx] = field_step(reinterpret_cast<const uint32_t*>(base + kStepOffset)[w.meta]);
         zeros[idx] = (base[kZeroOffset + (w.meta >> 1)] >> (4 * (w.meta & 1))) & 15;
     }
 }

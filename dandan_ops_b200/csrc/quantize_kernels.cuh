@@ -95,16 +95,16 @@ template <> struct Eight<__half> {
     }
 };
 
-// Reference word (nibble c = column c) -> native word of a whole word: even columns to the low half, odd ones to the high.
-__device__ __forceinline__ uint32_t split_nibbles(uint32_t ref) {
-    const uint32_t even = ref & 0x0F0F0F0Fu, odd = (ref >> 4) & 0x0F0F0F0Fu;
-    return __byte_perm(even | (even >> 4), odd | (odd >> 4), 0x6420);
-}
-
 __device__ __forceinline__ float reciprocal(float v) {       // to one unit in the last place
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
+}
+
+// Reference word (nibble c = column c) -> native word of a whole word: even columns to the low half, odd ones to the high.
+__device__ __forceinline__ uint32_t split_nibbles(uint32_t ref) {
+    const uint32_t even = ref & 0x0F0F0F0Fu, odd = (ref >> 4) & 0x0F0F0F0Fu;
+    return __byte_perm(even | (even >> 4), odd | (odd >> 4), 0x6420);
 }
 
 // Packed codes of eight weights: code = clamp(round_half_even(fl(fl(w / step) + zero)), 0, 15).
@@ -129,10 +129,17 @@ __device__ __forceinline__ uint32_t quantize_word(const float (&v)[8], float ste
     float off = step < 0x1p100f ? 0.0f : 1.0f;              // largest distance of a sum from the integer it rounds to
     int q[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float t = fmaf(v[c], inverse, zero), u = __fadd_rn(t, kRoundMagic);
-        off = fmaxf(off, fabsf(__fsub_rn(t, __fsub_rn(u, kRoundMagic))));
-        q[c] = code_of(u);
+    for (int c = 0; c < 8; c += 2) {                        // two weights per instruction, each rounded as if alone
+        float u0, u1, d0, d1;
+        asm("{\n\t.reg .b64 t, u, r, v, i, z, m;\n\t"
+            "mov.b64 v, {%4, %5};\n\tmov.b64 i, {%6, %6};\n\tmov.b64 z, {%7, %7};\n\tmov.b64 m, {%8, %8};\n\t"
+            "fma.rn.f32x2 t, v, i, z;\n\tadd.rn.f32x2 u, t, m;\n\tsub.rn.f32x2 r, u, m;\n\tsub.rn.f32x2 r, t, r;\n\t"
+            "mov.b64 {%0, %1}, u;\n\tmov.b64 {%2, %3}, r;\n\t}"
+            : "=f"(u0), "=f"(u1), "=f"(d0), "=f"(d1)
+            : "f"(v[c]), "f"(v[c + 1]), "f"(inverse), "f"(zero), "f"(kRoundMagic));
+        off = fmaxf(off, fmaxf(fabsf(d0), fabsf(d1)));
+        q[c] = code_of(u0);
+        q[c + 1] = code_of(u1);
     }
     if (off > 0.5f - 0x1p-16f) {
 #pragma unroll
@@ -196,7 +203,7 @@ quantize_kernel(const QuantizeArgs a) {
                 a.scales[int64_t(row) * d.groups + grp] = my_step;
                 a.zeros[int64_t(row) * d.groups + grp] = int32_t(my_zero);
             }
-            if (block) reinterpret_cast<float*>(block + kStepOffset)[(4 * (r & 7) + t) * 2 + (r >> 3)] = real ? my_step : 1.0f;
+            if (block) reinterpret_cast<uint32_t*>(block + kStepOffset)[(4 * (r & 7) + t) * 2 + (r >> 3)] = real ? __float_as_uint(my_step) : kPaddingField;
         }
         // zero points of rows r and r + 8 share a byte
         const unsigned z = real ? unsigned(int(my_zero)) : 0u, z8 = __shfl_xor_sync(kAll, z, 2);
@@ -284,7 +291,7 @@ dequantize_kernel(const uint8_t* __restrict__ native, const int32_t* __restrict_
                 const WordRef w = locate(d, row, col >> 3);
                 const uint8_t* base = native + w.block;
                 word[i] = __ldg(reinterpret_cast<const uint32_t*>(base) + w.word);
-                step[i] = __ldg(reinterpret_cast<const float*>(base + kStepOffset) + w.meta);
+                step[i] = field_step(__ldg(reinterpret_cast<const uint32_t*>(base + kStepOffset) + w.meta));
                 zero[i] = (__ldg(base + kZeroOffset + (w.meta >> 1)) >> (4 * (w.meta & 1))) & 15;
             } else {
                 const int64_t at = int64_t(row) * d.groups + (col >> 6);

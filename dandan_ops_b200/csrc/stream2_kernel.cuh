@@ -200,13 +200,13 @@ w4a16_stream2_kernel(const StreamArgs a) {
                     continue;
                 }
                 const uint8_t* slot = ring + stage * kBlockBytes;
-                const float2 step = *reinterpret_cast<const float2*>(slot + kStepOffset + lane * 8);
+                const uint2 field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
                 const uint32_t zero = slot[kZeroOffset + lane];
                 // -(1024 + z) and -(64 + z) as FP32 bit patterns: z sits in the mantissa
                 const uint32_t zlo = zero & 15u, zhi = zero >> 4;
                 const float cg = __uint_as_float(0xC4800000u + zlo * 8192u), ch = __uint_as_float(0xC4800000u + zhi * 8192u);
                 const float eg = __uint_as_float(0xC2800000u + zlo * 131072u), eh = __uint_as_float(0xC2800000u + zhi * 131072u);
-                const uint64_t sg = twice(step.x), sh = twice(step.y);
+                const uint64_t sg = twice(field_step(field.x)), sh = twice(field_step(field.y));
                 const uint8_t* xrow = xbase + kbl * 4 * kChunk;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {

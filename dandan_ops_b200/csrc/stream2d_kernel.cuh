@@ -141,7 +141,7 @@ w4a16_stream2d_kernel(const StreamArgs a) {
                 uint4 code[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) code[q] = *reinterpret_cast<const uint4*>(slot + q * 512 + lane * 16);
-                const float2 step = *reinterpret_cast<const float2*>(slot + kStepOffset + lane * 8);
+                const uint2 field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
                 const uint32_t zero = slot[kZeroOffset + lane];
                 __syncwarp();                                   // all lanes have read the slot
                 if (fs < b1) {
@@ -150,7 +150,8 @@ w4a16_stream2d_kernel(const StreamArgs a) {
                 }
                 if (++stage == kStages) { stage = 0; parity ^= 1u; }
 
-                const GroupConst<H16> gg = make_group<H16>(zero & 15u, step.x), gh = make_group<H16>(zero >> 4, step.y);
+                constexpr int CH = H16 ? kChainFp16 : kChainGeneral;
+                const GroupConst<CH> gg = make_group<CH>(zero & 15u, field.x), gh = make_group<CH>(zero >> 4, field.y);
                 const uint8_t* xchunk = (MT > 1 || g < xrows) ? xs + (jj * 4 + t) * kChunk + g * 144 : xzero;
 #pragma unroll
                 for (int wi = 0; wi < 8; ++wi) {
@@ -163,10 +164,7 @@ w4a16_stream2d_kernel(const StreamArgs a) {
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const uint32_t ua = wa >> (8 * e), ub = wb >> (8 * e);
-                        const uint32_t w[4] = {dq_even<H16>(and_or(ua, 0x000F000Fu, 0x64006400u), gg),
-                                               dq_even<H16>(and_or(ub, 0x000F000Fu, 0x64006400u), gh),
-                                               dq_odd<H16>(and_or(ua, 0x00F000F0u, 0x64006400u), gg),
-                                               dq_odd<H16>(and_or(ub, 0x00F000F0u, 0x64006400u), gh)};
+                        const uint32_t w[4] = {dq_even(ua, gg), dq_even(ub, gh), dq_odd(ua, gg), dq_odd(ub, gh)};
 #pragma unroll
                         for (int mt = 0; mt < MT; ++mt)
                             mma_16816(acc[mt], w, e ? xv[mt].z : xv[mt].x, e ? xv[mt].w : xv[mt].y, acc[mt]);

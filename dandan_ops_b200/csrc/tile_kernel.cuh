@@ -205,33 +205,35 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         const uint8_t* slot = blocks + b * kBlockBytes;
         const uint4 ca = *reinterpret_cast<const uint4*>(slot + h * 512 + lane * 16);         // row g
         const uint4 cb = *reinterpret_cast<const uint4*>(slot + (2 + h) * 512 + lane * 16);   // row g+8
-        const float2 step = *reinterpret_cast<const float2*>(slot + kStepOffset + lane * 8);
+        const uint2 field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
         const uint32_t zero = slot[kZeroOffset + lane];
-        const GroupConst<H16> gg = make_group<H16>(zero & 15u, step.x), gh = make_group<H16>(zero >> 4, step.y);
         const uint8_t* xchunk = xs + (b * 4 + t) * kChunk + g * 128;
+        auto multiply = [&](auto form) {
+            constexpr int CH = decltype(form)::value;
+            const GroupConst<CH> gg = make_group<CH>(zero & 15u, field.x), gh = make_group<CH>(zero >> 4, field.y);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t wa = pick(ca, i), wb = pick(cb, i);
-            uint4 xv[MT];
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t wa = pick(ca, i), wb = pick(cb, i);
+                uint4 xv[MT];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)      // rows of x that do not exist are not staged: their columns of the product are zero
-                xv[mt] = (FULL || mt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xchunk + mt * (8 * 128) + (((h * 4 + i) ^ g) << 4))
-                                                     : make_uint4(0, 0, 0, 0);
+                for (int mt = 0; mt < MT; ++mt)      // rows of x that do not exist are not staged: their columns of the product are zero
+                    xv[mt] = (FULL || mt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xchunk + mt * (8 * 128) + (((h * 4 + i) ^ g) << 4))
+                                                         : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const uint32_t ua = wa >> (8 * e), ub = wb >> (8 * e);
-                const uint32_t w[4] = {dq_even<H16>(and_or(ua, 0x000F000Fu, 0x64006400u), gg),
-                                       dq_even<H16>(and_or(ub, 0x000F000Fu, 0x64006400u), gh),
-                                       dq_odd<H16>(and_or(ua, 0x00F000F0u, 0x64006400u), gg),
-                                       dq_odd<H16>(and_or(ub, 0x00F000F0u, 0x64006400u), gh)};
-                const int chain = (kChains == 4 ? 2 * (i & 1) + e : e);       // compile-time under the unrolling
+                for (int e = 0; e < 2; ++e) {
+                    const uint32_t ua = wa >> (8 * e), ub = wb >> (8 * e);
+                    const uint32_t w[4] = {dq_even(ua, gg), dq_even(ub, gh), dq_odd(ua, gg), dq_odd(ub, gh)};
+                    const int chain = (kChains == 4 ? 2 * (i & 1) + e : e);       // compile-time under the unrolling
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    float (&dst)[4] = chain == 0 ? acc[mt] : accx[chain == 0 ? 0 : chain - 1][mt];
-                    mma_16816(dst, w, e ? xv[mt].z : xv[mt].x, e ? xv[mt].w : xv[mt].y, dst);
+                    for (int mt = 0; mt < MT; ++mt) {
+                        float (&dst)[4] = chain == 0 ? acc[mt] : accx[chain == 0 ? 0 : chain - 1][mt];
+                        mma_16816(dst, w, e ? xv[mt].z : xv[mt].x, e ? xv[mt].w : xv[mt].y, dst);
+                    }
                 }
             }
-        }
+        };
+        if (all_factored(field.x & field.y)) multiply(Chain<kChainFactored>{});
+        else multiply(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
