@@ -8,6 +8,9 @@
 //     anything else happens (kb * 2336 bytes in flight per CTA, several CTAs per SM);
 //   * the unit of work is half a block (eight of its sixteen MMA steps); up to 16 warps take
 //     consecutive units, so a block is decoded by two warps in parallel;
+//   * as a programmatic dependent a warp decodes its first unit before it waits for the previous kernel of the stream (up to
+//     8 rows of x; 4096 x 1024 at M = 1 / 8 in a chain of launches 3.3 / 3.4 -> 2.7 / 2.8 us, 6144 x 1024 3.4 / 3.6 -> 3.0 / 3.1;
+//     64 registers, so that two CTAs of 16 warps share an SM);
 //   * x for the CTA's K range is staged once, unpadded: rows of 128 bytes per 64-column chunk
 //     with the 16-byte pieces XOR-swizzled by the row, so the fragment reads are conflict-free
 //     and two CTAs of a 4096-column layer share an SM at M = 8;
@@ -149,7 +152,61 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     }
     // Kernels launched behind this one as programmatic dependents may start as soon as they find room.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // The weights are constant; x, the bias and y may belong to the previous kernel until it has completed.
+    // units = half blocks, dealt in consecutive runs to the warps
+    const int units = kbn * 2;
+    const int u0 = (units * warp) / a.warps, u1 = (units * (warp + 1)) / a.warps;
+    bool failed = false;
+    // Codes, step fields and zero points of the lane's two rows in half h of block b, and the fragments of word i of them.
+    struct Unit {
+        uint4 ca, cb;
+        uint2 field;
+        uint32_t zero;
+    };
+    auto fetch = [&](int u, Unit& o) -> bool {
+        const int b = u >> 1, h = u & 1;
+        if (!mbar_wait(bar0 + b * 8, 0, a.wait_limit)) {
+            if (lane == 0 && a.status) atomicOr(a.status, kStatusCopyTimeout);
+            return false;
+        }
+        const uint8_t* slot = blocks + b * kBlockBytes;
+        o.ca = *reinterpret_cast<const uint4*>(slot + h * 512 + lane * 16);           // row g
+        o.cb = *reinterpret_cast<const uint4*>(slot + (2 + h) * 512 + lane * 16);     // row g+8
+        o.field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
+        o.zero = slot[kZeroOffset + lane];
+        return true;
+    };
+    auto decode = [&](const Unit& o, int i, uint32_t (&w)[2][4], const auto& gg, const auto& gh) {
+        const uint32_t wa = pick(o.ca, i), wb = pick(o.cb, i);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const uint32_t ua = wa >> (8 * e), ub = wb >> (8 * e);
+            w[e][0] = dq_even(ua, gg); w[e][1] = dq_even(ub, gh);
+            w[e][2] = dq_odd(ua, gg); w[e][3] = dq_odd(ub, gh);
+        }
+    };
+    auto with_chain = [&](const Unit& o, auto f) {
+        auto go = [&](auto chain) {
+            constexpr int CH = decltype(chain)::value;
+            f(make_group<CH>(o.zero & 15u, o.field.x), make_group<CH>(o.zero >> 4, o.field.y));
+        };
+        if (all_factored(o.field.x & o.field.y)) go(Chain<kChainFactored>{});
+        else go(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
+    };
+    // The weights are constant; x, the bias and y may belong to the previous kernel until it has completed.  With one row tile
+    // of x (registers) a warp decodes its first unit meanwhile.
+    constexpr bool kAhead = MT == 1;
+    uint32_t first[kAhead ? 4 : 1][2][4];
+    if constexpr (kAhead) {
+        if (a.overlap) {
+            __syncthreads();        // barrier initialisation visible to every waiter
+            Unit o;
+            if (u0 < u1 && !(failed = !fetch(u0, o)))
+                with_chain(o, [&](const auto& gg, const auto& gh) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) decode(o, i, first[i], gg, gh);
+                });
+        }
+    }
     if (a.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
     // stage x for all columns (zero beyond M and K)
     {
@@ -179,9 +236,6 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     }
     __syncthreads();        // x staged; barrier initialisation visible to every waiter
 
-    // units = half blocks, dealt in consecutive runs to the warps
-    const int units = kbn * 2;
-    const int u0 = (units * warp) / a.warps, u1 = (units * (warp + 1)) / a.warps;
     // The eight MMAs of a unit would be one dependent chain per row tile of x; kChains accumulator tiles used in
     // turn cut it into chains of 8 / kChains (four at one row tile, two at two), added in a fixed order at the end.
     constexpr int kChains = MT == 1 ? 4 : 2;
@@ -194,46 +248,43 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
 #pragma unroll
             for (int q = 0; q < kChains - 1; ++q) accx[q][mt][c] = 0.0f;
         }
-    bool failed = false;
-    for (int u = u0; u < u1 && !failed; ++u) {
+    auto multiply = [&](int u, int i, const uint32_t (&w)[2][4]) {
         const int b = u >> 1, h = u & 1;
-        if (!mbar_wait(bar0 + b * 8, 0, a.wait_limit)) {
-            failed = true;
-            if (lane == 0 && a.status) atomicOr(a.status, kStatusCopyTimeout);
-            break;
-        }
-        const uint8_t* slot = blocks + b * kBlockBytes;
-        const uint4 ca = *reinterpret_cast<const uint4*>(slot + h * 512 + lane * 16);         // row g
-        const uint4 cb = *reinterpret_cast<const uint4*>(slot + (2 + h) * 512 + lane * 16);   // row g+8
-        const uint2 field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
-        const uint32_t zero = slot[kZeroOffset + lane];
         const uint8_t* xchunk = xs + (b * 4 + t) * kChunk + g * 128;
-        auto multiply = [&](auto form) {
-            constexpr int CH = decltype(form)::value;
-            const GroupConst<CH> gg = make_group<CH>(zero & 15u, field.x), gh = make_group<CH>(zero >> 4, field.y);
+        uint4 xv[MT];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)      // rows of x that do not exist are not staged: their columns of the product are zero
+            xv[mt] = (FULL || mt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xchunk + mt * (8 * 128) + (((h * 4 + i) ^ g) << 4))
+                                                 : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int chain = (kChains == 4 ? 2 * (i & 1) + e : e);       // compile-time under the unrolling
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                float (&dst)[4] = chain == 0 ? acc[mt] : accx[chain == 0 ? 0 : chain - 1][mt];
+                mma_16816(dst, w[e], e ? xv[mt].z : xv[mt].x, e ? xv[mt].w : xv[mt].y, dst);
+            }
+        }
+    };
+    int u = u0;
+    if constexpr (kAhead) {
+        if (a.overlap && u0 < u1 && !failed) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) multiply(u0, i, first[i]);
+            ++u;
+        }
+    }
+    for (; u < u1 && !failed; ++u) {
+        Unit o;
+        if ((failed = !fetch(u, o))) break;
+        with_chain(o, [&](const auto& gg, const auto& gh) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint32_t wa = pick(ca, i), wb = pick(cb, i);
-                uint4 xv[MT];
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)      // rows of x that do not exist are not staged: their columns of the product are zero
-                    xv[mt] = (FULL || mt * 8 + g < rows) ? *reinterpret_cast<const uint4*>(xchunk + mt * (8 * 128) + (((h * 4 + i) ^ g) << 4))
-                                                         : make_uint4(0, 0, 0, 0);
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const uint32_t ua = wa >> (8 * e), ub = wb >> (8 * e);
-                    const uint32_t w[4] = {dq_even(ua, gg), dq_even(ub, gh), dq_odd(ua, gg), dq_odd(ub, gh)};
-                    const int chain = (kChains == 4 ? 2 * (i & 1) + e : e);       // compile-time under the unrolling
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        float (&dst)[4] = chain == 0 ? acc[mt] : accx[chain == 0 ? 0 : chain - 1][mt];
-                        mma_16816(dst, w, e ? xv[mt].z : xv[mt].x, e ? xv[mt].w : xv[mt].y, dst);
-                    }
-                }
+                uint32_t w[2][4];
+                decode(o, i, w, gg, gh);
+                multiply(u, i, w);
             }
-        };
-        if (all_factored(field.x & field.y)) multiply(Chain<kChainFactored>{});
-        else multiply(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
+        });
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -329,13 +380,13 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
 }
 
 template <int MT, bool XVEC, bool FULL, bool H16 = false>
-__global__ void __launch_bounds__(kTileMaxWarps * 32)
+__global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_kernel(const TileArgs a) {
     tile_body<MT, XVEC, FULL, H16, false>(a, nullptr);
 }
 
 template <int MT, bool FULL, bool H16>
-__global__ void __launch_bounds__(kTileMaxWarps * 32)
+__global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_gather_kernel(const TileArgs a, const GatherArgs ga) {
     tile_body<MT, true, FULL, H16, true>(a, &ga);
 }
