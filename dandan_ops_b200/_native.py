@@ -59,6 +59,8 @@ _SIGNATURES = {
     "b2_w4a16_silu_mul_pairs": (_int, [_vp, _i64, _vp, _i64, _i64, _i64, _vp]),
     "b2_w4a16_rmsnorm_linear": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.c_float, _vp, _i64, _vp, _vp, _vp, _vp, _i64,
                                        _i64, _i64, _i64, _vp, _i64, _vp]),
+    "b2_w4a16_rmsnorm_linear_flags": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.c_float, _vp, _i64, _vp, _vp, _vp, _vp, _i64,
+                                             _i64, _i64, _i64, _vp, _i64, _vp, _int]),
     "b2_w4a16_residual_rms_norm": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.c_float, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
     "b2_w4a16_plan_flags": (_int, [_i64, _i64, _i64, _int, ctypes.POINTER(_int), ctypes.POINTER(_int),
                                    ctypes.POINTER(_int), ctypes.POINTER(_int)]),
@@ -474,7 +476,7 @@ def residual_rms_norm(x, residual, weight, eps, want_sum=True):
     return out, summed
 
 
-def rmsnorm_linear(x, residual, weight, eps, image, n, k, bias=None, want_sum=True):
+def rmsnorm_linear(x, residual, weight, eps, image, n, k, bias=None, want_sum=True, flags=0):
     """y = (RMSNorm(x + residual) * weight) @ W^T (+ bias) and the FP16 sum: the norm kernel, then
     the projection (see include/b2_w4a16.h)."""
     lib = load()
@@ -487,8 +489,8 @@ def rmsnorm_linear(x, residual, weight, eps, image, n, k, bias=None, want_sum=Tr
     with torch.cuda.device(device):
         scratch = torch.empty((m, k), dtype=torch.float16, device=device)
         ws = workspace(device, int(lib.b2_w4a16_workspace_bytes(m, n, k)))
-        _check(lib.b2_w4a16_rmsnorm_linear(x.data_ptr(), x.stride(0), _ptr(residual),
-                                           residual.stride(0) if residual is not None else 0, weight.data_ptr(),
-                                           float(eps), _ptr(summed), k, _ptr(scratch), image.data_ptr(), _ptr(bias),
-                                           y.data_ptr(), y.stride(0), m, n, k, ws.data_ptr(), ws.numel(), _stream()))
+        _check(lib.b2_w4a16_rmsnorm_linear_flags(x.data_ptr(), x.stride(0), _ptr(residual),
+                                                 residual.stride(0) if residual is not None else 0, weight.data_ptr(),
+                                                 float(eps), _ptr(summed), k, _ptr(scratch), image.data_ptr(), _ptr(bias),
+                                                 y.data_ptr(), y.stride(0), m, n, k, ws.data_ptr(), ws.numel(), _stream(), flags))
     return y, summed

@@ -991,6 +991,8 @@ residual_rms_norm_kernel(const __half* x, int64_t ldx, const __half* residual, i
     __shared__ b2::NormScratch scratch;
     // a projection launched behind this kernel as a programmatic dependent may fetch its weights meanwhile
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // as a dependent itself (B2_FLAG_OVERLAP_LAUNCH): everything it reads or writes may belong to the previous kernel
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int row = blockIdx.x;
     __half* o = out + row * ldo;
     b2::norm_row(x + row * ldx, residual ? residual + row * ldr : nullptr, weight, eps, summed ? summed + row * lds : o, o, k, scratch);
@@ -1137,6 +1139,15 @@ int b2_w4a16_rmsnorm_linear(const void* x, int64_t ldx, const void* residual, in
                             float eps, void* summed, int64_t lds, void* xn_scratch, const void* native,
                             const void* bias_fp16, void* y, int64_t ldy, int64_t m, int64_t n, int64_t k,
                             void* workspace, int64_t workspace_bytes, void* stream) {
+    return b2_w4a16_rmsnorm_linear_flags(x, ldx, residual, ldr, norm_weight, eps, summed, lds, xn_scratch, native, bias_fp16, y, ldy, m, n, k,
+                                         workspace, workspace_bytes, stream, 0);
+}
+
+int b2_w4a16_rmsnorm_linear_flags(const void* x, int64_t ldx, const void* residual, int64_t ldr, const void* norm_weight,
+                                  float eps, void* summed, int64_t lds, void* xn_scratch, const void* native,
+                                  const void* bias_fp16, void* y, int64_t ldy, int64_t m, int64_t n, int64_t k,
+                                  void* workspace, int64_t workspace_bytes, void* stream, int flags) {
+    if (flags & ~kLayerFlags) return fail(B2_ERR_ARGUMENT, "unknown flag");
     if (m < 0) return fail(B2_ERR_ARGUMENT, "m must be non-negative");
     if (int rc = check_dims(n, k)) return rc;
     if (m == 0) return B2_OK;
@@ -1156,16 +1167,17 @@ int b2_w4a16_rmsnorm_linear(const void* x, int64_t ldx, const void* residual, in
     const b2::Dims d = b2::make_dims(n, k);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (!xn_scratch) return fail(B2_ERR_ARGUMENT, "xn_scratch [M, K] is required");
-    residual_rms_norm_kernel<<<unsigned(m), b2::kNormThreads, 0, s>>>(
-        static_cast<const __half*>(x), ldx, static_cast<const __half*>(residual), ldr,
-        static_cast<const __half*>(norm_weight), eps, static_cast<__half*>(summed), lds,
-        static_cast<__half*>(xn_scratch), k, int(m), int(k));
-    if (int rc = after_launch("residual_rms_norm_kernel")) return rc;
+    if (int rc = launch_maybe_dependent("residual_rms_norm_kernel", residual_rms_norm_kernel, int(m), b2::kNormThreads, 0, s,
+                                        (flags & B2_FLAG_OVERLAP_LAUNCH) != 0, static_cast<const __half*>(x), ldx,
+                                        static_cast<const __half*>(residual), ldr, static_cast<const __half*>(norm_weight), eps,
+                                        static_cast<__half*>(summed), lds, static_cast<__half*>(xn_scratch), k, int(m), int(k)))
+        return rc;
     // The projection starts under the norm kernel (its weight copies do not depend on it) and reads xn_scratch
-    // after that kernel has completed.  The norm kernel itself is an ordinary launch, so everything issued
-    // before this call - including whatever wrote the weight image - has finished before either kernel runs.
+    // after that kernel has completed.  Without B2_FLAG_OVERLAP_LAUNCH the norm kernel itself is an ordinary launch, so
+    // everything issued before this call - including whatever wrote the weight image - has finished before either kernel
+    // runs; with it the norm kernel waits for its predecessor as the projection does for the norm.
     return linear_impl(xn_scratch, k, native, bias_fp16, y, ldy, m, n, k, workspace, workspace_bytes, stream, B2_ROUTE_AUTO, 0,
-                       B2_FLAG_OVERLAP_LAUNCH);
+                       flags | B2_FLAG_OVERLAP_LAUNCH);
 }
 
 int b2_w4a16_residual_rms_norm(const void* x, int64_t ldx, const void* residual, int64_t ldr, const void* norm_weight,

@@ -11,12 +11,11 @@ constexpr int kNormThreads = 32 * kNormSlices;       // the first 256 threads of
 
 struct NormScratch {                                   // shared memory of one row's reduction
     float slice[kNormSlices];
-    float inverse;
 };
 
 // One row: summed = fp16(x + residual) (to `sums`: the caller's `summed` row, or the output row when the sum is
 // not wanted), out = fp16(fp16(s * inverse_rms(s)) * weight).  Every thread of the CTA must call it (it
-// contains block-wide barriers); threads beyond kNormThreads only take part in the barriers.  The sum of
+// contains a block-wide barrier); threads beyond kNormThreads only take part in that.  The sum of
 // squares is added in eight lane-strided slices (one per warp), butterfly inside a slice, slices in order: a
 // fixed order, so the result does not depend on the launch.
 __device__ __forceinline__ void norm_row(const __half* x, const __half* residual, const __half* weight, float eps,
@@ -24,22 +23,28 @@ __device__ __forceinline__ void norm_row(const __half* x, const __half* residual
     const int pieces = k >> 3;
     constexpr int kStride = kNormThreads, kBatch = 4;  // loads in flight per thread; the sum keeps the order of the pieces
     const bool worker = threadIdx.x < kNormThreads;
+    // Up to 8192 columns a thread keeps its pieces of the sum (and has requested their weights) until the mean is known; longer
+    // rows are read back.  x and residual through L2: as a programmatic dependent the kernel is older than what the previous
+    // one has written.
+    const bool held = pieces <= kStride * kBatch;
+    uint4 v[kBatch], w[kBatch];
     float sq = 0.0f;
     if (worker) {
         for (int c0 = threadIdx.x; c0 < pieces; c0 += kStride * kBatch) {
-            uint4 v[kBatch], r[kBatch];
+            uint4 r[kBatch];
 #pragma unroll
             for (int j = 0; j < kBatch; ++j) {
                 const int cc = c0 + kStride * j;
-                v[j] = cc < pieces ? __ldg(reinterpret_cast<const uint4*>(x + cc * 8)) : make_uint4(0, 0, 0, 0);
-                r[j] = (cc < pieces && residual) ? __ldg(reinterpret_cast<const uint4*>(residual + cc * 8)) : make_uint4(0, 0, 0, 0);
+                v[j] = cc < pieces ? __ldcg(reinterpret_cast<const uint4*>(x + cc * 8)) : make_uint4(0, 0, 0, 0);
+                r[j] = (cc < pieces && residual) ? __ldcg(reinterpret_cast<const uint4*>(residual + cc * 8)) : make_uint4(0, 0, 0, 0);
+                if (held && cc < pieces) w[j] = __ldcg(reinterpret_cast<const uint4*>(weight + cc * 8));
             }
 #pragma unroll
             for (int j = 0; j < kBatch; ++j) {
                 const int cc = c0 + kStride * j;
                 if (cc < pieces) {
                     if (residual) v[j] = add_piece(v[j], r[j]);
-                    *reinterpret_cast<uint4*>(sums + cc * 8) = v[j];
+                    if (!held || sums != out) *reinterpret_cast<uint4*>(sums + cc * 8) = v[j];
                     sq = sumsq_piece(v[j], sq);
                 }
             }
@@ -48,23 +53,20 @@ __device__ __forceinline__ void norm_row(const __half* x, const __half* residual
         if ((threadIdx.x & 31) == 0) sm.slice[threadIdx.x >> 5] = sq;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float total = 0.0f;
+    float total = 0.0f;                                // (every thread for itself: no second barrier)
 #pragma unroll
-        for (int p = 0; p < kNormSlices; ++p) total += sm.slice[p];
-        sm.inverse = inverse_rms(total, k, eps);
-    }
-    __syncthreads();
+    for (int p = 0; p < kNormSlices; ++p) total += sm.slice[p];
+    const float inverse = inverse_rms(total, k, eps);
     if (worker) {
-        const float inverse = sm.inverse;
         for (int c0 = threadIdx.x; c0 < pieces; c0 += kStride * kBatch) {      // every thread re-reads only what it wrote itself
-            uint4 v[kBatch], w[kBatch];
+            if (!held) {
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
-                const int cc = c0 + kStride * j;
-                if (cc < pieces) {
-                    v[j] = *reinterpret_cast<const uint4*>(sums + cc * 8);
-                    w[j] = __ldg(reinterpret_cast<const uint4*>(weight + cc * 8));
+                for (int j = 0; j < kBatch; ++j) {
+                    const int cc = c0 + kStride * j;
+                    if (cc < pieces) {
+                        v[j] = *reinterpret_cast<const uint4*>(sums + cc * 8);
+                        w[j] = __ldcg(reinterpret_cast<const uint4*>(weight + cc * 8));
+                    }
                 }
             }
 #pragma unroll

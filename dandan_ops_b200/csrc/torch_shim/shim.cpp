@@ -186,7 +186,7 @@ at::Tensor silu_mul_image(const at::Tensor& x, const at::Tensor& image, int64_t 
 // Residual add + RMSNorm + projection: (y, x + residual) (as _native.rmsnorm_linear).
 std::tuple<at::Tensor, at::Tensor> rmsnorm_image(const at::Tensor& x, const c10::optional<at::Tensor>& residual, const at::Tensor& weight,
                                                  double eps, const at::Tensor& image, int64_t n, int64_t k,
-                                                 const c10::optional<at::Tensor>& bias) {
+                                                 const c10::optional<at::Tensor>& bias, int64_t flags) {
     check_image(x, image, n, k, bias);
     const bool with_residual = residual.has_value() && residual->defined();
     if (with_residual)
@@ -201,9 +201,9 @@ std::tuple<at::Tensor, at::Tensor> rmsnorm_image(const at::Tensor& x, const c10:
     at::Tensor scratch = at::empty({m, k}, x.options());
     cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
     at::Tensor ws = workspace_for(x.device(), stream, b2_w4a16_workspace_bytes(m, n, k));
-    check_rc(b2_w4a16_rmsnorm_linear(x.data_ptr(), x.stride(0), data_or_null(residual), with_residual ? residual->stride(0) : 0,
-                                     weight.data_ptr(), float(eps), summed.data_ptr(), k, scratch.data_ptr(), image.data_ptr(),
-                                     data_or_null(bias), y.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), stream));
+    check_rc(b2_w4a16_rmsnorm_linear_flags(x.data_ptr(), x.stride(0), data_or_null(residual), with_residual ? residual->stride(0) : 0,
+                                           weight.data_ptr(), float(eps), summed.data_ptr(), k, scratch.data_ptr(), image.data_ptr(),
+                                           data_or_null(bias), y.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), stream, int(flags)));
     return {y, summed};
 }
 
@@ -234,7 +234,7 @@ TORCH_LIBRARY_FRAGMENT(dandan_ops, m) {
     m.def("w4a16_small(Tensor x, Tensor packed_w, Tensor scales, Tensor zeros, int group_size) -> Tensor");
     m.def("w4a16_linear_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int route, int flags) -> Tensor");
     m.def("w4a16_silu_mul_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int flags) -> Tensor");
-    m.def("w4a16_rmsnorm_image(Tensor x, Tensor? residual, Tensor weight, float eps, Tensor image, int n, int k, Tensor? bias) -> (Tensor, Tensor)");
+    m.def("w4a16_rmsnorm_image(Tensor x, Tensor? residual, Tensor weight, float eps, Tensor image, int n, int k, Tensor? bias, int flags=0) -> (Tensor, Tensor)");
     m.def("w4a16_workspace_status() -> int", &status_all);
 }
 

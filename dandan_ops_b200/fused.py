@@ -192,9 +192,10 @@ class RmsNormLinear(nn.Module):
         residual = None if residual is None else residual.contiguous()
         if _plain(x) and (residual is None or _plain(residual)):
             return torch.ops.dandan_ops.w4a16_rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
-                                                            self.out_features, self.in_features, self.op._bias_fp16())
+                                                            self.out_features, self.in_features, self.op._bias_fp16(),
+                                                            self.op._image_flags)
         return _native.rmsnorm_linear(x, residual, self.norm_weight, self.eps, self.op._native_image(),
-                                      self.out_features, self.in_features, bias=self.op._bias_fp16())
+                                      self.out_features, self.in_features, bias=self.op._bias_fp16(), flags=self.op._image_flags)
 
 
 def fuse_named_projections(parent, names, fused_name=None):

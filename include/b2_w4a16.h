@@ -237,6 +237,12 @@ int b2_w4a16_rmsnorm_linear(const void* x, int64_t ldx, const void* residual, in
                             float eps, void* summed, int64_t lds, void* xn_scratch, const void* native,
                             const void* bias_fp16, void* y, int64_t ldy, int64_t m, int64_t n, int64_t k,
                             void* workspace, int64_t workspace_bytes, void* stream);
+/* Same with the layer flags of b2_w4a16_linear_flags; B2_FLAG_OVERLAP_LAUNCH lets the norm kernel, too, start before the
+ * previous kernel of the stream has completed (it waits for that before it reads or writes anything). */
+int b2_w4a16_rmsnorm_linear_flags(const void* x, int64_t ldx, const void* residual, int64_t ldr, const void* norm_weight,
+                                  float eps, void* summed, int64_t lds, void* xn_scratch, const void* native,
+                                  const void* bias_fp16, void* y, int64_t ldy, int64_t m, int64_t n, int64_t k,
+                                  void* workspace, int64_t workspace_bytes, void* stream, int flags);
 
 /* The norm alone (the first launch of b2_w4a16_rmsnorm_linear):
  * summed = fp16(x + residual) (optional output), out = RMSNorm(summed) * norm_weight. */
