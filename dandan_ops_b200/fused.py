@@ -135,7 +135,7 @@ class GateUpSilu(nn.Module):
             x = x.contiguous()
         image = self.op._native_image()
         if _plain(x) and (x.shape[0] <= 1 or x.stride(0) >= self.in_features):
-            return torch.ops.dandan_ops.w4a16_silu_mul_image(x, image, self.op.out_features, self.in_features, self.op._bias_fp16(),
+            return _ops.silu_mul_image(x, image, self.op.out_features, self.in_features, self.op._bias_fp16(),
                                                              self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
         return _native.linear_silu_mul(x, image, self.op.out_features, self.in_features, bias=self.op._bias_fp16(),
                                        flags=self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
@@ -191,7 +191,7 @@ class RmsNormLinear(nn.Module):
         x = x.contiguous()
         residual = None if residual is None else residual.contiguous()
         if _plain(x) and (residual is None or _plain(residual)):
-            return torch.ops.dandan_ops.w4a16_rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
+            return _ops.rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
                                                             self.out_features, self.in_features, self.op._bias_fp16(),
                                                             self.op._image_flags)
         return _native.rmsnorm_linear(x, residual, self.norm_weight, self.eps, self.op._native_image(),

@@ -72,6 +72,7 @@ _OPS = {"w4a16_gemv": _rule_gemv, "w4a16_small": _rule_small,
 
 
 SHIM_LOADED = False      # True when the ops come from the C++ operator library (lib/dandan_ops_b200_C.so)
+linear_image = silu_mul_image = rmsnorm_image = None     # its operators' one overload each, looked up once
 
 
 def register():
@@ -81,13 +82,16 @@ def register():
     with `torch.ops.load_library`, as the reference loads its `_C` module (dandan_ops/_extension.py:34); it
     registers the same names with TORCH_LIBRARY.  Where that file has not been built, the names are defined
     from Python over the ctypes binding instead - the same C-ABI kernels either way."""
-    global _registered, _library, SHIM_LOADED
+    global _registered, _library, SHIM_LOADED, linear_image, silu_mul_image, rmsnorm_image
     if _registered:
         return
     from . import build as _build
     if _build.SHIM_PATH.is_file() and _build.LIB_PATH.is_file():
         try:
             torch.ops.load_library(str(_build.SHIM_PATH))
+            linear_image = torch.ops.dandan_ops.w4a16_linear_image.default
+            silu_mul_image = torch.ops.dandan_ops.w4a16_silu_mul_image.default
+            rmsnorm_image = torch.ops.dandan_ops.w4a16_rmsnorm_image.default
             SHIM_LOADED = True
             _registered = True
             return

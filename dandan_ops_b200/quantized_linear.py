@@ -89,7 +89,7 @@ def _engine(x, image, rows, in_features, bias16, flags=0):
     if x.stride(1) != 1 or (x.shape[0] > 1 and x.stride(0) < in_features):
         x = x.contiguous()
     if _ops_module.SHIM_LOADED:       # C++ operator library: output, workspace and launch without a ctypes round trip
-        return torch.ops.dandan_ops.w4a16_linear_image(x, image, rows, in_features, bias16, 0, flags)
+        return _ops_module.linear_image(x, image, rows, in_features, bias16, 0, flags)
     return _native.linear(x, image, rows, in_features, bias=bias16, flags=flags)
 
 
@@ -225,9 +225,17 @@ class QuantizedLinear(torch.nn.Module):
         return self
 
     # -- native image ----------------------------------------------------------------------
+    def _state(self):
+        # (the buffers where Module keeps them: its attribute lookup takes longer than the rest of a key)
+        buffers = self._buffers
+        try:
+            return buffers["packed_weight"], buffers["scales"], buffers["zeros"]
+        except KeyError:                                     # turned into parameters or plain attributes
+            return self.packed_weight, self.scales, self.zeros
+
     def _state_key(self):
-        return (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
-                self.packed_weight._version, self.scales._version, self.zeros._version)
+        packed, scales, zeros = self._state()
+        return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(), packed._version, scales._version, zeros._version)
 
     _slice_flag = 0
 
@@ -275,11 +283,12 @@ class QuantizedLinear(torch.nn.Module):
 
     def _bias_fp16(self):
         """FP16 copy of the bias for the fused epilogue (derived, rebuilt when the bias changes)."""
-        if self.bias is None:
+        bias = self.bias
+        if bias is None:
             return None
-        key = (self.bias.data_ptr(), self.bias._version, self.bias.dtype)
+        key = (bias.data_ptr(), bias._version, bias.dtype)
         if self._bias16 is None or self._bias16_key != key:
-            self._bias16 = self.bias.detach().to(torch.float16).contiguous()
+            self._bias16 = bias.detach().to(torch.float16).contiguous()
             self._bias16_key = key
         return self._bias16
 
@@ -319,10 +328,11 @@ class QuantizedLinear(torch.nn.Module):
         return _native.dequantize(self._native_image(), self.out_features, self.in_features)
 
     def _forward_key(self):
+        packed, scales, zeros = self._state()
         bias = self.bias
-        return (self.packed_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
-                self.packed_weight._version, self.scales._version, self.zeros._version,
-                id(self.packed_weight), id(self.scales), id(self.zeros),
+        return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
+                packed._version, scales._version, zeros._version,
+                id(packed), id(scales), id(zeros),
                 self.in_features, self.group_size, self.backend,
                 None if bias is None else (bias.data_ptr(), bias._version, bias.dtype))
 
