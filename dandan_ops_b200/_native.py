@@ -3,6 +3,7 @@
 The library is the only compute path of the package: if it cannot be loaded, every
 operation that needs it raises ImportError - there is no eager or CPU stand-in.
 """
+import contextlib
 import ctypes
 import os
 import threading
@@ -107,6 +108,14 @@ def _ptr(t):
 
 def _stream():
     return torch.cuda.current_stream().cuda_stream
+
+
+_here = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context in which `device` is the current one (switching contexts takes longer than most launches)."""
+    return _here if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def launch_count():
@@ -216,7 +225,7 @@ def repack(packed, scales, zeros, k):
 
 def factor_steps(image, n, k):
     """Steps of a native image to the form that decodes fastest, in place (`b2_w4a16_factor_steps`)."""
-    with torch.cuda.device(image.device):
+    with _on(image.device):
         _check(load().b2_w4a16_factor_steps(image.data_ptr(), n, k, _stream()))
 
 
@@ -263,7 +272,7 @@ def quantize(weight, want_codes=False, want_layer=True):
     if size <= 0:
         raise RuntimeError("b2_w4a16: W4A16 dimensions exceed the kernel index range")
     words, groups = (k + 7) // 8, (k + 63) // 64
-    with torch.cuda.device(dev):
+    with _on(dev):
         codes = torch.empty((n, k), dtype=torch.uint8, device=dev) if want_codes else None
         packed = torch.empty((n, words), dtype=torch.int32, device=dev) if want_layer else None
         image = torch.empty(size, dtype=torch.uint8, device=dev) if want_layer else None
@@ -275,11 +284,27 @@ def quantize(weight, want_codes=False, want_layer=True):
         return codes, packed, scales, zeros, image, flags
 
 
+class HostWord:
+    """Copy of a one-element CUDA tensor to the host, in order on the current stream; `item()` waits for it, but for nothing
+    that is launched after this."""
+
+    def __init__(self, word):
+        with _on(word.device):
+            self._host = torch.empty(word.shape, dtype=word.dtype, pin_memory=True)
+            self._host.copy_(word, non_blocking=True)
+            self._done = torch.cuda.Event()
+            self._done.record()
+
+    def item(self):
+        self._done.synchronize()
+        return self._host.item()
+
+
 def dequantize_state(packed, scales, zeros, k):
     """Reference-layout CUDA tensors (group size 64) -> FP32 [N, K] weights."""
     lib = load()
     n = packed.shape[0]
-    with torch.cuda.device(packed.device):
+    with _on(packed.device):
         out = torch.empty((n, k), dtype=torch.float32, device=packed.device)
         _check(lib.b2_w4a16_dequantize_state(packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(), n, k,
                                              out.data_ptr(), k, _stream()))

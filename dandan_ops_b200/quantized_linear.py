@@ -155,12 +155,14 @@ class QuantizedLinear(torch.nn.Module):
             # points 0..15 by construction, so nothing is read back to check them.
             with torch.no_grad():
                 _, packed, steps, zero_points, image, flags = _native.quantize(weight.detach().contiguous())
+                flags = _native.HostWord(flags)
+                # (behind the flags, which are what is waited for: the image is complete with plain steps, and calls that use
+                # it may run beside this)
+                _native.factor_steps(image, *weight.shape)
                 layer = cls.__new__(cls)                      # (built while the kernel runs)
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
                 layer._set_image(image, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
-                # (the image is complete, with plain steps; the first calls may run beside this or before it)
-                _native.factor_steps(image, *weight.shape)
             return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)
