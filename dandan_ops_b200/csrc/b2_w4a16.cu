@@ -760,7 +760,10 @@ inline GemmShape gemm_shape(int64_t m, int64_t n, int kb, int sms, bool pairs_ok
             if (forced_splits && sp != std::min(forced_splits, smax)) continue;
             g.splits = sp;
             const int64_t steps = int64_t((kb + sp - 1) / sp) * 4 + 10 + (sp > 1 ? 4 + 2 * sp : 0);
-            const int64_t c = wave_cost(i, g, g.tiles(m, n) * sp) * steps;
+            // The partial tiles of a K-split are written and read back: 94 units are a microsecond, in which 2.4 MB make that
+            // trip (4096 x 12288 at M = 1024 / 2048: three / two CTAs along K 92 / 169 us, all of K on 256 rows 77 / 154; 4096 x
+            // 4096 at M = 512: two CTAs 25, one 29).
+            const int64_t c = wave_cost(i, g, g.tiles(m, n) * sp) * steps + g.partial_bytes(m, n) / 26000;
             if (c < best_cost) { best_cost = c; best = g; }
         }
     }
