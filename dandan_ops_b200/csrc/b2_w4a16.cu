@@ -606,7 +606,11 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 //                11.3 against 11.8.  One line for both kinds of steps: the flag must not change a bit.  Not below 4096
 //                output columns, the usual width of a slice: there a plain layer, too, has the bits of the kernels that
 //                carry the all-gather.
-//   9..16        above 4096 blocks, wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7, 24576 x 4096 26.8 -> 22.5,
+//                Up to 65536 blocks where K is 12288 or more: 4096 x 28672 at M = 1 / 8 22.9 / 22.5 -> 20.6 / 20.8, 6144 x 16384
+//                19.7 / 20.0 -> 17.4 / 17.7, 8192 x 28672 34.9 / 35.9 -> 34.7 / 34.8; 16384 x 8192 22.2 / 24.0 against 23.4 / 23.6.
+//   9..16        up to K = 3072 above 2304 blocks (8192 x 2048 at M = 16 9.5 -> 7.5, 6144 x 2048 8.1 -> 7.3, 12288 x 1024 7.4 -> 5.2,
+//                3072 x 3072 8.7 -> 6.6; 4096 x 2048 tile 5.0 against 6.3), else above 4096 (at 4096 x 4096, whose plan callers
+//                know as one CTA per tile, batch would be ahead, too: 10.3 against 7.4), wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7, 24576 x 4096 26.8 -> 22.5,
 //                57344 x 8192 90 -> 75; 57344 x 512 11.3 against 12.8
 //   17..32       from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
 //                1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 8.4 / 8.7, 57344 x 8192 121 / 125 -> 78
@@ -627,8 +631,8 @@ bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = fa
     if (m > 64) return !wide || tiles * d.kb >= 13 * sms;
     if (m > 32) return true;
     if (m > 16) return d.kb > 1 && (d.n > 512 || d.kb < 8 || d.kb >= 32);
-    if (m > 8) return blocks > 4096 && (!wide || d.kb > 2);
-    return blocks > 4096 && blocks <= 16384 && d.n >= 4096 && !wide;
+    if (m > 8) return blocks > (d.kb <= 12 ? 2304 : 4096) && (!wide || d.kb > 2);
+    return blocks > 4096 && blocks <= (d.kb >= 48 ? 65536 : 16384) && d.n >= 4096 && !wide;
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
