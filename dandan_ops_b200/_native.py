@@ -284,22 +284,6 @@ def quantize(weight, want_codes=False, want_layer=True):
         return codes, packed, scales, zeros, image, flags
 
 
-class HostWord:
-    """Copy of a one-element CUDA tensor to the host, in order on the current stream; `item()` waits for it, but for nothing
-    that is launched after this."""
-
-    def __init__(self, word):
-        with _on(word.device):
-            self._host = torch.empty(word.shape, dtype=word.dtype, pin_memory=True)
-            self._host.copy_(word, non_blocking=True)
-            self._done = torch.cuda.Event()
-            self._done.record()
-
-    def item(self):
-        self._done.synchronize()
-        return self._host.item()
-
-
 def dequantize_state(packed, scales, zeros, k):
     """Reference-layout CUDA tensors (group size 64) -> FP32 [N, K] weights."""
     lib = load()

@@ -70,7 +70,7 @@ int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream) {
     if (reinterpret_cast<uintptr_t>(native) % 4) return fail(B2_ERR_ARGUMENT, "misaligned native image");
     const b2::Dims d = b2::make_dims(n, k);
     const int64_t blocks = int64_t(d.n16) * d.kb;
-    b2::factor_steps_kernel<<<unsigned((blocks + 3) / 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint8_t*>(native), blocks);
+    b2::factor_steps_kernel<<<unsigned((blocks + b2::kFactorBlocks - 1) / b2::kFactorBlocks), b2::kFactorThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint8_t*>(native), blocks);
     return after_launch("factor_steps_kernel");
 }
 
@@ -107,7 +107,9 @@ int b2_w4a16_quantize(const void* weight, int weight_bits, int64_t n, int64_t k,
     a.native = static_cast<uint8_t*>(native);
     a.flags = flags;
     a.d = b2::make_dims(n, k);
-    return weight_bits == 16 ? run_quantize<__half>(a, static_cast<cudaStream_t>(stream)) : run_quantize<float>(a, static_cast<cudaStream_t>(stream));
+    if (int rc = weight_bits == 16 ? run_quantize<__half>(a, static_cast<cudaStream_t>(stream)) : run_quantize<float>(a, static_cast<cudaStream_t>(stream)))
+        return rc;
+    return native ? b2_w4a16_factor_steps(native, n, k, stream) : B2_OK;
 }
 
 int b2_w4a16_dequantize(const void* native, int64_t n, int64_t k, float* out, int64_t ldo, void* stream) {

@@ -3,8 +3,9 @@
 // quantize_kernel reads every weight once (2 or 4 bytes) and writes everything a layer keeps of it - packed codes, FP32
 // step, zero point, native image - in the same pass.  The same steps as separate
 // elementwise and reduction passes over an FP32 copy move about forty bytes per weight.  Measured on 4096 x 12288
-// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 51 us here
-// (2.0 TB/s of input, 3.2 TB/s with everything written): bound by the instructions of range and rounding.
+// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 46 us here
+// (2.2 TB/s of input, 3.5 TB/s with everything written; 51 us before the rounding took two weights per
+// instruction): bound by the instructions of range and rounding.
 #pragma once
 #include <cfloat>
 #include <type_traits>

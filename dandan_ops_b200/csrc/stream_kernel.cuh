@@ -1,8 +1,8 @@
 // Weight-streaming kernel for the decode regime (M <= 64 rows of x per launch).
 //
 // The kernel is bound by HBM and by instruction issue at the same time: every weight
-// byte is read exactly once (0.5703 B/weight) and every weight costs about three
-// instructions to decode exactly, so both the copy pipeline and the inner loop are kept
+// byte is read exactly once (0.5703 B/weight) and every weight costs 1.6 (factored steps) or
+// 2.6 instructions to decode exactly, so both the copy pipeline and the inner loop are kept
 // as lean as the arithmetic contract allows.
 //
 // Work split ("stream-K").  The layer is cut into steps = (group of 16 row tiles = 256

@@ -155,10 +155,6 @@ class QuantizedLinear(torch.nn.Module):
             # points 0..15 by construction, so nothing is read back to check them.
             with torch.no_grad():
                 _, packed, steps, zero_points, image, flags = _native.quantize(weight.detach().contiguous())
-                flags = _native.HostWord(flags)
-                # (behind the flags, which are what is waited for: the image is complete with plain steps, and calls that use
-                # it may run beside this)
-                _native.factor_steps(image, *weight.shape)
                 layer = cls.__new__(cls)                      # (built while the kernel runs)
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)

@@ -61,7 +61,7 @@ int b2_w4a16_contract_version(void);
 const char* b2_w4a16_last_error(void);
 
 /* Bytes of the device-native weight image for an [N, K] layer (0 on bad sizes).
- * The image holds the 4-bit codes, FP32 steps and 4-bit zero points tiled in
+ * The image holds the 4-bit codes, the FP32 steps (factored where that is exact) and 4-bit zero points tiled in
  * 16-row x 256-column blocks of 2336 bytes: 0.5703 bytes per weight when N and K are
  * multiples of 16 and 256.  The reference keeps 0.625 bytes per weight
  * (QuantizedLinear.storage_bytes, dandan_ops/quantized_linear.py:176-178). */
@@ -74,8 +74,8 @@ int64_t b2_w4a16_native_bytes(int64_t n, int64_t k);
 int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* zeros,
                     int64_t n, int64_t k, void* native, void* stream);
 /* Puts the steps of an image into the form that the kernels decode fastest, in place: the product of two FP16 numbers, for every
- * group whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() does so itself; the image
- * that b2_w4a16_quantize() writes has plain steps, which every kernel takes as well.  Calls that use the image may run at
+ * group whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() and
+ * b2_w4a16_quantize() do so themselves; every kernel takes plain steps as well.  Calls that use the image may run at
  * the same time: a field goes from one valid form to the other in one store. */
 int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream);
 
