@@ -107,9 +107,7 @@ int b2_w4a16_quantize(const void* weight, int weight_bits, int64_t n, int64_t k,
     a.native = static_cast<uint8_t*>(native);
     a.flags = flags;
     a.d = b2::make_dims(n, k);
-    if (int rc = weight_bits == 16 ? run_quantize<__half>(a, static_cast<cudaStream_t>(stream)) : run_quantize<float>(a, static_cast<cudaStream_t>(stream)))
-        return rc;
-    return native ? b2_w4a16_factor_steps(native, n, k, stream) : B2_OK;
+    return weight_bits == 16 ? run_quantize<__half>(a, static_cast<cudaStream_t>(stream)) : run_quantize<float>(a, static_cast<cudaStream_t>(stream));
 }
 
 int b2_w4a16_dequantize(const void* native, int64_t n, int64_t k, float* out, int64_t ldo, void* stream) {

@@ -159,6 +159,8 @@ class QuantizedLinear(torch.nn.Module):
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
                 layer._set_image(image, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
+                # (the image is complete, with plain steps; the first calls may run beside this or before it)
+                _native.factor_steps(image, *weight.shape)
             return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)

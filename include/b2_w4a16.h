@@ -74,8 +74,8 @@ int64_t b2_w4a16_native_bytes(int64_t n, int64_t k);
 int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* zeros,
                     int64_t n, int64_t k, void* native, void* stream);
 /* Puts the steps of an image into the form that the kernels decode fastest, in place: the product of two FP16 numbers, for every
- * group whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() and
- * b2_w4a16_quantize() do so themselves; every kernel takes plain steps as well.  Calls that use the image may run at
+ * group whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() does so itself; the image
+ * that b2_w4a16_quantize() writes has plain steps, which every kernel takes as well.  Calls that use the image may run at
  * the same time: a field goes from one valid form to the other in one store. */
 int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream);
 
