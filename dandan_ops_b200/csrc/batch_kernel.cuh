@@ -423,8 +423,9 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             };
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                if (all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
-                else convert(h, Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
+                if constexpr (H16) convert(h, Chain<kChainFp16>{});
+                else if (all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
+                else convert(h, Chain<kChainGeneral>{});
                 if (!ok) break;
             }
             if (!ok) break;

@@ -289,8 +289,9 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
                     o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
                 }
             };
-            if (all_factored(field)) convert(Chain<kChainFactored>{});
-            else convert(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
+            if constexpr (H16) convert(Chain<kChainFp16>{});
+            else if (all_factored(field)) convert(Chain<kChainFactored>{});
+            else convert(Chain<kChainGeneral>{});
             // the conversion happens in registers before the wait for the free tensor-memory stage
             if (s >= WS) ok = wait(DONE + (s - WS) % XS, ((s - WS) / XS) & 1);
             if (!ok) break;

@@ -189,8 +189,9 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
             constexpr int CH = decltype(chain)::value;
             f(make_group<CH>(o.zero & 15u, o.field.x), make_group<CH>(o.zero >> 4, o.field.y));
         };
-        if (all_factored(o.field.x & o.field.y)) go(Chain<kChainFactored>{});
-        else go(Chain<(H16 ? kChainFp16 : kChainGeneral)>{});
+        if constexpr (H16) go(Chain<kChainFp16>{});
+        else if (all_factored(o.field.x & o.field.y)) go(Chain<kChainFactored>{});
+        else go(Chain<kChainGeneral>{});
     };
     // The weights are constant; x, the bias and y may belong to the previous kernel until it has completed.  With one row tile
     // of x (registers) a warp decodes its first unit meanwhile.
