@@ -79,7 +79,8 @@ int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* z
  * the same time: a field goes from one valid form to the other in one store. */
 int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream);
 
-/* Native image -> reference layout (exact inverse of b2_w4a16_repack; codes beyond K
+/* Native image -> reference layout (exact inverse of b2_w4a16_repack for steps without a sign; a group whose step is negative, which
+ * no valid state has, comes back as the equal one with the absolute value of its step and 15 - code, 15 - zero; codes beyond K
  * in the last word come back as 0, as pack_int4 writes them). */
 int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed,
                       float* scales, int32_t* zeros, void* stream);
