@@ -2,6 +2,8 @@
 // Declarations and the per-function reference citations are in include/b2_w4a16.h.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/b2_w4a16.h"
 #include "factor_steps.cuh"
 #include "host_common.cuh"
@@ -33,13 +35,25 @@ int run_dequantize(const uint8_t* native, const int32_t* packed, const float* sc
     return after_launch("dequantize_kernel");
 }
 
+// Blocks of a warp: as few as let all warps run at once (40 on an SM; a 4096 x 12288 layer has three), for the shortest chain of
+// sets, up to eight, with which the lists of later sets fill most of a warp.
+int run_factor_steps(uint8_t* native, const b2::Dims& d, unsigned* flags, cudaStream_t s) {
+    constexpr int64_t kResident = 148 * 40;
+    const int64_t blocks = int64_t(d.n16) * d.kb;
+    const int64_t per_warp = std::min<int64_t>(b2::kFactorMaxBlocks, (blocks + kResident - 1) / kResident);
+    const int64_t per_cta = per_warp * b2::kFactorWarps;
+    b2::factor_steps_kernel<<<unsigned((blocks + per_cta - 1) / per_cta), b2::kFactorThreads, 0, s>>>(native, blocks, int(per_warp), flags);
+    return after_launch("factor_steps_kernel");
+}
+
 template <typename T>
 int run_quantize(const b2::QuantizeArgs& a, cudaStream_t s) {
     const unsigned blocks = unsigned(int64_t(a.d.n16) * a.d.kb);
     const bool vec = a.d.k % 8 == 0 && aligned16(a.weight) && reinterpret_cast<uintptr_t>(a.codes) % 8 == 0;
     if (vec) b2::quantize_kernel<T, true><<<blocks, 128, 0, s>>>(a);
     else b2::quantize_kernel<T, false><<<blocks, 128, 0, s>>>(a);
-    return after_launch("quantize_kernel");
+    if (int rc = after_launch("quantize_kernel")) return rc;
+    return a.native ? run_factor_steps(a.native, a.d, a.flags, s) : B2_OK;
 }
 
 }  // namespace
@@ -69,9 +83,7 @@ int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream) {
     if (int rc = check_dims(n, k)) return rc;
     if (reinterpret_cast<uintptr_t>(native) % 4) return fail(B2_ERR_ARGUMENT, "misaligned native image");
     const b2::Dims d = b2::make_dims(n, k);
-    const int64_t blocks = int64_t(d.n16) * d.kb;
-    b2::factor_steps_kernel<<<unsigned((blocks + b2::kFactorBlocks - 1) / b2::kFactorBlocks), b2::kFactorThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint8_t*>(native), blocks);
-    return after_launch("factor_steps_kernel");
+    return run_factor_steps(static_cast<uint8_t*>(native), d, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed, float* scales,

@@ -270,8 +270,9 @@ __device__ __forceinline__ uint32_t dequant_pair_odd(uint32_t h2, float c, uint6
 // in FP32 and fp16_rn(fp32(code - zero) * step) == hmul2(code - zero, step): one FP16 subtract (or fma by
 // 1/16 for the odd nibbles) and one FP16 multiply per pair, bit-identical to the general chain.
 // kChainFactored: for groups whose step field is factored (layout.cuh).  A pair of codes that is only masked out of its word
-// reads as the FP16 subnormals code * 2^-24 (odd nibbles: 2^-20), so one fma gives (code - zero) * a1 * 2^-14 - exact - and one
-// multiplication by a2 rounds to the weight: 1.6 instead of 2.6 instructions per weight, the same bits.
+// reads as the FP16 subnormals code * 2^-24 (odd nibbles: 2^-20), so one fma gives (code - zero) * a1 * 2^-14 and one
+// multiplication by a2 rounds to the weight: 1.6 instead of 2.6 instructions per weight, the same bits.  (The fma and its
+// addend can round, too; a field is factored only where these very operations were found to give the weights.)
 // A kernel takes the factored chain where all fields that a warp holds of a block are factored (`all_factored()`), else the
 // general one.  Under the FP16-step flag there is nothing to choose: that chain takes a weight in as many instructions as the
 // factored one and both forms of a field, and without vote and branch 57344 x 8192 takes 57.9 instead of 59.9 us at M = 1,

@@ -224,6 +224,26 @@ int64_t status_all() {
     return int64_t(all);
 }
 
+// One-pass quantizer (as _native.quantize for a layer): packed codes, steps, zero points, native image and the QUANT_* word, all of
+// them still being written when this returns.
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> quantize_image(const at::Tensor& weight) {
+    TORCH_CHECK(weight.is_cuda() && weight.dim() == 2 && weight.is_contiguous() &&
+                    (weight.scalar_type() == at::kHalf || weight.scalar_type() == at::kFloat),
+                "w4a16_quantize_image expects a contiguous CUDA FP16 or FP32 [N, K] weight");
+    c10::cuda::CUDAGuard guard(weight.device());
+    const int64_t n = weight.size(0), k = weight.size(1), groups = (k + 63) / 64, bytes = b2_w4a16_native_bytes(n, k);
+    TORCH_CHECK(bytes > 0, "b2_w4a16: W4A16 dimensions exceed the kernel index range");
+    const auto ints = weight.options().dtype(at::kInt);
+    at::Tensor packed = at::empty({n, (k + 7) / 8}, ints), image = at::empty({bytes}, weight.options().dtype(at::kByte));
+    at::Tensor scales = at::empty({n, groups}, weight.options().dtype(at::kFloat)), zeros = at::empty({n, groups}, ints);
+    at::Tensor flags = at::empty({1}, ints);
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    C10_CUDA_CHECK(cudaMemsetAsync(flags.data_ptr(), 0, 4, stream));
+    check_rc(b2_w4a16_quantize(weight.data_ptr(), int(weight.element_size()) * 8, n, k, nullptr, packed.data_ptr<int32_t>(), scales.data_ptr<float>(),
+                               zeros.data_ptr<int32_t>(), image.data_ptr(), reinterpret_cast<unsigned*>(flags.data_ptr<int32_t>()), stream));
+    return {packed, scales, zeros, image, flags};
+}
+
 }  // namespace
 
 TORCH_LIBRARY_FRAGMENT(dandan_ops, m) {
@@ -235,6 +255,7 @@ TORCH_LIBRARY_FRAGMENT(dandan_ops, m) {
     m.def("w4a16_linear_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int route, int flags) -> Tensor");
     m.def("w4a16_silu_mul_image(Tensor x, Tensor image, int n, int k, Tensor? bias, int flags) -> Tensor");
     m.def("w4a16_rmsnorm_image(Tensor x, Tensor? residual, Tensor weight, float eps, Tensor image, int n, int k, Tensor? bias, int flags=0) -> (Tensor, Tensor)");
+    m.def("w4a16_quantize_image(Tensor weight) -> (Tensor, Tensor, Tensor, Tensor, Tensor)");
     m.def("w4a16_workspace_status() -> int", &status_all);
 }
 
@@ -246,4 +267,5 @@ TORCH_LIBRARY_IMPL(dandan_ops, CUDA, m) {
     m.impl("w4a16_linear_image", &linear_image);
     m.impl("w4a16_silu_mul_image", &silu_mul_image);
     m.impl("w4a16_rmsnorm_image", &rmsnorm_image);
+    m.impl("w4a16_quantize_image", &quantize_image);
 }

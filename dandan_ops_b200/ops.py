@@ -72,7 +72,7 @@ _OPS = {"w4a16_gemv": _rule_gemv, "w4a16_small": _rule_small,
 
 
 SHIM_LOADED = False      # True when the ops come from the C++ operator library (lib/dandan_ops_b200_C.so)
-linear_image = silu_mul_image = rmsnorm_image = None     # its operators' one overload each, looked up once
+linear_image = silu_mul_image = rmsnorm_image = quantize_image = None     # its operators' one overload each, looked up once
 
 
 def register():
@@ -82,7 +82,7 @@ def register():
     with `torch.ops.load_library`, as the reference loads its `_C` module (dandan_ops/_extension.py:34); it
     registers the same names with TORCH_LIBRARY.  Where that file has not been built, the names are defined
     from Python over the ctypes binding instead - the same C-ABI kernels either way."""
-    global _registered, _library, SHIM_LOADED, linear_image, silu_mul_image, rmsnorm_image
+    global _registered, _library, SHIM_LOADED, linear_image, silu_mul_image, rmsnorm_image, quantize_image
     if _registered:
         return
     from . import build as _build
@@ -92,11 +92,16 @@ def register():
             linear_image = torch.ops.dandan_ops.w4a16_linear_image.default
             silu_mul_image = torch.ops.dandan_ops.w4a16_silu_mul_image.default
             rmsnorm_image = torch.ops.dandan_ops.w4a16_rmsnorm_image.default
+            quantize_image = torch.ops.dandan_ops.w4a16_quantize_image.default
             SHIM_LOADED = True
             _registered = True
             return
         except OSError:           # stale binary for another torch: fall through to the Python definitions
             pass
+        except AttributeError:    # an older build, without one of the operators above: its names stand, the modules call the C ABI
+            linear_image = silu_mul_image = rmsnorm_image = quantize_image = None
+            _registered = True
+            return
     _library = torch.library.Library("dandan_ops", "FRAGMENT")
     for name, rule in _OPS.items():
         _library.define(name + _SCHEMA)

@@ -154,13 +154,17 @@ class QuantizedLinear(torch.nn.Module):
             # One pass gives the state and the image of it.  Its steps are positive normal FP32 numbers and its zero
             # points 0..15 by construction, so nothing is read back to check them.
             with torch.no_grad():
-                _, packed, steps, zero_points, image, flags = _native.quantize(weight.detach().contiguous())
+                source = weight.detach().contiguous()
+                if (_ops_module.SHIM_LOADED and type(source) is torch.Tensor
+                        and not torch._C._functorch.is_functorch_wrapped_tensor(source)):
+                    packed, steps, zero_points, image, flags = _ops_module.quantize_image(source)
+                else:
+                    _, packed, steps, zero_points, image, flags = _native.quantize(source)
                 layer = cls.__new__(cls)                      # (built while the kernel runs)
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
-                layer._set_image(image, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
-                # (the image is complete, with plain steps; the first calls may run beside this or before it)
-                _native.factor_steps(image, *weight.shape)
+                key = layer._state_key()
+                layer._set_image(image, key, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
             return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)
@@ -245,9 +249,9 @@ class QuantizedLinear(torch.nn.Module):
         self._slice_flag = _native.FLAG_COLUMN_SLICE
         self._image_flags |= self._slice_flag
 
-    def _set_image(self, image, fp16_steps):
-        """Adopt an image of the current state that is complete in memory (its stream has been synchronized)."""
-        self._image, self._image_key = image, self._state_key()
+    def _set_image(self, image, key, fp16_steps):
+        """Adopt an image of the state with this key that is complete in memory (its stream has been synchronized)."""
+        self._image, self._image_key = image, key
         self._image_flags = ((_native.FLAG_FP16_STEPS if fp16_steps else 0)
                              | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0) | self._slice_flag)
 

@@ -73,10 +73,9 @@ int64_t b2_w4a16_native_bytes(int64_t n, int64_t k);
  * directly, this engine reads the tiled image. */
 int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* zeros,
                     int64_t n, int64_t k, void* native, void* stream);
-/* Puts the steps of an image into the form that the kernels decode fastest, in place: the product of two FP16 numbers, for every
- * group whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() does so itself; the image
- * that b2_w4a16_quantize() writes has plain steps, which every kernel takes as well.  Calls that use the image may run at
- * the same time: a field goes from one valid form to the other in one store. */
+/* Puts the steps of an image into the form that the kernels decode fastest, in place: the product of two FP16 numbers, for the
+ * groups whose sixteen weights that form reproduces bit for bit (csrc/layout.cuh).  b2_w4a16_repack() and b2_w4a16_quantize() do
+ * so themselves; images that hold plain steps (files of earlier versions) are read by every kernel as they are. */
 int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream);
 
 /* Native image -> reference layout (exact inverse of b2_w4a16_repack for steps without a sign; a group whose step is negative, which
@@ -93,7 +92,8 @@ int b2_w4a16_pack(const uint8_t* codes, int64_t n, int64_t k, int32_t* packed, v
  * (may be NULL), uint8 codes (may be NULL), FP32 steps, zero points and the native image (256-byte aligned, may be NULL).
  * Replaces quantize_int4 and pack_int4 (dandan_ops/quantization.py:62-103), bit for bit.  *flags must be zero before the
  * call and receives bit 0 = a weight is not finite (the results are then undefined), bit 1 = some step is not
- * representable in FP16 (B2_FLAG_FP16_STEPS does not apply). */
+ * representable in FP16 (B2_FLAG_FP16_STEPS does not apply), bit 2 = the image holds factored steps (two launches then: the
+ * second one looks for the factors). */
 int b2_w4a16_quantize(const void* weight, int weight_bits, int64_t n, int64_t k, uint8_t* codes, int32_t* packed,
                       float* scales, int32_t* zeros, void* native, unsigned* flags, void* stream);
 

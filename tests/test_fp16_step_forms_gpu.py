@@ -16,7 +16,7 @@ def _state(n, k, seed):
     codes = torch.randint(0, 16, (n, k), generator=g, dtype=torch.uint8)
     zeros = torch.randint(0, 16, (n, groups), generator=g, dtype=torch.int32)
     steps = torch.exp(torch.randn(n, groups, generator=g) * 0.5 - 5.0)
-    kind = torch.randint(0, 6, (n, groups), generator=g)
+    kind = torch.randint(0, 14, (n, groups), generator=g)
     steps = torch.where(kind == 1, torch.exp2(-24 + 14 * torch.rand(n, groups, generator=g)), steps)      # from FP16's smallest number on
     steps = torch.where(kind == 2, 4.0 + 4000.0 * torch.rand(n, groups, generator=g), steps)
     steps = steps.half().float().clamp_min(2.0 ** -24)
@@ -34,7 +34,7 @@ def test_both_forms_of_fp16_steps_give_the_weights(shape, route, m, n, k):
     packed, steps, zeros = _state(n, k, n + k + m)
     image = _native.repack(packed, steps, zeros, k)
     factored = image.view(-1, 2336)[:, 2048:2304].contiguous().view(torch.int32) < 0
-    assert (factored.any(1) & ~factored.all(1)).float().mean() > 0.4                   # blocks with both forms
+    assert (factored.any(1) & ~factored.all(1)).float().mean() > 0.4                    # blocks with both forms
     weights = ops.dequantize_int4(packed, steps, zeros, k).half()
     assert torch.isfinite(weights).all()
     _native.set_gemm_shape(shape)
