@@ -3,9 +3,9 @@
 // quantize_kernel reads every weight once (2 or 4 bytes) and writes everything a layer keeps of it - packed codes, FP32
 // step, zero point, native image - in the same pass.  The same steps as separate
 // elementwise and reduction passes over an FP32 copy move about forty bytes per weight.  Measured on 4096 x 12288
-// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 46 us here
-// (2.2 TB/s of input, 3.5 TB/s with everything written; 51 us before the rounding took two weights per
-// instruction): bound by the instructions of range and rounding.
+// FP16: 1690 us for the whole conversion as separate passes (with packing, value checks and relayout), 43 us here
+// (2.3 TB/s of input, 3.7 TB/s with everything written): bound by the instructions of range and rounding and, between them, by
+// the wait for the weights (nine CTAs of four warps on an SM instead of eight: 44.8 -> 43.2; FP32 weights ten, 46.8 -> 45.2).
 #pragma once
 #include <cfloat>
 #include <type_traits>
@@ -75,17 +75,16 @@ template <> struct Eight<__half> {
     __device__ __forceinline__ __half2 pair(int c) const { return *reinterpret_cast<const __half2*>(&p[c]); }
     __device__ __forceinline__ void range(float& lo, float& hi, bool& finite) const {      // two weights per instruction
         const __half2 zero = __half2half2(__ushort_as_half(0));
-        __half2 l = zero, h = zero, poison = zero;
+        __half2 l = zero, h = zero;                          // (a NaN stays in both, an infinity in one)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            l = __hmin2(l, pair(c));
-            h = __hmax2(h, pair(c));
-            poison = __hfma2(pair(c), zero, poison);
+            l = __hmin2_nan(l, pair(c));
+            h = __hmax2_nan(h, pair(c));
         }
         const float2 lf = __half22float2(l), hf = __half22float2(h);
         lo = fminf(lf.x, lf.y);
         hi = fmaxf(hf.x, hf.y);
-        finite = finite && __hbeq2(poison, zero);
+        finite = finite && (hf.x - lf.x) + (hf.y - lf.y) < 1e6f;
     }
     __device__ __forceinline__ void widen(float (&f)[8]) const {
 #pragma unroll
@@ -102,54 +101,66 @@ __device__ __forceinline__ float reciprocal(float v) {       // to one unit in t
     return r;
 }
 
-// Reference word (nibble c = column c) -> native word of a whole word: even columns to the low half, odd ones to the high.
-__device__ __forceinline__ uint32_t split_nibbles(uint32_t ref) {
-    const uint32_t even = ref & 0x0F0F0F0Fu, odd = (ref >> 4) & 0x0F0F0F0Fu;
-    return __byte_perm(even | (even >> 4), odd | (odd >> 4), 0x6420);
-}
-
 // Packed codes of eight weights: code = clamp(round_half_even(fl(fl(w / step) + zero)), 0, 15).
 //
 // The sum is first taken as w * (1 / step) + zero with the approximate reciprocal: |w / step| is at most 15 plus
 // rounding, so it is off by less than 2^-17 together with the two roundings of the definition.  Only a sum that close
 // to a half-integer can round to another code; where one of the eight is (one word in ~10^4), or where the
-// reciprocal of the step is not a normal number, the eight weights are divided.
+// reciprocal of the step is not a normal number, the eight weights are divided.  Only there, too, can a code be outside 0..15:
+// the ends of the range are at -0.5 and 15.5.
 //
-// Rounding is an addition of 1.5 * 2^23, whose ulp is 1: exact half-to-even for sums this small, and the code is then
-// in the low mantissa bits (rintf and the float-to-int conversion run at an eighth of the rate of an addition).
+// Rounding is an addition of 1.5 * 2^23, whose ulp is 1, in the fma that forms the sum: half-to-even for sums this small, and
+// the code is then in the low byte (rintf and the float-to-int conversion run at an eighth of the rate of an addition).
 constexpr float kRoundMagic = 12582912.0f;
 __device__ __forceinline__ int code_of(float u) { return __float_as_int(u) - 0x4B400000; }
-// Appends two codes, clamped to 0..15, in front of those that `words` already holds.
-__device__ __forceinline__ uint32_t push_codes(int high, int low, uint32_t words) {
-    uint32_t r;
-    asm("cvt.pack.sat.u4.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(high), "r"(low), "r"(words));
-    return r;
+// The eight codes of a word in the low halves of bytes: columns 0, 2, 4, 6 and columns 1, 3, 5, 7.
+struct Codes {
+    uint32_t even, odd;
+    __device__ __forceinline__ uint32_t reference() const { return even + (odd << 4); }            // nibble c = column c
+    __device__ __forceinline__ uint32_t native() const { return __byte_perm(even | even >> 4, odd | odd >> 4, 0x6420); }
+};
+__device__ __forceinline__ uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
-__device__ __forceinline__ uint32_t quantize_word(const float (&v)[8], float step, float zero) {
-    const float inverse = reciprocal(step);
+__device__ __forceinline__ Codes quantize_word(const float (&v)[8], float step, float zero) {
+    const float inverse = reciprocal(step), base = zero + kRoundMagic;
     float off = step < 0x1p100f ? 0.0f : 1.0f;              // largest distance of a sum from the integer it rounds to
-    int q[8];
+    uint32_t q[8];
 #pragma unroll
     for (int c = 0; c < 8; c += 2) {                        // two weights per instruction, each rounded as if alone
         float u0, u1, d0, d1;
-        asm("{\n\t.reg .b64 t, u, r, v, i, z, m;\n\t"
-            "mov.b64 v, {%4, %5};\n\tmov.b64 i, {%6, %6};\n\tmov.b64 z, {%7, %7};\n\tmov.b64 m, {%8, %8};\n\t"
-            "fma.rn.f32x2 t, v, i, z;\n\tadd.rn.f32x2 u, t, m;\n\tsub.rn.f32x2 r, u, m;\n\tsub.rn.f32x2 r, t, r;\n\t"
+        asm("{\n\t.reg .b64 u, r, v, i, z;\n\t"
+            "mov.b64 v, {%4, %5};\n\tmov.b64 i, {%6, %6};\n\tmov.b64 z, {%7, %7};\n\t"
+            "fma.rn.f32x2 u, v, i, z;\n\tsub.rn.f32x2 r, z, u;\n\tfma.rn.f32x2 r, v, i, r;\n\t"
             "mov.b64 {%0, %1}, u;\n\tmov.b64 {%2, %3}, r;\n\t}"
             : "=f"(u0), "=f"(u1), "=f"(d0), "=f"(d1)
-            : "f"(v[c]), "f"(v[c + 1]), "f"(inverse), "f"(zero), "f"(kRoundMagic));
-        off = fmaxf(off, fmaxf(fabsf(d0), fabsf(d1)));
-        q[c] = code_of(u0);
-        q[c + 1] = code_of(u1);
+            : "f"(v[c]), "f"(v[c + 1]), "f"(inverse), "f"(base));
+        asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(off) : "f"(off), "f"(d0), "f"(d1));
+        q[c] = __float_as_uint(u0);
+        q[c + 1] = __float_as_uint(u1);
     }
     if (off > 0.5f - 0x1p-16f) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) q[c] = code_of(__fadd_rn(__fadd_rn(__fdiv_rn(v[c], step), zero), kRoundMagic));
+        for (int c = 0; c < 8; ++c) q[c] = uint32_t(min(max(code_of(__fadd_rn(__fadd_rn(__fdiv_rn(v[c], step), zero), kRoundMagic)), 0), 15));
     }
-    uint32_t word = 0;
-#pragma unroll
-    for (int c = 6; c >= 0; c -= 2) word = push_codes(q[c + 1], q[c], word);
-    return word;
+    return Codes{low_bytes(q[0], q[2], q[4], q[6]), low_bytes(q[1], q[3], q[5], q[7])};
+}
+
+// v / 15, correctly rounded, in two operations: v times the high part of 1/15 plus (v times the low part), a division by a constant
+// after Brisebarre, Muller and Raina (IEEE Trans. Computers 53, 2004).  Equal to the division for all 2^23 mantissas as long as the
+// small product is a normal number; smaller and larger values are divided.
+__device__ __forceinline__ float fifteenth(float v) {
+    const float q = __fmaf_rn(v, 0x1.111112p-4f, __fmul_rn(v, -0x1.dddddep-29f));
+    return fabsf(v) > 0x1p-90f && fabsf(v) < 0x1p120f ? q : __fdiv_rn(v, 15.0f);
+}
+
+// clamp(round_half_even(fl(-lo / step)), 0, 15): as for a code, the quotient by the approximate reciprocal decides unless it is
+// close to a half-integer.
+__device__ __forceinline__ float zero_point(float lo, float step) {
+    const float inverse = reciprocal(step), u = __fmaf_rn(-lo, inverse, kRoundMagic), r = __fsub_rn(u, kRoundMagic);
+    const float off = fabsf(__fmaf_rn(-lo, inverse, -r));
+    const float zero = step < 0x1p100f && off < 0.5f - 0x1p-16f ? r : rintf(__fdiv_rn(-lo, step));
+    return fminf(fmaxf(zero, 0.0f), 15.0f);
 }
 
 // One CTA of four warps per 16 x 256 block; warp w takes the rows w, w + 4, w + 8 and w + 12, lane 8t + i word i of
@@ -157,7 +168,7 @@ __device__ __forceinline__ uint32_t quantize_word(const float (&v)[8], float ste
 // of rows a lane carries, so that lane i ends with the range of row i % 4 and computes that row's step and zero
 // point (IEEE divisions are what this kernel could least afford to repeat in every lane), which the others fetch.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, sizeof(T) == 2 ? 9 : 10)
 quantize_kernel(const QuantizeArgs a) {
     constexpr unsigned kAll = 0xffffffffu;
     const Dims& d = a.d;
@@ -191,9 +202,9 @@ quantize_kernel(const QuantizeArgs a) {
     exchange(lo[0], lo[0], lo[0], 4, true);                  // lanes i and i + 4 hold the same row
     exchange(hi[0], hi[0], hi[0], 4, false);
     // two quotients and a difference, each rounded; never below the smallest normal FP32; 1 for an all-zero group
-    float my_step = fmaxf(__fsub_rn(__fdiv_rn(hi[0], 15.0f), __fdiv_rn(lo[0], 15.0f)), FLT_MIN);
+    float my_step = fmaxf(__fsub_rn(fifteenth(hi[0]), fifteenth(lo[0])), FLT_MIN);
     if (hi[0] == 0.0f && lo[0] == 0.0f) my_step = 1.0f;
-    const float my_zero = fminf(fmaxf(rintf(__fdiv_rn(-lo[0], my_step)), 0.0f), 15.0f);
+    const float my_zero = zero_point(lo[0], my_step);
     uint8_t* block = a.native ? a.native + (int64_t(kb) * d.n16 + nt) * kBlockBytes : nullptr;
     {   // lane i < 4 of a group keeps the books of row w + 4i
         const int r = w + 4 * (wi & 3), row = nt * 16 + r;
@@ -217,7 +228,8 @@ quantize_kernel(const QuantizeArgs a) {
         const bool real = row < d.n && grp < d.groups;
         float f[8];
         v[p].widen(f);
-        uint32_t ref = quantize_word(f, step, zero);
+        const Codes codes = quantize_word(f, step, zero);
+        uint32_t ref = codes.reference();
         if (!VEC && valid < 8) ref &= valid > 0 ? 0xffffffffu >> (32 - 4 * valid) : 0u;
         if (real && valid > 0) {
             if (a.packed) a.packed[int64_t(row) * d.words + (k0 >> 3)] = int32_t(ref);
@@ -235,7 +247,7 @@ quantize_kernel(const QuantizeArgs a) {
         }
         if (block) {                   // rows and groups that do not exist: code 0; columns beyond K: the zero point
             const uint32_t fill = uint32_t(int(zero));
-            const uint32_t nat = !real ? 0u : valid >= 8 ? split_nibbles(ref) : permute_word(ref, max(valid, 0), fill);
+            const uint32_t nat = !real ? 0u : valid >= 8 ? codes.native() : permute_word(ref, max(valid, 0), fill);
             reinterpret_cast<uint32_t*>(block)[(2 * (r >> 3) + (wi >> 2)) * 128 + (4 * (r & 7) + t) * 4 + (wi & 3)] = nat;
         }
     }
