@@ -41,6 +41,7 @@ _SIGNATURES = {
     "b2_w4a16_native_bytes": (_i64, [_i64, _i64]),
     "b2_w4a16_repack": (_int, [_vp, _vp, _vp, _i64, _i64, _vp, _vp]),
     "b2_w4a16_factor_steps": (_int, [_vp, _i64, _i64, _vp]),
+    "b2_w4a16_image_flags": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "b2_w4a16_unrepack": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "b2_w4a16_pack": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "b2_w4a16_quantize": (_int, [_vp, _int, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
@@ -229,6 +230,20 @@ def factor_steps(image, n, k):
         _check(load().b2_w4a16_factor_steps(image.data_ptr(), n, k, _stream()))
 
 
+def image_flags(image, n, k):
+    """QUANT_STEP_NOT_FP16 and QUANT_FACTORED as they hold for a native image (`b2_w4a16_image_flags`; synchronizes)."""
+    with _on(image.device):
+        flags = torch.zeros(1, dtype=torch.int32, device=image.device)
+        _check(load().b2_w4a16_image_flags(image.data_ptr(), n, k, flags.data_ptr(), _stream()))
+        return flags.item()
+
+
+def step_flags(found):
+    """Layer flags that follow from the QUANT_* bits of an image."""
+    return ((0 if found & QUANT_STEP_NOT_FP16 else FLAG_FP16_STEPS) | (0 if found & QUANT_FACTORED else FLAG_PLAIN_STEPS)
+            | (FLAG_OVERLAP_LAUNCH if OVERLAP_LAUNCH else 0))
+
+
 def image_from_host(host_bytes, device):
     """A native image read back from storage (uint8 CPU tensor) -> uint8 tensor on `device`."""
     if host_bytes.dtype != torch.uint8 or host_bytes.ndim != 1:
@@ -258,7 +273,7 @@ def pack(codes):
     return out
 
 
-QUANT_NONFINITE, QUANT_STEP_NOT_FP16 = 1, 2
+QUANT_NONFINITE, QUANT_STEP_NOT_FP16, QUANT_FACTORED = 1, 2, 4
 
 
 def quantize(weight, want_codes=False, want_layer=True):
@@ -404,6 +419,7 @@ def linear_static(x, image, n, k, out):
 
 
 FLAG_FP16_STEPS = 1
+FLAG_PLAIN_STEPS = 32        # no group of the image has a factored step
 FLAG_COLUMN_SLICE = 16       # up to 16 rows the kernels that carry the all-gather (see include/b2_w4a16.h)
 FLAG_OVERLAP_LAUNCH = 2      # tile, streaming and batch kernel may start under the previous kernel's tail
 OVERLAP_LAUNCH = os.environ.get("B2_W4A16_OVERLAP", "1") != "0"

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "../../include/b2_w4a16.h"
 #include "host_common.cuh"
@@ -193,12 +194,20 @@ int launch_maybe_dependent(const char* name, Kernel kernel, int grid, int thread
 // Up to this many rows of x the streaming kernel stages only the rows that exist (template parameter XROWS).
 constexpr int kStreamExactRows = 4;
 
-template <int MT, bool XVEC, int W, bool H16 = false, bool XROWS = false>
+// f(integral constant of what is known of the layer's step fields).
+template <typename F>
+int with_steps(int steps, const F& f) {
+    if (steps == b2::kStepsFp16) return f(std::integral_constant<int, b2::kStepsFp16>{});
+    if (steps == b2::kStepsPlain) return f(std::integral_constant<int, b2::kStepsPlain>{});
+    return f(std::integral_constant<int, b2::kStepsMixed>{});
+}
+
+template <int MT, bool XVEC, int W, int STEPS = b2::kStepsMixed, bool XROWS = false>
 int launch_stream_one(const b2::StreamArgs& a, int grid, cudaStream_t s) {
     if constexpr (MT == 1 && !XROWS) {
-        if (a.m <= kStreamExactRows) return launch_stream_one<MT, XVEC, W, H16, true>(a, grid, s);
+        if (a.m <= kStreamExactRows) return launch_stream_one<MT, XVEC, W, STEPS, true>(a, grid, s);
     }
-    auto kernel = b2::w4a16_stream_kernel<MT, XVEC, W, H16, XROWS>;
+    auto kernel = b2::w4a16_stream_kernel<MT, XVEC, W, STEPS, XROWS>;
     constexpr int smem = b2::stream_smem_bytes(W);
     // Opt in to >48 KB of dynamic shared memory once per device and instantiation.
     static std::atomic<uint64_t> configured{0};
@@ -217,12 +226,12 @@ constexpr int kNotFused = -1000;            // internal: the fused projection + 
 
 // Projection + all-gather in one launch (w4a16_stream_gather_kernel).  Its CTAs wait for packets from other
 // GPUs, so the whole grid must be resident at once: checked against the occupancy the runtime reports.
-template <int MT, int W, bool H16, bool XROWS = false>
+template <int MT, int W, int STEPS, bool XROWS = false>
 int launch_stream_gather_one(const b2::StreamArgs& a, const b2::GatherArgs& ga, int grid, int sms, cudaStream_t s) {
     if constexpr (MT == 1 && !XROWS) {
-        if (a.m <= kStreamExactRows) return launch_stream_gather_one<MT, W, H16, true>(a, ga, grid, sms, s);
+        if (a.m <= kStreamExactRows) return launch_stream_gather_one<MT, W, STEPS, true>(a, ga, grid, sms, s);
     }
-    auto kernel = b2::w4a16_stream_gather_kernel<MT, W, H16, XROWS>;
+    auto kernel = b2::w4a16_stream_gather_kernel<MT, W, STEPS, XROWS>;
     constexpr int smem = b2::stream_smem_bytes(W);
     static std::atomic<uint64_t> configured{0};
     static std::atomic<int> per_sm[64];
@@ -260,9 +269,9 @@ int launch_stream2_one(const b2::StreamArgs& a, int grid, cudaStream_t s) {
     return after_launch("w4a16_stream2_kernel");
 }
 
-template <int MT, bool XVEC, bool H16>
+template <int MT, bool XVEC, int STEPS>
 int launch_stream2d_one(const b2::StreamArgs& a, int grid, cudaStream_t s) {
-    auto kernel = b2::w4a16_stream2d_kernel<MT, XVEC, H16>;
+    auto kernel = b2::w4a16_stream2d_kernel<MT, XVEC, STEPS>;
     constexpr int smem = b2::stream_smem_bytes(16);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -278,15 +287,17 @@ int launch_stream2d_one(const b2::StreamArgs& a, int grid, cudaStream_t s) {
 }
 
 template <int MT>
-int launch_stream(const b2::StreamArgs& a, bool xvec, int warps, int grid, cudaStream_t s, bool h16) {
+int launch_stream(const b2::StreamArgs& a, bool xvec, int warps, int grid, cudaStream_t s, int steps) {
     if constexpr (MT <= 2) {
         if (a.nchunks > 1) {
-            if (h16 && xvec) return launch_stream2d_one<MT, true, true>(a, grid, s);
-            return xvec ? launch_stream2d_one<MT, true, false>(a, grid, s) : launch_stream2d_one<MT, false, false>(a, grid, s);
+            if (steps == b2::kStepsFp16 && xvec) return launch_stream2d_one<MT, true, b2::kStepsFp16>(a, grid, s);
+            return xvec ? launch_stream2d_one<MT, true, b2::kStepsMixed>(a, grid, s) : launch_stream2d_one<MT, false, b2::kStepsMixed>(a, grid, s);
         }
-        // FP16-step chain: up to 16 rows of an aligned x (the decode case it was built for)
-        if (h16 && xvec && warps == 16) return launch_stream_one<MT, true, 16, true>(a, grid, s);
-        if (h16 && xvec && warps == 4) return launch_stream_one<MT, true, 4, true>(a, grid, s);
+        // what is known of the steps is used for up to 16 rows of an aligned x (the decode case these forms were built for)
+        if (steps != b2::kStepsMixed && xvec && (warps == 16 || warps == 4))
+            return with_steps(steps, [&](auto t) {
+                return warps == 16 ? launch_stream_one<MT, true, 16, decltype(t)::value>(a, grid, s) : launch_stream_one<MT, true, 4, decltype(t)::value>(a, grid, s);
+            });
         if (warps == 32) return xvec ? launch_stream2_one<MT, true, 32>(a, grid, s) : launch_stream2_one<MT, false, 32>(a, grid, s);
         if (warps == 16 && g_stream_variant.load(std::memory_order_relaxed) == 3)
             return xvec ? launch_stream2_one<MT, true, 16>(a, grid, s) : launch_stream2_one<MT, false, 16>(a, grid, s);
@@ -331,9 +342,9 @@ bool tile_applicable(int64_t rows, const b2::Dims& d, int split) {
 
 bool pair_available();
 
-template <int MT, bool XVEC, bool FULL, bool H16 = false>
+template <int MT, bool XVEC, bool FULL, int STEPS = b2::kStepsMixed>
 int launch_tile_one(const b2::TileArgs& a, int smem, cudaStream_t s) {
-    auto kernel = b2::w4a16_tile_kernel<MT, XVEC, FULL, H16>;
+    auto kernel = b2::w4a16_tile_kernel<MT, XVEC, FULL, STEPS>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -381,9 +392,9 @@ bool tile_gather_pays(int64_t m, const b2::Dims& d, int ksplit, int world, int64
     return int64_t(world - 1) * m * (slice_cols / 2) <= 4LL * warps * 32;
 }
 
-template <int MT, bool FULL, bool H16>
+template <int MT, bool FULL, int STEPS>
 int launch_tile_gather_one(const b2::TileArgs& a, const b2::GatherArgs& ga, int smem, cudaStream_t s) {
-    auto kernel = b2::w4a16_tile_gather_kernel<MT, FULL, H16>;
+    auto kernel = b2::w4a16_tile_gather_kernel<MT, FULL, STEPS>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -420,7 +431,7 @@ int launch_tile_gather_one(const b2::TileArgs& a, const b2::GatherArgs& ga, int 
 
 int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t rows,
              const b2::Dims& d, void* workspace, bool xvec, cudaStream_t s, const void* bias, int act = 0, int sms = 148,
-             bool h16 = false, bool overlap = false, const b2::GatherArgs* ga = nullptr) {
+             int steps = b2::kStepsMixed, bool overlap = false, const b2::GatherArgs* ga = nullptr) {
     if (ga && (!xvec || act)) return kNotFused;       // the gather form exists for an aligned x and the plain output
     if (ga && !tile_gather_pays(rows, d, tile_ksplit(d, sms > 0 ? sms : 148, pair_available()), ga->world, ga->slice_cols))
         return kNotFused;
@@ -445,10 +456,14 @@ int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
     if (a.ksplit > 1) {
         const int smem2 = b2::tile_smem_bytes(kb_cta, mt * 8, a.warps) + a.ksplit * mt * 512;      // padded rows: the grid is small
         if (ga) {
-            if (mt == 1) return h16 ? launch_tile_gather_one<1, true, true>(a, *ga, smem2, s) : launch_tile_gather_one<1, true, false>(a, *ga, smem2, s);
-            return h16 ? launch_tile_gather_one<2, true, true>(a, *ga, smem2, s) : launch_tile_gather_one<2, true, false>(a, *ga, smem2, s);
+            return with_steps(steps, [&](auto t) {
+                return mt == 1 ? launch_tile_gather_one<1, true, decltype(t)::value>(a, *ga, smem2, s) : launch_tile_gather_one<2, true, decltype(t)::value>(a, *ga, smem2, s);
+            });
         }
-        if (h16 && xvec) return mt == 1 ? launch_tile_one<1, true, true, true>(a, smem2, s) : launch_tile_one<2, true, true, true>(a, smem2, s);
+        if (steps != b2::kStepsMixed && xvec)
+            return with_steps(steps, [&](auto t) {
+                return mt == 1 ? launch_tile_one<1, true, true, decltype(t)::value>(a, smem2, s) : launch_tile_one<2, true, true, decltype(t)::value>(a, smem2, s);
+            });
         if (mt == 1) return xvec ? launch_tile_one<1, true, true>(a, smem2, s) : launch_tile_one<1, false, true>(a, smem2, s);
         return xvec ? launch_tile_one<2, true, true>(a, smem2, s) : launch_tile_one<2, false, true>(a, smem2, s);
     }
@@ -459,17 +474,16 @@ int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
     const bool full = rows == mt * 8 || int64_t(d.n16) <= int64_t(per_sm) * (sms > 0 ? sms : 148);
     const int smem = b2::tile_smem_bytes(d.kb, full ? mt * 8 : int(rows), a.warps);
     if (ga) {
-        if (mt == 1) {
-            if (full) return h16 ? launch_tile_gather_one<1, true, true>(a, *ga, smem, s) : launch_tile_gather_one<1, true, false>(a, *ga, smem, s);
-            return h16 ? launch_tile_gather_one<1, false, true>(a, *ga, smem, s) : launch_tile_gather_one<1, false, false>(a, *ga, smem, s);
-        }
-        if (full) return h16 ? launch_tile_gather_one<2, true, true>(a, *ga, smem, s) : launch_tile_gather_one<2, true, false>(a, *ga, smem, s);
-        return h16 ? launch_tile_gather_one<2, false, true>(a, *ga, smem, s) : launch_tile_gather_one<2, false, false>(a, *ga, smem, s);
+        return with_steps(steps, [&](auto t) {
+            if (mt == 1) return full ? launch_tile_gather_one<1, true, decltype(t)::value>(a, *ga, smem, s) : launch_tile_gather_one<1, false, decltype(t)::value>(a, *ga, smem, s);
+            return full ? launch_tile_gather_one<2, true, decltype(t)::value>(a, *ga, smem, s) : launch_tile_gather_one<2, false, decltype(t)::value>(a, *ga, smem, s);
+        });
     }
-    if (h16 && xvec) {
-        if (mt == 1) return full ? launch_tile_one<1, true, true, true>(a, smem, s) : launch_tile_one<1, true, false, true>(a, smem, s);
-        return full ? launch_tile_one<2, true, true, true>(a, smem, s) : launch_tile_one<2, true, false, true>(a, smem, s);
-    }
+    if (steps != b2::kStepsMixed && xvec)
+        return with_steps(steps, [&](auto t) {
+            if (mt == 1) return full ? launch_tile_one<1, true, true, decltype(t)::value>(a, smem, s) : launch_tile_one<1, true, false, decltype(t)::value>(a, smem, s);
+            return full ? launch_tile_one<2, true, true, decltype(t)::value>(a, smem, s) : launch_tile_one<2, true, false, decltype(t)::value>(a, smem, s);
+        });
     if (mt == 1) {
         if (full) return xvec ? launch_tile_one<1, true, true>(a, smem, s) : launch_tile_one<1, false, true>(a, smem, s);
         return xvec ? launch_tile_one<1, true, false>(a, smem, s) : launch_tile_one<1, false, false>(a, smem, s);
@@ -480,7 +494,7 @@ int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
 
 int run_stream(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t m,
                const b2::Dims& d, void* workspace, int64_t workspace_bytes, cudaStream_t s,
-               const DeviceInfo& dev, const void* bias, int act = 0, bool h16 = false,
+               const DeviceInfo& dev, const void* bias, int act = 0, int steps = b2::kStepsMixed,
                const b2::GatherArgs* ga = nullptr, bool overlap = false) {
     const int64_t ticket_bytes = B2_W4A16_TICKET_BYTES;
     const bool xvec = (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (ldx % 8 == 0) && (d.k % 8 == 0);
@@ -511,18 +525,17 @@ int run_stream(const void* x, int64_t ldx, const void* native, void* y, int64_t 
             // one launch for projection and gather: 16 rows at most, aligned x, the shipped 16- or 4-warp kernel
             if (!xvec || p.mt > 2 || (p.warps != 16 && p.warps != 4) || p.nchunks > 1 || act) return kNotFused;
             const int sms = dev.sm_count > 0 ? dev.sm_count : 148;
-            if (p.mt == 1) {
-                if (p.warps == 16) return h16 ? launch_stream_gather_one<1, 16, true>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<1, 16, false>(a, *ga, p.grid, sms, s);
-                return h16 ? launch_stream_gather_one<1, 4, true>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<1, 4, false>(a, *ga, p.grid, sms, s);
-            }
-            if (p.warps == 16) return h16 ? launch_stream_gather_one<2, 16, true>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<2, 16, false>(a, *ga, p.grid, sms, s);
-            return h16 ? launch_stream_gather_one<2, 4, true>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<2, 4, false>(a, *ga, p.grid, sms, s);
+            return with_steps(steps, [&](auto t) {
+                if (p.mt == 1)
+                    return p.warps == 16 ? launch_stream_gather_one<1, 16, decltype(t)::value>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<1, 4, decltype(t)::value>(a, *ga, p.grid, sms, s);
+                return p.warps == 16 ? launch_stream_gather_one<2, 16, decltype(t)::value>(a, *ga, p.grid, sms, s) : launch_stream_gather_one<2, 4, decltype(t)::value>(a, *ga, p.grid, sms, s);
+            });
         }
         switch (p.mt) {
-            case 1: rc = launch_stream<1>(a, xvec, p.warps, p.grid, s, h16); break;
-            case 2: rc = launch_stream<2>(a, xvec, p.warps, p.grid, s, h16); break;
-            case 4: rc = launch_stream<4>(a, xvec, p.warps, p.grid, s, h16); break;
-            default: rc = launch_stream<8>(a, xvec, p.warps, p.grid, s, h16); break;
+            case 1: rc = launch_stream<1>(a, xvec, p.warps, p.grid, s, steps); break;
+            case 2: rc = launch_stream<2>(a, xvec, p.warps, p.grid, s, steps); break;
+            case 4: rc = launch_stream<4>(a, xvec, p.warps, p.grid, s, steps); break;
+            default: rc = launch_stream<8>(a, xvec, p.warps, p.grid, s, steps); break;
         }
         if (rc != B2_OK) return rc;
     }
@@ -590,7 +603,7 @@ bool gemm_preferred(int64_t m, const b2::Dims& d) {
 }
 
 // The batch kernel reads x by TMA; the product of its steps and CTAs stays inside 32 bits.
-constexpr int kLayerFlags = B2_FLAG_FP16_STEPS | B2_FLAG_OVERLAP_LAUNCH | B2_FLAG_COLUMN_SLICE;
+constexpr int kLayerFlags = B2_FLAG_FP16_STEPS | B2_FLAG_PLAIN_STEPS | B2_FLAG_OVERLAP_LAUNCH | B2_FLAG_COLUMN_SLICE;
 constexpr int64_t kBatchMaxM = 128;
 constexpr int64_t kGatherMaxM = 16;      // rows of x up to which projection and all-gather run as one launch
 bool batch_applicable(int64_t m, const b2::Dims& d) {
@@ -656,9 +669,9 @@ int launch_gemm_one(const CUtensorMap& map, const b2::GemmArgs& a, dim3 grid, cu
     return after_launch("w4a16_gemm_kernel");
 }
 
-template <int MT, bool TMA_Y, bool H16 = false>
+template <int MT, bool TMA_Y, int STEPS = b2::kStepsMixed>
 int launch_gemm_pair(const CUtensorMap& map, const CUtensorMap& ymap, const b2::GemmArgs& a, dim3 grid, cudaStream_t s) {
-    auto kernel = b2::w4a16_gemm_pair_kernel<MT, TMA_Y, H16>;
+    auto kernel = b2::w4a16_gemm_pair_kernel<MT, TMA_Y, STEPS>;
     constexpr int smem = b2::pair_smem_bytes<MT>();
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -783,7 +796,7 @@ GemmShape gemm_shape_for_call(int64_t m, const b2::Dims& d, int sms, int64_t wor
 
 int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t m,
              const b2::Dims& d, void* workspace, int64_t workspace_bytes, cudaStream_t s, int sms, const void* bias,
-             int act = 0, bool h16 = false) {
+             int act = 0, int steps = b2::kStepsMixed) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return fail(B2_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available from the driver");
     if (workspace == nullptr) return fail(B2_ERR_WORKSPACE, "workspace smaller than b2_w4a16_workspace_bytes()");
@@ -824,8 +837,9 @@ int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
             if (encode(&ymap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, y, ydims, ystrides, ybox, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return fail(B2_ERR_CUDA, "cuTensorMapEncodeTiled failed for y");
-            if (h16) return pair_mt == 256 ? launch_gemm_pair<256, true, true>(map, ymap, a, pgrid, s) : launch_gemm_pair<192, true, true>(map, ymap, a, pgrid, s);
-            return pair_mt == 256 ? launch_gemm_pair<256, true>(map, ymap, a, pgrid, s) : launch_gemm_pair<192, true>(map, ymap, a, pgrid, s);
+            return with_steps(steps, [&](auto t) {
+                return pair_mt == 256 ? launch_gemm_pair<256, true, decltype(t)::value>(map, ymap, a, pgrid, s) : launch_gemm_pair<192, true, decltype(t)::value>(map, ymap, a, pgrid, s);
+            });
         }
         return pair_mt == 256 ? launch_gemm_pair<256, false>(map, ymap, a, pgrid, s) : launch_gemm_pair<192, false>(map, ymap, a, pgrid, s);
     }
@@ -838,7 +852,7 @@ int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
 
 // x [M <= 128, K] through the batch kernel.
 int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t m, const b2::Dims& d, void* workspace,
-              int64_t workspace_bytes, cudaStream_t s, int sms, const void* bias, int act, bool h16, bool overlap) {
+              int64_t workspace_bytes, cudaStream_t s, int sms, const void* bias, int act, int steps, bool overlap) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return fail(B2_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available from the driver");
     const b2host::BatchPlan p = b2host::plan_batch(m, d, sms);
@@ -865,7 +879,7 @@ int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t l
     a.act = act;
     a.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
     a.fault_block = g_fault_step.exchange(-1, std::memory_order_relaxed);
-    return b2host::launch_batch(p, map, a, h16, overlap, s);
+    return b2host::launch_batch(p, map, a, steps, overlap, s);
 }
 
 }  // namespace
@@ -1050,7 +1064,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
                 int64_t ldy, int64_t m, int64_t n, int64_t k, void* workspace,
                 int64_t workspace_bytes, void* stream, int route, int act, int flags = 0,
                 const b2::GatherArgs* ga = nullptr) {
-    const bool h16 = (flags & B2_FLAG_FP16_STEPS) != 0;
+    const int steps = flags & B2_FLAG_FP16_STEPS ? b2::kStepsFp16 : flags & B2_FLAG_PLAIN_STEPS ? b2::kStepsPlain : b2::kStepsMixed;
     const void* bias = bias_fp16;
     if (bias && reinterpret_cast<uintptr_t>(bias) % 4) return fail(B2_ERR_ARGUMENT, "bias must be 4-byte aligned");
     if (m < 0) return fail(B2_ERR_ARGUMENT, "m must be non-negative");
@@ -1090,24 +1104,24 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
         if (!tile_applicable(m, d, tile_split))
             return fail(B2_ERR_UNSUPPORTED, "the tile route needs M <= 16 and a layer whose K range fits in shared memory");
         const bool xvec = (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (ldx % 8 == 0) && (d.k % 8 == 0);
-        return run_tile(x, ldx, native, y, ldy, m, d, workspace, xvec, static_cast<cudaStream_t>(stream), bias, act, dev.sm_count, h16,
+        return run_tile(x, ldx, native, y, ldy, m, d, workspace, xvec, static_cast<cudaStream_t>(stream), bias, act, dev.sm_count, steps,
                         (flags & B2_FLAG_OVERLAP_LAUNCH) != 0, ga);
     }
     if (route == B2_ROUTE_STREAM)
         return run_stream(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes,
-                          static_cast<cudaStream_t>(stream), dev, bias, act, h16, ga, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
+                          static_cast<cudaStream_t>(stream), dev, bias, act, steps, ga, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
     if (route == B2_ROUTE_TCGEN05) {
         if (!gemm_applicable(x, ldx, d))
             return fail(B2_ERR_UNSUPPORTED, "the tcgen05 route needs K % 8 == 0 and a 16-byte aligned x");
         if (workspace_bytes < B2_W4A16_TICKET_BYTES)
             return fail(B2_ERR_WORKSPACE, "workspace smaller than b2_w4a16_workspace_bytes()");
-        return run_gemm(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count, bias, act, h16);
+        return run_gemm(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count, bias, act, steps);
     }
     if (route == B2_ROUTE_BATCH) {
         if (!batch_applicable(m, d) || !gemm_applicable(x, ldx, d))
             return fail(B2_ERR_UNSUPPORTED, "the batch route needs M <= 128, K % 8 == 0 and a 16-byte aligned x");
         return run_batch(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count,
-                         bias, act, h16, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
+                         bias, act, steps, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
     }
     return fail(B2_ERR_UNSUPPORTED, "unknown route");
 }

@@ -22,9 +22,9 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
 
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
-template <int NX, bool H16>
+template <int NX, int STEPS>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
-    auto kernel = b2::w4a16_batch_kernel<NX, H16>;
+    auto kernel = b2::w4a16_batch_kernel<NX, STEPS>;
     constexpr int smem = b2::batch_smem_bytes(NX);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -75,12 +75,19 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     return p;
 }
 
-int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool h16, bool overlap, cudaStream_t s) {
+template <int NX>
+int launch_known(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, int steps, bool overlap, cudaStream_t s) {
+    if (steps == b2::kStepsFp16) return launch_one<NX, b2::kStepsFp16>(xmap, a, grid, overlap, s);
+    if (steps == b2::kStepsPlain) return launch_one<NX, b2::kStepsPlain>(xmap, a, grid, overlap, s);
+    return launch_one<NX, b2::kStepsMixed>(xmap, a, grid, overlap, s);
+}
+
+int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
     switch (p.nx) {
-        case 16: return h16 ? launch_one<16, true>(xmap, a, p.grid, overlap, s) : launch_one<16, false>(xmap, a, p.grid, overlap, s);
-        case 32: return h16 ? launch_one<32, true>(xmap, a, p.grid, overlap, s) : launch_one<32, false>(xmap, a, p.grid, overlap, s);
-        case 64: return h16 ? launch_one<64, true>(xmap, a, p.grid, overlap, s) : launch_one<64, false>(xmap, a, p.grid, overlap, s);
-        default: return h16 ? launch_one<128, true>(xmap, a, p.grid, overlap, s) : launch_one<128, false>(xmap, a, p.grid, overlap, s);
+        case 16: return launch_known<16>(xmap, a, p.grid, steps, overlap, s);
+        case 32: return launch_known<32>(xmap, a, p.grid, steps, overlap, s);
+        case 64: return launch_known<64>(xmap, a, p.grid, steps, overlap, s);
+        default: return launch_known<128>(xmap, a, p.grid, steps, overlap, s);
     }
 }
 

@@ -24,6 +24,6 @@ inline int64_t batch_workspace(int64_t m, const b2::Dims& d, int sm_count) {
 }
 
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count);
-int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool h16, bool overlap, cudaStream_t s);
+int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s);
 
 }  // namespace b2host

@@ -124,7 +124,7 @@ __device__ __forceinline__ void batch_sums(uint32_t taddr, float (&f)[CW]) {
 __device__ __forceinline__ int batch_begin(int steps, int ctas, int c) { return int(unsigned(steps) * unsigned(c) / unsigned(ctas)); }
 __device__ __forceinline__ int batch_owner(int s, int steps, int ctas) { return int((unsigned(s + 1) * unsigned(ctas) - 1u) / unsigned(steps)); }
 
-template <int NX, bool H16>
+template <int NX, int STEPS>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
     constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
@@ -407,7 +407,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             const uint32_t fields[2] = {*reinterpret_cast<const uint32_t*>(raw + step_at), *reinterpret_cast<const uint32_t*>(raw + step_at + 8)};
             const uint32_t zeros = *reinterpret_cast<const uint16_t*>(raw + zero_at) >> (4 * hi8);
             auto convert = [&](int h, auto chain) {
-                const auto gc = make_group<decltype(chain)::value>((zeros >> (8 * h)) & 15u, fields[h]);
+                const auto gc = make_group<decltype(chain)::value, STEPS == kStepsPlain>((zeros >> (8 * h)) & 15u, fields[h]);
                 const uint32_t words[8] = {code[2 * h].x, code[2 * h].y, code[2 * h].z, code[2 * h].w,
                                            code[2 * h + 1].x, code[2 * h + 1].y, code[2 * h + 1].z, code[2 * h + 1].w};
                 const uint32_t to = tmem_base + lane_addr + kWBase + slot * kWStage + (2 * v + h) * kBatchWCols;
@@ -423,8 +423,8 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             };
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                if constexpr (H16) convert(h, Chain<kChainFp16>{});
-                else if (all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
+                if constexpr (STEPS == kStepsFp16) convert(h, Chain<kChainFp16>{});
+                else if (STEPS == kStepsMixed && all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
                 else convert(h, Chain<kChainGeneral>{});
                 if (!ok) break;
             }

@@ -86,6 +86,16 @@ int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream) {
     return run_factor_steps(static_cast<uint8_t*>(native), d, nullptr, static_cast<cudaStream_t>(stream));
 }
 
+int b2_w4a16_image_flags(const void* native, int64_t n, int64_t k, unsigned* flags, void* stream) {
+    if (!native || !flags) return fail(B2_ERR_ARGUMENT, "null pointer");
+    if (int rc = check_dims(n, k)) return rc;
+    if (reinterpret_cast<uintptr_t>(native) % 4) return fail(B2_ERR_ARGUMENT, "misaligned native image");
+    const b2::Dims d = b2::make_dims(n, k);
+    const int64_t fields = int64_t(d.n16) * d.kb * 64;
+    b2::image_flags_kernel<<<unsigned((fields + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint8_t*>(native), d, flags);
+    return after_launch("image_flags_kernel");
+}
+
 int b2_w4a16_unrepack(const void* native, int64_t n, int64_t k, int32_t* packed, float* scales,
                       int32_t* zeros, void* stream) {
     if (!packed || !scales || !zeros || !native) return fail(B2_ERR_ARGUMENT, "null pointer");

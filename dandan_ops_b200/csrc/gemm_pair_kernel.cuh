@@ -135,7 +135,7 @@ __device__ __forceinline__ void tma_store_wait_read() {
 // TMA_Y: y is 16-byte aligned with a row stride that is a multiple of 16 bytes; the epilogue
 // then transposes through shared memory (the idle x ring) and stores each warp's 32 columns x
 // MT/2 rows with one TMA store.  Otherwise every thread stores its 2-byte results itself.
-template <int MT, bool TMA_Y, bool H16 = false>
+template <int MT, bool TMA_Y, int STEPS = kStepsMixed>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, PairShape<MT>::CTAS)
 w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap ymap, const GemmArgs a) {
     constexpr int XS = PairShape<MT>::XS, WS = PairShape<MT>::WS, RS = PairShape<MT>::RS;
@@ -282,15 +282,15 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_co
             const uint32_t words[8] = {code0.x, code0.y, code0.z, code0.w, code1.x, code1.y, code1.z, code1.w};
             uint32_t o[32];
             auto convert = [&](auto chain) {
-                const auto gc = make_group<decltype(chain)::value>(z, field);
+                const auto gc = make_group<decltype(chain)::value, STEPS == kStepsPlain>(z, field);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const uint4 q = dequant_word(words[i], gc);
                     o[4 * i] = q.x; o[4 * i + 1] = q.y; o[4 * i + 2] = q.z; o[4 * i + 3] = q.w;
                 }
             };
-            if constexpr (H16) convert(Chain<kChainFp16>{});
-            else if (all_factored(field)) convert(Chain<kChainFactored>{});
+            if constexpr (STEPS == kStepsFp16) convert(Chain<kChainFp16>{});
+            else if (STEPS == kStepsMixed && all_factored(field)) convert(Chain<kChainFactored>{});
             else convert(Chain<kChainGeneral>{});
             // the conversion happens in registers before the wait for the free tensor-memory stage
             if (s >= WS) ok = wait(DONE + (s - WS) % XS, ((s - WS) / XS) & 1);

@@ -102,7 +102,10 @@ __host__ __device__ inline uint32_t unpermute_word(uint32_t nat, int valid) {
     return out;
 }
 
-constexpr unsigned kQuantFactored = 4u;      // image flag: some group that exists has a factored field
+// Flags of a conversion and of an image.
+constexpr unsigned kQuantNonFinite = 1u;     // a weight is NaN or infinite
+constexpr unsigned kQuantStepNotFp16 = 2u;   // some step is not exactly representable in FP16
+constexpr unsigned kQuantFactored = 4u;      // some group that exists has a factored field
 
 constexpr uint32_t kFactored = 0x80000000u;
 __host__ __device__ constexpr uint32_t factored_field(uint32_t i, uint32_t a2_bits, int remainder) {

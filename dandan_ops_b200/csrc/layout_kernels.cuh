@@ -47,6 +47,24 @@ repack_kernel(const int32_t* __restrict__ packed, const float* __restrict__ scal
     }
 }
 
+// kQuant* bits of the steps of an image, a thread per field.
+__global__ void __launch_bounds__(256)
+image_flags_kernel(const uint8_t* __restrict__ native, Dims d, unsigned* flags) {
+    const int64_t idx = int64_t(blockIdx.x) * 256 + threadIdx.x, block = idx >> 6;
+    const int f = int(idx & 63);
+    unsigned found = 0;
+    if (block < int64_t(d.n16) * d.kb) {
+        const int kb = int(block / d.n16), nt = int(block - int64_t(kb) * d.n16);
+        if (nt * 16 + (f >> 3) + 8 * (f & 1) < d.n && kb * 4 + ((f >> 1) & 3) < d.groups) {
+            const uint32_t field = reinterpret_cast<const uint32_t*>(native + block * kBlockBytes + kStepOffset)[f];
+            const float s = field_step(field);
+            found = (int32_t(field) < 0 ? kQuantFactored : 0u) | (__half2float(__float2half_rn(s)) != s ? kQuantStepNotFp16 : 0u);
+        }
+    }
+    found = __reduce_or_sync(0xffffffffu, found);
+    if ((threadIdx.x & 31) == 0 && (found & ~*static_cast<volatile unsigned*>(flags))) atomicOr(flags, found);
+}
+
 // One thread per reference word / per (row, group) entry.
 __global__ void __launch_bounds__(256)
 unrepack_kernel(const uint8_t* __restrict__ native, Dims d, int32_t* __restrict__ packed,

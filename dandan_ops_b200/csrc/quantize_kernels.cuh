@@ -13,9 +13,6 @@
 
 namespace b2 {
 
-constexpr unsigned kQuantNonFinite = 1u;     // a weight is NaN or infinite
-constexpr unsigned kQuantStepNotFp16 = 2u;   // some step is not exactly representable in FP16
-
 struct QuantizeArgs {
     const void* weight;      // [N, K] contiguous
     uint8_t* codes;          // [N, K], may be null

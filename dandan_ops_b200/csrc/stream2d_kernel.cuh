@@ -38,7 +38,7 @@ struct Split2D {
     }
 };
 
-template <int MT, bool XVEC, bool H16>
+template <int MT, bool XVEC, int STEPS>
 __global__ void __launch_bounds__(16 * 32, 1)
 w4a16_stream2d_kernel(const StreamArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -150,7 +150,7 @@ w4a16_stream2d_kernel(const StreamArgs a) {
                 }
                 if (++stage == kStages) { stage = 0; parity ^= 1u; }
 
-                constexpr int CH = H16 ? kChainFp16 : kChainGeneral;
+                constexpr int CH = STEPS == kStepsFp16 ? kChainFp16 : kChainGeneral;
                 const GroupConst<CH> gg = make_group<CH>(zero & 15u, field.x), gh = make_group<CH>(zero >> 4, field.y);
                 const uint8_t* xchunk = (MT > 1 || g < xrows) ? xs + (jj * 4 + t) * kChunk + g * 144 : xzero;
 #pragma unroll

@@ -277,6 +277,12 @@ __device__ __forceinline__ uint32_t dequant_pair_odd(uint32_t h2, float c, uint6
 // general one.  Under the FP16-step flag there is nothing to choose: that chain takes a weight in as many instructions as the
 // factored one and both forms of a field, and without vote and branch 57344 x 8192 takes 57.9 instead of 59.9 us at M = 1,
 // 64.6 instead of 67.3 at M = 16 and 234 instead of 240 at M = 256.
+//
+// What the caller knows of a layer's step fields, as a template parameter of the kernels: nothing (a vote per block), that FP16 holds
+// every step (B2_FLAG_FP16_STEPS), or that none is factored (B2_FLAG_PLAIN_STEPS: weights whose steps lie outside the factored
+// range.  The vote, always lost, and a step that might be factored cost them 2 to 10 %: 24576 x 4096 at M = 1 / 8 / 16 / 64 23.0 / 24.5 /
+// 24.2 / 28.0 us, without 21.0 / 22.9 / 22.7 / 26.8, 57344 x 8192 at M = 8 82.9 and 75.8).
+enum : int { kStepsMixed = 0, kStepsFp16 = 1, kStepsPlain = 2 };
 enum : int { kChainGeneral = 0, kChainFp16 = 1, kChainFactored = 2 };
 template <int CH> struct Chain { static constexpr int value = CH; };
 template <int CH> struct GroupConst;
@@ -294,7 +300,8 @@ template <> struct GroupConst<kChainFactored> {
 };
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ bool all_factored(uint32_t field) { return __all_sync(0xffffffffu, int32_t(field) < 0); }
-template <int CH>
+// PLAIN: the field is known not to be factored.
+template <int CH, bool PLAIN = false>
 __device__ __forceinline__ GroupConst<CH> make_group(uint32_t z, uint32_t field) {
     GroupConst<CH> g;
     if constexpr (CH == kChainFactored) {
@@ -314,7 +321,7 @@ __device__ __forceinline__ GroupConst<CH> make_group(uint32_t z, uint32_t field)
         // -(1024 + z) and -(64 + z) as FP32 bit patterns: z sits in the mantissa, no int-to-float conversion
         g.c_even = __uint_as_float(0xC4800000u + z * 8192u);
         g.c_odd = __uint_as_float(0xC2800000u + z * 131072u);
-        g.s2 = twice(field_step(field));
+        g.s2 = twice(PLAIN ? __uint_as_float(field) : field_step(field));
     }
     return g;
 }
@@ -465,7 +472,7 @@ __device__ __forceinline__ int owner_of(int s, int steps, int ctas) {
 // XROWS (MT = 1 only): stage just the rows of x that exist.  The row count is then a run-time number in the
 // x addressing of every block (measured: 28 more instructions per block at M = 8, 13 fewer at M = 1, where most
 // lanes read the zero row), so batches of 5 to 8 rows use the compile-time layout of all 8 rows instead.
-template <int MT, bool XVEC, int W, bool H16, bool GATHER, bool XROWS>
+template <int MT, bool XVEC, int W, int STEPS, bool GATHER, bool XROWS>
 __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArgs* ga) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int MP = MT * 8;
@@ -592,11 +599,16 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
                 }
                 const uint8_t* slot = ring + stage * kBlockBytes;
                 // fields first: which chain follows is known before the codes arrive (57344 x 8192 at M = 1 62.1 -> 59.4 us)
-                const uint2 field = load_fields(slot + kStepOffset + lane * 8);
-                const bool factored = !H16 && all_factored(field.x & field.y);
+                uint2 field;
+                bool factored = false;
+                if constexpr (STEPS == kStepsMixed) {
+                    field = load_fields(slot + kStepOffset + lane * 8);
+                    factored = all_factored(field.x & field.y);
+                }
                 uint4 code[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) code[j] = *reinterpret_cast<const uint4*>(slot + j * 512 + lane * 16);
+                if constexpr (STEPS != kStepsMixed) field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
                 const uint32_t zero = slot[kZeroOffset + lane];
                 __syncwarp();                              // all lanes have read the slot
                 if (lane == 0 && fetch < wb1) {
@@ -606,9 +618,7 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
                 if (++stage == kStages) { stage = 0; parity ^= 1u; }
 
                 const uint8_t* xchunk = (MT > 1 || g < xrows) ? xs + ((kb - xorigin) * 4 + t) * kChunk + g * 144 : xzero;
-                auto multiply = [&](auto chain) {
-                    constexpr int CH = decltype(chain)::value;
-                    const GroupConst<CH> gg = make_group<CH>(zero & 15u, field.x), gh = make_group<CH>(zero >> 4, field.y);
+                auto multiply = [&](const auto& gg, const auto& gh) {
 #pragma unroll
                     for (int wi = 0; wi < 8; ++wi) {
                         const uint32_t wa = pick(code[wi >> 2], wi & 3);        // row g
@@ -628,9 +638,11 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
                         }
                     }
                 };
-                if constexpr (H16) multiply(Chain<kChainFp16>{});
-                else if (factored) multiply(Chain<kChainFactored>{});
-                else multiply(Chain<kChainGeneral>{});
+                const uint32_t zg = zero & 15u, zh = zero >> 4;
+                if constexpr (STEPS == kStepsFp16) multiply(make_group<kChainFp16>(zg, field.x), make_group<kChainFp16>(zh, field.y));
+                else if constexpr (STEPS == kStepsPlain) multiply(make_group<kChainGeneral, true>(zg, field.x), make_group<kChainGeneral, true>(zh, field.y));
+                else if (factored) multiply(make_group<kChainFactored>(zg, field.x), make_group<kChainFactored>(zh, field.y));
+                else multiply(make_group<kChainGeneral>(zg, field.x), make_group<kChainGeneral>(zh, field.y));
             }
         }
 
@@ -747,16 +759,16 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
     }
 }
 
-template <int MT, bool XVEC, int W, bool H16 = false, bool XROWS = false>
+template <int MT, bool XVEC, int W, int STEPS = kStepsMixed, bool XROWS = false>
 __global__ void __launch_bounds__(W * 32, (W == 16 ? B2_STREAM_CTAS16 : 4))
 w4a16_stream_kernel(const StreamArgs a) {
-    stream_body<MT, XVEC, W, H16, false, XROWS>(a, nullptr);
+    stream_body<MT, XVEC, W, STEPS, false, XROWS>(a, nullptr);
 }
 
-template <int MT, int W, bool H16, bool XROWS = false>
+template <int MT, int W, int STEPS, bool XROWS = false>
 __global__ void __launch_bounds__(W * 32, (W == 16 ? B2_STREAM_CTAS16 : 4))
 w4a16_stream_gather_kernel(const StreamArgs a, const GatherArgs ga) {
-    stream_body<MT, true, W, H16, true, XROWS>(a, &ga);
+    stream_body<MT, true, W, STEPS, true, XROWS>(a, &ga);
 }
 
 }  // namespace b2

@@ -115,7 +115,7 @@ __device__ __forceinline__ void tile_collect(const TileArgs& a, const GatherArgs
 // for a peer while others are still to be scheduled: the CTAs count themselves on the flag block's ticket
 // when their tile is out, and only the LAST one - by then every packet of this rank has left - collects the
 // packets the peers sent (bounded as everywhere) and publishes the epoch.
-template <int MT, bool XVEC, bool FULL, bool H16, bool GATHER>
+template <int MT, bool XVEC, bool FULL, int STEPS, bool GATHER>
 __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* ga) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int rows = FULL ? MT * 8 : a.m;
@@ -187,10 +187,11 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     auto with_chain = [&](const Unit& o, auto f) {
         auto go = [&](auto chain) {
             constexpr int CH = decltype(chain)::value;
-            f(make_group<CH>(o.zero & 15u, o.field.x), make_group<CH>(o.zero >> 4, o.field.y));
+            constexpr bool kPlain = STEPS == kStepsPlain;
+            f(make_group<CH, kPlain>(o.zero & 15u, o.field.x), make_group<CH, kPlain>(o.zero >> 4, o.field.y));
         };
-        if constexpr (H16) go(Chain<kChainFp16>{});
-        else if (all_factored(o.field.x & o.field.y)) go(Chain<kChainFactored>{});
+        if constexpr (STEPS == kStepsFp16) go(Chain<kChainFp16>{});
+        else if (STEPS == kStepsMixed && all_factored(o.field.x & o.field.y)) go(Chain<kChainFactored>{});
         else go(Chain<kChainGeneral>{});
     };
     // The weights are constant; x, the bias and y may belong to the previous kernel until it has completed.  With one row tile
@@ -380,16 +381,16 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     if constexpr (GATHER) tile_collect(a, ga);
 }
 
-template <int MT, bool XVEC, bool FULL, bool H16 = false>
+template <int MT, bool XVEC, bool FULL, int STEPS = kStepsMixed>
 __global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_kernel(const TileArgs a) {
-    tile_body<MT, XVEC, FULL, H16, false>(a, nullptr);
+    tile_body<MT, XVEC, FULL, STEPS, false>(a, nullptr);
 }
 
-template <int MT, bool FULL, bool H16>
+template <int MT, bool FULL, int STEPS>
 __global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_gather_kernel(const TileArgs a, const GatherArgs ga) {
-    tile_body<MT, true, FULL, H16, true>(a, &ga);
+    tile_body<MT, true, FULL, STEPS, true>(a, &ga);
 }
 
 }  // namespace b2

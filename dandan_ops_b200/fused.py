@@ -15,6 +15,9 @@ from . import ops as _ops
 from .quantized_linear import QuantizedLinear
 
 
+_GATE_UP_FLAGS = _native.FLAG_OVERLAP_LAUNCH | _native.FLAG_PLAIN_STEPS
+
+
 def _plain(x):
     """Whether the C++ operator library runs this call: an ordinary tensor outside autograd and functorch transforms
     (vmap, jvp: the operators have no rules for them, and the ctypes path refuses their wrappers, which have no storage),
@@ -136,9 +139,9 @@ class GateUpSilu(nn.Module):
         image = self.op._native_image()
         if _plain(x) and (x.shape[0] <= 1 or x.stride(0) >= self.in_features):
             return _ops.silu_mul_image(x, image, self.op.out_features, self.in_features, self.op._bias_fp16(),
-                                                             self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
+                                       self.op._image_flags & _GATE_UP_FLAGS)
         return _native.linear_silu_mul(x, image, self.op.out_features, self.in_features, bias=self.op._bias_fp16(),
-                                       flags=self.op._image_flags & _native.FLAG_OVERLAP_LAUNCH)
+                                       flags=self.op._image_flags & _GATE_UP_FLAGS)
 
     def unfuse(self):
         """The original (gate, up) layers, state bit-identical."""
@@ -192,8 +195,7 @@ class RmsNormLinear(nn.Module):
         residual = None if residual is None else residual.contiguous()
         if _plain(x) and (residual is None or _plain(residual)):
             return _ops.rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
-                                                            self.out_features, self.in_features, self.op._bias_fp16(),
-                                                            self.op._image_flags)
+                                      self.out_features, self.in_features, self.op._bias_fp16(), self.op._image_flags)
         return _native.rmsnorm_linear(x, residual, self.norm_weight, self.eps, self.op._native_image(),
                                       self.out_features, self.in_features, bias=self.op._bias_fp16(), flags=self.op._image_flags)
 

@@ -164,7 +164,7 @@ class QuantizedLinear(torch.nn.Module):
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
                 key = layer._state_key()
-                layer._set_image(image, key, not read_quantizer_flags(flags) & _native.QUANT_STEP_NOT_FP16)
+                layer._set_image(image, key, read_quantizer_flags(flags))
             return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)
@@ -249,11 +249,11 @@ class QuantizedLinear(torch.nn.Module):
         self._slice_flag = _native.FLAG_COLUMN_SLICE
         self._image_flags |= self._slice_flag
 
-    def _set_image(self, image, key, fp16_steps):
-        """Adopt an image of the state with this key that is complete in memory (its stream has been synchronized)."""
+    def _set_image(self, image, key, found):
+        """Adopt an image of the state with this key that is complete in memory (its stream has been synchronized); `found`: its
+        QUANT_* bits."""
         self._image, self._image_key = image, key
-        self._image_flags = ((_native.FLAG_FP16_STEPS if fp16_steps else 0)
-                             | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0) | self._slice_flag)
+        self._image_flags = _native.step_flags(found) | self._slice_flag
 
     def _native_image(self):
         key = self._state_key()
@@ -264,16 +264,16 @@ class QuantizedLinear(torch.nn.Module):
         return self._image
 
     def _layer_flags(self):
-        """Flags of the C ABI for this state.  FLAG_FP16_STEPS when every step is exactly representable in
+        """Flags of the C ABI for this layer's image.  FLAG_FP16_STEPS when every step is exactly representable in
         FP16 (checkpoints with FP16 scales): the decode kernels then use the FP16-only dequantization, which
-        is bit-identical for such steps; FLAG_OVERLAP_LAUNCH unless switched off (B2_W4A16_OVERLAP=0).  Reads the steps once (a host sync), only when an image is (re)built -
+        is bit-identical for such steps; FLAG_PLAIN_STEPS when none is factored; FLAG_OVERLAP_LAUNCH unless switched off
+        (B2_W4A16_OVERLAP=0).  Reads the image's steps once (a host sync), only when an image is (re)built -
         never on the per-token path - and not while a stream is being captured."""
         if not self.scales.is_cuda or torch.cuda.is_current_stream_capturing():
             return 0
-        flags = _native.FLAG_FP16_STEPS if bool((self.scales.half().float() == self.scales).all()) else 0
-        # The read above has synchronized the stream, so the image is complete in memory from here on: the
+        # The read synchronizes the stream, so the image is complete in memory from here on: the
         # decode kernel may start under the tail of whatever kernel precedes it (FLAG_OVERLAP_LAUNCH).
-        return flags | (_native.FLAG_OVERLAP_LAUNCH if _native.OVERLAP_LAUNCH else 0)
+        return _native.step_flags(_native.image_flags(self._image, self.out_features, self.in_features))
 
     def attach_native_image(self, image):
         """Use a prebuilt device image of THIS layer's state (e.g. from `checkpoint.ImageCache`)

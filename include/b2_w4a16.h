@@ -78,6 +78,9 @@ int b2_w4a16_repack(const int32_t* packed, const float* scales, const int32_t* z
  * so themselves; images that hold plain steps (files of earlier versions) are read by every kernel as they are. */
 int b2_w4a16_factor_steps(void* native, int64_t n, int64_t k, void* stream);
 
+/* ORs into *flags (device memory) what holds for the steps of an image: bit 1 and bit 2 as b2_w4a16_quantize(). */
+int b2_w4a16_image_flags(const void* native, int64_t n, int64_t k, unsigned* flags, void* stream);
+
 /* Native image -> reference layout (exact inverse of b2_w4a16_repack for steps without a sign; a group whose step is negative, which
  * no valid state has, comes back as the equal one with the absolute value of its step and 15 - code, 15 - zero; codes beyond K
  * in the last word come back as 0, as pack_int4 writes them). */
@@ -187,6 +190,9 @@ int b2_w4a16_linear_bias(const void* x, int64_t ldx, const void* native, const v
  * set on a layer with other steps it gives wrong weights.  No counterpart in the reference (its kernels
  * multiply in FP32 throughout, kernels/w4a16_small.cuh:39). */
 #define B2_FLAG_FP16_STEPS 1
+/* B2_FLAG_PLAIN_STEPS: the caller asserts that no group of the image has a factored step (bit 2 of b2_w4a16_image_flags()
+ * is clear: weights whose steps lie outside the factored range); the kernels then do not look.  Same bits. */
+#define B2_FLAG_PLAIN_STEPS 32
 /* B2_FLAG_OVERLAP_LAUNCH: the tile, streaming and batch kernels may start before the previous kernel of the
  * stream has finished (programmatic dependent launch).  As that kernel drains, CTAs of this one move in, set
  * up their barriers, request their weight blocks (the tile kernel all of them, the others the first ring) and
