@@ -777,10 +777,13 @@ inline GemmShape gemm_shape(int64_t m, int64_t n, int kb, int sms, bool pairs_ok
             if (forced_splits && sp != std::min(forced_splits, smax)) continue;
             g.splits = sp;
             const int64_t steps = int64_t((kb + sp - 1) / sp) * 4 + 10 + (sp > 1 ? 4 + 2 * sp : 0);
-            // The partial tiles of a K-split are written and read back: 94 units are a microsecond, in which 2.4 MB make that
-            // trip (4096 x 12288 at M = 1024 / 2048: three / two CTAs along K 92 / 169 us, all of K on 256 rows 77 / 154; 4096 x
-            // 4096 at M = 512: two CTAs 25, one 29).
-            const int64_t c = wave_cost(i, g, g.tiles(m, n) * sp) * steps + g.partial_bytes(m, n) / 26000;
+            // The partial tiles of a K-split are written and read back: 94 units are a microsecond, in which 4.9 MB make that
+            // trip.  The rate is the one with which the model chooses best on 65 problems of 1.5 to 235 M weights at 136 to 3072
+            // rows, all splits measured (0.5 % over the fastest in the mean; 1.8 % without this term, 1.4 and 0.9 % with
+            // half and 1.5 times the time for it; anything from 48000 to 60000 chooses the same): 4096 x 12288 at M = 1024
+            // three CTAs along K 103 us, one 86; 6144 x 4096 at M = 256 two 24.0, three 22.0; 8192 x 28672 at M = 2048 one
+            // 845, two 761.
+            const int64_t c = wave_cost(i, g, g.tiles(m, n) * sp) * steps + g.partial_bytes(m, n) / 52000;
             if (c < best_cost) { best_cost = c; best = g; }
         }
     }
