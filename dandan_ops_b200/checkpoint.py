@@ -92,6 +92,12 @@ def write_image_file(path, image_bytes, n, k):
 
 def read_image_file(path, n, k, expected_bytes):
     """uint8 numpy array of the image, or None when the file does not describe this layer."""
+    found = _read_image_file(path, n, k, expected_bytes)
+    return None if found is None else found[0]
+
+
+def _read_image_file(path, n, k, expected_bytes):
+    """(image bytes, layout) or None."""
     try:
         with open(path, "rb") as f:
             head = f.read(_HEADER.size)
@@ -106,7 +112,27 @@ def read_image_file(path, n, k, expected_bytes):
         return None
     if data.size != expected_bytes or zlib.crc32(data.tobytes()) != crc:      # truncated or damaged file: a miss
         return None
-    return data
+    return data, layout
+
+
+def _factored(data, n, k):
+    """Whether some group of an image (its bytes, on the host) has a factored step."""
+    rows, columns = -(-n // 16), -(-k // 256)
+    fields = data.view(np.int32).reshape(columns, rows, 584)[:, :, 512:576].reshape(columns, rows, 8, 4, 2)      # (g, t, h): row g + 8h, group t
+    factored = (fields < 0).transpose(1, 4, 2, 0, 3).reshape(rows * 16, columns * 4)
+    return bool(factored[:n, : -(-k // 64)].any())
+
+
+def _attach(layer, data, layout):
+    """Give `layer` the image of a file; the steps of a file of layout 1 are brought to the form that decodes fastest."""
+    n, k = layer.out_features, layer.in_features
+    image = _native.image_from_host(torch.from_numpy(data), layer.packed_weight.device)
+    if layout == 1:
+        _native.factor_steps(image, n, k)
+        factored = bool(_native.image_flags(image, n, k) & _native.QUANT_FACTORED)
+    else:
+        factored = _factored(data, n, k)
+    layer.attach_native_image(image, factored)
 
 
 class ImageCache:
@@ -144,13 +170,13 @@ class ImageCache:
                                 in_features=k, group_size=meta["group_size"], bias=None if bias is None else bias.to(device),
                                 backend=backend, defer_image=True)
         layer.set_extra_state(meta)
-        data = read_image_file(path, n, k, _native.native_bytes(n, k))
-        if data is None:
+        found = _read_image_file(path, n, k, _native.native_bytes(n, k))
+        if found is None:
             self.misses += 1
             write_image_file(path, layer._native_image().cpu().numpy(), n, k)
             return layer, False
         self.hits += 1
-        layer.attach_native_image(_native.image_from_host(torch.from_numpy(data), layer.packed_weight.device))
+        _attach(layer, *found)
         return layer, True
 
     def attach(self, layer):
@@ -159,11 +185,11 @@ class ImageCache:
             raise ValueError("the native image lives on a CUDA device")
         path = self.path_for(layer)
         nbytes = _native.native_bytes(layer.out_features, layer.in_features)
-        data = read_image_file(path, layer.out_features, layer.in_features, nbytes)
-        if data is None:
+        found = _read_image_file(path, layer.out_features, layer.in_features, nbytes)
+        if found is None:
             self.misses += 1
             self.store(layer)
             return False
         self.hits += 1
-        layer.attach_native_image(_native.image_from_host(torch.from_numpy(data), layer.packed_weight.device))
+        _attach(layer, *found)
         return True

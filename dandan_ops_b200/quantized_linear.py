@@ -275,15 +275,19 @@ class QuantizedLinear(torch.nn.Module):
         # decode kernel may start under the tail of whatever kernel precedes it (FLAG_OVERLAP_LAUNCH).
         return _native.step_flags(_native.image_flags(self._image, self.out_features, self.in_features))
 
-    def attach_native_image(self, image):
+    def attach_native_image(self, image, factored=True):
         """Use a prebuilt device image of THIS layer's state (e.g. from `checkpoint.ImageCache`)
-        instead of repacking.  The image is dropped again if the state tensors change."""
+        instead of repacking.  The image is dropped again if the state tensors change.  `factored=False` asserts that
+        none of its steps is factored (FLAG_PLAIN_STEPS)."""
         if image.dtype != torch.uint8 or image.device != self.packed_weight.device or \
                 image.numel() != _native.native_bytes(self.out_features, self.in_features):
             raise ValueError("not a native image of this layer")
         self._image = image
         self._image_key = self._state_key()
-        self._image_flags = self._layer_flags() | self._slice_flag
+        self._image_flags = self._slice_flag
+        if self.scales.is_cuda and not torch.cuda.is_current_stream_capturing():
+            fp16 = bool((self.scales.half().float() == self.scales).all())             # (synchronizes, as _layer_flags)
+            self._image_flags |= _native.step_flags((0 if fp16 else _native.QUANT_STEP_NOT_FP16) | (_native.QUANT_FACTORED if factored else 0))
 
     def _bias_fp16(self):
         """FP16 copy of the bias for the fused epilogue (derived, rebuilt when the bias changes)."""

@@ -20,8 +20,10 @@ def test_who_has_the_flag():
         again = ops.QuantizedLinear.from_state_dict(layer.state_dict())
         assert again._image_flags == layer._image_flags == layer._layer_flags()
         other = ops.QuantizedLinear(layer.packed_weight, layer.scales, layer.zeros, in_features=520, defer_image=True)
-        other.attach_native_image(layer._native_image())
+        other.attach_native_image(layer._native_image(), factored=not layer._image_flags & PLAIN)
         assert other._image_flags == layer._image_flags
+        other.attach_native_image(layer._native_image())     # (nothing said about its steps)
+        assert other._image_flags == layer._image_flags & ~PLAIN
     small.scales.mul_(100.0)                                 # the image and its flags are rebuilt
     small._native_image()
     assert not small._image_flags & PLAIN
