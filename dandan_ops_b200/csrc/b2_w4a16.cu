@@ -619,12 +619,16 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 //                11.3 against 11.8.  One line for both kinds of steps: the flag must not change a bit.  Not below 4096
 //                output columns, the usual width of a slice: there a plain layer, too, has the bits of the kernels that
 //                carry the all-gather.
-//                Up to 65536 blocks where K is 12288 or more: 4096 x 28672 at M = 1 / 8 22.9 / 22.5 -> 20.6 / 20.8, 6144 x 16384
-//                19.7 / 20.0 -> 17.4 / 17.7, 8192 x 28672 34.9 / 35.9 -> 34.7 / 34.8; 16384 x 8192 22.2 / 24.0 against 23.4 / 23.6.
-//   9..16        up to K = 3072 above 2304 blocks (8192 x 2048 at M = 16 9.5 -> 7.5, 6144 x 2048 8.1 -> 7.3, 12288 x 1024 7.4 -> 5.2,
-//                3072 x 3072 8.7 -> 6.6; 4096 x 2048 tile 5.0 against 6.3), else above 4096 (at 4096 x 4096, whose plan callers
-//                know as one CTA per tile, batch would be ahead, too: 10.3 against 7.4), wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7, 24576 x 4096 26.8 -> 22.5,
-//                57344 x 8192 90 -> 75; 57344 x 512 11.3 against 12.8
+//                Up to 65536 blocks where K is 12288 or more: 4096 x 28672 at M = 1 / 8 21.9 / 22.3 -> 20.7 / 20.9, 6144 x 16384
+//                19.1 / 19.9 -> 17.6 / 17.9, 8192 x 28672 34.9 / 36.0 -> 34.7 / 34.9 (with FP16 steps 21.0 / 21.5 -> 19.9 / 20.2, 18.4 /
+//                19.2 -> 16.8 / 17.0, 33.1 / 34.5 -> 33.0 / 33.3); 16384 x 8192 22.2 / 24.0 against 23.4 / 23.6.
+//   9..16        up to K = 3072 above 2304 blocks (8192 x 2048 at M = 16 9.5 -> 7.5, 6144 x 2048 8.1 -> 7.3, 12288 x 1024 7.4 ->
+//                5.2; 4096 x 2048 tile 5.0 against 6.3; on the line 3072 x 3072 stays with the tile kernel, 6.1 against 6.5 at M =
+//                9, 8.8 against 6.7 at M = 16), else above 4096, wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7,
+//                24576 x 4096 26.8 -> 22.5, 57344 x 8192 90 -> 75; 57344 x 512 11.3 against 12.8.  Longer K up to 4096 blocks
+//                keeps the tile kernel although batch would be ahead from K = 3329 on (M = 9 / 16: 4096 x 4096, whose plan
+//                callers know as one CTA per tile, 10.2 / 10.2 against 7.2 / 7.4, 4096 x 3840 10.2 / 10.0 against 7.6 / 7.8, 3072 x
+//                4096 9.7 / 10.0 against 7.2 / 7.4; 4096 x 3328 7.0 / 9.4 against 7.2 / 7.3).
 //   17..32       from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
 //                1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 8.4 / 8.7, 57344 x 8192 121 / 125 -> 78
 //                / 80; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4, 256 x 4096 6.2 / 6.2
