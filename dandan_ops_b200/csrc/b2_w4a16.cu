@@ -656,9 +656,9 @@ bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
     return reinterpret_cast<uintptr_t>(x) % 16 == 0 && ldx % 8 == 0 && d.k % 8 == 0;
 }
 
-template <int MA, int BN, bool VEC>
+template <int MA, int BN, bool VEC, int STEPS = b2::kStepsMixed>
 int launch_gemm_one(const CUtensorMap& map, const b2::GemmArgs& a, dim3 grid, cudaStream_t s) {
-    auto kernel = b2::w4a16_gemm_kernel<MA, BN, VEC>;
+    auto kernel = b2::w4a16_gemm_kernel<MA, BN, VEC, STEPS>;
     constexpr int smem = b2::gemm_smem_bytes(MA, BN);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -852,6 +852,10 @@ int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
     }
     const int ma = shape.ma, bn = shape.bn;
     const dim3 grid((d.n + bn - 1) / bn, unsigned((m + 128 * ma - 1) / (128 * ma)));
+    if (steps == b2::kStepsPlain && vec) {
+        if (ma == 1) return launch_gemm_one<1, 128, true, b2::kStepsPlain>(map, a, grid, s);
+        return bn == 128 ? launch_gemm_one<2, 128, true, b2::kStepsPlain>(map, a, grid, s) : launch_gemm_one<2, 192, true, b2::kStepsPlain>(map, a, grid, s);
+    }
     if (ma == 1) return vec ? launch_gemm_one<1, 128, true>(map, a, grid, s) : launch_gemm_one<1, 128, false>(map, a, grid, s);
     if (bn == 128) return vec ? launch_gemm_one<2, 128, true>(map, a, grid, s) : launch_gemm_one<2, 128, false>(map, a, grid, s);
     return vec ? launch_gemm_one<2, 192, true>(map, a, grid, s) : launch_gemm_one<2, 192, false>(map, a, grid, s);

@@ -142,7 +142,7 @@ __device__ __forceinline__ uint4 dequant_word(uint32_t w, const GroupConst<CH>& 
 
 // MA = accumulators of 128 rows of x each (1 or 2).  VEC: y rows may be written with
 // 16-byte stores (N % 8 == 0, ldy % 8 == 0, y 16-byte aligned).
-template <int MA, int BN, bool VEC>
+template <int MA, int BN, bool VEC, int STEPS = kStepsMixed>
 __global__ void __launch_bounds__(gemm_threads(BN), 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
     constexpr int kGemmBN = BN, kGemmRawStages = gemm_raw_stages(BN), kGemmRawBytes = gemm_raw_bytes(BN);
@@ -272,11 +272,11 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
             uint8_t* brow = stage_base + st * kStageBytes + r * 128;
             const uint32_t words[4] = {code.x, code.y, code.z, code.w};
             auto convert = [&](auto chain) {
-                const auto gc = make_group<decltype(chain)::value>(z, field);
+                const auto gc = make_group<decltype(chain)::value, STEPS == kStepsPlain>(z, field);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(brow + (((4 * h + i) ^ (r & 7)) << 4)) = dequant_word(words[i], gc);
             };
-            if (all_factored(field)) convert(Chain<kChainFactored>{});
+            if (STEPS != kStepsPlain && all_factored(field)) convert(Chain<kChainFactored>{});
             else convert(Chain<kChainGeneral>{});
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // generic-proxy stores -> MMA (async proxy)
             __syncwarp();
