@@ -17,6 +17,9 @@ def pytest_configure(config):
 def pytest_collection_modifyitems(config, items):
     import torch
 
+    # The first CPU exp() of a process gives other last bits about once in 750 processes when several threads enter it together (4 of
+    # 3000 fresh processes with torch alone, 0 of 6000 after this call).  Seeded inputs are compared by digest.
+    torch.exp(torch.zeros(64))
     if torch.cuda.is_available():
         return
     skip = pytest.mark.skip(reason="no CUDA device")
