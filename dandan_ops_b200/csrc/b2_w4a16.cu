@@ -887,6 +887,7 @@ int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t l
     a.ldy = ldy;
     a.m = int(m); a.n = d.n; a.n16 = d.n16; a.kb = d.kb;
     a.steps = p.steps;
+    a.cluster = p.cluster;
     a.act = act;
     a.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
     a.fault_block = g_fault_step.exchange(-1, std::memory_order_relaxed);

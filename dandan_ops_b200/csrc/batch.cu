@@ -22,10 +22,10 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
 
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
-template <int NX, int STEPS>
+template <int NX, int STEPS, bool CL>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
-    auto kernel = b2::w4a16_batch_kernel<NX, STEPS>;
-    constexpr int smem = b2::batch_smem_bytes(NX);
+    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, CL>;
+    constexpr int smem = b2::batch_smem_bytes(NX, CL);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -40,11 +40,20 @@ int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool o
     cfg.blockDim = dim3(b2::kBatchThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int count = 0;
+    if (CL) {
+        attr[count].id = cudaLaunchAttributeClusterDimension;
+        attr[count].val.clusterDim.x = unsigned(a.cluster); attr[count].val.clusterDim.y = 1; attr[count].val.clusterDim.z = 1;
+        ++count;
+    }
+    if (overlap) {
+        attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[count].val.programmaticStreamSerializationAllowed = 1;
+        ++count;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = unsigned(count);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xmap, a);
     if (e != cudaSuccess) return b2host::fail(B2_ERR_CUDA, std::string("w4a16_batch_kernel: ") + cudaGetErrorString(e));
     return b2host::after_launch("w4a16_batch_kernel");
@@ -54,14 +63,60 @@ int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool o
 
 namespace b2host {
 
+// Clusters of c CTAs of the kernel that the device runs at the same time (asked once per device and size; without a device, for
+// planning alone, those of a B200).
+int cluster_capacity(int c) {
+    static std::atomic<int> known[64][9];                    // 0 = not asked yet, else capacity + 1
+    static constexpr int kB200[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return kB200[c];
+    }
+    std::atomic<int>& at = known[dev][c];
+    if (const int v = at.load(std::memory_order_acquire)) return v - 1;
+    auto kernel = b2::w4a16_batch_kernel<16, b2::kStepsMixed, true>;
+    constexpr int smem = 232448;                             // (no form uses more)
+    int clusters = 0;
+    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    if (ok) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(c));
+        cfg.blockDim = dim3(b2::kBatchThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = unsigned(c); attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        ok = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess;
+    }
+    if (!ok) {
+        cudaGetLastError();                                  // clear the error of a failed query
+        clusters = 0;
+    }
+    at.store(clusters + 1, std::memory_order_release);
+    return clusters;
+}
+
+// Estimated time of a launch with c CTAs per tile (one: whole tiles, no sums to send) beyond its fixed start, in ns: the blocks of a
+// CTA, and, the more SMs a launch takes, the later the next one finds room to start under it.  Fitted to 33 layers of 512 x 1024
+// to 9216 x 4096 at 1 to 128 rows in chains of launches, all cluster sizes measured: off by 2 to 6 % (rms), the chosen size
+// 0.7 % slower than the fastest in the mean.
+int cluster_cost(int nx, int tiles, int kb, int c) {
+    const int block_ns = nx <= 32 ? 455 : nx == 64 ? 525 : 750, exchange_ns = nx == 16 ? 350 : nx == 32 ? 700 : nx == 64 ? 1100 : 1400;
+    const int blocks = (kb + c - 1) / c, ctas = tiles * c;
+    return blocks * block_ns + ctas * (2000 + 85 * blocks) / 148 + (c > 1 ? exchange_ns : 0);
+}
+
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     BatchPlan p;
     p.nx = b2::batch_nx(m);
+    p.cluster = 1;
     const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows, tsteps = d.kb * 4;
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);
-    // Either equal ranges over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle):
-    // 4096 x 4096 at M = 16 / 64: 148 CTAs 9.1 / 13.0 us, 4 per tile 7.3 / 10.9; 1024 x 2048 at M = 32: 85 CTAs 7.9 us, 24 CTAs 5.8.
+    // Either equal ranges over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle).
     const int sms = int(std::min<int64_t>(sm_count > 0 ? sm_count : 148, steps));
     int best_cost = launch_cost(p.nx, p.steps, tsteps, sms);
     p.grid = sms;
@@ -72,22 +127,41 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     const int64_t range = (steps + p.grid - 1) / p.grid;
     p.max_parts = p.grid % tiles == 0 ? p.grid / tiles : int(std::min<int64_t>(p.grid, (tsteps + range - 1) / range + 1));
     p.partial_bytes = b2::batch_partial_bytes(p.nx, p.grid);
+    // A layer whose tiles all find a cluster at the same time (74 of two CTAs on a B200) takes one, or one CTA, per tile: us with the
+    // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.2 / 7.0, 8.7 / 7.2, 11.5 / 9.4, 16.2 / 13.2; 4096 x 12288
+    // (four) 11.3 / 10.1, 11.7 / 10.3, 15.1 / 12.2, 22.1 / 16.9; 1024 x 2048 (six) 4.7 / 3.0, 5.2 / 3.4, 8.3 / 5.0, 12.6 / 7.7; 8192 x 8192 (two)
+    // 13.6 / 11.8, 14.2 / 12.0, 17.0 / 14.4, 23.2 / 20.4.  No cluster but whole tiles: 8192 x 1024 at M = 16 4.0 against 4.9.
+    if (tiles <= cluster_capacity(2)) {
+        int best = cluster_cost(p.nx, tiles, d.kb, 1), c = 1;
+        for (const int size : b2::kBatchClusters) {
+            if (d.kb < size || tiles > cluster_capacity(size)) continue;
+            const int cost = cluster_cost(p.nx, tiles, d.kb, size);
+            if (cost < best) { best = cost; c = size; }
+        }
+        p.cluster = p.max_parts = c;
+        p.grid = tiles * c;
+    }
     return p;
 }
 
+template <int NX, int STEPS>
+int launch_form(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool overlap, cudaStream_t s) {
+    return p.cluster > 1 ? launch_one<NX, STEPS, true>(xmap, a, p.grid, overlap, s) : launch_one<NX, STEPS, false>(xmap, a, p.grid, overlap, s);
+}
+
 template <int NX>
-int launch_known(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, int steps, bool overlap, cudaStream_t s) {
-    if (steps == b2::kStepsFp16) return launch_one<NX, b2::kStepsFp16>(xmap, a, grid, overlap, s);
-    if (steps == b2::kStepsPlain) return launch_one<NX, b2::kStepsPlain>(xmap, a, grid, overlap, s);
-    return launch_one<NX, b2::kStepsMixed>(xmap, a, grid, overlap, s);
+int launch_known(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
+    if (steps == b2::kStepsFp16) return launch_form<NX, b2::kStepsFp16>(p, xmap, a, overlap, s);
+    if (steps == b2::kStepsPlain) return launch_form<NX, b2::kStepsPlain>(p, xmap, a, overlap, s);
+    return launch_form<NX, b2::kStepsMixed>(p, xmap, a, overlap, s);
 }
 
 int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
     switch (p.nx) {
-        case 16: return launch_known<16>(xmap, a, p.grid, steps, overlap, s);
-        case 32: return launch_known<32>(xmap, a, p.grid, steps, overlap, s);
-        case 64: return launch_known<64>(xmap, a, p.grid, steps, overlap, s);
-        default: return launch_known<128>(xmap, a, p.grid, steps, overlap, s);
+        case 16: return launch_known<16>(p, xmap, a, steps, overlap, s);
+        case 32: return launch_known<32>(p, xmap, a, steps, overlap, s);
+        case 64: return launch_known<64>(p, xmap, a, steps, overlap, s);
+        default: return launch_known<128>(p, xmap, a, steps, overlap, s);
     }
 }
 

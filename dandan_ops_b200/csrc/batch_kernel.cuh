@@ -8,11 +8,15 @@
 //   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x; batch_chains(NX) of them, added on reading)
 //     += A[n][k] (weights, FP16, tensor memory, written by the converter warps) * B[m][k] (x, shared memory, TMA)
 //
-// Work split ("stream-K"): the layer is cut into steps = (tile of 128 weight rows) x (64 columns of K), numbered
-// tile by tile and dealt out in equal contiguous ranges to one persistent CTA per SM (a block of 256 columns that two
-// CTAs share is fetched and decoded by both, each multiplying its own steps).  A tile that several CTAs share is added up
-// by the last of them to arrive (a ticket per tile and warp, nobody waits), in CTA order, so the result does not depend
-// on which that is.
+// Work split, one of two forms (plan_batch() in batch.cu chooses):
+//   ranges    ("stream-K") The layer is cut into steps = (tile of 128 weight rows) x (64 columns of K), numbered tile by tile and
+//             dealt out in equal contiguous ranges to one persistent CTA per SM (a block of 256 columns that two CTAs share is
+//             fetched and decoded by both, each multiplying its own steps).  A tile that several CTAs share is added up by the
+//             last of them to arrive (a ticket per tile and warp, nobody waits), in CTA order, so the result does not depend on
+//             which that is.
+//   clusters  (CL) A cluster of CTAs per tile, each with an equal share of the blocks of K.  The sums meet in shared memory: of
+//             every four columns of D one CTA is the owner, to which the others send theirs (st.async, counted on its barrier) and
+//             which adds them in CTA order.  One trip between SMs instead of store, fence, ticket and load through L2.
 //
 // Roles (20 warps):
 //   warp 0      bulk copies of the raw blocks: one copy per 256 columns of K (8 native blocks, contiguous)
@@ -31,6 +35,7 @@
 //   full[b % R]           the x tiles (bytes) and the eight converter warps' weights of block b are in place
 //   done[b % R]           tcgen05.commit: the MMAs of block b have completed
 //   acc_full/acc_free[b]  accumulator b complete (commit) / read by all converter warps
+//   sums                  (CL) the other CTAs' sums have landed (bytes)
 #pragma once
 #include "gemm_kernel.cuh"
 
@@ -56,12 +61,23 @@ __host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; 
 __host__ __device__ constexpr int batch_chains(int nx) { return nx <= 32 ? 4 : 2; }
 __host__ __device__ constexpr int batch_accs(int nx) { return nx == 16 ? 2 : 1; }
 __host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
-__host__ __device__ constexpr int batch_raw_stages(int nx) {
-    const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx) * batch_x_bytes(nx)) / kBatchRawBytes;
+// Sums a CTA of a cluster receives: from every other one, of the units (four columns x 128 weight rows) that it owns.
+constexpr int kBatchUnitBytes = kBatchRows * 16;
+__host__ __device__ constexpr int batch_sums_bytes(int nx, int c) { return (c - 1) * ((nx / 4 + c - 1) / c) * kBatchUnitBytes; }
+// Cluster sizes in use; what they need beside the rings.  With 128 rows of x there is no room left, and the sums go to the x tiles
+// (which no CTA of the cluster may still be reading then, see `ready` in the kernel).
+constexpr int kBatchClusters[] = {2, 3, 4, 6, 8};
+__host__ __device__ constexpr int batch_sums_area(int nx, bool cl) {
+    int most = 0;
+    for (int c : kBatchClusters) most = batch_sums_bytes(nx, c) > most ? batch_sums_bytes(nx, c) : most;
+    return cl && nx <= 64 ? most : 0;
+}
+__host__ __device__ constexpr int batch_raw_stages(int nx, bool cl) {
+    const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx) * batch_x_bytes(nx) - batch_sums_area(nx, cl)) / kBatchRawBytes;
     return fit < 8 ? fit : 8;
 }
-__host__ __device__ constexpr int batch_smem_bytes(int nx) {
-    return 1024 + 4 * batch_ring(nx) * batch_x_bytes(nx) + batch_raw_stages(nx) * kBatchRawBytes + 512;
+__host__ __device__ constexpr int batch_smem_bytes(int nx, bool cl) {
+    return 1024 + 4 * batch_ring(nx) * batch_x_bytes(nx) + batch_raw_stages(nx, cl) * kBatchRawBytes + batch_sums_area(nx, cl) + 512;
 }
 // Bytes of all partial tiles of a launch: a CTA has at most two tiles that it shares.
 __host__ __device__ constexpr int64_t batch_partial_bytes(int nx, int grid) { return int64_t(grid) * 2 * nx * kBatchRows * 4; }
@@ -77,6 +93,7 @@ struct BatchArgs {
     int m, n;
     int n16, kb;
     int steps;              // tiles * kb * 4
+    int cluster;            // CTAs per tile (CL)
     int act;                // as StreamArgs::act
     int wait_limit;
     int fault_block;        // -1; a test passes b >= 0: CTA 0 arms the barrier of its b-th block but skips the copy
@@ -124,10 +141,20 @@ __device__ __forceinline__ void batch_sums(uint32_t taddr, float (&f)[CW]) {
 __device__ __forceinline__ int batch_begin(int steps, int ctas, int c) { return int(unsigned(steps) * unsigned(c) / unsigned(ctas)); }
 __device__ __forceinline__ int batch_owner(int s, int steps, int ctas) { return int((unsigned(s + 1) * unsigned(ctas) - 1u) / unsigned(steps)); }
 
-template <int NX, int STEPS>
+__device__ __forceinline__ uint32_t peer_address(uint32_t own, int rank) {                // the same place in another CTA of the cluster
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(own), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void send_sums(uint32_t to, float4 v, uint32_t barrier) {        // 16 bytes counted on the receiver's barrier
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(barrier) : "memory");
+}
+
+template <int NX, int STEPS, bool CL>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
-    constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
+    constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX, CL), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
     constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
     constexpr int C = batch_chains(NX), ACCS = batch_accs(NX);
     static_assert(ACCS * C * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
@@ -135,9 +162,10 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_base = smem;                                                // [R][4][kXBytes]
     uint8_t* raw_base = x_base + R * kXStage;                              // [RS][18688]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes);
+    uint8_t* sums = NX <= 64 ? raw_base + RS * kBatchRawBytes : x_base;    // (CL) [other CTA][unit of this one][weight row] x 4 columns
+    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes + batch_sums_area(NX, CL));
     constexpr int RAW_FULL = 0, RAW_FREE = RAW_FULL + RS, FULL = RAW_FREE + RS, DONE = FULL + R, ACC_FULL = DONE + R,
-                  ACC_FREE = ACC_FULL + 2, DRAIN = ACC_FREE + 2, NBARS = DRAIN + 1;
+                  ACC_FREE = ACC_FULL + 2, DRAIN = ACC_FREE + 2, SUMS = DRAIN + 1, NBARS = SUMS + 1;
     static_assert(NBARS * 8 + 8 <= 512, "barrier area");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
     volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -146,7 +174,16 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ctas = gridDim.x;
-    const int b0 = batch_begin(a.steps, ctas, blockIdx.x), nsteps = batch_begin(a.steps, ctas, blockIdx.x + 1) - b0;
+    const int rank = CL ? int(blockIdx.x) % a.cluster : 0;                 // (CL) of the CTA in its cluster
+    int b0, nsteps;                                                        // its range of steps
+    if constexpr (CL) {                                                    // whole blocks of one tile
+        const int k0 = rank * a.kb / a.cluster;
+        b0 = (int(blockIdx.x) / a.cluster * a.kb + k0) * 4;
+        nsteps = ((rank + 1) * a.kb / a.cluster - k0) * 4;
+    } else {
+        b0 = batch_begin(a.steps, ctas, blockIdx.x);
+        nsteps = batch_begin(a.steps, ctas, blockIdx.x + 1) - b0;
+    }
     const int tsteps = a.kb * 4;                                           // steps of a tile
     const int gb0 = b0 >> 2, nblocks = ((b0 + nsteps - 1) >> 2) - gb0 + 1; // blocks of 8 x 256 columns, tile by tile
 
@@ -176,17 +213,27 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + 8); mbar_init(bar(DONE + i), 1); }
             for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
             mbar_init(bar(DRAIN), 1);
+            if constexpr (CL) mbar_init(bar(SUMS), 1);
             *abort_flag = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if constexpr (CL) {
+                const int units = (a.m + 3) / 4;                           // in use; this CTA owns every a.cluster-th
+                mbar_expect_tx(bar(SUMS), uint32_t((a.cluster - 1) * ((units - rank + a.cluster - 1) / a.cluster) * kBatchUnitBytes));
+            }
         }
         __syncwarp();
     }
+    // Phases of the cluster barrier, the same in every thread: `ready` - the others may write to this CTA's `sums` - and
+    // `sent` - this thread writes to nobody any more; a CTA leaves only when all threads of its cluster have got that far.
+    auto cluster_arrive = [] { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); };
+    auto cluster_wait = [] { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); };
     if (warp == 3) tmem_alloc(smem_u32(tmem_slot), 512);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if constexpr (CL && NX <= 64) cluster_arrive();                        // `sums` has a place of its own: ready from the start
 
     // Bounded; the lanes of a warp go on or leave together.  As a programmatic dependent the kernel may have been held up by
     // the one before it, which can last longer than the limit (a gather that waits for its peers): a limit that has run
@@ -299,6 +346,29 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         bool ok = true;
         int read = 0;                                                      // tiles of the range that this warp has read
 
+        // The sums of this lane's weight row and the rows m0.. of x -> y.
+        auto emit = [&](int tile, int m0, const auto& f) {
+            constexpr int W = sizeof(f) / sizeof(float);
+            const int n = tile * kBatchRows + row;
+            if (a.act) {
+                // lanes l and l ^ 4 hold the gate and the up sum of one output column: the gate lane
+                // finishes the even rows of x, the up lane the odd ones
+                const int out = (n >> 4) * 8 + g;
+#pragma unroll
+                for (int i = 0; i < W; i += 2) {
+                    const float theirs = __shfl_xor_sync(0xffffffffu, hi8 ? f[i] : f[i + 1], 4);
+                    const float gate = hi8 ? theirs : f[i], up = hi8 ? f[i + 1] : theirs;
+                    const int m = m0 + i + hi8;
+                    if (m < a.m && (n | 8) < a.n)
+                        a.y[int64_t(m) * a.ldy + out] = silu_mul(finish_output(gate, a.bias, n & ~8), finish_output(up, a.bias, n | 8));
+                }
+            } else if (n < a.n) {
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    if (m0 + i < a.m) a.y[int64_t(m0 + i) * a.ldy + n] = finish_output(f[i], a.bias, n);
+            }
+        };
+
         auto epilogue = [&](int seg) {
             const int tile = tile0 + seg;                                  // (of the accumulator read here)
             if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // bias, tickets, partial tiles, y
@@ -338,7 +408,6 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 if (mine) __threadfence();
             }
             if (mine) {
-                const int n = tile * kBatchRows + row;
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
                     const int m0 = u * (NX / 4) + c0;
@@ -366,23 +435,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                                     }
                             }
                         }
-                        if (a.act) {
-                            // lanes l and l ^ 4 hold the gate and the up sum of one output column: the gate lane
-                            // finishes the even rows of x, the up lane the odd ones
-                            const int out = (n >> 4) * 8 + g;
-#pragma unroll
-                            for (int i = 0; i < CW; i += 2) {
-                                const float theirs = __shfl_xor_sync(0xffffffffu, hi8 ? f[i] : f[i + 1], 4);
-                                const float gate = hi8 ? theirs : f[i], up = hi8 ? f[i + 1] : theirs;
-                                const int m = m0 + i + hi8;
-                                if (m < a.m && (n | 8) < a.n)
-                                    a.y[int64_t(m) * a.ldy + out] = silu_mul(finish_output(gate, a.bias, n & ~8), finish_output(up, a.bias, n | 8));
-                            }
-                        } else if (n < a.n) {
-#pragma unroll
-                            for (int i = 0; i < CW; ++i)
-                                if (m0 + i < a.m) a.y[int64_t(m0 + i) * a.ldy + n] = finish_output(f[i], a.bias, n);
-                        }
+                        emit(tile, m0, f);
                     }
                 }
             }
@@ -390,6 +443,53 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(ACC_FREE + seg % ACCS));
+            }
+        };
+
+        // Clusters: unit U (columns 4U..4U + 3) belongs to CTA U % cluster, as its unit U / cluster.
+        auto exchange = [&] {
+            ok = ok && wait(ACC_FULL, 0);
+            if (ok) tcgen05_fence_after();
+            __syncwarp();
+            if constexpr (NX > 64) cluster_arrive();                       // all products of this CTA are done: nothing reads its x tiles
+            cluster_wait();
+            constexpr int kUnits = NX / 16;                                // of this warp
+            const int c = a.cluster, own_units = (NX / 4 + c - 1) / c, inverse = 65536 / c + 1;      // U / c for U < 32
+            const uint32_t lane_at = uint32_t(quad * 32 + lane) * 16, acc0 = tmem_base + lane_addr + u * (NX / 4);
+            if (ok)
+#pragma unroll
+                for (int c0 = 0; c0 < NX / 4; c0 += CW)
+                    if (u * (NX / 4) + c0 < a.m) {
+                        float f[CW];
+                        batch_sums<NX, CW>(acc0 + c0, f);
+#pragma unroll
+                        for (int q = 0; q < CW / 4; ++q) {
+                            const int U = u * kUnits + c0 / 4 + q, i = U * inverse >> 16, owner = U - i * c;
+                            if (owner == rank || 4 * U >= a.m) continue;
+                            const int from = rank < owner ? rank : rank - 1;
+                            send_sums(peer_address(smem_u32(sums) + (from * own_units + i) * kBatchUnitBytes + lane_at, owner),
+                                      make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]), peer_address(bar(SUMS), owner));
+                        }
+                    }
+            __syncwarp();
+            cluster_arrive();                                              // sent
+            if (!ok) return;
+            asm volatile("griddepcontrol.wait;" ::: "memory");             // bias, y
+            bool landed = false;
+#pragma unroll 1
+            for (int U = u * kUnits; U < (u + 1) * kUnits && 4 * U < a.m; ++U) {
+                const int i = U * inverse >> 16;
+                if (U - i * c != rank) continue;
+                if (!landed && !(ok = wait(SUMS, 0))) return;
+                landed = true;
+                float mine[4], f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                batch_sums<NX, 4>(acc0 + (U - u * kUnits) * 4, mine);
+                for (int q = 0; q < c; ++q) {                              // in CTA order
+                    float4 p = make_float4(mine[0], mine[1], mine[2], mine[3]);
+                    if (q != rank) p = *reinterpret_cast<const float4*>(sums + ((q < rank ? q : q - 1) * own_units + i) * kBatchUnitBytes + lane_at);
+                    f[0] += p.x; f[1] += p.y; f[2] += p.z; f[3] += p.w;
+                }
+                emit(tile0, 4 * U, f);
             }
         };
 
@@ -436,20 +536,35 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 mbar_arrive(bar(FULL + slot));
                 if (b + RS < nblocks) mbar_arrive(bar(RAW_FREE + r));      // the last copies are not waited for
             }
-            while (read < seg && ok) epilogue(read++);
-            if (!ok) break;
+            if constexpr (!CL) {
+                while (read < seg && ok) epilogue(read++);
+                if (!ok) break;
+            }
             left -= kBatchSets;
             if ((slot += kBatchSets) >= R) { slot -= R; free_parity ^= 1; }
             if ((r += kBatchSets) >= RS) { r -= RS; raw_parity ^= 1; }
         }
-        const int segs = (b0 + nsteps - 1) / tsteps - tile0 + 1;
-        while (read < segs && ok) epilogue(read++);
+        if constexpr (CL) {
+            exchange();
+        } else {
+            const int segs = (b0 + nsteps - 1) / tsteps - tile0 + 1;
+            while (read < segs && ok) epilogue(read++);
+        }
     }
     __syncwarp();
+    if constexpr (CL) {
+        if (warp < 4) {                                // (the converters have been through these)
+            if constexpr (NX > 64) cluster_arrive();
+            cluster_wait();
+            cluster_arrive();
+        }
+        cluster_wait();                                // nobody writes to this CTA any more
+    }
     tcgen05_fence_before();
     __syncthreads();
-    // After an abort x tiles may be on their way to stages whose barrier the converters never completed, which nothing
-    // can wait for: whoever gave up, all roles have stopped requesting, and the last loads get 0.1 ms to land.
+    // After an abort x tiles may be on their way to stages whose barrier the converters never completed, and sums of other CTAs
+    // to a place that this one does not wait for: whoever gave up, all roles have stopped requesting, and the last loads and
+    // stores get 0.1 ms to land.
     for (int p = 0; p < 64 && *abort_flag; ++p) __nanosleep(2000);
     if (warp == 3) {
         tcgen05_fence_after();

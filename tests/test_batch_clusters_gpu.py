@@ -1,0 +1,38 @@
+"""w4a16_batch_kernel with a cluster of CTAs per tile, whose sums meet in shared memory: every cluster size and number of
+rows of x at the edges of its units of four columns, with K that does not divide evenly and a last tile that is not whole."""
+import pytest
+import torch
+
+import dandan_ops_b200 as ops
+from dandan_ops_b200 import _native
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k,act", [
+    (1, 8192, 4096, False), (5, 6144, 4104, True), (4, 5120, 5120, False), (13, 4097, 5000, False), (16, 1024, 3080, True),
+    (17, 1000, 1544, False), (24, 5008, 5128, True), (32, 512, 8192, False), (33, 304, 2056, True), (61, 256, 8192, False),
+    (64, 6144, 2048, False), (65, 129, 8200, False), (100, 5001, 5128, False), (128, 1024, 2304, True), (126, 7680, 2056, False)])
+def test_against_64_bit_sums(m, n, k, act):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    layer = ops.QuantizedLinear.from_float((torch.randn(n, k, generator=g, device="cuda") * 0.02).half())
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    bias = torch.randn(n, generator=g, device="cuda").half()
+    image, flags = layer._native_image(), layer._image_flags
+    assert _native.plan(m, n, k)["k_splits"] > 1
+    y = _native.linear(x, image, n, k, route=_native.ROUTE_BATCH, flags=flags)
+    # FP32 sums of at most K products and one rounding to FP16 (2^-11); the tensor core truncates, which the floor covers
+    exact = x.double() @ layer.dequantize().half().double().t()
+    assert ((y.double() - exact).abs() <= 2.0 ** -10 * exact.abs() + 2e-4).all()
+    for _ in range(5):                                                       # neither timing nor the launch attribute shows
+        assert torch.equal(_native.linear(x, image, n, k, route=_native.ROUTE_BATCH, flags=flags), y)
+    assert torch.equal(_native.linear(x, image, n, k, route=_native.ROUTE_BATCH), y)
+    assert torch.equal(_native.linear(x, image, n, k, route=_native.ROUTE_BATCH, bias=bias), y + bias)
+    if act:                                                                  # the rows of the layer taken as gate/up pairs
+        lib, out = _native.load(), torch.zeros(m, n // 2, dtype=torch.float16, device="cuda")
+        ws = torch.zeros(int(lib.b2_w4a16_workspace_bytes(m, n, k)), dtype=torch.uint8, device="cuda")
+        if _native.plan(m, n, k)["route"] == "b200_batch":
+            assert lib.b2_w4a16_linear_silu_mul(x.data_ptr(), k, image.data_ptr(), None, out.data_ptr(), n // 2, m, n, k, ws.data_ptr(),
+                                                ws.numel(), torch.cuda.current_stream().cuda_stream) == 0
+            assert torch.equal(out, _native.silu_mul_pairs(y))
+    assert _native.status() == 0
