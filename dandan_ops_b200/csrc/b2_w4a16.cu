@@ -887,7 +887,13 @@ int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t l
     a.ldy = ldy;
     a.m = int(m); a.n = d.n; a.n16 = d.n16; a.kb = d.kb;
     a.steps = p.steps;
+    a.shared_tiles = p.shared_tiles;
+    a.whole = p.whole;
     a.cluster = p.cluster;
+    a.parts = p.parts;
+    const int share = p.cluster > 1 ? p.cluster : p.parts;
+    a.kb_each = d.kb / share;
+    a.kb_more = d.kb % share;
     a.act = act;
     a.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
     a.fault_block = g_fault_step.exchange(-1, std::memory_order_relaxed);

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <climits>
 
 #include "../../include/b2_w4a16.h"
 #include "batch.cuh"
@@ -20,11 +21,13 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
     return range * step_ns + (parts == 1 ? 0 : (aligned ? 1 : 2) * 1300 + parts * (200 + 7 * nx));
 }
 
+constexpr int kRangeBlocks = 11, kRangeBlocksCluster = 8;   // blocks of K that equal ranges must gain per SM to pay for their hand-over
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
-template <int NX, int STEPS, bool CL>
+template <int NX, int STEPS, int FORM>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
-    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, CL>;
+    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, FORM>;
+    constexpr bool CL = FORM == b2::kClusters;
     constexpr int smem = b2::batch_smem_bytes(NX, CL);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -75,7 +78,7 @@ int cluster_capacity(int c) {
     }
     std::atomic<int>& at = known[dev][c];
     if (const int v = at.load(std::memory_order_acquire)) return v - 1;
-    auto kernel = b2::w4a16_batch_kernel<16, b2::kStepsMixed, true>;
+    auto kernel = b2::w4a16_batch_kernel<16, b2::kStepsMixed, b2::kClusters>;
     constexpr int smem = 232448;                             // (no form uses more)
     int clusters = 0;
     bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
@@ -109,14 +112,24 @@ int cluster_cost(int nx, int tiles, int kb, int c) {
     return blocks * block_ns + ctas * (2000 + 85 * blocks) / 148 + (c > 1 ? exchange_ns : 0);
 }
 
+// Time that the tiles left over by whole rounds take, in ns, if each is shared by `parts` CTAs: their blocks, the slower the more
+// of the SMs are at it, and the trip of the partial sums.  Fitted to 54 layers of 149 to 592 tiles and K = 512 to 8192 at 16 to 128
+// rows, every number of CTAs measured: off by 5 % of a launch (rms), the chosen number 1 % slower than the fastest in the mean.
+int shared_cost(int nx, int tiles, int kb, int parts, int sms) {
+    const int alone_ns = nx <= 32 ? 290 : nx == 64 ? 350 : 670, crowd_ns = nx <= 32 ? 435 : nx == 64 ? 500 : 630;
+    const int share_ns = nx <= 32 ? 1400 : nx == 64 ? 2200 : 2600, part_ns = nx == 16 ? 0 : nx == 32 ? 30 : nx == 64 ? 110 : 270;
+    return (kb + parts - 1) / parts * (alone_ns + crowd_ns * tiles * parts / sms) + (parts > 1 ? share_ns + part_ns * parts : 0);
+}
+
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     BatchPlan p;
     p.nx = b2::batch_nx(m);
-    p.cluster = 1;
+    p.cluster = p.parts = 1;
+    p.whole = p.shared_tiles = 0;
     const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows, tsteps = d.kb * 4;
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);
-    // Either equal ranges over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle).
+    // Ranges: equal ones over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle).
     const int sms = int(std::min<int64_t>(sm_count > 0 ? sm_count : 148, steps));
     int best_cost = launch_cost(p.nx, p.steps, tsteps, sms);
     p.grid = sms;
@@ -127,26 +140,56 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     const int64_t range = (steps + p.grid - 1) / p.grid;
     p.max_parts = p.grid % tiles == 0 ? p.grid / tiles : int(std::min<int64_t>(p.grid, (tsteps + range - 1) / range + 1));
     p.partial_bytes = b2::batch_partial_bytes(p.nx, p.grid);
-    // A layer whose tiles all find a cluster at the same time (74 of two CTAs on a B200) takes one, or one CTA, per tile: us with the
-    // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.2 / 7.0, 8.7 / 7.2, 11.5 / 9.4, 16.2 / 13.2; 4096 x 12288
-    // (four) 11.3 / 10.1, 11.7 / 10.3, 15.1 / 12.2, 22.1 / 16.9; 1024 x 2048 (six) 4.7 / 3.0, 5.2 / 3.4, 8.3 / 5.0, 12.6 / 7.7; 8192 x 8192 (two)
-    // 13.6 / 11.8, 14.2 / 12.0, 17.0 / 14.4, 23.2 / 20.4.  No cluster but whole tiles: 8192 x 1024 at M = 16 4.0 against 4.9.
-    if (tiles <= cluster_capacity(2)) {
+    bool one_round = false;
+    if (tiles >= sms) {
+        // Rounds: 28672 x 1024 at M = 16 / 128 12.0 -> 8.3, 20.5 -> 13.7 us, 24576 x 4096 20.0 -> 18.1, 37.0 -> 34.5, 57344 x 8192 at M = 16
+        // 71.0 -> 67.9; a fifth less in the mean over the 54 layers of shared_cost(), at worst level.
+        p.grid = sms;
+        p.whole = tiles / sms;
+        p.shared_tiles = tiles % sms;
+        int best = INT_MAX;
+        for (int parts = 1; p.shared_tiles && parts <= std::min({kMaxPerTile, sms / p.shared_tiles, d.kb}); ++parts) {
+            const int cost = shared_cost(p.nx, p.shared_tiles, d.kb, parts, sms);
+            if (cost < best) { best = cost; p.parts = parts; }
+        }
+        p.max_parts = p.parts;
+    } else if (tiles <= cluster_capacity(2)) {
+        // A layer whose tiles all find a cluster at the same time (74 of two CTAs on a B200) takes one, or one CTA, per tile: us with the
+        // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.2 / 6.7, 8.7 / 7.0, 11.5 / 9.1, 16.2 / 13.1; 4096 x 12288
+        // (four) 11.3 / 9.9, 11.7 / 10.2, 15.1 / 11.9, 22.1 / 16.7; 1024 x 2048 (six) 4.7 / 3.0, 5.2 / 3.4, 8.3 / 5.0, 12.6 / 7.7; 8192 x 8192 (two)
+        // 13.6 / 11.8, 14.2 / 12.0, 17.0 / 14.4, 23.2 / 20.4.  One CTA: 8192 x 1024 at M = 16 4.0 against 4.9.
+        // Sizes above two leave a cluster free (5760 x 12288 with all 45 clusters of three at M = 16 14.3 -> 15.6).  Where so few CTAs per
+        // tile fit that many SMs idle, ranges over all of them win on the longest K: 6144 x 28672 at M = 16 26.8 against 31.2, 6144 x
+        // 12288 16.8 against 17.5; 7168 x 16384 23.2 against 21.6.
         int best = cluster_cost(p.nx, tiles, d.kb, 1), c = 1;
         for (const int size : b2::kBatchClusters) {
-            if (d.kb < size || tiles > cluster_capacity(size)) continue;
+            if (d.kb < size || tiles > cluster_capacity(size) - (size > 2 ? 1 : 0)) continue;
             const int cost = cluster_cost(p.nx, tiles, d.kb, size);
             if (cost < best) { best = cost; c = size; }
         }
-        p.cluster = p.max_parts = c;
-        p.grid = tiles * c;
+        if (((d.kb + c - 1) / c) * (sms - tiles * c) <= (c > 1 ? kRangeBlocksCluster : kRangeBlocks) * sms) {
+            p.cluster = p.max_parts = c;
+            p.grid = tiles * c;
+            one_round = c == 1;
+        }
+    } else {
+        // One whole tile per CTA as long as what the other SMs could have taken off them is little: ranges / whole tiles at M = 16, 76 x 128
+        // columns with K = 4096 14.1 / 12.1, 5120 15.2 / 15.5, 8192 18.5 / 20.2, 97 x 128 with 5120 15.3 / 13.7, 8192 20.5 / 20.8, 12288 26.3 / 28.9.
+        one_round = d.kb * (sms - tiles) <= kRangeBlocks * sms;
+    }
+    if (one_round) {
+        p.grid = tiles;
+        p.max_parts = 1;
+        p.whole = p.nx >= 64 || d.kb >= 8 ? 1 : 0;       // (as ranges of a tile each: 12416 x 1024 at M = 16 / 64 4.8 / 6.1, as a round 4.9 / 6.0)
     }
     return p;
 }
 
 template <int NX, int STEPS>
 int launch_form(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool overlap, cudaStream_t s) {
-    return p.cluster > 1 ? launch_one<NX, STEPS, true>(xmap, a, p.grid, overlap, s) : launch_one<NX, STEPS, false>(xmap, a, p.grid, overlap, s);
+    if (p.cluster > 1) return launch_one<NX, STEPS, b2::kClusters>(xmap, a, p.grid, overlap, s);
+    if (p.whole) return launch_one<NX, STEPS, b2::kRounds>(xmap, a, p.grid, overlap, s);
+    return launch_one<NX, STEPS, b2::kRanges>(xmap, a, p.grid, overlap, s);
 }
 
 template <int NX>

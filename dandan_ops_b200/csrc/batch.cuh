@@ -11,7 +11,10 @@ namespace b2host {
 struct BatchPlan {
     int nx;                // rows of x the accumulator holds: 16, 32, 64 or 128
     int steps;             // 64-column steps of all tiles
-    int cluster;           // CTAs of a cluster, which share a tile; 1: equal ranges of steps
+    int cluster;           // CTAs of a cluster, which share a tile; 1: ranges or rounds
+    int whole;             // tiles that every CTA takes by itself; 0: equal ranges of steps
+    int shared_tiles;      // the others, and the CTAs of each (rounds)
+    int parts;
     int grid;
     int max_parts;         // most CTAs that share a tile
     int64_t partial_bytes;

@@ -8,7 +8,7 @@
 //   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x; batch_chains(NX) of them, added on reading)
 //     += A[n][k] (weights, FP16, tensor memory, written by the converter warps) * B[m][k] (x, shared memory, TMA)
 //
-// Work split, one of two forms (plan_batch() in batch.cu chooses):
+// Work split, one of three forms (plan_batch() in batch.cu chooses):
 //   ranges    ("stream-K") The layer is cut into steps = (tile of 128 weight rows) x (64 columns of K), numbered tile by tile and
 //             dealt out in equal contiguous ranges to one persistent CTA per SM (a block of 256 columns that two CTAs share is
 //             fetched and decoded by both, each multiplying its own steps).  A tile that several CTAs share is added up by the
@@ -17,6 +17,10 @@
 //   clusters  (CL) A cluster of CTAs per tile, each with an equal share of the blocks of K.  The sums meet in shared memory: of
 //             every four columns of D one CTA is the owner, to which the others send theirs (st.async, counted on its barrier) and
 //             which adds them in CTA order.  One trip between SMs instead of store, fence, ticket and load through L2.
+//   rounds    More tiles than CTAs: every CTA takes the same number of whole tiles, all CTAs the same columns of K at a time, which
+//             streams faster than ranges that begin anywhere.  The tiles left over are shared, each by as many CTAs with an
+//             equal share of K as there are, and come first: their sums travel (as those of ranges do) under the products of
+//             the whole tiles, and the launch ends with plain stores.
 //
 // Roles (20 warps):
 //   warp 0      bulk copies of the raw blocks: one copy per 256 columns of K (8 native blocks, contiguous)
@@ -92,8 +96,10 @@ struct BatchArgs {
     int64_t ldy;
     int m, n;
     int n16, kb;
-    int steps;              // tiles * kb * 4
-    int cluster;            // CTAs per tile (CL)
+    int steps;              // tiles * kb * 4 (ranges)
+    int shared_tiles, whole;    // tiles that several CTAs share, and that every CTA takes by itself (rounds)
+    int cluster, parts;     // CTAs per tile (clusters), per shared tile (rounds); their blocks of K: kb_each, the first kb_more of them one more
+    int kb_each, kb_more;
     int act;                // as StreamArgs::act
     int wait_limit;
     int fault_block;        // -1; a test passes b >= 0: CTA 0 arms the barrier of its b-th block but skips the copy
@@ -151,9 +157,12 @@ __device__ __forceinline__ void send_sums(uint32_t to, float4 v, uint32_t barrie
                  ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(barrier) : "memory");
 }
 
-template <int NX, int STEPS, bool CL>
+enum : int { kRanges = 0, kClusters = 1, kRounds = 2 };
+
+template <int NX, int STEPS, int FORM>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
+    constexpr bool CL = FORM == kClusters;
     constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX, CL), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
     constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
     constexpr int C = batch_chains(NX), ACCS = batch_accs(NX);
@@ -174,18 +183,43 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ctas = gridDim.x;
-    const int rank = CL ? int(blockIdx.x) % a.cluster : 0;                 // (CL) of the CTA in its cluster
-    int b0, nsteps;                                                        // its range of steps
-    if constexpr (CL) {                                                    // whole blocks of one tile
-        const int k0 = rank * a.kb / a.cluster;
-        b0 = (int(blockIdx.x) / a.cluster * a.kb + k0) * 4;
-        nsteps = ((rank + 1) * a.kb / a.cluster - k0) * 4;
+    const int tsteps = a.kb * 4;                                           // steps of a tile
+    int rank = 0, tile0, kb0, b0 = 0, nsteps = 0, nblocks;                 // first tile and block; range of steps; blocks of 8 x 256 columns
+    int nshared = 0;                                                       // (rounds) blocks of a shared tile, before the whole ones
+    if constexpr (CL) {                                                    // whole blocks of one tile, without a division
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%clusterid.x;" : "=r"(tile0));
+        kb0 = rank * a.kb_each + min(rank, a.kb_more);
+        nblocks = a.kb_each + (rank < a.kb_more ? 1 : 0);
+    } else if constexpr (FORM == kRounds) {
+        tile0 = int(blockIdx.x) / a.parts;
+        rank = int(blockIdx.x) - tile0 * a.parts;
+        kb0 = rank * a.kb_each + min(rank, a.kb_more);
+        if (tile0 < a.shared_tiles) {
+            nshared = a.kb_each + (rank < a.kb_more ? 1 : 0);
+        } else {
+            tile0 = a.shared_tiles + int(blockIdx.x);
+            kb0 = 0;
+        }
+        nblocks = nshared + a.whole * a.kb;
     } else {
         b0 = batch_begin(a.steps, ctas, blockIdx.x);
         nsteps = batch_begin(a.steps, ctas, blockIdx.x + 1) - b0;
+        nblocks = ((b0 + nsteps - 1) >> 2) - (b0 >> 2) + 1;
+        tile0 = (b0 >> 2) / a.kb;
+        kb0 = (b0 >> 2) - tile0 * a.kb;
     }
-    const int tsteps = a.kb * 4;                                           // steps of a tile
-    const int gb0 = b0 >> 2, nblocks = ((b0 + nsteps - 1) >> 2) - gb0 + 1; // blocks of 8 x 256 columns, tile by tile
+    int tile = tile0, kb = kb0;                                            // (warps 0 and 2: of the block at hand)
+    auto next_block = [&](int b) {                                         // from block b - 1 to b
+        if (FORM == kRounds && b == nshared) {
+            tile = a.shared_tiles + int(blockIdx.x);
+            kb = 0;
+        } else if (++kb == a.kb) {
+            kb = 0;
+            tile += FORM == kRounds ? ctas : 1;
+        }
+    };
+    const int first_end = FORM == kRounds && nshared ? nshared : a.kb - kb0;                // blocks up to the end of the first tile
 
     auto request = [&](int b, int tile, int kb) {                           // block b of the range
         const int r = b % RS;
@@ -197,25 +231,23 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     };
     // The first blocks are on their way before anything else happens: their trip is the longest part of the start.  (Not a
     // whole ring of them: x would queue up behind all CTAs' rings.)
-    int tile = gb0 / a.kb, kb = gb0 - tile * a.kb, issued = 0;             // (warp 0: next block to request)
+    int issued = 0;                                                        // (warp 0: next block to request)
     if (warp == 0) {
-        if (elect_one()) {
-            for (int i = 0; i < RS; ++i) mbar_init(bar(RAW_FULL + i), 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
+        static_assert(RS <= 32 && NBARS - RS <= 32, "a lane per barrier");
+        if (lane < RS) mbar_init(bar(RAW_FULL + lane), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
         for (; issued < min(kBatchEarly, nblocks); ++issued) {
             if (elect_one()) request(issued, tile, kb);
             __syncwarp();
-            if (++kb == a.kb) { kb = 0; ++tile; }
+            next_block(issued + 1);
         }
+        if (const int i = RAW_FREE + lane; i < NBARS)
+            mbar_init(bar(i), i < FULL ? 8 : i < DONE ? 1 + 8 : i >= ACC_FREE && i < DRAIN ? kBatchWarps : 1);
+        if (lane == 0) *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
         if (elect_one()) {
-            for (int i = 0; i < RS; ++i) mbar_init(bar(RAW_FREE + i), 8);
-            for (int i = 0; i < R; ++i) { mbar_init(bar(FULL + i), 1 + 8); mbar_init(bar(DONE + i), 1); }
-            for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), kBatchWarps); }
-            mbar_init(bar(DRAIN), 1);
-            if constexpr (CL) mbar_init(bar(SUMS), 1);
-            *abort_flag = 0;
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             if constexpr (CL) {
                 const int units = (a.m + 3) / 4;                           // in use; this CTA owns every a.cluster-th
                 mbar_expect_tx(bar(SUMS), uint32_t((a.cluster - 1) * ((units - rank + a.cluster - 1) / a.cluster) * kBatchUnitBytes));
@@ -223,6 +255,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         }
         __syncwarp();
     }
+    if (warp == 2 && elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
     // Phases of the cluster barrier, the same in every thread: `ready` - the others may write to this CTA's `sums` - and
     // `sent` - this thread writes to nobody any more; a CTA leaves only when all threads of its cluster have got that far.
     auto cluster_arrive = [] { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); };
@@ -262,7 +295,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             if (issued >= RS && !wait(RAW_FREE + r, ((issued / RS) - 1) & 1)) break;
             if (elect_one()) request(issued, tile, kb);
             __syncwarp();
-            if (++kb == a.kb) { kb = 0; ++tile; }
+            next_block(issued + 1);
         }
         // after an abort: the last copies land before the shared memory is released
         for (int i = max(0, issued - RS); i < issued; ++i)
@@ -272,7 +305,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         // D = F32, A = B = F16, both K-major, M = 128 weight rows, N = NX rows of x
         const uint32_t idesc = (1u << 4) | (uint32_t(NX >> 3) << 17) | (uint32_t(kBatchRows >> 4) << 24);
         const uint64_t desc0 = umma_desc_sw128(smem_u32(x_base));
-        int left = a.kb - gb0 % a.kb;                 // blocks to the end of the tile
+        int left = first_end;                         // blocks to the end of the tile
         int seg = 0;
         bool fresh = true;                            // the accumulator starts with this block
         bool ok = true;
@@ -293,7 +326,8 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                                     kk < C ? accumulate : 1u);
                     accumulate = 1;
                 };
-                const int t0 = b == 0 ? b0 & 3 : 0, t1 = b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;     // steps of the range in this block
+                const int t0 = FORM == kRanges && b == 0 ? b0 & 3 : 0;                                      // steps of the range in this block
+                const int t1 = FORM == kRanges && b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
                 if (t0 == 0 && t1 == 3) {
 #pragma unroll
                     for (int t = 0; t < 4; ++t) step(t);
@@ -319,18 +353,17 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     } else if (warp == 2) {
         // ------------------------------ x tiles ------------------------------------------
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        kb = gb0 % a.kb;
         for (int b = 0; b < nblocks; ++b) {
             const int slot = b % R;
             if (b >= R && !wait(DONE + slot, ((b / R) - 1) & 1)) break;
             if (elect_one()) {
-                const int t0 = b == 0 ? b0 & 3 : 0, t1 = b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
+                const int t0 = FORM == kRanges && b == 0 ? b0 & 3 : 0, t1 = FORM == kRanges && b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
                 mbar_expect_tx(bar(FULL + slot), uint32_t(t1 - t0 + 1) * kXBytes);
                 for (int t = t0; t <= t1; ++t)
                     tma_load_2d(smem_u32(x_base + slot * kXStage + t * kXBytes), &xmap, (kb * 4 + t) * kGemmBK, 0, bar(FULL + slot));
             }
             __syncwarp();
-            if (++kb == a.kb) kb = 0;
+            next_block(b + 1);
         }
     } else if (warp >= 4) {
         // ------------------------------ converters ---------------------------------------
@@ -341,7 +374,6 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         const int code_at = (quad * 2 + blk) * kBlockBytes + (2 * hi8) * 512 + (4 * g + 2 * v) * 16;
         const int step_at = (quad * 2 + blk) * kBlockBytes + kStepOffset + (4 * g + 2 * v) * 8 + hi8 * 4;
         const int zero_at = (quad * 2 + blk) * kBlockBytes + kZeroOffset + 4 * g + 2 * v;
-        const int tile0 = b0 / tsteps;
         constexpr int CW = NX >= 64 ? 16 : NX / 4;                         // accumulator columns per read
         bool ok = true;
         int read = 0;                                                      // tiles of the range that this warp has read
@@ -369,21 +401,88 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             }
         };
 
+        // A tile that other CTAs share, in three steps: partial sums out, ticket drawn, and, if it was the last, all sums read back.
+        // Rounds take a block of the next tile between them, so that none waits for the one before.
+        int pending = 0, shared_tile = 0, first = 0, last = 0;              // steps done, of which tile, and its CTAs
+        unsigned prior = 0;
+        auto slot_of = [&](int c) {                                        // partial tile of CTA c, this warp's columns and lanes
+            return a.partial + ((int64_t(c) * 2 + (c == first ? 1 : 0)) * (NX / 4) + u * (NX / 16)) * kBatchRows + quad * 32 + lane;
+        };
+        auto draw_ticket = [&] {
+            __threadfence();
+            __syncwarp();
+            unsigned* ticket = a.tickets + first * kBatchWarps + (warp - 4);
+            if (lane == 0) {
+                prior = atomicAdd(ticket, 1u);
+                if (prior == unsigned(last - first)) *ticket = 0u;
+            }
+            pending = 2;
+        };
+        auto read_back = [&] {
+            pending = 0;
+            if (__shfl_sync(0xffffffffu, prior, 0) != unsigned(last - first)) return;
+            __threadfence();
+            constexpr int RW = CW < 8 ? CW : 8, PARTS = 32 / RW;           // partial tiles requested together, added in CTA order
+#pragma unroll 1
+            for (int c0 = 0; c0 < NX / 4; c0 += RW) {
+                const int m0 = u * (NX / 4) + c0;
+                if (m0 >= a.m) break;
+                float f[RW];
+#pragma unroll
+                for (int i = 0; i < RW; ++i) f[i] = 0.0f;
+                for (int c = first; c <= last; c += PARTS) {
+                    float4 p[PARTS][RW / 4];
+#pragma unroll
+                    for (int j = 0; j < PARTS; ++j)
+#pragma unroll
+                        for (int q = 0; q < RW / 4; ++q)
+                            if (c + j <= last && m0 + 4 * q < a.m) p[j][q] = __ldcg(slot_of(c + j) + (c0 / 4 + q) * kBatchRows);
+                            else p[j][q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                    for (int j = 0; j < PARTS; ++j)
+#pragma unroll
+                        for (int q = 0; q < RW / 4; ++q) {
+                            f[4 * q] += p[j][q].x; f[4 * q + 1] += p[j][q].y; f[4 * q + 2] += p[j][q].z; f[4 * q + 3] += p[j][q].w;
+                        }
+                }
+                emit(shared_tile, m0, f);
+            }
+        };
+        auto advance = [&] {
+            if (pending == 1) draw_ticket();
+            else if (pending == 2) read_back();
+        };
         auto epilogue = [&](int seg) {
-            const int tile = tile0 + seg;                                  // (of the accumulator read here)
+            const int tile = FORM == kRounds ? (seg == 0 ? tile0 : a.shared_tiles + int(blockIdx.x) + (seg - (nshared ? 1 : 0)) * ctas) : tile0 + seg;
             if (seg == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // bias, tickets, partial tiles, y
             ok = ok && wait(ACC_FULL + seg % ACCS, (seg / ACCS) & 1);
             if (!ok) return;
             tcgen05_fence_after();
-            const int t0 = tile * tsteps, t1 = t0 + tsteps;
-            const bool whole = b0 <= t0 && t1 <= b0 + nsteps;
-            const int first = whole ? 0 : batch_owner(t0, a.steps, ctas), last = whole ? 0 : batch_owner(t1 - 1, a.steps, ctas);
+            bool whole;
+            if constexpr (FORM == kRounds) {
+                whole = seg > 0 || nshared == 0 || a.parts == 1;
+                if (!whole) {                                              // (a whole tile may be read while a shared one is pending)
+                    first = tile * a.parts;
+                    last = first + a.parts - 1;
+                }
+            } else {
+                const int t0 = tile * tsteps, t1 = t0 + tsteps;
+                whole = b0 <= t0 && t1 <= b0 + nsteps;
+                first = whole ? 0 : batch_owner(t0, a.steps, ctas);
+                last = whole ? 0 : batch_owner(t1 - 1, a.steps, ctas);
+            }
             const uint32_t acc = tmem_base + lane_addr + seg % ACCS * (C * NX) + u * (NX / 4);
-            auto slot_of = [&](int c) {                                    // partial tile of CTA c, this warp's columns and lanes
-                return a.partial + ((int64_t(c) * 2 + (c == first ? 1 : 0)) * (NX / 4) + u * (NX / 16)) * kBatchRows + quad * 32 + lane;
-            };
-            bool mine = whole;
-            if (!whole) {
+            if (whole) {
+#pragma unroll
+                for (int c0 = 0; c0 < NX / 4; c0 += CW) {
+                    const int m0 = u * (NX / 4) + c0;
+                    if (m0 < a.m) {
+                        float f[CW];
+                        batch_sums<NX, CW>(acc + c0, f);
+                        emit(tile, m0, f);
+                    }
+                }
+            } else {
                 float4* dst = slot_of(int(blockIdx.x));
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
@@ -394,55 +493,15 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                         if (u * (NX / 4) + c0 + 4 * q < a.m)
                             __stcg(dst + (c0 / 4 + q) * kBatchRows, make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]));
                 }
-                tcgen05_fence_before();
-                __threadfence();
-                __syncwarp();
-                unsigned prior = 0;
-                unsigned* ticket = a.tickets + first * kBatchWarps + (warp - 4);
-                if (lane == 0) {
-                    mbar_arrive(bar(ACC_FREE + seg % ACCS));
-                    prior = atomicAdd(ticket, 1u);
-                    if (prior == unsigned(last - first)) *ticket = 0u;
-                }
-                mine = __shfl_sync(0xffffffffu, prior, 0) == unsigned(last - first);
-                if (mine) __threadfence();
+                pending = 1;
+                shared_tile = tile;
             }
-            if (mine) {
-#pragma unroll
-                for (int c0 = 0; c0 < NX / 4; c0 += CW) {
-                    const int m0 = u * (NX / 4) + c0;
-                    if (m0 < a.m) {
-                        float f[CW];
-                        if (whole) {
-                            batch_sums<NX, CW>(acc + c0, f);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < CW; ++i) f[i] = 0.0f;
-                            constexpr int PARTS = 32 / CW;                 // partial tiles requested together, added in CTA order
-                            for (int c = first; c <= last; c += PARTS) {
-                                float4 p[PARTS][CW / 4];
-#pragma unroll
-                                for (int j = 0; j < PARTS; ++j)
-#pragma unroll
-                                    for (int q = 0; q < CW / 4; ++q)
-                                        if (c + j <= last && m0 + 4 * q < a.m) p[j][q] = __ldcg(slot_of(c + j) + (c0 / 4 + q) * kBatchRows);
-                                        else p[j][q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-                                for (int j = 0; j < PARTS; ++j)
-#pragma unroll
-                                    for (int q = 0; q < CW / 4; ++q) {
-                                        f[4 * q] += p[j][q].x; f[4 * q + 1] += p[j][q].y; f[4 * q + 2] += p[j][q].z; f[4 * q + 3] += p[j][q].w;
-                                    }
-                            }
-                        }
-                        emit(tile, m0, f);
-                    }
-                }
-            }
-            if (whole) {
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(ACC_FREE + seg % ACCS));
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(ACC_FREE + seg % ACCS));
+            if (FORM == kRanges && !whole) {
+                draw_ticket();
+                read_back();
             }
         };
 
@@ -456,99 +515,102 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             constexpr int kUnits = NX / 16;                                // of this warp
             const int c = a.cluster, own_units = (NX / 4 + c - 1) / c, inverse = 65536 / c + 1;      // U / c for U < 32
             const uint32_t lane_at = uint32_t(quad * 32 + lane) * 16, acc0 = tmem_base + lane_addr + u * (NX / 4);
-            if (ok)
+            float f[NX / 4];
+            if (ok) {
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW)
                     if (u * (NX / 4) + c0 < a.m) {
-                        float f[CW];
-                        batch_sums<NX, CW>(acc0 + c0, f);
+                        float (&mine)[CW] = *reinterpret_cast<float (*)[CW]>(f + c0);
+                        batch_sums<NX, CW>(acc0 + c0, mine);
 #pragma unroll
                         for (int q = 0; q < CW / 4; ++q) {
                             const int U = u * kUnits + c0 / 4 + q, i = U * inverse >> 16, owner = U - i * c;
                             if (owner == rank || 4 * U >= a.m) continue;
                             const int from = rank < owner ? rank : rank - 1;
                             send_sums(peer_address(smem_u32(sums) + (from * own_units + i) * kBatchUnitBytes + lane_at, owner),
-                                      make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]), peer_address(bar(SUMS), owner));
+                                      make_float4(mine[4 * q], mine[4 * q + 1], mine[4 * q + 2], mine[4 * q + 3]), peer_address(bar(SUMS), owner));
                         }
                     }
+            }
             __syncwarp();
             cluster_arrive();                                              // sent
             if (!ok) return;
             asm volatile("griddepcontrol.wait;" ::: "memory");             // bias, y
-            bool landed = false;
-#pragma unroll 1
-            for (int U = u * kUnits; U < (u + 1) * kUnits && 4 * U < a.m; ++U) {
-                const int i = U * inverse >> 16;
-                if (U - i * c != rank) continue;
-                if (!landed && !(ok = wait(SUMS, 0))) return;
-                landed = true;
-                float mine[4], f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                batch_sums<NX, 4>(acc0 + (U - u * kUnits) * 4, mine);
-                for (int q = 0; q < c; ++q) {                              // in CTA order
-                    float4 p = make_float4(mine[0], mine[1], mine[2], mine[3]);
-                    if (q != rank) p = *reinterpret_cast<const float4*>(sums + ((q < rank ? q : q - 1) * own_units + i) * kBatchUnitBytes + lane_at);
-                    f[0] += p.x; f[1] += p.y; f[2] += p.z; f[3] += p.w;
+            if (!(ok = wait(SUMS, 0))) return;
+#pragma unroll
+            for (int q = 0; q < kUnits; ++q) {
+                const int U = u * kUnits + q, i = U * inverse >> 16;
+                if (U - i * c != rank || 4 * U >= a.m) continue;
+                float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 2
+                for (int r = 0; r < c; ++r) {                              // in CTA order
+                    float4 p = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+                    if (r != rank) p = *reinterpret_cast<const float4*>(sums + ((r < rank ? r : r - 1) * own_units + i) * kBatchUnitBytes + lane_at);
+                    t[0] += p.x; t[1] += p.y; t[2] += p.z; t[3] += p.w;
                 }
-                emit(tile0, 4 * U, f);
+                emit(tile0, 4 * U, t);
             }
         };
 
-        int slot = set, r = set, seg = 0, left = a.kb - gb0 % a.kb - set;  // rings and tile of the warp's block
+        int slot = set, r = set, b = set;                                  // rings, and the warp's block
         uint32_t free_parity = 1, raw_parity = 0;                          // (the first round of the stages is free)
-        for (int b = set; b < nblocks; b += kBatchSets) {
-            while (left <= 0) {
-                left += a.kb;
-                ++seg;
-            }
-            if (!(ok = wait(RAW_FULL + r, raw_parity))) break;
-            const uint8_t* raw = raw_base + r * kBatchRawBytes;
-            const uint4 code[4] = {*reinterpret_cast<const uint4*>(raw + code_at), *reinterpret_cast<const uint4*>(raw + code_at + 512),
-                                   *reinterpret_cast<const uint4*>(raw + code_at + 16), *reinterpret_cast<const uint4*>(raw + code_at + 528)};
-            const uint32_t fields[2] = {*reinterpret_cast<const uint32_t*>(raw + step_at), *reinterpret_cast<const uint32_t*>(raw + step_at + 8)};
-            const uint32_t zeros = *reinterpret_cast<const uint16_t*>(raw + zero_at) >> (4 * hi8);
-            auto convert = [&](int h, auto chain) {
-                const auto gc = make_group<decltype(chain)::value, STEPS == kStepsPlain>((zeros >> (8 * h)) & 15u, fields[h]);
-                const uint32_t words[8] = {code[2 * h].x, code[2 * h].y, code[2 * h].z, code[2 * h].w,
-                                           code[2 * h + 1].x, code[2 * h + 1].y, code[2 * h + 1].z, code[2 * h + 1].w};
-                const uint32_t to = tmem_base + lane_addr + kWBase + slot * kWStage + (2 * v + h) * kBatchWCols;
+        // Up to and with the first block behind the oldest tile that has not been read (`tile_end`): its products are in the making
+        // while that tile is read.
+        int tile_end = first_end;
+        while (ok && b < nblocks) {
+            const int stop = CL ? nblocks : min(nblocks, FORM == kRounds && pending ? b + kBatchSets : tile_end + kBatchSets);
+            for (; b < stop; b += kBatchSets) {
+                if (!(ok = wait(RAW_FULL + r, raw_parity))) break;
+                const uint8_t* raw = raw_base + r * kBatchRawBytes;
+                const uint4 code[4] = {*reinterpret_cast<const uint4*>(raw + code_at), *reinterpret_cast<const uint4*>(raw + code_at + 512),
+                                       *reinterpret_cast<const uint4*>(raw + code_at + 16), *reinterpret_cast<const uint4*>(raw + code_at + 528)};
+                const uint32_t fields[2] = {*reinterpret_cast<const uint32_t*>(raw + step_at), *reinterpret_cast<const uint32_t*>(raw + step_at + 8)};
+                const uint32_t zeros = *reinterpret_cast<const uint16_t*>(raw + zero_at) >> (4 * hi8);
+                auto convert = [&](int h, auto chain) {
+                    const auto gc = make_group<decltype(chain)::value, STEPS == kStepsPlain>((zeros >> (8 * h)) & 15u, fields[h]);
+                    const uint32_t words[8] = {code[2 * h].x, code[2 * h].y, code[2 * h].z, code[2 * h].w,
+                                               code[2 * h + 1].x, code[2 * h + 1].y, code[2 * h + 1].z, code[2 * h + 1].w};
+                    const uint32_t to = tmem_base + lane_addr + kWBase + slot * kWStage + (2 * v + h) * kBatchWCols;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint4 p = dequant_word(words[2 * i], gc), q = dequant_word(words[2 * i + 1], gc);
-                    if (h == 0 && i == 0) {
-                        if (!(ok = wait(DONE + slot, free_parity))) return;
-                        tcgen05_fence_after();
+                    for (int i = 0; i < 4; ++i) {
+                        const uint4 p = dequant_word(words[2 * i], gc), q = dequant_word(words[2 * i + 1], gc);
+                        if (h == 0 && i == 0) {
+                            if (!(ok = wait(DONE + slot, free_parity))) return;
+                            tcgen05_fence_after();
+                        }
+                        tmem_st8(to + 8 * i, p, q);
                     }
-                    tmem_st8(to + 8 * i, p, q);
-                }
-            };
+                };
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if constexpr (STEPS == kStepsFp16) convert(h, Chain<kChainFp16>{});
-                else if (STEPS == kStepsMixed && all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
-                else convert(h, Chain<kChainGeneral>{});
+                for (int h = 0; h < 2; ++h) {
+                    if constexpr (STEPS == kStepsFp16) convert(h, Chain<kChainFp16>{});
+                    else if (STEPS == kStepsMixed && all_factored(fields[h])) convert(h, Chain<kChainFactored>{});
+                    else convert(h, Chain<kChainGeneral>{});
+                    if (!ok) break;
+                }
                 if (!ok) break;
-            }
-            if (!ok) break;
-            tmem_st_wait();
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(bar(FULL + slot));
-                if (b + RS < nblocks) mbar_arrive(bar(RAW_FREE + r));      // the last copies are not waited for
+                tmem_st_wait();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(bar(FULL + slot));
+                    if (b + RS < nblocks) mbar_arrive(bar(RAW_FREE + r));      // the last copies are not waited for
+                }
+                if ((slot += kBatchSets) >= R) { slot -= R; free_parity ^= 1; }
+                if ((r += kBatchSets) >= RS) { r -= RS; raw_parity ^= 1; }
             }
             if constexpr (!CL) {
-                while (read < seg && ok) epilogue(read++);
-                if (!ok) break;
+                if (FORM == kRounds && pending) advance();
+                for (; ok && tile_end <= b - kBatchSets; tile_end += a.kb) epilogue(read++);
             }
-            left -= kBatchSets;
-            if ((slot += kBatchSets) >= R) { slot -= R; free_parity ^= 1; }
-            if ((r += kBatchSets) >= RS) { r -= RS; raw_parity ^= 1; }
         }
         if constexpr (CL) {
             exchange();
         } else {
-            const int segs = (b0 + nsteps - 1) / tsteps - tile0 + 1;
+            const int segs = FORM == kRounds ? a.whole + (nshared ? 1 : 0) : (b0 + nsteps - 1) / tsteps - tile0 + 1;
             while (read < segs && ok) epilogue(read++);
+            if constexpr (FORM == kRounds)
+                while (pending) advance();
         }
     }
     __syncwarp();
