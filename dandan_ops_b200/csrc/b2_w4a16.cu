@@ -610,37 +610,39 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
     return m <= kBatchMaxM && d.k % 8 == 0 && (int64_t(d.n) + 127) / 128 * d.kb * 4 < (int64_t(1) << 23);
 }
 
-// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of what ran before (us in a chain of dependent launches,
-// tile / streaming / GEMM -> batch).  A wide layer has more tiles of 128 columns than SMs: its CTAs pay for reading more than
-// one tile's sums back, which a short K does not carry.
-//   up to 8 rows above 4096 native blocks (~10 MB), where the tile kernel runs out, up to 16384, not on wide layers: 6144 x 4096
-//                at M = 1 / 8 10.1 / 10.4 -> 9.2 / 9.5, 4096 x 12288 14.1 / 14.2 -> 12.7 / 12.9, 14336 x 2048 at M = 8
-//                11.5 -> 8.5; 4096 x 4096 6.2 / 6.7 against 7.3, 24576 x 4096 21.7 / 22.4 against 21.9 / 22.2, 28672 x 1024
-//                11.3 against 11.8.  One line for both kinds of steps: the flag must not change a bit.  Not below 4096
-//                output columns, the usual width of a slice: there a plain layer, too, has the bits of the kernels that
-//                carry the all-gather.
-//                Up to 65536 blocks where K is 12288 or more: 4096 x 28672 at M = 1 / 8 21.9 / 22.3 -> 20.7 / 20.9, 6144 x 16384
-//                19.1 / 19.9 -> 17.6 / 17.9, 8192 x 28672 34.9 / 36.0 -> 34.7 / 34.9 (with FP16 steps 21.0 / 21.5 -> 19.9 / 20.2, 18.4 /
-//                19.2 -> 16.8 / 17.0, 33.1 / 34.5 -> 33.0 / 33.3); 16384 x 8192 22.2 / 24.0 against 23.4 / 23.6.
-//   9..16        up to K = 3072 above 2304 blocks (8192 x 2048 at M = 16 9.5 -> 7.5, 6144 x 2048 8.1 -> 7.3, 12288 x 1024 7.4 ->
-//                5.2; 4096 x 2048 tile 5.0 against 6.3; on the line 3072 x 3072 stays with the tile kernel, 6.1 against 6.5 at M =
-//                9, 8.8 against 6.7 at M = 16), else above 4096, wide ones from K = 513 on: 6144 x 4096 at M = 16 14.8 -> 9.7,
-//                24576 x 4096 26.8 -> 22.5, 57344 x 8192 90 -> 75; 57344 x 512 11.3 against 12.8.  Longer K up to 4096 blocks
-//                keeps the tile kernel although batch would be ahead from K = 3329 on (M = 9 / 16: 4096 x 4096, whose plan
-//                callers know as one CTA per tile, 10.2 / 10.2 against 7.2 / 7.4, 4096 x 3840 10.2 / 10.0 against 7.6 / 7.8, 3072 x
-//                4096 9.7 / 10.0 against 7.2 / 7.4; 4096 x 3328 7.0 / 9.4 against 7.2 / 7.3).
-//   17..32       from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
-//                1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 8.4 / 8.7, 57344 x 8192 121 / 125 -> 78
-//                / 80; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4, 256 x 4096 6.2 / 6.2
-//                against 6.8 / 7.2.  (Behind a kernel that does not let it start early the batch kernel's own start shows:
-//                up to 1024 blocks 0.5 to 2.4 us more than the streaming kernel, 1024 x 1024 at M = 17 7.3 against 5.5.  The
-//                two cannot be told apart here, and of a decoder layer's four projections most are in the first position.)
-//   33..64       always: 1024 x 1024 at M = 64 12.4 -> 5.2, 4096 x 4096 19.9 -> 11.1, 57344 x 8192 147 -> 93, 28672 x 1024 16.4
-//                -> 15.5
-//   65..128      wide layers from 13 blocks of 256 columns per SM on: 57344 x 8192 at M = 128 184 -> 125, 40960 x 2048 40.0 ->
-//                33.6, 28672 x 3072 33.2 -> 32.7; 28672 x 2048 25.8 against 27.3, 28672 x 1024 17.2 against 21.6; others
-//                always (4096 x 4096 20.2 -> 15.7, 1024 x 1024 11.2 -> 7.6, 18944 x 1024 13.3 -> 10.1)
-// A column slice (B2_FLAG_COLUMN_SLICE) keeps the kernels that carry the all-gather wherever that runs in the same launch.
+// B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of the kernel that runs otherwise (us in a chain of dependent
+// launches, tile / streaming / GEMM -> batch), on 150 layers of 512 x 1024 to 57344 x 8192 at 1 to 16 rows and 33 to 128 rows.
+//   up to 8 rows   K above 4864 from 1536 native blocks (3.6 MB) on: 1536 x 6144 at M = 1 / 8 5.0 / 5.7 -> 4.5 / 4.6, 2048 x 5120 5.4 / 6.0 -> 4.3 /
+//                  4.4, 2560 x 12288 15.5 / 10.7 -> 7.7; 1536 x 4096 3.4 / 4.3 against 4.0 / 4.1.  Not up to 1024 columns, the usual
+//                  width of a slice: there a plain layer, too, has the bits of the kernels that carry the all-gather (1024 x 8192
+//                  4.8 / 4.9 against 4.5 / 4.7);
+//                  any K above 1024 with more row tiles than the tile kernel runs at once (two per SM): 5120 x 1536 5.2 / 5.8 -> 4.0 / 4.2,
+//                  7168 x 2048 6.8 / 7.3 -> 5.1 / 5.3; 4096 x 2048 3.7 / 3.9 against 4.6 / 4.7, 8192 x 1024 3.3 / 3.5 against 3.7 / 3.8;
+//                  all others above 4096 blocks (9.6 MB), where the tile kernel runs out: 6144 x 4096 8.3 / 8.5 -> 6.7 / 6.8.
+//                  Up to 65536 blocks (8192 x 28672 33.9 / 34.8 -> 31.1 / 31.2); on wide layers (more tiles of 128 columns than SMs) up to
+//                  49152, above which the streaming kernel is level (57344 x 8192 63.9 / 68.4, 62.4 / 66.8), with K above 1024: 24576 x 4096 18.2 / 19.0 -> 17.5 / 17.8, 28672 x 2048 13.6 / 14.5 -> 11.1 /
+//                  11.4, 57344 x 2048 20.5 / 20.9 -> 19.5 / 19.8.
+//   9..16          K above 1024 above 768 blocks (1024 x 4096 at M = 16 4.4 -> 3.9, 2048 x 2048 4.5 -> 3.3, 2048 x 5120 9.1 -> 4.5, 24576 x 4096 20.1 ->
+//                  18.1; up to there the kernels are less than a microsecond apart and callers know the tile kernel's bits; narrow
+//                  slices, below 512 columns, keep those of the all-gather's kernels) but for
+//                  one to two tiles per SM at K up to 2048 (4096 x 1536 4.0 against 4.3, 3584 x 2048 4.5 / 4.8 against 4.5 / 4.6);
+//                  K of 769 to 1024 from 512 blocks on (2048 x 1024 3.5 -> 3.0, 28672 x 1024 11.4 -> 7.5; 1024 x 1024 2.7 against 3.0); shorter
+//                  K above 2304 blocks, wide ones from K = 513 on (57344 x 512 11.3 against 12.8).  Layers with one to two row tiles per
+//                  SM, K of 3073 to 4352 and up to 4096 blocks keep the tile kernel, whose plan of one CTA per tile callers know (4096 x
+//                  4096 at M = 16).
+//   17..32         from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
+//                  1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 6.9 / 7.0, 57344 x 8192 121 / 125 -> 72
+//                  / 74; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4.
+//                  (Behind a kernel that does not let it start early the batch kernel's own start shows:
+//                  up to 1024 blocks 0.5 to 2.4 us more than the streaming kernel, 1024 x 1024 at M = 17 7.3 against 5.5.  The
+//                  two cannot be told apart here, and of a decoder layer's four projections most are in the first position.)
+//   33..64         always: 1024 x 1024 at M = 64 12.4 -> 4.4, 4096 x 4096 19.9 -> 7.5, 57344 x 8192 147 -> 93, 28672 x 1024 16.4
+//                  -> 9.6
+//   65..128        wide layers from 13 blocks of 256 columns per SM on: 57344 x 8192 at M = 128 184 -> 125, 40960 x 2048 40.0 ->
+//                  33.6, 28672 x 3072 33.2 -> 32.7; others always (4096 x 4096 20.2 -> 10.4, 1024 x 1024 11.2 -> 6.5, 18944 x 1024
+//                  13.3 -> 10.1)
+// One line for both kinds of steps: the flag must not change a bit.  A column slice (B2_FLAG_COLUMN_SLICE) keeps the kernels that carry
+// the all-gather wherever that runs in the same launch.
 bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = false) {
     if ((slice && m <= kGatherMaxM) || !batch_applicable(m, d)) return false;
     const int64_t blocks = int64_t(d.n16) * d.kb, tiles = (int64_t(d.n) + 127) / 128, sms = sm_count > 0 ? sm_count : 148;
@@ -648,8 +650,17 @@ bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = fa
     if (m > 64) return !wide || tiles * d.kb >= 13 * sms;
     if (m > 32) return true;
     if (m > 16) return d.kb > 1 && (d.n > 512 || d.kb < 8 || d.kb >= 32);
-    if (m > 8) return blocks > (d.kb <= 12 ? 2304 : 4096) && (!wide || d.kb > 2);
-    return blocks > 4096 && blocks <= (d.kb >= 48 ? 65536 : 16384) && d.n >= 4096 && !wide;
+    const bool second = d.n16 > sms && d.n16 <= 2 * sms;     // row tiles: one to two for every SM
+    if (m > 8) {
+        if (d.kb < 4) return blocks > 2304 && (!wide || d.kb > 2);
+        if (d.kb == 4) return blocks >= 512;
+        if (second && (d.kb <= 8 || (d.kb > 12 && d.kb <= 17 && blocks <= 4096))) return false;
+        return blocks > 768 && d.n >= 512;
+    }
+    if (blocks > (wide ? 49152 : 65536)) return false;
+    if (wide) return d.kb > 4;
+    if (d.kb > 19) return blocks >= 1536 && d.n > 1024;
+    return blocks > 4096 || (d.kb > 4 && d.n16 > 2 * sms);
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {
