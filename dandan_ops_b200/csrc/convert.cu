@@ -19,20 +19,30 @@ using b2host::fail;
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
-template <typename Out, bool IMAGE>
-int run_dequantize(const uint8_t* native, const int32_t* packed, const float* scales, const int32_t* zeros, const b2::Dims& d,
-                   Out* out, int64_t ldo, cudaStream_t s) {
+template <typename Out>
+int run_dequantize(const uint8_t* native, const b2::Dims& d, Out* out, int64_t ldo, cudaStream_t s) {
     constexpr int kVec = 16 / int(sizeof(Out));
     constexpr int64_t kPerCta = 256 * b2::kDequantUnits;
     const int64_t elements = int64_t(d.n) * d.k;
     // 16-byte stores need rows that are whole, aligned units
     if (d.k % kVec == 0 && ldo % kVec == 0 && aligned16(out)) {
         const int64_t units = elements / kVec;
-        b2::dequantize_kernel<Out, kVec, IMAGE><<<unsigned((units + kPerCta - 1) / kPerCta), 256, 0, s>>>(native, packed, scales, zeros, d, out, ldo);
+        b2::dequantize_kernel<Out, kVec><<<unsigned((units + kPerCta - 1) / kPerCta), 256, 0, s>>>(native, d, out, ldo);
     } else {
-        b2::dequantize_kernel<Out, 1, IMAGE><<<unsigned((elements + kPerCta - 1) / kPerCta), 256, 0, s>>>(native, packed, scales, zeros, d, out, ldo);
+        b2::dequantize_kernel<Out, 1><<<unsigned((elements + kPerCta - 1) / kPerCta), 256, 0, s>>>(native, d, out, ldo);
     }
     return after_launch("dequantize_kernel");
+}
+
+int run_dequantize_state(const int32_t* packed, const float* scales, const int32_t* zeros, const b2::Dims& d, float* out, int64_t ldo,
+                         cudaStream_t s) {
+    constexpr int64_t kRuns = int64_t(b2::kStateWarps) * b2::kStateRuns;
+    const unsigned ctas = unsigned((int64_t(d.n) * d.kb + kRuns - 1) / kRuns);
+    if (d.k % 4 == 0 && ldo % 4 == 0 && aligned16(out))
+        b2::dequantize_state_kernel<true><<<ctas, b2::kStateWarps * 32, 0, s>>>(packed, scales, zeros, d, out, ldo);
+    else
+        b2::dequantize_state_kernel<false><<<ctas, b2::kStateWarps * 32, 0, s>>>(packed, scales, zeros, d, out, ldo);
+    return after_launch("dequantize_state_kernel");
 }
 
 // Blocks of a warp: as few as let all warps run at once (40 on an SM; a 4096 x 12288 layer has three), for the shortest chain of
@@ -136,16 +146,15 @@ int b2_w4a16_dequantize(const void* native, int64_t n, int64_t k, float* out, in
     if (!native || !out) return fail(B2_ERR_ARGUMENT, "null pointer");
     if (int rc = check_dims(n, k)) return rc;
     if (ldo < k) return fail(B2_ERR_ARGUMENT, "ldo must be at least k");
-    return run_dequantize<float, true>(static_cast<const uint8_t*>(native), nullptr, nullptr, nullptr, b2::make_dims(n, k), out, ldo,
-                                       static_cast<cudaStream_t>(stream));
+    return run_dequantize<float>(static_cast<const uint8_t*>(native), b2::make_dims(n, k), out, ldo, static_cast<cudaStream_t>(stream));
 }
 
 int b2_w4a16_dequantize_fp16(const void* native, int64_t n, int64_t k, void* out, int64_t ldo, void* stream) {
     if (!native || !out) return fail(B2_ERR_ARGUMENT, "null pointer");
     if (int rc = check_dims(n, k)) return rc;
     if (ldo < k) return fail(B2_ERR_ARGUMENT, "ldo must be at least k");
-    return run_dequantize<__half, true>(static_cast<const uint8_t*>(native), nullptr, nullptr, nullptr, b2::make_dims(n, k),
-                                        static_cast<__half*>(out), ldo, static_cast<cudaStream_t>(stream));
+    return run_dequantize<__half>(static_cast<const uint8_t*>(native), b2::make_dims(n, k), static_cast<__half*>(out), ldo,
+                                  static_cast<cudaStream_t>(stream));
 }
 
 int b2_w4a16_dequantize_state(const int32_t* packed, const float* scales, const int32_t* zeros, int64_t n, int64_t k, float* out,
@@ -153,7 +162,7 @@ int b2_w4a16_dequantize_state(const int32_t* packed, const float* scales, const 
     if (!packed || !scales || !zeros || !out) return fail(B2_ERR_ARGUMENT, "null pointer");
     if (int rc = check_dims(n, k)) return rc;
     if (ldo < k) return fail(B2_ERR_ARGUMENT, "ldo must be at least k");
-    return run_dequantize<float, false>(nullptr, packed, scales, zeros, b2::make_dims(n, k), out, ldo, static_cast<cudaStream_t>(stream));
+    return run_dequantize_state(packed, scales, zeros, b2::make_dims(n, k), out, ldo, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -275,16 +275,73 @@ __device__ __forceinline__ void store_unit(Out* dst, const float (&v)[V]) {
     }
 }
 
+// Checkpoint tensors -> FP32.  A warp takes kStateRuns runs of 256 columns of a row (consecutive runs, so nearly always one row): lane i
+// loads word i of a run, lanes 0..3 its four steps and zero points, and the lanes of a store, four columns each (VEC; else one), fetch
+// theirs by shuffle: a word is loaded once, a store is 512 (128) consecutive bytes, and a run costs no division.  Bound by the stores:
+// 6144 x 4096 17.4 us (6.6 TB/s into L2 and memory; a fill of the output 15.0), 4096 x 12288 34.8 (28.7); with a thread per four
+// columns that found its row, word, step and zero point by itself, bound by instructions, 24.0 and 46.5.  Codes become floats as
+// 2^23 + code, from which 2^23 + zero is subtracted exactly.
+constexpr int kStateRuns = 4;
+constexpr int kStateWarps = 8;
+template <bool VEC>
+__global__ void __launch_bounds__(kStateWarps * 32)
+dequantize_state_kernel(const int32_t* __restrict__ packed, const float* __restrict__ scales, const int32_t* __restrict__ zeros, Dims d,
+                        float* __restrict__ out, int64_t ldo) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned first = (blockIdx.x * kStateWarps + (threadIdx.x >> 5)) * kStateRuns, total = unsigned(d.n) * unsigned(d.kb);
+    if (first >= total) return;
+    int row = int(first / unsigned(d.kb)), run = int(first - unsigned(row) * unsigned(d.kb));
+    const int64_t row0 = row;
+    const int run0 = run;
+    uint32_t word[kStateRuns];
+    float step[kStateRuns];
+    int zero[kStateRuns];
+#pragma unroll
+    for (int i = 0; i < kStateRuns; ++i) {
+        word[i] = 0; step[i] = 0.0f; zero[i] = 0;
+        if (row < d.n) {
+            const int w = run * 32 + lane, g = run * 4 + lane;
+            if (w < d.words) word[i] = uint32_t(__ldg(packed + int64_t(row) * d.words + w));
+            if (lane < 4 && g < d.groups) {
+                step[i] = __ldg(scales + int64_t(row) * d.groups + g);
+                zero[i] = __ldg(zeros + int64_t(row) * d.groups + g) & 15;         // as the image holds it
+            }
+        }
+        if (++run == d.kb) { run = 0; ++row; }
+    }
+    row = int(row0);
+    run = run0;
+#pragma unroll
+    for (int i = 0; i < kStateRuns; ++i) {
+        if (row >= d.n) break;
+        constexpr int V = VEC ? 4 : 1, kStores = 8 / V;
+        float* dst = out + int64_t(row) * ldo + run * kBlockCols + lane * V;
+#pragma unroll
+        for (int j = 0; j < kStores; ++j) {
+            const int col = j * 32 * V + lane * V, grp = VEC ? col >> 6 : j >> 1;         // of the run
+            const uint32_t codes = __shfl_sync(kAll, word[i], col >> 3) >> (4 * (col & 7));
+            const float s = __shfl_sync(kAll, step[i], grp), base = __int_as_float(0x4B000000 + __shfl_sync(kAll, zero[i], grp));
+            float v[V];
+#pragma unroll
+            for (int c = 0; c < V; ++c)
+                v[c] = __fmul_rn(__fsub_rn(__uint_as_float(0x4B000000u | ((codes >> (4 * c)) & 15u)), base), s);
+            if (run * kBlockCols + col < d.k) {
+                if constexpr (VEC) __stcs(reinterpret_cast<float4*>(dst + j * 128), make_float4(v[0], v[1], v[2], v[3]));
+                else __stcs(dst + j * 32, v[0]);
+            }
+        }
+        if (++run == d.kb) { run = 0; ++row; }
+    }
+}
+
 // Unit = V consecutive columns of a row, one 16-byte store (V = 1: one element, for rows that are not whole
-// units); the lanes of a warp write consecutive units.  Bound by the FP32 (FP16) stores: 6144 x 4096 to FP32, through
-// the image and with a thread per eight columns 96 us, straight from the checkpoint tensors 27 us (4.3 TB/s).  A thread takes
-// kDequantUnits units a CTA apart so that their loads are in flight together.
-// IMAGE: from the native image, else from the checkpoint tensors.
+// units); the lanes of a warp write consecutive units.  A thread takes kDequantUnits units a CTA apart so that their loads are in
+// flight together.
 constexpr int kDequantUnits = 4;
-template <typename Out, int V, bool IMAGE>
+template <typename Out, int V>
 __global__ void __launch_bounds__(256)
-dequantize_kernel(const uint8_t* __restrict__ native, const int32_t* __restrict__ packed, const float* __restrict__ scales,
-                  const int32_t* __restrict__ zeros, Dims d, Out* __restrict__ out, int64_t ldo) {
+dequantize_kernel(const uint8_t* __restrict__ native, Dims d, Out* __restrict__ out, int64_t ldo) {
     const unsigned per_row = unsigned(d.k) / V;
     const int64_t total = int64_t(d.n) * per_row;
     const int64_t u0 = int64_t(blockIdx.x) * (256 * kDequantUnits) + threadIdx.x;
@@ -297,18 +354,11 @@ dequantize_kernel(const uint8_t* __restrict__ native, const int32_t* __restrict_
         word[i] = 0; step[i] = 0.0f; zero[i] = 0;
         if (u < total) {
             const int row = int(unsigned(u) / per_row), col = int(unsigned(u) - unsigned(row) * per_row) * V;
-            if constexpr (IMAGE) {
-                const WordRef w = locate(d, row, col >> 3);
-                const uint8_t* base = native + w.block;
-                word[i] = __ldg(reinterpret_cast<const uint32_t*>(base) + w.word);
-                step[i] = field_step(__ldg(reinterpret_cast<const uint32_t*>(base + kStepOffset) + w.meta));
-                zero[i] = (__ldg(base + kZeroOffset + (w.meta >> 1)) >> (4 * (w.meta & 1))) & 15;
-            } else {
-                const int64_t at = int64_t(row) * d.groups + (col >> 6);
-                word[i] = uint32_t(__ldg(packed + int64_t(row) * d.words + (col >> 3)));
-                step[i] = __ldg(scales + at);
-                zero[i] = __ldg(zeros + at) & 15;          // as the image holds it
-            }
+            const WordRef w = locate(d, row, col >> 3);
+            const uint8_t* base = native + w.block;
+            word[i] = __ldg(reinterpret_cast<const uint32_t*>(base) + w.word);
+            step[i] = field_step(__ldg(reinterpret_cast<const uint32_t*>(base + kStepOffset) + w.meta));
+            zero[i] = (__ldg(base + kZeroOffset + (w.meta >> 1)) >> (4 * (w.meta & 1))) & 15;
         }
     }
 #pragma unroll
@@ -320,7 +370,7 @@ dequantize_kernel(const uint8_t* __restrict__ native, const int32_t* __restrict_
 #pragma unroll
         for (int c = 0; c < V; ++c) {
             const int cc = (col & 7) + c;
-            v[c] = dequantize_one((word[i] >> (4 * (IMAGE ? nibble_slot(cc) : cc))) & 15u, zero[i], step[i]);
+            v[c] = dequantize_one((word[i] >> (4 * nibble_slot(cc))) & 15u, zero[i], step[i]);
         }
         store_unit<Out, V>(out + int64_t(row) * ldo + col, v);
     }
