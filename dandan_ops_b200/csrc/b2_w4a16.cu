@@ -713,13 +713,15 @@ struct GemmShape {
     int ma, bn;      // single-CTA kernel: accumulators of 128 x rows, output columns
     int pair_mt;     // pair kernel: rows of x per CTA pair (256 or 192), 0 = single-CTA kernel
     int splits;      // pair kernel: CTAs along K per tile
+    int batch = 0;   // the batch kernel's tiles of 128 x 128: CTAs of the launch (`splits` per tile)
+    bool fuses_silu() const { return pair_mt || batch; }
     int64_t tiles(int64_t m, int64_t n) const {
         if (pair_mt) return ((n + 255) / 256) * ((m + pair_mt - 1) / pair_mt);
         return ((n + bn - 1) / bn) * ((m + 128 * ma - 1) / (128 * ma));
     }
-    int64_t ctas(int64_t m, int64_t n) const { return tiles(m, n) * (pair_mt ? 2 * splits : 1); }
+    int64_t ctas(int64_t m, int64_t n) const { return batch ? batch : tiles(m, n) * (pair_mt ? 2 * splits : 1); }
     int64_t partial_bytes(int64_t m, int64_t n) const {
-        return splits > 1 ? tiles(m, n) * splits * 256 * pair_mt * int64_t(sizeof(float)) : 0;
+        return splits > 1 && !batch ? tiles(m, n) * splits * 256 * pair_mt * int64_t(sizeof(float)) : 0;
     }
 };
 constexpr GemmShape kGemmShapes[5] = {{1, 128, 0, 1}, {2, 128, 0, 1}, {2, 192, 0, 1}, {0, 0, 256, 1}, {0, 0, 192, 1}};
@@ -805,9 +807,39 @@ inline GemmShape gemm_shape(int64_t m, int64_t n, int kb, int sms, bool pairs_ok
     return best;
 }
 
-// Shape the GEMM would take for this call (workspace permitting the K-split).
+// The batch kernel's 128 x 128 tiles as a shape of the GEMM, for 129 to 1024 rows of x wherever all tiles run at once, one CTA or a
+// cluster of them each: the pair kernel's 256-column tiles leave most SMs idle there and it starts later (us in a chain of launches, pair
+// kernel / 128 x 128 tiles, at M = 129, 256, 512 and 1024: 1024 x 2048 15.8 / 7.5, 16.1 / 7.7, 16.2 / 9.0, 16.2 / 10.7; 1024 x 3072 17.0 / 8.5, 17.2 /
+// 9.3, 17.7 / 9.8, 18.4 / 12.3; 4096 x 1024 12.8 / 8.1, 11.3 / 7.6, 11.5 / 8.8, two rounds 12.6 / 14.5; 6144 x 2048 16.8 / 11.0, 17.6 / 11.6, two rounds
+// 17.9 / 20.2).  Not where K is so long that the batch kernel would take equal ranges over all SMs (1024 x 8192 at M = 1536 28.9 /
+// 32.4).  More rows, and layers from 4096 native blocks on (3072 from K = 3841 on, where the pair kernel splits K), keep the
+// pair kernel's plans, which callers know.
+constexpr int64_t kBatchTilesMaxM = 1024;
+int batch_tiles(int64_t m, const b2::Dims& d, int sms, int* parts) {
+    if (m <= b2::batch_nx(m) || m > kBatchTilesMaxM || d.k % 8 != 0 || g_forced_shape.load(std::memory_order_relaxed) ||
+        g_forced_splits.load(std::memory_order_relaxed) || int64_t(d.n16) * d.kb >= (d.kb < 16 ? 4096 : 3072))
+        return 0;
+    if ((int64_t(d.n) + 127) / 128 * ((m + 127) / 128) > sms) return 0;
+    const b2host::BatchPlan p = b2host::plan_batch(m, d, sms);
+    if (p.cluster == 1 && p.max_parts > 1) return 0;
+    *parts = p.max_parts;
+    return p.grid;
+}
+
+// Shape of the GEMM for a problem, the batch kernel's among them.
+GemmShape gemm_shape(int64_t m, const b2::Dims& d, int sms, bool pairs_ok = true) {
+    int parts = 1;
+    if (const int grid = batch_tiles(m, d, sms, &parts)) {
+        GemmShape shape{1, 128, 0, parts};
+        shape.batch = grid;
+        return shape;
+    }
+    return gemm_shape(m, d.n, d.kb, sms, pairs_ok);
+}
+
+// Shape the GEMM would take for this call (workspace permitting the K-split; the batch kernel needs none for these tiles).
 GemmShape gemm_shape_for_call(int64_t m, const b2::Dims& d, int sms, int64_t workspace_bytes) {
-    GemmShape shape = gemm_shape(m, d.n, d.kb, sms, pair_available());
+    GemmShape shape = gemm_shape(m, d, sms, pair_available());
     if (B2_W4A16_TICKET_BYTES + shape.partial_bytes(m, d.n) > workspace_bytes) shape.splits = 1;   // no room: one CTA per tile
     return shape;
 }
@@ -902,6 +934,7 @@ int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t l
     a.whole = p.whole;
     a.cluster = p.cluster;
     a.parts = p.parts;
+    a.row_tiles = p.row_tiles;
     const int share = p.cluster > 1 ? p.cluster : p.parts;
     a.kb_each = d.kb / share;
     a.kb_more = d.kb % share;
@@ -964,7 +997,7 @@ int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, 
         return B2_OK;
     }
     if (gemm_preferred(m, d) && d.k % 8 == 0) {
-        const GemmShape shape = gemm_shape(m, d.n, d.kb, dev.sm_count > 0 ? dev.sm_count : 148);
+        const GemmShape shape = gemm_shape(m, d, dev.sm_count > 0 ? dev.sm_count : 148);
         if (route) *route = B2_ROUTE_TCGEN05;
         if (k_splits) *k_splits = shape.splits;
         if (grid) *grid = int(shape.ctas(m, d.n));
@@ -1121,7 +1154,7 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
     if (route == B2_ROUTE_AUTO)
         route = tile_applicable(m, d, tile_split) ? B2_ROUTE_TILE
               : (gemm_preferred(m, d) && gemm_applicable(x, ldx, d)) ? B2_ROUTE_TCGEN05 : B2_ROUTE_STREAM;
-    if (act && route == B2_ROUTE_TCGEN05 && !gemm_shape_for_call(m, d, dev.sm_count, workspace_bytes).pair_mt) {
+    if (act && route == B2_ROUTE_TCGEN05 && !gemm_shape_for_call(m, d, dev.sm_count, workspace_bytes).fuses_silu()) {
         // the single-CTA GEMM has no such epilogue: small batches stream, larger ones take two launches (unless the batch
         // kernel would have taken them with a larger workspace: b2_w4a16_silu_mul_is_fused() says one launch)
         if (m > B2_STREAM_MAX_M && !batch)
@@ -1144,6 +1177,9 @@ int linear_impl(const void* x, int64_t ldx, const void* native, const void* bias
             return fail(B2_ERR_UNSUPPORTED, "the tcgen05 route needs K % 8 == 0 and a 16-byte aligned x");
         if (workspace_bytes < B2_W4A16_TICKET_BYTES)
             return fail(B2_ERR_WORKSPACE, "workspace smaller than b2_w4a16_workspace_bytes()");
+        if (gemm_shape_for_call(m, d, dev.sm_count, workspace_bytes).batch)
+            return run_batch(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count,
+                             bias, act, steps, (flags & B2_FLAG_OVERLAP_LAUNCH) != 0);
         return run_gemm(x, ldx, native, y, ldy, m, d, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), dev.sm_count, bias, act, steps);
     }
     if (route == B2_ROUTE_BATCH) {
@@ -1258,7 +1294,7 @@ int b2_w4a16_silu_mul_is_fused(int64_t m, int64_t n, int64_t k) {
     if (device_info(dev) != B2_OK) dev.sm_count = 148;
     const b2::Dims d = b2::make_dims(n, k);
     if (d.k % 8 != 0 || batch_preferred(m, d, dev.sm_count)) return 1;   // the streaming kernel in chunks of 64 rows, or the batch kernel
-    return gemm_shape_for_call(m, d, dev.sm_count > 0 ? dev.sm_count : 148, INT64_MAX).pair_mt != 0 ? 1 : 0;
+    return gemm_shape_for_call(m, d, dev.sm_count > 0 ? dev.sm_count : 148, INT64_MAX).fuses_silu() ? 1 : 0;
 }
 
 int b2_w4a16_silu_mul_pairs(const void* y_pairs, int64_t ld_in, void* out, int64_t ld_out, int64_t m, int64_t n,

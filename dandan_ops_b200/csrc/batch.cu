@@ -24,9 +24,9 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
 constexpr int kRangeBlocks = 11, kRangeBlocksCluster = 8;   // blocks of K that equal ranges must gain per SM to pay for their hand-over
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
-template <int NX, int STEPS, int FORM>
+template <int NX, int STEPS, int FORM, bool MANY = false>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
-    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, FORM>;
+    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, FORM, MANY>;
     constexpr bool CL = FORM == b2::kClusters;
     constexpr int smem = b2::batch_smem_bytes(NX, CL);
     static std::atomic<uint64_t> configured{0};
@@ -124,9 +124,10 @@ int shared_cost(int nx, int tiles, int kb, int parts, int sms) {
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     BatchPlan p;
     p.nx = b2::batch_nx(m);
+    p.row_tiles = int((m + p.nx - 1) / p.nx);
     p.cluster = p.parts = 1;
     p.whole = p.shared_tiles = 0;
-    const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows, tsteps = d.kb * 4;
+    const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows * p.row_tiles, tsteps = d.kb * 4;
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);
     // Ranges: equal ones over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle).
@@ -189,11 +190,20 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
         p.max_parts = 1;
         p.whole = p.nx >= 64 || d.kb >= 8 ? 1 : 0;       // (as ranges of a tile each: 12416 x 1024 at M = 16 / 64 4.8 / 6.1, as a round 4.9 / 6.0)
     }
+    // (up to 128 rows a smaller workspace than that of the ranges is refused whatever the form)
+    if (p.row_tiles > 1 && (p.cluster > 1 || p.max_parts == 1)) p.partial_bytes = 0;
     return p;
 }
 
 template <int NX, int STEPS>
 int launch_form(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool overlap, cudaStream_t s) {
+    if constexpr (NX == 128) {
+        if (p.row_tiles > 1) {
+            if (p.cluster > 1) return launch_one<NX, STEPS, b2::kClusters, true>(xmap, a, p.grid, overlap, s);
+            if (p.whole) return launch_one<NX, STEPS, b2::kRounds, true>(xmap, a, p.grid, overlap, s);
+            return launch_one<NX, STEPS, b2::kRanges, true>(xmap, a, p.grid, overlap, s);
+        }
+    }
     if (p.cluster > 1) return launch_one<NX, STEPS, b2::kClusters>(xmap, a, p.grid, overlap, s);
     if (p.whole) return launch_one<NX, STEPS, b2::kRounds>(xmap, a, p.grid, overlap, s);
     return launch_one<NX, STEPS, b2::kRanges>(xmap, a, p.grid, overlap, s);

@@ -100,6 +100,7 @@ struct BatchArgs {
     int shared_tiles, whole;    // tiles that several CTAs share, and that every CTA takes by itself (rounds)
     int cluster, parts;     // CTAs per tile (clusters), per shared tile (rounds); their blocks of K: kb_each, the first kb_more of them one more
     int kb_each, kb_more;
+    int row_tiles;          // tiles of NX rows of x (MANY)
     int act;                // as StreamArgs::act
     int wait_limit;
     int fault_block;        // -1; a test passes b >= 0: CTA 0 arms the barrier of its b-th block but skips the copy
@@ -159,7 +160,9 @@ __device__ __forceinline__ void send_sums(uint32_t to, float4 v, uint32_t barrie
 
 enum : int { kRanges = 0, kClusters = 1, kRounds = 2 };
 
-template <int NX, int STEPS, int FORM>
+// MANY: x has more than NX rows.  A tile is then NX rows of x by 128 weight rows, numbered with the rows of x inside, so that CTAs side by
+// side read the same weights.
+template <int NX, int STEPS, int FORM, bool MANY = false>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
     constexpr bool CL = FORM == kClusters;
@@ -209,6 +212,8 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         tile0 = (b0 >> 2) / a.kb;
         kb0 = (b0 >> 2) - tile0 * a.kb;
     }
+    auto weight_tile = [&](int tile) { return MANY ? tile / a.row_tiles : tile; };
+    auto first_row = [&](int tile) { return MANY ? tile % a.row_tiles * NX : 0; };          // of x
     int tile = tile0, kb = kb0;                                            // (warps 0 and 2: of the block at hand)
     auto next_block = [&](int b) {                                         // from block b - 1 to b
         if (FORM == kRounds && b == nshared) {
@@ -238,7 +243,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         __syncwarp();
         for (; issued < min(kBatchEarly, nblocks); ++issued) {
-            if (elect_one()) request(issued, tile, kb);
+            if (elect_one()) request(issued, weight_tile(tile), kb);
             __syncwarp();
             next_block(issued + 1);
         }
@@ -249,7 +254,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         __syncwarp();
         if (elect_one()) {
             if constexpr (CL) {
-                const int units = (a.m + 3) / 4;                           // in use; this CTA owns every a.cluster-th
+                const int units = (min(a.m - first_row(tile0), NX) + 3) / 4;        // in use; this CTA owns every a.cluster-th
                 mbar_expect_tx(bar(SUMS), uint32_t((a.cluster - 1) * ((units - rank + a.cluster - 1) / a.cluster) * kBatchUnitBytes));
             }
         }
@@ -293,7 +298,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         for (; issued < nblocks; ++issued) {
             const int r = issued % RS;
             if (issued >= RS && !wait(RAW_FREE + r, ((issued / RS) - 1) & 1)) break;
-            if (elect_one()) request(issued, tile, kb);
+            if (elect_one()) request(issued, weight_tile(tile), kb);
             __syncwarp();
             next_block(issued + 1);
         }
@@ -360,7 +365,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 const int t0 = FORM == kRanges && b == 0 ? b0 & 3 : 0, t1 = FORM == kRanges && b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
                 mbar_expect_tx(bar(FULL + slot), uint32_t(t1 - t0 + 1) * kXBytes);
                 for (int t = t0; t <= t1; ++t)
-                    tma_load_2d(smem_u32(x_base + slot * kXStage + t * kXBytes), &xmap, (kb * 4 + t) * kGemmBK, 0, bar(FULL + slot));
+                    tma_load_2d(smem_u32(x_base + slot * kXStage + t * kXBytes), &xmap, (kb * 4 + t) * kGemmBK, first_row(tile), bar(FULL + slot));
             }
             __syncwarp();
             next_block(b + 1);
@@ -381,7 +386,8 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
         // The sums of this lane's weight row and the rows m0.. of x -> y.
         auto emit = [&](int tile, int m0, const auto& f) {
             constexpr int W = sizeof(f) / sizeof(float);
-            const int n = tile * kBatchRows + row;
+            const int n = weight_tile(tile) * kBatchRows + row, base = first_row(tile), rows = a.m - base;
+            __half* y = a.y + int64_t(base) * a.ldy;
             if (a.act) {
                 // lanes l and l ^ 4 hold the gate and the up sum of one output column: the gate lane
                 // finishes the even rows of x, the up lane the odd ones
@@ -391,13 +397,13 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     const float theirs = __shfl_xor_sync(0xffffffffu, hi8 ? f[i] : f[i + 1], 4);
                     const float gate = hi8 ? theirs : f[i], up = hi8 ? f[i + 1] : theirs;
                     const int m = m0 + i + hi8;
-                    if (m < a.m && (n | 8) < a.n)
-                        a.y[int64_t(m) * a.ldy + out] = silu_mul(finish_output(gate, a.bias, n & ~8), finish_output(up, a.bias, n | 8));
+                    if (m < rows && (n | 8) < a.n)
+                        y[int64_t(m) * a.ldy + out] = silu_mul(finish_output(gate, a.bias, n & ~8), finish_output(up, a.bias, n | 8));
                 }
             } else if (n < a.n) {
 #pragma unroll
                 for (int i = 0; i < W; ++i)
-                    if (m0 + i < a.m) a.y[int64_t(m0 + i) * a.ldy + n] = finish_output(f[i], a.bias, n);
+                    if (m0 + i < rows) y[int64_t(m0 + i) * a.ldy + n] = finish_output(f[i], a.bias, n);
             }
         };
 
@@ -422,11 +428,12 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             pending = 0;
             if (__shfl_sync(0xffffffffu, prior, 0) != unsigned(last - first)) return;
             __threadfence();
+            const int rows = a.m - first_row(shared_tile);
             constexpr int RW = CW < 8 ? CW : 8, PARTS = 32 / RW;           // partial tiles requested together, added in CTA order
 #pragma unroll 1
             for (int c0 = 0; c0 < NX / 4; c0 += RW) {
                 const int m0 = u * (NX / 4) + c0;
-                if (m0 >= a.m) break;
+                if (m0 >= rows) break;
                 float f[RW];
 #pragma unroll
                 for (int i = 0; i < RW; ++i) f[i] = 0.0f;
@@ -436,7 +443,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     for (int j = 0; j < PARTS; ++j)
 #pragma unroll
                         for (int q = 0; q < RW / 4; ++q)
-                            if (c + j <= last && m0 + 4 * q < a.m) p[j][q] = __ldcg(slot_of(c + j) + (c0 / 4 + q) * kBatchRows);
+                            if (c + j <= last && m0 + 4 * q < rows) p[j][q] = __ldcg(slot_of(c + j) + (c0 / 4 + q) * kBatchRows);
                             else p[j][q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
                     for (int j = 0; j < PARTS; ++j)
@@ -472,11 +479,12 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 last = whole ? 0 : batch_owner(t1 - 1, a.steps, ctas);
             }
             const uint32_t acc = tmem_base + lane_addr + seg % ACCS * (C * NX) + u * (NX / 4);
+            const int rows = a.m - first_row(tile);
             if (whole) {
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
                     const int m0 = u * (NX / 4) + c0;
-                    if (m0 < a.m) {
+                    if (m0 < rows) {
                         float f[CW];
                         batch_sums<NX, CW>(acc + c0, f);
                         emit(tile, m0, f);
@@ -490,7 +498,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     batch_sums<NX, CW>(acc + c0, f);
 #pragma unroll
                     for (int q = 0; q < CW / 4; ++q)
-                        if (u * (NX / 4) + c0 + 4 * q < a.m)
+                        if (u * (NX / 4) + c0 + 4 * q < rows)
                             __stcg(dst + (c0 / 4 + q) * kBatchRows, make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]));
                 }
                 pending = 1;
@@ -513,19 +521,20 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
             if constexpr (NX > 64) cluster_arrive();                       // all products of this CTA are done: nothing reads its x tiles
             cluster_wait();
             constexpr int kUnits = NX / 16;                                // of this warp
+            const int rows = a.m - first_row(tile0);
             const int c = a.cluster, own_units = (NX / 4 + c - 1) / c, inverse = 65536 / c + 1;      // U / c for U < 32
             const uint32_t lane_at = uint32_t(quad * 32 + lane) * 16, acc0 = tmem_base + lane_addr + u * (NX / 4);
             float f[NX / 4];
             if (ok) {
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW)
-                    if (u * (NX / 4) + c0 < a.m) {
+                    if (u * (NX / 4) + c0 < rows) {
                         float (&mine)[CW] = *reinterpret_cast<float (*)[CW]>(f + c0);
                         batch_sums<NX, CW>(acc0 + c0, mine);
 #pragma unroll
                         for (int q = 0; q < CW / 4; ++q) {
                             const int U = u * kUnits + c0 / 4 + q, i = U * inverse >> 16, owner = U - i * c;
-                            if (owner == rank || 4 * U >= a.m) continue;
+                            if (owner == rank || 4 * U >= rows) continue;
                             const int from = rank < owner ? rank : rank - 1;
                             send_sums(peer_address(smem_u32(sums) + (from * own_units + i) * kBatchUnitBytes + lane_at, owner),
                                       make_float4(mine[4 * q], mine[4 * q + 1], mine[4 * q + 2], mine[4 * q + 3]), peer_address(bar(SUMS), owner));
@@ -540,7 +549,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 #pragma unroll
             for (int q = 0; q < kUnits; ++q) {
                 const int U = u * kUnits + q, i = U * inverse >> 16;
-                if (U - i * c != rank || 4 * U >= a.m) continue;
+                if (U - i * c != rank || 4 * U >= rows) continue;
                 float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 2
                 for (int r = 0; r < c; ++r) {                              // in CTA order
