@@ -342,9 +342,9 @@ bool tile_applicable(int64_t rows, const b2::Dims& d, int split) {
 
 bool pair_available();
 
-template <int MT, bool XVEC, bool FULL, int STEPS = b2::kStepsMixed>
+template <int MT, bool XVEC, bool FULL, int STEPS = b2::kStepsMixed, bool SPLIT = false>
 int launch_tile_one(const b2::TileArgs& a, int smem, cudaStream_t s) {
-    auto kernel = b2::w4a16_tile_kernel<MT, XVEC, FULL, STEPS>;
+    auto kernel = b2::w4a16_tile_kernel<MT, XVEC, FULL, STEPS, SPLIT>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -462,10 +462,11 @@ int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
         }
         if (steps != b2::kStepsMixed && xvec)
             return with_steps(steps, [&](auto t) {
-                return mt == 1 ? launch_tile_one<1, true, true, decltype(t)::value>(a, smem2, s) : launch_tile_one<2, true, true, decltype(t)::value>(a, smem2, s);
+                return mt == 1 ? launch_tile_one<1, true, true, decltype(t)::value, true>(a, smem2, s) : launch_tile_one<2, true, true, decltype(t)::value, true>(a, smem2, s);
             });
-        if (mt == 1) return xvec ? launch_tile_one<1, true, true>(a, smem2, s) : launch_tile_one<1, false, true>(a, smem2, s);
-        return xvec ? launch_tile_one<2, true, true>(a, smem2, s) : launch_tile_one<2, false, true>(a, smem2, s);
+        if (mt == 1)
+            return xvec ? launch_tile_one<1, true, true, b2::kStepsMixed, true>(a, smem2, s) : launch_tile_one<1, false, true, b2::kStepsMixed, true>(a, smem2, s);
+        return xvec ? launch_tile_one<2, true, true, b2::kStepsMixed, true>(a, smem2, s) : launch_tile_one<2, false, true, b2::kStepsMixed, true>(a, smem2, s);
     }
     // Stage all mt * 8 rows (zeros beyond M) unless that costs occupancy: the padded layout is the
     // faster one as long as every CTA of the grid still finds a place in the first wave.

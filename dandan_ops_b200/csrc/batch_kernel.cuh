@@ -153,10 +153,6 @@ __device__ __forceinline__ uint32_t peer_address(uint32_t own, int rank) {      
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(own), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void send_sums(uint32_t to, float4 v, uint32_t barrier) {        // 16 bytes counted on the receiver's barrier
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(barrier) : "memory");
-}
 
 enum : int { kRanges = 0, kClusters = 1, kRounds = 2 };
 

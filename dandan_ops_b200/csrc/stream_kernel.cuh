@@ -400,6 +400,12 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
+// 16 bytes to the shared memory of another CTA of the cluster, counted on a barrier there.
+__device__ __forceinline__ void send_sums(uint32_t to, float4 v, uint32_t barrier) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(barrier) : "memory");
+}
+
 __device__ __forceinline__ uint32_t pick(const uint4& v, int i) {
     return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }

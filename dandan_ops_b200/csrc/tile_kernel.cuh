@@ -105,6 +105,18 @@ __device__ __forceinline__ void tile_collect(const TileArgs& a, const GatherArgs
     }
 }
 
+// The warps' tiles added in warp order, for the fragment at `red` of the first warp's.
+template <int MT>
+__device__ __forceinline__ float4 tile_sum(const float4* red, int warps) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int w = 0; w < warps; ++w) {
+        const float4 f = red[w * (MT * 32)];
+        v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+    }
+    return v;
+}
+
 // FULL: all MT * 8 rows of x are staged (zeros beyond M): compile-time layout, no row predicates -
 // the faster form whenever the padded rows do not cost occupancy.  Otherwise only the M rows that
 // exist are staged and lanes of missing rows use zero fragments.
@@ -115,33 +127,42 @@ __device__ __forceinline__ void tile_collect(const TileArgs& a, const GatherArgs
 // for a peer while others are still to be scheduled: the CTAs count themselves on the flag block's ticket
 // when their tile is out, and only the LAST one - by then every packet of this rank has left - collects the
 // packets the peers sent (bounded as everywhere) and publishes the epoch.
-template <int MT, bool XVEC, bool FULL, int STEPS, bool GATHER>
+//
+// SPLIT: a cluster of a.ksplit CTAs per row tile (always FULL: those grids are small).  A kernel of its own, so that layers of one CTA
+// per tile do not carry it: 6144 x 1024 at M = 1 / 4 3.00 / 3.08 -> 2.71 / 2.95 us, a chain of 3072 x 2048, 2048 x 2048, 8192 x 2048 and
+// 2048 x 4096 16.4 / 16.8 -> 15.2 / 16.2.  (A chain that takes both in turn starts each with cold instructions: the projections of a
+// 0.6B layer 11.1 against 11.2 in one kernel at M = 1, 12.0 against 11.9 at M = 4.)
+template <int MT, bool XVEC, bool FULL, int STEPS, bool GATHER, bool SPLIT>
 __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* ga) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int rows = FULL ? MT * 8 : a.m;
+    const int ksplit = SPLIT ? a.ksplit : 1;
     const int kChunk = tile_x_chunk_bytes(rows);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     // this CTA's share of the row tile: blocks kb0 .. kb0 + kbn - 1 of K
     uint32_t part = 0;
-    if (a.ksplit > 1) {
+    if (ksplit > 1) {
         asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
         // first phase of "both CTAs are running", completed before the hand-over below touches the
         // other CTA's shared memory
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     }
-    const int nt = blockIdx.x / a.ksplit;
-    const int kb0 = int(part) * a.kb / a.ksplit, kbn = (int(part) + 1) * a.kb / a.ksplit - kb0;
-    const int kb_max = (a.kb + a.ksplit - 1) / a.ksplit;     // both CTAs of a pair use one layout
+    const int nt = blockIdx.x / ksplit;
+    const int kb0 = int(part) * a.kb / ksplit, kbn = (int(part) + 1) * a.kb / ksplit - kb0;
+    const int kb_max = (a.kb + ksplit - 1) / ksplit;     // both CTAs of a pair use one layout
     const int bar_bytes = ((kb_max * 8 + 127) / 128) * 128;
     uint8_t* blocks = smem + bar_bytes;
     uint8_t* xs = blocks + kb_max * kBlockBytes;
     float4* red = reinterpret_cast<float4*>(xs + kb_max * 4 * kChunk);
     const uint32_t bar0 = smem_u32(smem);
 
+    auto sums_bar = [&] { return smem_u32(red + a.warps * MT * 32); };       // (clusters) behind the reduction tiles
     if (threadIdx.x == 0) {
         for (int b = 0; b < kbn; ++b) mbar_init(bar0 + b * 8, 1);
+        if (!GATHER && ksplit > 1 && part == 0) mbar_init(sums_bar(), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (!GATHER && ksplit > 1 && part == 0) mbar_expect_tx(sums_bar(), uint32_t(ksplit - 1) * (MT * 512));
         const uint8_t* src = a.native + (int64_t(kb0) * a.n16 + nt) * kBlockBytes;
         const int64_t stride = int64_t(a.n16) * kBlockBytes;
         for (int b = 0; b < kbn; ++b) {
@@ -234,7 +255,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
             }
             if constexpr (XVEC && kAsync) stage_wait();
         };
-        if (a.ksplit > 1) stage(std::true_type{}); else stage(std::false_type{});
+        if (ksplit > 1) stage(std::true_type{}); else stage(std::false_type{});
     }
     __syncthreads();        // x staged; barrier initialisation visible to every waiter
 
@@ -307,7 +328,54 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     for (int mt = 0; mt < MT; ++mt)
         red[(warp * MT + mt) * 32 + lane] = make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
     __syncthreads();
-    if (a.ksplit > 1) {
+    if constexpr (SPLIT && !GATHER) {
+        // The CTAs of a cluster share the row tile.  Each adds its warps' tiles in warp order; the others send their sums to the
+        // first one's shared memory, counted on its barrier, and it adds them to its own in CTA order and writes y.  (Against plain
+        // remote stores between two cluster barriers 1024 x 2048 at M = 1 / 8 / 16 2.74 / 2.98 / 3.97 -> 2.47 / 2.75 / 3.66 us.)
+        const float4* peer = red + (a.warps + 1) * MT * 32;                // [ksplit - 1][MT * 32] the others' sums
+        const bool adds = threadIdx.x < MT * 32;                           // a thread per fragment of the sums
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (adds) v = tile_sum<MT>(red + threadIdx.x, a.warps);
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // CTA 0 runs, its barrier is set up
+        if (adds && part != 0) {
+            uint32_t to, bar;
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(smem_u32(peer + (part - 1) * (MT * 32) + threadIdx.x)));
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(bar) : "r"(sums_bar()));
+            send_sums(to, v, bar);
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this thread sends nothing any more
+        if (adds && part == 0) {
+            const bool landed = __all_sync(0xffffffffu, mbar_wait(sums_bar(), 0, a.wait_limit));
+            if (landed) {
+                for (int p = 0; p + 1 < ksplit; ++p) {
+                    const float4 f = peer[p * (MT * 32) + threadIdx.x];
+                    v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+                }
+                const int m = int(threadIdx.x >> 5) * 8 + 2 * t, n = nt * 16 + g;
+                if (a.act) {                                               // gate (row g) and up (row g + 8) of two rows of x
+                    if (n + 8 < a.n) {
+                        if (m < a.m) a.y[int64_t(m) * a.ldy + nt * 8 + g] = silu_mul(finish_output(v.x, a.bias, n), finish_output(v.z, a.bias, n + 8));
+                        if (m + 1 < a.m) a.y[int64_t(m + 1) * a.ldy + nt * 8 + g] = silu_mul(finish_output(v.y, a.bias, n), finish_output(v.w, a.bias, n + 8));
+                    }
+                } else {
+                    __half* y = a.y + int64_t(m) * a.ldy + n;
+                    if (m < a.m && n < a.n) y[0] = finish_output(v.x, a.bias, n);
+                    if (m + 1 < a.m && n < a.n) y[a.ldy] = finish_output(v.y, a.bias, n);
+                    if (m < a.m && n + 8 < a.n) y[8] = finish_output(v.z, a.bias, n + 8);
+                    if (m + 1 < a.m && n + 8 < a.n) y[a.ldy + 8] = finish_output(v.w, a.bias, n + 8);
+                }
+            } else if (lane == 0 && a.status) {
+                atomicOr(a.status, kStatusCopyTimeout);
+            }
+            failed = !landed;
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");        // nobody writes to this CTA any more
+        if (__syncthreads_or(failed)) __nanosleep(100000);                 // (but for sums that were on their way when it gave up)
+        return;
+    }
+    if (ksplit > 1) {
         // The CTAs of a cluster share the row tile.  Each adds its warps' tiles in warp order; CTA p > 0
         // puts its 128 * MT sums into slot p - 1 of the first one's shared memory, and after the cluster
         // barrier the first adds the slots to its own sums in CTA order and writes y.
@@ -334,7 +402,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
                 const int mt = e >> 6, rl = (e >> 1) & 31, c = e & 1;
                 const int at = (mt * 32 + rl) * 4 + c;
                 float gate = tot[at], up = tot[at + 2];
-                for (int p = 0; p + 1 < a.ksplit; ++p) {
+                for (int p = 0; p + 1 < ksplit; ++p) {
                     gate += peer[p * (MT * 128) + at];
                     up += peer[p * (MT * 128) + at + 2];
                 }
@@ -347,7 +415,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         }
         for (int e = threadIdx.x; e < MT * 128; e += blockDim.x) {
             float sum = tot[e];
-            for (int p = 0; p + 1 < a.ksplit; ++p) sum += peer[p * (MT * 128) + e];
+            for (int p = 0; p + 1 < ksplit; ++p) sum += peer[p * (MT * 128) + e];
             tile_emit<GATHER>(a, ga, nt, e, sum);
         }
         if constexpr (GATHER) tile_collect(a, ga);
@@ -381,16 +449,16 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     if constexpr (GATHER) tile_collect(a, ga);
 }
 
-template <int MT, bool XVEC, bool FULL, int STEPS = kStepsMixed>
+template <int MT, bool XVEC, bool FULL, int STEPS = kStepsMixed, bool SPLIT = false>
 __global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_kernel(const TileArgs a) {
-    tile_body<MT, XVEC, FULL, STEPS, false>(a, nullptr);
+    tile_body<MT, XVEC, FULL, STEPS, false, SPLIT>(a, nullptr);
 }
 
 template <int MT, bool FULL, int STEPS>
 __global__ void __launch_bounds__(kTileMaxWarps * 32, 2)
 w4a16_tile_gather_kernel(const TileArgs a, const GatherArgs ga) {
-    tile_body<MT, true, FULL, STEPS, true>(a, &ga);
+    tile_body<MT, true, FULL, STEPS, true, FULL>(a, &ga);
 }
 
 }  // namespace b2
