@@ -19,6 +19,7 @@
 #include "gemm_kernel.cuh"
 #include "gemm_pair_kernel.cuh"
 #include "tile_kernel.cuh"
+#include "tile_pair_kernel.cuh"
 #include "gather_kernel.cuh"
 #include "rmsnorm.cuh"
 #include "batch.cuh"
@@ -340,6 +341,14 @@ bool tile_applicable(int64_t rows, const b2::Dims& d, int split) {
     return int64_t(d.n16) * d.kb <= limit && smem <= kTileSmemLimit;
 }
 
+constexpr int kTilePairSmemLimit = 232448;
+
+// Whether the tile route takes two row tiles per CTA (tile_pair_kernel.cuh; an aligned x, and not the gather form).
+bool tile_pair_applicable(int64_t rows, const b2::Dims& d, int split, int sms) {
+    return rows > 8 && split == 1 && d.n16 > sms && d.n16 <= 2 * sms && d.k % 8 == 0 && d.kb >= b2::kTilePairMinBlocks &&
+           b2::tile_pair_smem_bytes(d.kb) <= kTilePairSmemLimit;
+}
+
 bool pair_available();
 
 template <int MT, bool XVEC, bool FULL, int STEPS = b2::kStepsMixed, bool SPLIT = false>
@@ -381,6 +390,22 @@ int launch_tile_one(const b2::TileArgs& a, int smem, cudaStream_t s) {
     const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, a);
     if (le != cudaSuccess) return cuda_fail("w4a16_tile_kernel", le);
     return B2_OK;
+}
+
+template <int STEPS>
+int launch_tile_pair(const b2::TileArgs& a, cudaStream_t s) {
+    auto kernel = b2::w4a16_tile_pair_kernel<STEPS>;
+    static std::atomic<uint64_t> configured{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTilePairSmemLimit);
+        if (e != cudaSuccess) return cuda_fail("cudaFuncSetAttribute", e);
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    return launch_maybe_dependent("w4a16_tile_pair_kernel", kernel, (a.n16 + 1) / 2, b2::kTilePairWarps * 32, b2::tile_pair_smem_bytes(a.kb),
+                                  s, a.overlap != 0, a);
 }
 
 // The gather form of the tile kernel collects the peers' packets with the threads of ONE CTA (the last to
@@ -468,6 +493,8 @@ int run_tile(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
             return xvec ? launch_tile_one<1, true, true, b2::kStepsMixed, true>(a, smem2, s) : launch_tile_one<1, false, true, b2::kStepsMixed, true>(a, smem2, s);
         return xvec ? launch_tile_one<2, true, true, b2::kStepsMixed, true>(a, smem2, s) : launch_tile_one<2, false, true, b2::kStepsMixed, true>(a, smem2, s);
     }
+    if (!ga && xvec && tile_pair_applicable(rows, d, a.ksplit, sms > 0 ? sms : 148))
+        return with_steps(steps, [&](auto t) { return launch_tile_pair<decltype(t)::value>(a, s); });
     // Stage all mt * 8 rows (zeros beyond M) unless that costs occupancy: the padded layout is the
     // faster one as long as every CTA of the grid still finds a place in the first wave.
     const int padded = b2::tile_smem_bytes(d.kb, mt * 8, a.warps);
@@ -628,9 +655,9 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 //                  slices, below 512 columns, keep those of the all-gather's kernels) but for
 //                  one to two tiles per SM at K up to 2048 (4096 x 1536 4.0 against 4.3, 3584 x 2048 4.5 / 4.8 against 4.5 / 4.6);
 //                  K of 769 to 1024 from 512 blocks on (2048 x 1024 3.5 -> 3.0, 28672 x 1024 11.4 -> 7.5; 1024 x 1024 2.7 against 3.0); shorter
-//                  K above 2304 blocks, wide ones from K = 513 on (57344 x 512 11.3 against 12.8).  Layers with one to two row tiles per
-//                  SM, K of 3073 to 4352 and up to 4096 blocks keep the tile kernel, whose plan of one CTA per tile callers know (4096 x
-//                  4096 at M = 16).
+//                  K above 2304 blocks, wide ones from K = 513 on (57344 x 512 11.3 against 12.8).  Layers with one and a half to two row tiles
+//                  per SM, K of 3073 to 4352 and up to 4096 blocks keep the tile kernel, whose plan without a split callers know
+//                  (4096 x 4096 at M = 16, two tiles per CTA 7.3 against 6.1).
 //   17..32         from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
 //                  1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 6.9 / 7.0, 57344 x 8192 121 / 125 -> 72
 //                  / 74; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4.
@@ -655,7 +682,7 @@ bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = fa
     if (m > 8) {
         if (d.kb < 4) return blocks > 2304 && (!wide || d.kb > 2);
         if (d.kb == 4) return blocks >= 512;
-        if (second && (d.kb <= 8 || (d.kb > 12 && d.kb <= 17 && blocks <= 4096))) return false;
+        if (second && (d.kb <= 8 || (d.kb > 12 && d.kb <= 17 && 2 * d.n16 > 3 * sms && blocks <= 4096))) return false;
         return blocks > 768 && d.n >= 512;
     }
     if (blocks > (wide ? 49152 : 65536)) return false;
@@ -1009,7 +1036,7 @@ int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, 
     if (m > 0 && tile_applicable(m, d, split)) {   // whole K of a row tile per CTA, or per cluster of 2 or 4 CTAs
         if (route) *route = B2_ROUTE_TILE;
         if (k_splits) *k_splits = split;
-        if (grid) *grid = d.n16 * split;
+        if (grid) *grid = tile_pair_applicable(m, d, split, dev.sm_count > 0 ? dev.sm_count : 148) ? (d.n16 + 1) / 2 : d.n16 * split;
         if (rows_per_launch) *rows_per_launch = int(m);
         return B2_OK;
     }
