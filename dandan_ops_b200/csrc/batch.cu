@@ -24,83 +24,9 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
 constexpr int kRangeBlocks = 11, kRangeBlocksCluster = 8;   // blocks of K that equal ranges must gain per SM to pay for their hand-over
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
-template <int NX, int STEPS, int FORM, bool MANY = false>
-int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
-    auto kernel = b2::w4a16_batch_kernel<NX, STEPS, FORM, MANY>;
-    constexpr bool CL = FORM == b2::kClusters;
-    constexpr int smem = b2::batch_smem_bytes(NX, CL);
-    static std::atomic<uint64_t> configured{0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured.load(std::memory_order_acquire) & bit)) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return b2host::fail(B2_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        configured.fetch_or(bit, std::memory_order_release);
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(grid));
-    cfg.blockDim = dim3(b2::kBatchThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    int count = 0;
-    if (CL) {
-        attr[count].id = cudaLaunchAttributeClusterDimension;
-        attr[count].val.clusterDim.x = unsigned(a.cluster); attr[count].val.clusterDim.y = 1; attr[count].val.clusterDim.z = 1;
-        ++count;
-    }
-    if (overlap) {
-        attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[count].val.programmaticStreamSerializationAllowed = 1;
-        ++count;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = unsigned(count);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xmap, a);
-    if (e != cudaSuccess) return b2host::fail(B2_ERR_CUDA, std::string("w4a16_batch_kernel: ") + cudaGetErrorString(e));
-    return b2host::after_launch("w4a16_batch_kernel");
-}
-
 }  // namespace
 
 namespace b2host {
-
-// Clusters of c CTAs of the kernel that the device runs at the same time (asked once per device and size; without a device, for
-// planning alone, those of a B200).
-int cluster_capacity(int c) {
-    static std::atomic<int> known[64][9];                    // 0 = not asked yet, else capacity + 1
-    static constexpr int kB200[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-        cudaGetLastError();
-        return kB200[c];
-    }
-    std::atomic<int>& at = known[dev][c];
-    if (const int v = at.load(std::memory_order_acquire)) return v - 1;
-    auto kernel = b2::w4a16_batch_kernel<16, b2::kStepsMixed, b2::kClusters>;
-    constexpr int smem = 232448;                             // (no form uses more)
-    int clusters = 0;
-    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
-    if (ok) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(c));
-        cfg.blockDim = dim3(b2::kBatchThreads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = unsigned(c); attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        ok = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess;
-    }
-    if (!ok) {
-        cudaGetLastError();                                  // clear the error of a failed query
-        clusters = 0;
-    }
-    at.store(clusters + 1, std::memory_order_release);
-    return clusters;
-}
 
 // Estimated time of a launch with c CTAs per tile (one: whole tiles, no sums to send) beyond its fixed start, in ns: the blocks of a
 // CTA, and, the more SMs a launch takes, the later the next one finds room to start under it.  Fitted to 33 layers of 512 x 1024
@@ -195,34 +121,10 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     return p;
 }
 
-template <int NX, int STEPS>
-int launch_form(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, bool overlap, cudaStream_t s) {
-    if constexpr (NX == 128) {
-        if (p.row_tiles > 1) {
-            if (p.cluster > 1) return launch_one<NX, STEPS, b2::kClusters, true>(xmap, a, p.grid, overlap, s);
-            if (p.whole) return launch_one<NX, STEPS, b2::kRounds, true>(xmap, a, p.grid, overlap, s);
-            return launch_one<NX, STEPS, b2::kRanges, true>(xmap, a, p.grid, overlap, s);
-        }
-    }
-    if (p.cluster > 1) return launch_one<NX, STEPS, b2::kClusters>(xmap, a, p.grid, overlap, s);
-    if (p.whole) return launch_one<NX, STEPS, b2::kRounds>(xmap, a, p.grid, overlap, s);
-    return launch_one<NX, STEPS, b2::kRanges>(xmap, a, p.grid, overlap, s);
-}
-
-template <int NX>
-int launch_known(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
-    if (steps == b2::kStepsFp16) return launch_form<NX, b2::kStepsFp16>(p, xmap, a, overlap, s);
-    if (steps == b2::kStepsPlain) return launch_form<NX, b2::kStepsPlain>(p, xmap, a, overlap, s);
-    return launch_form<NX, b2::kStepsMixed>(p, xmap, a, overlap, s);
-}
-
 int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
-    switch (p.nx) {
-        case 16: return launch_known<16>(p, xmap, a, steps, overlap, s);
-        case 32: return launch_known<32>(p, xmap, a, steps, overlap, s);
-        case 64: return launch_known<64>(p, xmap, a, steps, overlap, s);
-        default: return launch_known<128>(p, xmap, a, steps, overlap, s);
-    }
+    if (p.row_tiles > 1) return launch_batch_row_tiles(p, xmap, a, steps, overlap, s);
+    if (p.cluster > 1) return launch_batch_clusters(p, xmap, a, steps, overlap, s);
+    return p.whole ? launch_batch_rounds(p, xmap, a, steps, overlap, s) : launch_batch_ranges(p, xmap, a, steps, overlap, s);
 }
 
 }  // namespace b2host

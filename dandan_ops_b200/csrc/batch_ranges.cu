@@ -1,0 +1,10 @@
+// The batch kernel's ranges.
+#include "batch_launch.cuh"
+
+namespace b2host {
+
+int launch_batch_ranges(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
+    return launch_rows<b2::kRanges>(p, xmap, a, steps, overlap, s);
+}
+
+}  // namespace b2host
