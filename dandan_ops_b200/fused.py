@@ -27,6 +27,12 @@ def _plain(x):
             and not (x.requires_grad and torch.is_grad_enabled()))
 
 
+def _held(module, name="op"):
+    """A child module, from where Module keeps it (an attribute lookup takes half a microsecond, several times per call)."""
+    children = module._modules
+    return children[name] if name in children else getattr(module, name)
+
+
 def concat_layers(layers, backend=None):
     """One QuantizedLinear whose rows are the rows of `layers` in order (same in_features,
     group size and device).  A missing bias counts as zeros when any layer has one."""
@@ -132,16 +138,16 @@ class GateUpSilu(nn.Module):
     def forward(self, x):
         if not isinstance(x, torch.Tensor) or x.ndim != 2 or x.shape[1] != self.in_features:
             raise ValueError("x must have shape [M, in_features]")
-        if x.dtype != torch.float16 or not x.is_cuda or x.device != self.op.packed_weight.device:
+        op = _held(self)
+        if x.dtype != torch.float16 or not x.is_cuda or x.device != op._state()[0].device:
             raise ValueError("the fused gate/up projection requires CUDA FP16 input on the layer's device")
         if x.stride(1) != 1:
             x = x.contiguous()
-        image = self.op._native_image()
+        image = op._native_image()
         if _plain(x) and (x.shape[0] <= 1 or x.stride(0) >= self.in_features):
-            return _ops.silu_mul_image(x, image, self.op.out_features, self.in_features, self.op._bias_fp16(),
-                                       self.op._image_flags & _GATE_UP_FLAGS)
-        return _native.linear_silu_mul(x, image, self.op.out_features, self.in_features, bias=self.op._bias_fp16(),
-                                       flags=self.op._image_flags & _GATE_UP_FLAGS)
+            return _ops.silu_mul_image(x, image, op.out_features, self.in_features, op._bias_fp16(), op._image_flags & _GATE_UP_FLAGS)
+        return _native.linear_silu_mul(x, image, op.out_features, self.in_features, bias=op._bias_fp16(),
+                                       flags=op._image_flags & _GATE_UP_FLAGS)
 
     def unfuse(self):
         """The original (gate, up) layers, state bit-identical."""
@@ -182,22 +188,26 @@ class RmsNormLinear(nn.Module):
         self.eval()
 
     def forward(self, x, residual=None):
+        op = _held(self)
+        device = op._state()[0].device
         for t in (x, residual):
             if t is None:
                 continue
             if not isinstance(t, torch.Tensor) or t.ndim != 2 or t.shape[1] != self.in_features:
                 raise ValueError("x and residual must have shape [M, in_features]")
-            if t.dtype != torch.float16 or t.device != self.op.packed_weight.device or not t.is_cuda:
+            if t.dtype != torch.float16 or t.device != device or not t.is_cuda:
                 raise ValueError("the RMSNorm prologue requires CUDA FP16 inputs on the layer's device")
         if residual is not None and residual.shape != x.shape:
             raise ValueError("x and residual must have the same shape")
         x = x.contiguous()
         residual = None if residual is None else residual.contiguous()
+        buffers = self._buffers
+        weight = buffers["norm_weight"] if "norm_weight" in buffers else self.norm_weight
+        image = op._native_image()                           # (before the flags, which it renews)
         if _plain(x) and (residual is None or _plain(residual)):
-            return _ops.rmsnorm_image(x, residual, self.norm_weight, self.eps, self.op._native_image(),
-                                      self.out_features, self.in_features, self.op._bias_fp16(), self.op._image_flags)
-        return _native.rmsnorm_linear(x, residual, self.norm_weight, self.eps, self.op._native_image(),
-                                      self.out_features, self.in_features, bias=self.op._bias_fp16(), flags=self.op._image_flags)
+            return _ops.rmsnorm_image(x, residual, weight, self.eps, image, self.out_features, self.in_features, op._bias_fp16(), op._image_flags)
+        return _native.rmsnorm_linear(x, residual, weight, self.eps, image, self.out_features, self.in_features, bias=op._bias_fp16(),
+                                      flags=op._image_flags)
 
 
 def fuse_named_projections(parent, names, fused_name=None):

@@ -291,7 +291,7 @@ class QuantizedLinear(torch.nn.Module):
 
     def _bias_fp16(self):
         """FP16 copy of the bias for the fused epilogue (derived, rebuilt when the bias changes)."""
-        bias = self.bias
+        bias = self._bias()
         if bias is None:
             return None
         key = (bias.data_ptr(), bias._version, bias.dtype)
@@ -335,9 +335,13 @@ class QuantizedLinear(torch.nn.Module):
             raise ValueError("dequantize " + CUDA_ONLY.replace(" FP16", ""))
         return _native.dequantize(self._native_image(), self.out_features, self.in_features)
 
+    def _bias(self):
+        buffers = self._buffers                              # (as _state: a lookup through Module takes half a microsecond)
+        return buffers["bias"] if "bias" in buffers else self.bias
+
     def _forward_key(self):
         packed, scales, zeros = self._state()
-        bias = self.bias
+        bias = self._bias()
         return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                 packed._version, scales._version, zeros._version,
                 id(packed), id(scales), id(zeros),
@@ -352,7 +356,8 @@ class QuantizedLinear(torch.nn.Module):
         if (key == self._checked_key and type(x) is torch.Tensor and x.dtype is torch.float16 and x.ndim == 2
                 and x.shape[1] == self.in_features and x.device == self._checked_device
                 and not (x.requires_grad and torch.is_grad_enabled())):
-            return _engine(x, self._image, self.out_features, self.in_features, self._bias_fp16(), self._image_flags)
+            bias16 = None if key[-1] is None else self._bias16 if self._bias16_key == key[-1] else self._bias_fp16()
+            return _engine(x, self._image, self.out_features, self.in_features, bias16, self._image_flags)
         y = self._forward_checked(x)
         if self.backend in ("auto", "cuda", "tensorcore", "naive") and not self.scales.requires_grad \
                 and self._image is not None:
