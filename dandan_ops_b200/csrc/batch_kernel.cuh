@@ -62,8 +62,10 @@ __host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; 
 // 4096 x 12288 at M = 16 1.4 % -> 0.4 % (0.6 %), M = 24 1.4 -> 0.5 (0.7), M = 64 1.4 -> 0.8 (0.75); 6144 x 4096 at M = 16
 // 0.7 -> 0.2 (0.4).  Reading the chains takes 0.1 us of a launch.  As many as fit beside the weight ring: the accumulator is
 // double-buffered only where that leaves four chains (one buffer is level: a tile's products wait for one read).
-__host__ __device__ constexpr int batch_chains(int nx) { return nx <= 32 ? 4 : 2; }
-__host__ __device__ constexpr int batch_accs(int nx) { return nx == 16 ? 2 : 1; }
+// (A cluster has one tile, and at up to 16 rows eight chains instead of two accumulators of four: 8192 x 12288 at M = 8 0.77 -> 0.43 %, 2048 x 5120
+// 0.20 -> 0.11 %; at the same time, since the loads of all chains share a wait.)
+__host__ __device__ constexpr int batch_chains(int nx, bool cl) { return nx == 16 && cl ? 8 : nx <= 32 ? 4 : 2; }
+__host__ __device__ constexpr int batch_accs(int nx, bool cl) { return nx == 16 && !cl ? 2 : 1; }
 __host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
 // Sums a CTA of a cluster receives: from every other one, of the units (four columns x 128 weight rows) that it owns.
 constexpr int kBatchUnitBytes = kBatchRows * 16;
@@ -123,23 +125,23 @@ __device__ __forceinline__ void batch_ld(uint32_t taddr, uint32_t (&v)[CW]) {
                      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                      : "r"(taddr) : "memory");
 }
-// The sums of CW accumulator columns: the chains (NX columns apart) added in a fixed order.
-template <int NX, int CW>
+// The sums of CW accumulator columns: the C chains (NX columns apart), all requested before one wait, added in a fixed order.
+template <int NX, int C, int CW>
 __device__ __forceinline__ void batch_sums(uint32_t taddr, float (&f)[CW]) {
-    constexpr int C = batch_chains(NX), W = CW < 8 ? CW : 8;
+    constexpr int W = CW < 8 ? CW : 8;
 #pragma unroll
     for (int at = 0; at < CW; at += W) {
+        uint32_t v[C][W];
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-            uint32_t v[W];
-            batch_ld<W>(taddr + c * NX + at, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int c = 0; c < C; ++c) batch_ld<W>(taddr + c * NX + at, v[c]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < C; ++c)
 #pragma unroll
             for (int i = 0; i < W; ++i) {
-                asm volatile("" : "+r"(v[i]));                                 // (not used before the wait)
-                f[at + i] = c == 0 ? __uint_as_float(v[i]) : __fadd_rn(f[at + i], __uint_as_float(v[i]));
+                asm volatile("" : "+r"(v[c][i]));                              // (not used before the wait)
+                f[at + i] = c == 0 ? __uint_as_float(v[c][i]) : __fadd_rn(f[at + i], __uint_as_float(v[c][i]));
             }
-        }
     }
 }
 
@@ -164,7 +166,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
     constexpr bool CL = FORM == kClusters;
     constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX, CL), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
     constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
-    constexpr int C = batch_chains(NX), ACCS = batch_accs(NX);
+    constexpr int C = batch_chains(NX, CL), ACCS = batch_accs(NX, CL);
     static_assert(ACCS * C * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -322,10 +324,12 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 uint32_t accumulate = fresh ? 0u : 1u;
                 auto step = [&](int t) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        umma_f16_ts(d + kk % C * NX, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc,
-                                    kk < C ? accumulate : 1u);
-                    accumulate = 1;
+                    for (int kk = 0; kk < 4; ++kk) {
+                        const int chain = C == 8 ? (t & 1) * 4 + kk : kk % C;
+                        umma_f16_ts(d + chain * NX, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc,
+                                    C == 8 ? (t < 2 ? accumulate : 1u) : kk < C ? accumulate : 1u);
+                    }
+                    if (C < 8) accumulate = 1;
                 };
                 const int t0 = FORM == kRanges && b == 0 ? b0 & 3 : 0;                                      // steps of the range in this block
                 const int t1 = FORM == kRanges && b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
@@ -482,7 +486,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     const int m0 = u * (NX / 4) + c0;
                     if (m0 < rows) {
                         float f[CW];
-                        batch_sums<NX, CW>(acc + c0, f);
+                        batch_sums<NX, C, CW>(acc + c0, f);
                         emit(tile, m0, f);
                     }
                 }
@@ -491,7 +495,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
                     float f[CW];
-                    batch_sums<NX, CW>(acc + c0, f);
+                    batch_sums<NX, C, CW>(acc + c0, f);
 #pragma unroll
                     for (int q = 0; q < CW / 4; ++q)
                         if (u * (NX / 4) + c0 + 4 * q < rows)
@@ -526,7 +530,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 for (int c0 = 0; c0 < NX / 4; c0 += CW)
                     if (u * (NX / 4) + c0 < rows) {
                         float (&mine)[CW] = *reinterpret_cast<float (*)[CW]>(f + c0);
-                        batch_sums<NX, CW>(acc0 + c0, mine);
+                        batch_sums<NX, C, CW>(acc0 + c0, mine);
 #pragma unroll
                         for (int q = 0; q < CW / 4; ++q) {
                             const int U = u * kUnits + c0 / 4 + q, i = U * inverse >> 16, owner = U - i * c;

@@ -10,6 +10,7 @@
 #include "host_common.cuh"
 
 namespace b2host {
+namespace {                       // (what is configured is known per copy of the library: no symbol shared between two of them)
 
 template <int NX, int STEPS, int FORM, bool MANY>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
@@ -66,4 +67,5 @@ int launch_rows(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs
     }
 }
 
+}  // namespace
 }  // namespace b2host
