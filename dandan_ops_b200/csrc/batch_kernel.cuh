@@ -5,7 +5,7 @@
 // (eight per fragment at 64 rows).  Here the decoded weights go to tensor memory as the A operand of one
 // tcgen05.mma per 16 columns of K, issued by a single thread and the same instruction whatever the number of rows:
 //
-//   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x; batch_chains(NX) of them, added on reading)
+//   D[n][m] (FP32, tensor memory: 128 lanes = weight rows, NX columns = rows of x; batch_chains() of them, added on reading)
 //     += A[n][k] (weights, FP16, tensor memory, written by the converter warps) * B[m][k] (x, shared memory, TMA)
 //
 // Work split, one of three forms (plan_batch() in batch.cu chooses):
