@@ -142,12 +142,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     const int g = lane >> 2, t = lane & 3;
     // this CTA's share of the row tile: blocks kb0 .. kb0 + kbn - 1 of K
     uint32_t part = 0;
-    if (ksplit > 1) {
-        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
-        // first phase of "both CTAs are running", completed before the hand-over below touches the
-        // other CTA's shared memory
-        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    }
+    if (ksplit > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
     const int nt = blockIdx.x / ksplit;
     const int kb0 = int(part) * a.kb / ksplit, kbn = (int(part) + 1) * a.kb / ksplit - kb0;
     const int kb_max = (a.kb + ksplit - 1) / ksplit;     // both CTAs of a pair use one layout
@@ -170,6 +165,13 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
             if (!(blockIdx.x == 0 && b == a.fault_block))
                 bulk_copy_g2s(smem_u32(blocks + b * kBlockBytes), src + b * stride, kBlockBytes, bar0 + b * 8);
         }
+    }
+    if (ksplit > 1) {
+        // First phase of "every CTA of the cluster runs and the first one's barrier for the sums is set up", completed before the
+        // hand-over below touches another CTA's shared memory: thread 0 arrives behind its initialisation, made visible to the cluster
+        // by the fence.  (Nobody waits for this phase until its products are done.)
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     }
     // Kernels launched behind this one as programmatic dependents may start as soon as they find room.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
