@@ -37,8 +37,9 @@
 // fragment is x^T (8 rows of x per MMA) and whose accumulators are FP32.
 //
 // Every wait in the kernel is bounded: a warp that gives up on an mbarrier records
-// kStatusCopyTimeout in the status word, stops computing and leaves through the normal
-// exit (its outputs are then undefined; the host reads the status word on demand).
+// kStatusCopyTimeout in the status word, asks for no more copies, drops its sums and leaves
+// through the normal exit (its outputs are then undefined; the host reads the status word on
+// demand).
 #pragma once
 #include "layout.cuh"
 #include "gather_kernel.cuh"
@@ -388,11 +389,12 @@ __device__ __forceinline__ bool mbar_try_wait_long(uint32_t bar, uint32_t parity
                  : "=r"(done) : "r"(bar), "r"(parity), "r"(kWaitHint) : "memory");
     return done != 0;
 }
-// Bounded wait: false if the phase did not complete within `limit` polls.
+// Bounded wait of a whole warp: false if the phase did not complete within `limit` polls.  The lanes go on or give up together: what
+// follows has votes, shuffles and products of the whole warp, and a lane that had left alone would hold up the others for good.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int limit = kWaitLimit) {
-    if (mbar_try_wait(bar, parity)) return true;           // the common case costs no loop bookkeeping
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;           // the common case costs no loop bookkeeping
     for (int i = 1; i < limit; ++i)
-        if (mbar_try_wait_long(bar, parity)) return true;
+        if (__all_sync(0xffffffffu, mbar_try_wait_long(bar, parity))) return true;
     return false;
 }
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -566,7 +568,27 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
     float acc[MT][4], acc2[kTwoChains ? MT : 1][4];
     int stage = 0;
     uint32_t parity = 0;
-    bool failed = false;
+    bool failed = false, given_up = false;         // this lane gave up a wait; a lane of the warp did
+
+    // The copies that lane 0 has asked for and nobody will wait for get time to land (bounded) before the slots are released.
+    auto give_up = [&](int slot, uint32_t phase) {
+        failed = true;
+        if (lane != 0) return;
+        fetch = wb1;                                       // no more of them
+        for (int s = 0; s < kStages; ++s) {
+            for (int i = 0; i < 4096 && !mbar_try_wait(bar0 + slot * 8, phase); ++i) {}
+            if (++slot == kStages) { slot = 0; phase ^= 1u; }
+        }
+    };
+    // Up to 16 rows: a wait that does not succeed at once, bounded.  A lane that gives up goes through the products with whatever is in
+    // the slot - they are instructions of the whole warp, and the other lanes may have seen the copy land - and the warp's sums are
+    // dropped behind them.  (A vote behind every wait instead, as from 17 rows on, costs 57344 x 8192 at M = 1 / 8 1.3 / 1.0 %;
+    // there it gains 6 % at M = 64 and this form loses 3 at M = 32, 24576 x 4096.)
+    auto await = [&](int slot, uint32_t phase) {
+        for (int i = failed ? a.wait_limit : 1; i < a.wait_limit; ++i)
+            if (mbar_try_wait_long(bar0 + slot * 8, phase)) return;
+        if (!failed) give_up(slot, phase);
+    };
 
     if (whole_x) {
         stage_wait();
@@ -596,11 +618,12 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
                 __syncthreads();
             }
             const int xorigin = whole_x ? 0 : p0;          // column block that the x buffer starts at
-            if (!active || failed) continue;
+            if (!active || given_up) continue;
             for (int kb = p0; kb < p1; ++kb) {
-                if (!mbar_wait(bar0 + stage * 8, parity, a.wait_limit)) {
-                    failed = true;
-                    if (lane == 0) atomicOr(a.status, kStatusCopyTimeout);
+                if constexpr (MT <= 2) {
+                    if (!mbar_try_wait(bar0 + stage * 8, parity)) await(stage, parity);
+                } else if (!mbar_wait(bar0 + stage * 8, parity, a.wait_limit)) {
+                    give_up(stage, parity);
                     break;
                 }
                 const uint8_t* slot = ring + stage * kBlockBytes;
@@ -650,6 +673,7 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
                 else if (factored) multiply(make_group<kChainFactored>(zg, field.x), make_group<kChainFactored>(zh, field.y));
                 else multiply(make_group<kChainGeneral>(zg, field.x), make_group<kChainGeneral>(zh, field.y));
             }
+            given_up = MT <= 2 ? __any_sync(0xffffffffu, failed) : failed;
         }
 
         if constexpr (kTwoChains) {            // (a fixed order: results do not depend on timing)
@@ -658,7 +682,7 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[mt][c] += acc2[mt][c];
         }
-        if (active && !failed) {
+        if (active && !given_up) {
             const bool whole = (k_lo == 0 && k_hi == a.kb);
             bool write_out = whole;
             if (!whole) {
@@ -748,15 +772,7 @@ __device__ __forceinline__ void stream_body(const StreamArgs& a, const GatherArg
         s0 += k_hi - k_lo;
     }
 
-    if (failed) {
-        // Let copies that are still in flight land before the CTA's shared memory is released
-        // (a bounded look at every slot of this warp's ring).
-        for (int s = 0; s < kStages; ++s) {
-            bool landed = false;
-            for (int i = 0; i < 4096 && !landed; ++i) landed = mbar_try_wait(bar0 + stage * 8, parity);
-            if (++stage == kStages) { stage = 0; parity ^= 1u; }
-        }
-    }
+    if (given_up && lane == 0) atomicOr(a.status, kStatusCopyTimeout);
 
     if constexpr (GATHER) {
         const unsigned epoch = mailbox_epoch(*ga);

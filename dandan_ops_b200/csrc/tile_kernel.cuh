@@ -185,18 +185,29 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         uint2 field;
         uint32_t zero;
     };
-    auto fetch = [&](int u, Unit& o) -> bool {
-        const int b = u >> 1, h = u & 1;
-        if (!mbar_wait(bar0 + b * 8, 0, a.wait_limit)) {
-            if (lane == 0 && a.status) atomicOr(a.status, kStatusCopyTimeout);
-            return false;
+    // A lane that gives up a wait goes on with whatever is in the block: products and votes are instructions of the whole warp, and the
+    // other lanes may have seen the copy land.  (A vote behind the wait costs 1024 x 2048 at M = 1 / 8 5 / 1 %, 6144 x 1024 1 / 0; where
+    // K is split at 9 to 16 rows it gains 3.)
+    constexpr bool kVote = SPLIT && MT == 2;
+    auto await = [&](uint32_t barrier) {
+        if constexpr (kVote) {
+            if (failed || mbar_wait(barrier, 0, a.wait_limit)) return;
+        } else {
+            if (mbar_try_wait(barrier, 0)) return;
+            for (int i = failed ? a.wait_limit : 1; i < a.wait_limit; ++i)
+                if (mbar_try_wait_long(barrier, 0)) return;
         }
+        if (!failed && a.status) atomicOr(a.status, kStatusCopyTimeout);
+        failed = true;
+    };
+    auto fetch = [&](int u, Unit& o) {
+        const int b = u >> 1, h = u & 1;
+        await(bar0 + b * 8);
         const uint8_t* slot = blocks + b * kBlockBytes;
         o.ca = *reinterpret_cast<const uint4*>(slot + h * 512 + lane * 16);           // row g
         o.cb = *reinterpret_cast<const uint4*>(slot + (2 + h) * 512 + lane * 16);     // row g+8
         o.field = *reinterpret_cast<const uint2*>(slot + kStepOffset + lane * 8);
         o.zero = slot[kZeroOffset + lane];
-        return true;
     };
     auto decode = [&](const Unit& o, int i, uint32_t (&w)[2][4], const auto& gg, const auto& gh) {
         const uint32_t wa = pick(o.ca, i), wb = pick(o.cb, i);
@@ -225,11 +236,13 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         if (a.overlap) {
             __syncthreads();        // barrier initialisation visible to every waiter
             Unit o;
-            if (u0 < u1 && !(failed = !fetch(u0, o)))
+            if (u0 < u1) {
+                fetch(u0, o);
                 with_chain(o, [&](const auto& gg, const auto& gh) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) decode(o, i, first[i], gg, gh);
                 });
+            }
         }
     }
     if (a.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -293,15 +306,15 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     };
     int u = u0;
     if constexpr (kAhead) {
-        if (a.overlap && u0 < u1 && !failed) {
+        if (a.overlap && u0 < u1) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) multiply(u0, i, first[i]);
             ++u;
         }
     }
-    for (; u < u1 && !failed; ++u) {
+    for (; u < u1; ++u) {
         Unit o;
-        if ((failed = !fetch(u, o))) break;
+        fetch(u, o);
         with_chain(o, [&](const auto& gg, const auto& gh) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -348,7 +361,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         __syncwarp();
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this thread sends nothing any more
         if (adds && part == 0) {
-            const bool landed = __all_sync(0xffffffffu, mbar_wait(sums_bar(), 0, a.wait_limit));
+            const bool landed = mbar_wait(sums_bar(), 0, a.wait_limit);
             if (landed) {
                 for (int p = 0; p + 1 < ksplit; ++p) {
                     const float4 f = peer[p * (MT * 32) + threadIdx.x];
