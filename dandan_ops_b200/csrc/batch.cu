@@ -24,6 +24,14 @@ int launch_cost(int nx, int steps, int tsteps, int grid) {
 constexpr int kRangeBlocks = 11, kRangeBlocksCluster = 8;   // blocks of K that equal ranges must gain per SM to pay for their hand-over
 constexpr int kMaxPerTile = 16;      // CTAs per tile looked at: beyond, the partial sums cost more than the shorter ranges give
 
+// Clusters of c CTAs of the kernel that a device of so many SMs runs at the same time: those of a B200 (what
+// cudaOccupancyMaxActiveClusters() says of its 148 SMs), in proportion.  Not asked of the device at hand: which of its SMs are there
+// differs from one to the next, and the plan, and with it the order of the sums, must not.  (A cluster that finds no place waits for one.)
+int cluster_capacity(int c, int sms) {
+    static constexpr int kB200[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    return kB200[c] * sms / 148;
+}
+
 }  // namespace
 
 namespace b2host {
@@ -57,7 +65,7 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);
     // Ranges: equal ones over all SMs, or the same number of CTAs for every tile (shorter hand-over, a few SMs idle).
-    const int sms = int(std::min<int64_t>(sm_count > 0 ? sm_count : 148, steps));
+    const int device_sms = sm_count > 0 ? sm_count : 148, sms = int(std::min<int64_t>(device_sms, steps));
     int best_cost = launch_cost(p.nx, p.steps, tsteps, sms);
     p.grid = sms;
     for (int g = tiles; g <= std::min(sms, kMaxPerTile * tiles); g += tiles) {
@@ -87,7 +95,7 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
             p.parts = 1;
             p.max_parts = int(std::min<int64_t>(p.grid, (tsteps + range - 1) / range + 1));
         }
-    } else if (tiles <= cluster_capacity(2)) {
+    } else if (tiles <= cluster_capacity(2, device_sms)) {
         // A layer whose tiles all find a cluster at the same time (74 of two CTAs on a B200) takes one, or one CTA, per tile: us with the
         // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.2 / 6.7, 8.7 / 7.0, 11.5 / 9.1, 16.2 / 13.1; 4096 x 12288
         // (four) 11.3 / 9.9, 11.7 / 10.2, 15.1 / 11.9, 22.1 / 16.7; 1024 x 2048 (six) 4.7 / 3.0, 5.2 / 3.4, 8.3 / 5.0, 12.6 / 7.7; 8192 x 8192 (two)
@@ -97,7 +105,7 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
         // 12288 16.8 against 17.5; 7168 x 16384 23.2 against 21.6.
         int best = cluster_cost(p.nx, tiles, d.kb, 1), c = 1;
         for (const int size : b2::kBatchClusters) {
-            if (d.kb < size || tiles > cluster_capacity(size) - (size > 2 ? 1 : 0)) continue;
+            if (d.kb < size || tiles > cluster_capacity(size, device_sms) - (size > 2 ? 1 : 0)) continue;
             const int cost = cluster_cost(p.nx, tiles, d.kb, size);
             if (cost < best) { best = cost; c = size; }
         }

@@ -29,7 +29,6 @@ inline int64_t batch_workspace(int64_t m, const b2::Dims& d, int sm_count) {
 }
 
 BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count);
-int cluster_capacity(int c);               // clusters of c CTAs of the kernel that the device runs at the same time
 int launch_batch_ranges(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s);
 int launch_batch_clusters(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s);
 int launch_batch_rounds(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s);
