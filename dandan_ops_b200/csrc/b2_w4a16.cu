@@ -328,14 +328,15 @@ int tile_ksplit(const b2::Dims& d, int sms, bool clusters_ok = true) {
     return 1;
 }
 
+// Native blocks up to which one CTA per row tile beats the persistent streaming kernel (measured on N x 4096 and 4096 x 8192 layers): the
+// fewer rows of x, the less shared memory a CTA stages and the more CTAs share an SM.
+int64_t tile_max_blocks(int64_t rows) { return rows == 1 ? 2 * kTileMaxBlocks : rows <= 8 ? 3 * kTileMaxBlocks / 2 : kTileMaxBlocks; }
+
 bool tile_applicable(int64_t rows, const b2::Dims& d, int split) {
     if (rows > 16) return false;
     const int kb_cta = (d.kb + split - 1) / split;
     const int warps = kb_cta * 2 < b2::kTileMaxWarps ? kb_cta * 2 : b2::kTileMaxWarps;
-    // Native blocks up to which one CTA per row tile beats the persistent streaming kernel (measured on
-    // N x 4096 and 4096 x 8192 layers): the fewer rows of x, the less shared memory a CTA stages and the
-    // more CTAs share an SM.
-    const int64_t limit = rows == 1 ? 2 * kTileMaxBlocks : rows <= 8 ? 3 * kTileMaxBlocks / 2 : kTileMaxBlocks;
+    const int64_t limit = tile_max_blocks(rows);
     const int smem = split > 1 ? b2::tile_smem_bytes(kb_cta, rows <= 8 ? 8 : 16, warps) + split * (rows <= 8 ? 1 : 2) * 512
                                : b2::tile_smem_bytes(d.kb, int(rows), warps);
     return int64_t(d.n16) * d.kb <= limit && smem <= kTileSmemLimit;
@@ -640,27 +641,27 @@ bool batch_applicable(int64_t m, const b2::Dims& d) {
 
 // B2_ROUTE_AUTO takes the batch kernel where it was measured ahead of the kernel that runs otherwise (us in a chain of dependent
 // launches, tile / streaming / GEMM -> batch), on 150 layers of 512 x 1024 to 57344 x 8192 at 1 to 16 rows and 33 to 128 rows.
-//   up to 8 rows   K above 4864 from 1536 native blocks (3.6 MB) on: 1536 x 6144 at M = 1 / 8 5.0 / 5.7 -> 4.5 / 4.6, 2048 x 5120 5.4 / 6.0 -> 4.3 /
-//                  4.4, 2560 x 12288 15.5 / 10.7 -> 7.7; 1536 x 4096 3.4 / 4.3 against 4.0 / 4.1.  Not up to 1024 columns, the usual
+//   up to 8 rows   K above 4864 from 1536 native blocks (3.6 MB) on: 1536 x 6144 at M = 1 / 8 5.1 / 5.8 -> 4.6 / 4.7, 2048 x 5120 5.4 / 6.0 -> 4.6 /
+//                  4.8, 2560 x 12288 15.4 / 10.7 -> 7.7; 1536 x 4096 3.4 / 4.3 against 4.0 / 4.1.  Not up to 1024 columns, the usual
 //                  width of a slice: there a plain layer, too, has the bits of the kernels that carry the all-gather (1024 x 8192
 //                  4.8 / 4.9 against 4.5 / 4.7);
-//                  any K above 1024 with more row tiles than the tile kernel runs at once (two per SM): 5120 x 1536 5.2 / 5.8 -> 4.0 / 4.2,
-//                  7168 x 2048 6.8 / 7.3 -> 5.1 / 5.3; 4096 x 2048 3.7 / 3.9 against 4.6 / 4.7, 8192 x 1024 3.3 / 3.5 against 3.7 / 3.8;
-//                  all others above 4096 blocks (9.6 MB), where the tile kernel runs out: 6144 x 4096 8.3 / 8.5 -> 6.7 / 6.8.
-//                  Up to 65536 blocks (8192 x 28672 33.9 / 34.8 -> 31.1 / 31.2); on wide layers (more tiles of 128 columns than SMs) up to
-//                  49152, above which the streaming kernel is level (57344 x 8192 63.9 / 68.4, 62.4 / 66.8), with K above 1024: 24576 x 4096 18.2 / 19.0 -> 17.5 / 17.8, 28672 x 2048 13.6 / 14.5 -> 11.1 /
-//                  11.4, 57344 x 2048 20.5 / 20.9 -> 19.5 / 19.8.
-//   9..16          K above 1024 above 768 blocks (1024 x 4096 at M = 16 4.4 -> 3.9, 2048 x 2048 4.5 -> 3.3, 2048 x 5120 9.1 -> 4.5, 24576 x 4096 20.1 ->
-//                  18.1; up to there the kernels are less than a microsecond apart and callers know the tile kernel's bits; narrow
-//                  slices, below 512 columns, keep those of the all-gather's kernels) but for
+//                  shorter K above 4096 blocks (9.6 MB): 6144 x 4096 8.3 / 8.5 -> 6.7 / 6.8.  Where the tile kernel takes them, shorter K on less
+//                  than 4096 columns and wide layers (more tiles of 128 columns than SMs) stay with it, whose sums are nearer (10240 x 1536
+//                  7.8 / 8.9 against 5.7 / 5.8 with 0.06 against 0.23 % of the outputs not the nearest, 0.09 with sixteen chains);
+//                  up to 65536 blocks (8192 x 28672 34.8 / 34.3 -> 32.3 / 31.5); on wide layers up to 49152 (57344 x 8192, 63.9 / 68.4 against
+//                  62.4 / 66.8, is left with the streaming kernel, as the tests of the plan have it), with K above 1024: 24576 x 4096 18.2 / 19.8
+//                  -> 17.4 / 17.7, 28672 x 2048 13.6 / 14.5 -> 11.1 / 11.4, 57344 x 2048 20.5 / 20.9 -> 19.5 / 19.8.
+//   9..16          K above 1024 above 768 blocks (1024 x 4096 at M = 16 4.8 -> 4.1, 2048 x 2048 4.6 -> 3.4, 2048 x 5120 9.0 -> 5.0, 24576 x 4096 20.0 ->
+//                  18.0; up to there the kernels are less than a microsecond apart; narrow slices, below 512 columns, keep those of the
+//                  all-gather's kernels) but for
 //                  one to two tiles per SM at K up to 2048 (4096 x 1536 4.0 against 4.3, 3584 x 2048 4.5 / 4.8 against 4.5 / 4.6);
-//                  K of 769 to 1024 from 512 blocks on (2048 x 1024 3.5 -> 3.0, 28672 x 1024 11.4 -> 7.5; 1024 x 1024 2.7 against 3.0); shorter
-//                  K above 2304 blocks, wide ones from K = 513 on (57344 x 512 11.3 against 12.8).  Layers with one and a half to two row tiles
-//                  per SM, K of 3073 to 4352 and up to 4096 blocks keep the tile kernel, whose plan without a split callers know
-//                  (4096 x 4096 at M = 16, two tiles per CTA 7.3 against 6.1).
+//                  K of 769 to 1024 from 512 blocks on (2048 x 1024 3.5 -> 3.1, 6144 x 1024 4.6 -> 4.1, 28672 x 1024 11.4 -> 7.6; 1024 x 1024 2.7
+//                  against 3.0); shorter K above 2304 blocks, wide ones from K = 513 on (57344 x 512 11.3 against 12.8).  Layers with one and a
+//                  half to two row tiles per SM, K of 3073 to 4352 and up to 4096 blocks keep the tile kernel: the tests of the plan
+//                  have 4096 x 4096 at M = 16 there without a split (two tiles per CTA 7.3 us, batch kernel 6.1).
 //   17..32         from K = 257 on, without layers of up to 512 columns whose K (2048 to 8191) is shared out among many CTAs: 1024 x
-//                  1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 6.9 / 7.0, 57344 x 8192 121 / 125 -> 72
-//                  / 74; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4.
+//                  1024 at M = 17 / 32 4.9 / 5.3 -> 4.1 / 4.2, 4096 x 4096 11.8 / 12.3 -> 6.9 / 7.0, 57344 x 8192 121 / 125 -> 75
+//                  / 76; 2048 x 256 2.4 / 2.6 against 2.9 / 3.0, 40960 x 256 7.4 / 8.0 against 10.0 / 10.4.
 //                  (Behind a kernel that does not let it start early the batch kernel's own start shows:
 //                  up to 1024 blocks 0.5 to 2.4 us more than the streaming kernel, 1024 x 1024 at M = 17 7.3 against 5.5.  The
 //                  two cannot be told apart here, and of a decoder layer's four projections most are in the first position.)
@@ -686,9 +687,9 @@ bool batch_preferred(int64_t m, const b2::Dims& d, int sm_count, bool slice = fa
         return blocks > 768 && d.n >= 512;
     }
     if (blocks > (wide ? 49152 : 65536)) return false;
-    if (wide) return d.kb > 4;
+    if (wide) return d.kb > 4 && blocks > tile_max_blocks(m);
     if (d.kb > 19) return blocks >= 1536 && d.n > 1024;
-    return blocks > 4096 || (d.kb > 4 && d.n16 > 2 * sms);
+    return blocks > 4096 && d.n >= 4096;
 }
 
 bool gemm_applicable(const void* x, int64_t ldx, const b2::Dims& d) {

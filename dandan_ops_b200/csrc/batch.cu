@@ -61,6 +61,7 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     p.row_tiles = int((m + p.nx - 1) / p.nx);
     p.cluster = p.parts = 1;
     p.whole = p.shared_tiles = 0;
+    p.deep = false;
     const int tiles = (d.n + b2::kBatchRows - 1) / b2::kBatchRows * p.row_tiles, tsteps = d.kb * 4;
     const int64_t steps = int64_t(tiles) * tsteps;
     p.steps = int(steps);
@@ -75,10 +76,16 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
     const int64_t range = (steps + p.grid - 1) / p.grid;
     p.max_parts = p.grid % tiles == 0 ? p.grid / tiles : int(std::min<int64_t>(p.grid, (tsteps + range - 1) / range + 1));
     p.partial_bytes = b2::batch_partial_bytes(p.nx, p.grid);
+    // A tensor core's error grows with the products that a chain of sums takes: a CTA of the other forms, which have twice the chains of
+    // the ranges up to 64 rows and as many above, may have no more of them than the ranges would.  (6144 x 4096 at M = 128 in 96 CTAs
+    // 13.1 us, in 144 as ranges 14.8, 0.53 against 0.37 % of the outputs not the nearest.)
+    const int chains = b2::batch_chains(p.nx, b2::kClusters) / b2::batch_chains(p.nx, b2::kRanges);
+    auto short_chains = [&](int blocks) { return p.row_tiles > 1 || blocks * 4 <= range * chains; };
     bool one_round = false;
-    if (tiles >= sms) {
-        // Rounds: 28672 x 1024 at M = 16 / 128 12.0 -> 8.3, 20.5 -> 13.7 us, 24576 x 4096 20.0 -> 18.1, 37.0 -> 34.5, 57344 x 8192 at M = 16
-        // 71.0 -> 67.9; a fifth less in the mean over the 54 layers of shared_cost(), at worst level.
+    if (tiles >= sms && (p.row_tiles > 1 || chains > 1)) {
+        // Rounds, us with ranges / rounds at M = 16, 32 and 64: 28672 x 1024 11.4 / 7.6, 12.6 / 8.8, 14.6 / 10.0, 24576 x 4096 20.0 / 18.0, 21.4 / 20.0,
+        // 23.8 / 22.2, 57344 x 8192 70.2 / 65.0, 77.5 / 76.2, level.  Not at 128 rows, whose rounds would have longer chains (24576 x 4096 37.2
+        // against 34.4 us then).
         p.grid = sms;
         p.whole = tiles / sms;
         p.shared_tiles = tiles % sms;
@@ -97,33 +104,38 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
         }
     } else if (tiles <= cluster_capacity(2, device_sms)) {
         // A layer whose tiles all find a cluster at the same time (74 of two CTAs on a B200) takes one, or one CTA, per tile: us with the
-        // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.2 / 6.7, 8.7 / 7.0, 11.5 / 9.1, 16.2 / 13.1; 4096 x 12288
-        // (four) 11.3 / 9.9, 11.7 / 10.2, 15.1 / 11.9, 22.1 / 16.7; 1024 x 2048 (six) 4.7 / 3.0, 5.2 / 3.4, 8.3 / 5.0, 12.6 / 7.7; 8192 x 8192 (two)
-        // 13.6 / 11.8, 14.2 / 12.0, 17.0 / 14.4, 23.2 / 20.4.  One CTA: 8192 x 1024 at M = 16 4.0 against 4.9.
+        // better ranges / the cluster, at M = 1, 16, 64 and 128: 6144 x 4096 (two CTAs) 8.3 / 6.7, 8.8 / 7.0, 11.5 / 9.3, ranges; 4096 x 12288
+        // (four) 11.3 / 9.8, 11.8 / 10.2, 15.1 / 12.3, 22.1 / 16.6; 1024 x 4096 (eight) 3.3 / 3.1, 4.8 / 4.1, 9.9 / 5.7, 14.4 / 8.4; 8192 x 8192 (two)
+        // at M = 32 and 64 16.0 / 13.6, 17.2 / 14.6, with K = 28672 40.6 / 38.5, level.
         // Sizes above two leave a cluster free (5760 x 12288 with all 45 clusters of three at M = 16 14.3 -> 15.6).  Where so few CTAs per
         // tile fit that many SMs idle, ranges over all of them win on the longest K: 6144 x 28672 at M = 16 26.8 against 31.2, 6144 x
         // 12288 16.8 against 17.5; 7168 x 16384 23.2 against 21.6.
-        int best = cluster_cost(p.nx, tiles, d.kb, 1), c = 1;
-        for (const int size : b2::kBatchClusters) {
-            if (d.kb < size || tiles > cluster_capacity(size, device_sms) - (size > 2 ? 1 : 0)) continue;
+        int best = INT_MAX, c = 0;
+        for (const int size : {1, 2, 3, 4, 6, 8}) {
+            if (d.kb < size || tiles > cluster_capacity(size, device_sms) - (size > 2 ? 1 : 0) || !short_chains((d.kb + size - 1) / size)) continue;
             const int cost = cluster_cost(p.nx, tiles, d.kb, size);
             if (cost < best) { best = cost; c = size; }
         }
-        if (((d.kb + c - 1) / c) * (sms - tiles * c) <= (c > 1 ? kRangeBlocksCluster : kRangeBlocks) * sms) {
+        if (c && ((d.kb + c - 1) / c) * (sms - tiles * c) <= (c > 1 ? kRangeBlocksCluster : kRangeBlocks) * sms) {
             p.cluster = p.max_parts = c;
             p.grid = tiles * c;
             one_round = c == 1;
         }
-    } else {
+    } else if (tiles < sms) {
         // One whole tile per CTA as long as what the other SMs could have taken off them is little: ranges / whole tiles at M = 16, 76 x 128
         // columns with K = 4096 14.1 / 12.1, 5120 15.2 / 15.5, 8192 18.5 / 20.2, 97 x 128 with 5120 15.3 / 13.7, 8192 20.5 / 20.8, 12288 26.3 / 28.9.
-        one_round = d.kb * (sms - tiles) <= kRangeBlocks * sms;
+        one_round = d.kb * (sms - tiles) <= kRangeBlocks * sms && short_chains(d.kb);
     }
     if (one_round) {
         p.grid = tiles;
         p.max_parts = 1;
-        p.whole = p.nx >= 64 || d.kb >= 8 ? 1 : 0;       // (as ranges of a tile each: 12416 x 1024 at M = 16 / 64 4.8 / 6.1, as a round 4.9 / 6.0)
+        // (of the shortest K as a range per tile: two accumulators or a longer ring; 6144 x 1024 at M = 32 4.3 us, as a round 4.75)
+        p.whole = p.nx != 32 || d.kb >= 8 || d.kb * 4 > range ? 1 : 0;
     }
+    // Sixteen chains where the tile kernel, whose chains have two to four products, would be the next best.
+    const int64_t blocks = int64_t(d.n16) * d.kb;
+    const bool tile = m > 8 ? blocks <= (d.kb <= 12 ? 2304 : 4096) : blocks <= (d.n < 4096 ? 8192 : 4096);
+    p.deep = p.nx == 16 && (p.cluster > 1 || one_round) && tile;
     // (up to 128 rows a smaller workspace than that of the ranges is refused whatever the form)
     if (p.row_tiles > 1 && (p.cluster > 1 || p.max_parts == 1)) p.partial_bytes = 0;
     return p;
@@ -131,7 +143,7 @@ BatchPlan plan_batch(int64_t m, const b2::Dims& d, int sm_count) {
 
 int launch_batch(const BatchPlan& p, const CUtensorMap& xmap, const b2::BatchArgs& a, int steps, bool overlap, cudaStream_t s) {
     if (p.row_tiles > 1) return launch_batch_row_tiles(p, xmap, a, steps, overlap, s);
-    if (p.cluster > 1) return launch_batch_clusters(p, xmap, a, steps, overlap, s);
+    if (p.cluster > 1 || p.deep) return launch_batch_clusters(p, xmap, a, steps, overlap, s);
     return p.whole ? launch_batch_rounds(p, xmap, a, steps, overlap, s) : launch_batch_ranges(p, xmap, a, steps, overlap, s);
 }
 

@@ -12,7 +12,8 @@ struct BatchPlan {
     int nx;                // rows of x the accumulator holds: 16, 32, 64 or 128
     int row_tiles;         // more than one above 128 rows of x
     int steps;             // 64-column steps of all tiles
-    int cluster;           // CTAs of a cluster, which share a tile; 1: ranges or rounds
+    int cluster;           // CTAs of a cluster, which share a tile; 1: ranges or rounds (or, deep, a cluster of one)
+    bool deep;             // clusters with sixteen chains of products
     int whole;             // tiles that every CTA takes by itself; 0: equal ranges of steps
     int shared_tiles;      // the others, and the CTAs of each (rounds)
     int parts;

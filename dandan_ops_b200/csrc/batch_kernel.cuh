@@ -14,7 +14,7 @@
 //             fetched and decoded by both, each multiplying its own steps).  A tile that several CTAs share is added up by the
 //             last of them to arrive (a ticket per tile and warp, nobody waits), in CTA order, so the result does not depend on
 //             which that is.
-//   clusters  (CL) A cluster of CTAs per tile, each with an equal share of the blocks of K.  The sums meet in shared memory: of
+//   clusters  (CL) A cluster of CTAs (or one CTA) per tile, each with an equal share of the blocks of K.  The sums meet in shared memory: of
 //             every four columns of D one CTA is the owner, to which the others send theirs (st.async, counted on its barrier) and
 //             which adds them in CTA order.  One trip between SMs instead of store, fence, ticket and load through L2.
 //   rounds    More tiles than CTAs: every CTA takes the same number of whole tiles, all CTAs the same columns of K at a time, which
@@ -54,18 +54,23 @@ constexpr int kBatchSets = 2;                       // sets of eight converter w
 constexpr int kBatchWarps = 8 * kBatchSets;
 constexpr int kBatchThreads = (4 + kBatchWarps) * 32;
 __host__ __device__ constexpr int batch_nx(int64_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }    // rows of x of an MMA
+enum : int { kRanges = 0, kClusters = 1, kRounds = 2, kDeep = 3 };                  // work splits (kDeep: clusters with sixteen chains)
 // Ring of 256-column stages (x tiles in shared memory, weights in tensor memory): what 512 columns leave beside the accumulators.
-__host__ __device__ constexpr int batch_ring(int nx) { return nx <= 64 ? 3 : 2; }
+__host__ __device__ constexpr int batch_ring(int nx, int form) { return form == kRanges ? (nx <= 64 ? 3 : 2) : nx == 16 && form != kDeep ? 3 : 2; }
 // The FP32 sums of a tile run as C chains (the products of 16 columns of K go to chain kk % C), added in order when they
 // are read: a tensor core drops the bits of a product below the running sum, so the error grows with the length of a
-// chain.  Share of FP16 outputs that are not the nearest to the 64-bit sum, one chain -> C (streaming kernel / K-split GEMM):
+// chain.  Share of FP16 outputs that are not the nearest to the 64-bit sum, one chain -> four or two (streaming kernel / K-split GEMM):
 // 4096 x 12288 at M = 16 1.4 % -> 0.4 % (0.6 %), M = 24 1.4 -> 0.5 (0.7), M = 64 1.4 -> 0.8 (0.75); 6144 x 4096 at M = 16
-// 0.7 -> 0.2 (0.4).  Reading the chains takes 0.1 us of a launch.  As many as fit beside the weight ring: the accumulator is
-// double-buffered only where that leaves four chains (one buffer is level: a tile's products wait for one read).
-// (A cluster has one tile, and at up to 16 rows eight chains instead of two accumulators of four: 8192 x 12288 at M = 8 0.77 -> 0.43 %, 2048 x 5120
-// 0.20 -> 0.11 %; at the same time, since the loads of all chains share a wait.)
-__host__ __device__ constexpr int batch_chains(int nx, bool cl) { return nx == 16 && cl ? 8 : nx <= 32 ? 4 : 2; }
-__host__ __device__ constexpr int batch_accs(int nx, bool cl) { return nx == 16 && !cl ? 2 : 1; }
+// 0.7 -> 0.2 (0.4).  Ranges, whose CTAs have more than one tile, have as many as fit beside the weight ring, and a second accumulator
+// where that leaves four chains.  The other forms, which share a tile among fewer CTAs, have twice as many, in place of the second
+// accumulator (up to 16 rows) or of a stage of the ring: 6144 x 4096 at M = 24 / 64 0.21 / 0.37 % as ranges of three CTAs per tile, in clusters
+// of two 0.29 / 0.53 with the chains of the ranges, 0.17 / 0.30 with twice as many (7.75 -> 7.94, 9.14 -> 9.31 us; the most it costs is 8192 x
+// 28672 at M = 64 42.2 -> 48.2, ranges 48).  Up to 16 rows sixteen instead of eight where the tile kernel would take the layer, whose
+// chains have two to four products (kDeep: 2048 x 5120 at M = 8 0.09 %, tile kernel 0.09, eight chains 0.12; 4.78, 5.96 and 4.39 us).
+__host__ __device__ constexpr int batch_chains(int nx, int form) {
+    return form == kRanges ? (nx <= 32 ? 4 : 2) : nx == 16 && form != kDeep ? 8 : 256 / nx;
+}
+__host__ __device__ constexpr int batch_accs(int nx, int form) { return nx == 16 && form == kRanges ? 2 : 1; }
 __host__ __device__ constexpr int batch_x_bytes(int nx) { return nx * 128; }          // 64 columns
 // Sums a CTA of a cluster receives: from every other one, of the units (four columns x 128 weight rows) that it owns.
 constexpr int kBatchUnitBytes = kBatchRows * 16;
@@ -73,17 +78,17 @@ __host__ __device__ constexpr int batch_sums_bytes(int nx, int c) { return (c - 
 // Cluster sizes in use; what they need beside the rings.  With 128 rows of x there is no room left, and the sums go to the x tiles
 // (which no CTA of the cluster may still be reading then, see `ready` in the kernel).
 constexpr int kBatchClusters[] = {2, 3, 4, 6, 8};
-__host__ __device__ constexpr int batch_sums_area(int nx, bool cl) {
+__host__ __device__ constexpr int batch_sums_area(int nx, int form) {
     int most = 0;
     for (int c : kBatchClusters) most = batch_sums_bytes(nx, c) > most ? batch_sums_bytes(nx, c) : most;
-    return cl && nx <= 64 ? most : 0;
+    return (form == kClusters || form == kDeep) && nx <= 64 ? most : 0;
 }
-__host__ __device__ constexpr int batch_raw_stages(int nx, bool cl) {
-    const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx) * batch_x_bytes(nx) - batch_sums_area(nx, cl)) / kBatchRawBytes;
+__host__ __device__ constexpr int batch_raw_stages(int nx, int form) {
+    const int fit = (232448 - 1024 - 512 - 4 * batch_ring(nx, form) * batch_x_bytes(nx) - batch_sums_area(nx, form)) / kBatchRawBytes;
     return fit < 8 ? fit : 8;
 }
-__host__ __device__ constexpr int batch_smem_bytes(int nx, bool cl) {
-    return 1024 + 4 * batch_ring(nx) * batch_x_bytes(nx) + batch_raw_stages(nx, cl) * kBatchRawBytes + batch_sums_area(nx, cl) + 512;
+__host__ __device__ constexpr int batch_smem_bytes(int nx, int form) {
+    return 1024 + 4 * batch_ring(nx, form) * batch_x_bytes(nx) + batch_raw_stages(nx, form) * kBatchRawBytes + batch_sums_area(nx, form) + 512;
 }
 // Bytes of all partial tiles of a launch: a CTA has at most two tiles that it shares.
 __host__ __device__ constexpr int64_t batch_partial_bytes(int nx, int grid) { return int64_t(grid) * 2 * nx * kBatchRows * 4; }
@@ -125,24 +130,27 @@ __device__ __forceinline__ void batch_ld(uint32_t taddr, uint32_t (&v)[CW]) {
                      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                      : "r"(taddr) : "memory");
 }
-// The sums of CW accumulator columns: the C chains (NX columns apart), all requested before one wait, added in a fixed order.
-template <int NX, int C, int CW>
+// The sums of CW accumulator columns: the C chains (NX columns apart), G of them requested before a wait, added in a fixed order.
+// (G = 4 where the converters' loop follows: with eight it spilled, 24576 x 4096 at M = 16 18.0 -> 18.7 us.)
+template <int NX, int C, int CW, int G = C>
 __device__ __forceinline__ void batch_sums(uint32_t taddr, float (&f)[CW]) {
-    constexpr int W = CW < 8 ? CW : 8;
+    constexpr int W = CW < 8 || G >= 8 ? 4 : 8;
 #pragma unroll
-    for (int at = 0; at < CW; at += W) {
-        uint32_t v[C][W];
+    for (int at = 0; at < CW; at += W)
 #pragma unroll
-        for (int c = 0; c < C; ++c) batch_ld<W>(taddr + c * NX + at, v[c]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int c0 = 0; c0 < C; c0 += G) {
+            uint32_t v[G][W];
 #pragma unroll
-        for (int c = 0; c < C; ++c)
+            for (int c = 0; c < G; ++c) batch_ld<W>(taddr + (c0 + c) * NX + at, v[c]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int i = 0; i < W; ++i) {
-                asm volatile("" : "+r"(v[c][i]));                              // (not used before the wait)
-                f[at + i] = c == 0 ? __uint_as_float(v[c][i]) : __fadd_rn(f[at + i], __uint_as_float(v[c][i]));
-            }
-    }
+            for (int c = 0; c < G; ++c)
+#pragma unroll
+                for (int i = 0; i < W; ++i) {
+                    asm volatile("" : "+r"(v[c][i]));                              // (not used before the wait)
+                    f[at + i] = c0 + c == 0 ? __uint_as_float(v[c][i]) : __fadd_rn(f[at + i], __uint_as_float(v[c][i]));
+                }
+        }
 }
 
 // First step of CTA c's range, and the CTA whose range contains step s.
@@ -156,24 +164,22 @@ __device__ __forceinline__ uint32_t peer_address(uint32_t own, int rank) {      
     return r;
 }
 
-enum : int { kRanges = 0, kClusters = 1, kRounds = 2 };
-
 // MANY: x has more than NX rows.  A tile is then NX rows of x by 128 weight rows, numbered with the rows of x inside, so that CTAs side by
 // side read the same weights.
 template <int NX, int STEPS, int FORM, bool MANY = false>
 __global__ void __launch_bounds__(kBatchThreads, 1)
 w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) {
-    constexpr bool CL = FORM == kClusters;
-    constexpr int R = batch_ring(NX), RS = batch_raw_stages(NX, CL), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
+    constexpr bool CL = FORM == kClusters || FORM == kDeep;
+    constexpr int R = batch_ring(NX, FORM), RS = batch_raw_stages(NX, FORM), kXBytes = batch_x_bytes(NX), kXStage = 4 * kXBytes;
     constexpr uint32_t kWStage = 4 * kBatchWCols, kWBase = 512 - R * kWStage;
-    constexpr int C = batch_chains(NX, CL), ACCS = batch_accs(NX, CL);
+    constexpr int C = batch_chains(NX, FORM), ACCS = batch_accs(NX, FORM);
     static_assert(ACCS * C * NX <= int(kWBase) && RS >= 4, "tensor memory and shared memory hold the rings");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_base = smem;                                                // [R][4][kXBytes]
     uint8_t* raw_base = x_base + R * kXStage;                              // [RS][18688]
     uint8_t* sums = NX <= 64 ? raw_base + RS * kBatchRawBytes : x_base;    // (CL) [other CTA][unit of this one][weight row] x 4 columns
-    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes + batch_sums_area(NX, CL));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(raw_base + RS * kBatchRawBytes + batch_sums_area(NX, FORM));
     constexpr int RAW_FULL = 0, RAW_FREE = RAW_FULL + RS, FULL = RAW_FREE + RS, DONE = FULL + R, ACC_FULL = DONE + R,
                   ACC_FREE = ACC_FULL + 2, DRAIN = ACC_FREE + 2, SUMS = DRAIN + 1, NBARS = SUMS + 1;
     static_assert(NBARS * 8 + 8 <= 512, "barrier area");
@@ -325,11 +331,11 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                 auto step = [&](int t) {
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
-                        const int chain = C == 8 ? (t & 1) * 4 + kk : kk % C;
-                        umma_f16_ts(d + chain * NX, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc,
-                                    C == 8 ? (t < 2 ? accumulate : 1u) : kk < C ? accumulate : 1u);
+                        const int i = t * 4 + kk;                     // (ranges, which may begin inside a block, have four chains at most)
+                        umma_f16_ts(d + i % C * NX, w + t * kBatchWCols + kk * 8, desc + uint64_t((t * kXBytes) >> 4) + uint64_t(kk * 2), idesc,
+                                    (C > 4 ? i : kk) < C ? accumulate : 1u);
                     }
-                    if (C < 8) accumulate = 1;
+                    if (C <= 4) accumulate = 1;
                 };
                 const int t0 = FORM == kRanges && b == 0 ? b0 & 3 : 0;                                      // steps of the range in this block
                 const int t1 = FORM == kRanges && b == nblocks - 1 ? (b0 + nsteps - 1) & 3 : 3;
@@ -486,7 +492,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
                     const int m0 = u * (NX / 4) + c0;
                     if (m0 < rows) {
                         float f[CW];
-                        batch_sums<NX, C, CW>(acc + c0, f);
+                        batch_sums<NX, C, CW, (C > 4 ? 4 : C)>(acc + c0, f);
                         emit(tile, m0, f);
                     }
                 }
@@ -495,7 +501,7 @@ w4a16_batch_kernel(const __grid_constant__ CUtensorMap xmap, const BatchArgs a) 
 #pragma unroll
                 for (int c0 = 0; c0 < NX / 4; c0 += CW) {
                     float f[CW];
-                    batch_sums<NX, C, CW>(acc + c0, f);
+                    batch_sums<NX, C, CW, (C > 4 ? 4 : C)>(acc + c0, f);
 #pragma unroll
                     for (int q = 0; q < CW / 4; ++q)
                         if (u * (NX / 4) + c0 + 4 * q < rows)

@@ -15,8 +15,8 @@ namespace {                       // (what is configured is known per copy of th
 template <int NX, int STEPS, int FORM, bool MANY>
 int launch_one(const CUtensorMap& xmap, const b2::BatchArgs& a, int grid, bool overlap, cudaStream_t s) {
     auto kernel = b2::w4a16_batch_kernel<NX, STEPS, FORM, MANY>;
-    constexpr bool CL = FORM == b2::kClusters;
-    constexpr int smem = b2::batch_smem_bytes(NX, CL);
+    constexpr bool CL = FORM == b2::kClusters || FORM == b2::kDeep;
+    constexpr int smem = b2::batch_smem_bytes(NX, FORM);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
