@@ -841,9 +841,16 @@ inline GemmShape gemm_shape(int64_t m, int64_t n, int kb, int sms, bool pairs_ok
 // kernel / 128 x 128 tiles, at M = 129, 256, 512 and 1024: 1024 x 2048 15.8 / 7.5, 16.1 / 7.7, 16.2 / 9.0, 16.2 / 10.7; 1024 x 3072 17.0 / 8.5, 17.2 /
 // 9.3, 17.7 / 9.8, 18.4 / 12.3; 4096 x 1024 12.8 / 8.1, 11.3 / 7.6, 11.5 / 8.8, two rounds 12.6 / 14.5; 6144 x 2048 16.8 / 11.0, 17.6 / 11.6, two rounds
 // 17.9 / 20.2).  Not where K is so long that the batch kernel would take equal ranges over all SMs (1024 x 8192 at M = 1536 28.9 /
-// 32.4).  More rows, and layers from 4096 native blocks on (3072 from K = 3841 on, where the pair kernel splits K), keep the
-// pair kernel's plans, which callers know.
+// 32.4), nor where their chains of products, two per share of K, would be longer than the pair kernel's one, whose error grows with
+// them (3072 x 3072 at M = 512 19.6 / 15.3 us, 0.53 / 0.74 % of the outputs not the nearest).  More rows, and layers from 4096 native blocks
+// on (3072 from K = 3841 on, where the pair kernel splits K), keep the pair kernel, as the tests of its cost model have it (4096 x
+// 4096 at M = 256 20.5 / 14.1).
 constexpr int64_t kBatchTilesMaxM = 1024;
+// Native blocks of K that a CTA pair takes.
+int pair_chain(int64_t m, const b2::Dims& d, int sms) {
+    const int splits = gemm_shape(m, d.n, d.kb, sms).splits;
+    return (d.kb + splits - 1) / splits;
+}
 int batch_tiles(int64_t m, const b2::Dims& d, int sms, int* parts) {
     if (m <= b2::batch_nx(m) || m > kBatchTilesMaxM || d.k % 8 != 0 || g_forced_shape.load(std::memory_order_relaxed) ||
         g_forced_splits.load(std::memory_order_relaxed) || int64_t(d.n16) * d.kb >= (d.kb < 16 ? 4096 : 3072))
@@ -851,6 +858,9 @@ int batch_tiles(int64_t m, const b2::Dims& d, int sms, int* parts) {
     if ((int64_t(d.n) + 127) / 128 * ((m + 127) / 128) > sms) return 0;
     const b2host::BatchPlan p = b2host::plan_batch(m, d, sms);
     if (p.cluster == 1 && p.max_parts > 1) return 0;
+    // (a pair's share is at least four blocks)
+    const int blocks = (d.kb + p.max_parts - 1) / p.max_parts;
+    if (blocks > 8 && pair_chain(m, d, sms) * 2 < blocks) return 0;
     *parts = p.max_parts;
     return p.grid;
 }
@@ -933,7 +943,7 @@ int run_gemm(const void* x, int64_t ldx, const void* native, void* y, int64_t ld
     return vec ? launch_gemm_one<2, 192, true>(map, a, grid, s) : launch_gemm_one<2, 192, false>(map, a, grid, s);
 }
 
-// x [M <= 128, K] through the batch kernel.
+// x [M, K] through the batch kernel: up to 128 rows, or what batch_tiles() takes.
 int run_batch(const void* x, int64_t ldx, const void* native, void* y, int64_t ldy, int64_t m, const b2::Dims& d, void* workspace,
               int64_t workspace_bytes, cudaStream_t s, int sms, const void* bias, int act, int steps, bool overlap) {
     EncodeTiledFn encode = encode_tiled();
