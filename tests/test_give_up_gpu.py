@@ -50,3 +50,17 @@ def test_tile_kernel(m, n, k, offset, skipped, flags):
                                                   (24, 8192, 4096, 1, 1), (64, 2048, 4096, 1, 0)])
 def test_streaming_kernel(m, n, k, offset, skipped, flags):
     check(STREAM, m, n, k, skipped, 1, offset, flags)
+
+
+@pytest.mark.parametrize("flags", [0, _native.FLAG_OVERLAP_LAUNCH])
+@pytest.mark.parametrize("m,n,k,skipped,grid,parts", [
+    (16, 5760, 16384, 0, 135, 3), (64, 12288, 8192, 9, 148, 3), (128, 24576, 4104, 3, 148, 2),                   # ranges
+    (16, 24576, 2064, 1, 148, 3), (64, 20480, 3080, 0, 148, 7), (17, 20480, 3080, 9, 148, 7),                    # rounds, shared tiles first
+    (20, 18952, 264, 0, 148, 1), (24, 16384, 520, 2, 128, 1), (60, 37888, 264, 3, 148, 1),                       # rounds of whole tiles
+    (12, 16384, 4104, 4, 128, 1), (9, 1024, 4104, 1, 48, 6), (16, 8192, 1032, 2, 64, 1),                         # clusters, sixteen chains
+    (17, 6144, 4096, 7, 96, 2), (100, 4096, 8200, 8, 128, 4), (129, 1000, 520, 1, 16, 1), (300, 1024, 2048, 0, 96, 4)])
+def test_batch_kernel(m, n, k, skipped, grid, parts, flags):
+    """The tickets of a shared tile are drawn, and the sums of a cluster waited for, after an abort too."""
+    plan = _native.plan(m, n, k)
+    assert plan["route"] == ("b200_batch" if m <= 128 else "b200_tcgen05") and plan["grid"] == grid and plan["k_splits"] == parts
+    check(_native.ROUTE_AUTO, m, n, k, skipped, 2, flags=flags)
