@@ -58,10 +58,23 @@ def _resolve(x, scales, group_size, backend):
     return None
 
 
+class _Source:
+    """The tensors that something was derived from, held weakly.  They are recognised by themselves: an address, a version and an
+    id come back with other tensors.  A copy or a pickle of this knows none."""
+
+    __slots__ = ("refs",)
+
+    def __init__(self, *tensors):
+        self.refs = tuple(map(weakref.ref, tensors)) or (lambda: None,) * 3
+
+    def __reduce__(self):
+        return _Source, ()
+
+
 # ------------------------------------------------------------------------------------------
 # Native images for callers that hold only reference-layout tensors (the functional form
 # and the torch.ops entry points).  Keyed by tensor identity and version counter; entries
-# die with their tensors.
+# die with their packed weights.
 # ------------------------------------------------------------------------------------------
 _images = {}
 
@@ -75,11 +88,11 @@ def _image_for(packed, scales, zeros, in_features):
     ident = id(packed)
     entry = _images.get(ident)
     key = _state_key(packed, scales, zeros)
-    if entry is not None and entry[0] == key and entry[1]() is packed:
-        return entry[2]
+    if entry is not None and entry[0] == key and entry[1]() is packed and entry[2]() is scales and entry[3]() is zeros:
+        return entry[4]
     image = _native.repack(packed, scales, zeros, in_features)
     ref = weakref.ref(packed, lambda _r, i=ident: _images.pop(i, None))
-    _images[ident] = (key, ref, image)
+    _images[ident] = (key, ref, weakref.ref(scales), weakref.ref(zeros), image)
     return image
 
 
@@ -163,8 +176,8 @@ class QuantizedLinear(torch.nn.Module):
                 layer = cls.__new__(cls)                      # (built while the kernel runs)
                 torch.nn.Module.__init__(layer)
                 layer._set_state(packed, steps, zero_points, weight.shape[1], group_size, bias, backend)
-                key = layer._state_key()
-                layer._set_image(image, key, read_quantizer_flags(flags))
+                key, source = layer._state_key(), _Source(*layer._state())
+                layer._set_image(image, key, source, read_quantizer_flags(flags))
             return layer
         with torch.no_grad():
             codes, steps, zero_points = quantize_int4(weight, group_size)
@@ -242,6 +255,7 @@ class QuantizedLinear(torch.nn.Module):
         return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(), packed._version, scales._version, zeros._version)
 
     _slice_flag = 0
+    _image_source = _checked_source = _bias16_source = _Source()
 
     def serve_as_column_slice(self):
         """This layer is one rank's slice of a column-sharded layer: up to 16 rows of x every call runs the kernels that
@@ -249,17 +263,19 @@ class QuantizedLinear(torch.nn.Module):
         self._slice_flag = _native.FLAG_COLUMN_SLICE
         self._image_flags |= self._slice_flag
 
-    def _set_image(self, image, key, found):
+    def _set_image(self, image, key, source, found):
         """Adopt an image of the state with this key that is complete in memory (its stream has been synchronized); `found`: its
         QUANT_* bits."""
-        self._image, self._image_key = image, key
+        self._image, self._image_key, self._image_source, self._checked_key = image, key, source, None
         self._image_flags = _native.step_flags(found) | self._slice_flag
 
     def _native_image(self):
         key = self._state_key()
-        if self._image is None or self._image_key != key:
-            self._image = _native.repack(self.packed_weight, self.scales, self.zeros, self.in_features)
-            self._image_key = key
+        packed, scales, zeros = self._state()
+        of_packed, of_scales, of_zeros = self._image_source.refs
+        if self._image is None or self._image_key != key or of_packed() is not packed or of_scales() is not scales or of_zeros() is not zeros:
+            self._image = _native.repack(packed, scales, zeros, self.in_features)
+            self._image_key, self._image_source, self._checked_key = key, _Source(packed, scales, zeros), None
             self._image_flags = self._layer_flags() | self._slice_flag
         return self._image
 
@@ -283,7 +299,7 @@ class QuantizedLinear(torch.nn.Module):
                 image.numel() != _native.native_bytes(self.out_features, self.in_features):
             raise ValueError("not a native image of this layer")
         self._image = image
-        self._image_key = self._state_key()
+        self._image_key, self._image_source, self._checked_key = self._state_key(), _Source(*self._state()), None
         self._image_flags = self._slice_flag
         if self.scales.is_cuda and not torch.cuda.is_current_stream_capturing():
             fp16 = bool((self.scales.half().float() == self.scales).all())             # (synchronizes, as _layer_flags)
@@ -295,9 +311,9 @@ class QuantizedLinear(torch.nn.Module):
         if bias is None:
             return None
         key = (bias.data_ptr(), bias._version, bias.dtype)
-        if self._bias16 is None or self._bias16_key != key:
+        if self._bias16 is None or self._bias16_key != key or self._bias16_source.refs[0]() is not bias:
             self._bias16 = bias.detach().to(torch.float16).contiguous()
-            self._bias16_key = key
+            self._bias16_key, self._bias16_source = key, _Source(bias)
         return self._bias16
 
     # -- introspection ---------------------------------------------------------------------
@@ -339,29 +355,32 @@ class QuantizedLinear(torch.nn.Module):
         buffers = self._buffers                              # (as _state: a lookup through Module takes half a microsecond)
         return buffers["bias"] if "bias" in buffers else self.bias
 
-    def _forward_key(self):
-        packed, scales, zeros = self._state()
-        bias = self._bias()
+    def _forward_key(self, packed, scales, zeros, bias):
         return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
                 packed._version, scales._version, zeros._version,
-                id(packed), id(scales), id(zeros),
                 self.in_features, self.group_size, self.backend,
                 None if bias is None else (bias.data_ptr(), bias._version, bias.dtype))
 
     def forward(self, x):
         # Per-token fast path: the metadata checks below depend only on the layer's state, so they
-        # are repeated only when a state tensor was replaced or written (data pointer / version
-        # counter), an attribute was reassigned, or x is not the plain CUDA FP16 case.
-        key = self._forward_key()
-        if (key == self._checked_key and type(x) is torch.Tensor and x.dtype is torch.float16 and x.ndim == 2
+        # are repeated only when a state tensor was replaced or written (the tensor itself, data pointer,
+        # version counter), an attribute was reassigned, or x is not the plain CUDA FP16 case.
+        packed, scales, zeros = self._state()
+        bias = self._bias()
+        key = self._forward_key(packed, scales, zeros, bias)
+        of_packed, of_scales, of_zeros = self._checked_source.refs
+        if (key == self._checked_key and of_packed() is packed and of_scales() is scales and of_zeros() is zeros
+                and (bias is None or (self._bias16_key == key[-1] and self._bias16_source.refs[0]() is bias))
+                and type(x) is torch.Tensor and x.dtype is torch.float16 and x.ndim == 2
                 and x.shape[1] == self.in_features and x.device == self._checked_device
                 and not (x.requires_grad and torch.is_grad_enabled())):
-            bias16 = None if key[-1] is None else self._bias16 if self._bias16_key == key[-1] else self._bias_fp16()
-            return _engine(x, self._image, self.out_features, self.in_features, bias16, self._image_flags)
+            return _engine(x, self._image, self.out_features, self.in_features, None if bias is None else self._bias16, self._image_flags)
         y = self._forward_checked(x)
         if self.backend in ("auto", "cuda", "tensorcore", "naive") and not self.scales.requires_grad \
                 and self._image is not None:
-            self._checked_key, self._checked_device = self._forward_key(), self.packed_weight.device
+            packed, scales, zeros = self._state()
+            self._checked_key, self._checked_source = self._forward_key(packed, scales, zeros, self._bias()), _Source(packed, scales, zeros)
+            self._checked_device = packed.device
         return y
 
     def check_input(self, x):
