@@ -56,8 +56,9 @@ void check_rc(int rc) {
 }
 
 // ---- native images of reference-layout state, for the four legacy ops ---------------------------
+using WeakTensor = c10::weak_intrusive_ptr<c10::TensorImpl>;
 struct ImageEntry {
-    c10::weak_intrusive_ptr<c10::TensorImpl> owner;
+    WeakTensor packed, scales, zeros;      // recognised by themselves: other tensors turn up at the same addresses
     std::tuple<void*, void*, void*, uint32_t, uint32_t, uint32_t, int64_t, int64_t> stamp;
     at::Tensor image;
 };
@@ -73,9 +74,12 @@ at::Tensor image_for(const at::Tensor& packed, const at::Tensor& scales, const a
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         auto it = images().find(id);
-        if (it != images().end() && !it->second.owner.expired() && it->second.stamp == stamp) return it->second.image;
+        auto same = [](const WeakTensor& was, const at::Tensor& is) { return !was.expired() && was._unsafe_get_target() == is.unsafeGetTensorImpl(); };
+        if (it != images().end() && same(it->second.packed, packed) && same(it->second.scales, scales) && same(it->second.zeros, zeros) &&
+            it->second.stamp == stamp)
+            return it->second.image;
         for (auto e = images().begin(); e != images().end();)            // drop entries whose tensors are gone
-            e = e->second.owner.expired() ? images().erase(e) : std::next(e);
+            e = e->second.packed.expired() ? images().erase(e) : std::next(e);
     }
     const int64_t bytes = b2_w4a16_native_bytes(packed.size(0), k);
     TORCH_CHECK(bytes > 0, "W4A16 dimensions exceed the kernel index range");
@@ -84,7 +88,8 @@ at::Tensor image_for(const at::Tensor& packed, const at::Tensor& scales, const a
                              image.data_ptr(), at::cuda::getCurrentCUDAStream().stream()));
     std::lock_guard<std::mutex> lock(g_mutex);
     images().erase(id);
-    images().emplace(id, ImageEntry{c10::weak_intrusive_ptr<c10::TensorImpl>(packed.getIntrusivePtr()), stamp, image});
+    images().emplace(id, ImageEntry{WeakTensor(packed.getIntrusivePtr()), WeakTensor(scales.getIntrusivePtr()), WeakTensor(zeros.getIntrusivePtr()),
+                                    stamp, image});
     return image;
 }
 

@@ -79,11 +79,17 @@ def test_a_state_that_comes_back():
 
 
 @pytest.mark.gpu
-def test_the_functional_form_with_temporary_scales():
-    """Temporaries of one size follow each other at one address."""
+@pytest.mark.parametrize("operator", [False, True])
+def test_state_by_value_with_temporary_scales(operator):
+    """Temporaries of one size follow each other at one address, given to the functional form and to the operators of the reference."""
     g = torch.Generator(device="cuda").manual_seed(3)
     layer = ops.QuantizedLinear.from_float(torch.randn(64, 128, generator=g, device="cuda").half())
     x = torch.randn(3, 128, generator=g, device="cuda").half()
-    call = lambda factor: ops.quantized_linear(x, layer.packed_weight, layer.scales * factor, layer.zeros, in_features=128)
+
+    def call(factor):
+        if operator:
+            return torch.ops.dandan_ops.w4a16_tensorcore(x, layer.packed_weight, layer.scales * factor, layer.zeros, 64)
+        return ops.quantized_linear(x, layer.packed_weight, layer.scales * factor, layer.zeros, in_features=128)
+
     once = call(1.0)
     assert torch.equal(call(2.0), once * 2) and torch.equal(call(1.0), once)
