@@ -20,7 +20,7 @@
 #include "gemm_pair_kernel.cuh"
 #include "tile_kernel.cuh"
 #include "tile_pair_kernel.cuh"
-#include "gather_kernel.cuh"
+#include "gather_mailbox.cuh"
 #include "rmsnorm.cuh"
 #include "batch.cuh"
 

@@ -17,7 +17,7 @@
 //   * the per-warp FP32 accumulator tiles are added in warp order through shared memory, so
 //     the result is bit-reproducible and no workspace, ticket or partial tile is needed;
 //   * layers with few row tiles and a long K run a cluster of 2 or 4 CTAs per row tile, each
-//     on its share of K; the sums of CTAs 1.. reach CTA 0 through distributed shared memory.
+//     on its share of K; the sums of CTAs 1.. are sent to CTA 0's shared memory (st.async, counted on a barrier there).
 // The dequantization chain and the MMA fragment layout are those of stream_kernel.cuh.
 #pragma once
 #include <type_traits>
@@ -42,8 +42,8 @@ struct TileArgs {
     int wait_limit;         // mbarrier polls before a warp gives up (a test passes a small number)
     int fault_block;        // -1; a test passes b >= 0: CTA 0 arms the barrier of its b-th block but skips the copy
     int ksplit;             // 1, 2 or 4: a cluster of that many CTAs shares a row tile, each takes its share
-                            // of the K blocks and the others hand their 16 x 8*MT sums to the first through
-                            // distributed shared memory (layers whose row tiles leave most SMs idle)
+                            // of the K blocks and the others send their 16 x 8*MT sums to the first one's shared
+                            // memory (layers whose row tiles leave most SMs idle)
     int overlap;            // launched as a programmatic dependent of the previous kernel: all weight copies are
                             // requested first, then the kernel waits for that one before it reads x
 };
@@ -145,7 +145,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
     if (ksplit > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
     const int nt = blockIdx.x / ksplit;
     const int kb0 = int(part) * a.kb / ksplit, kbn = (int(part) + 1) * a.kb / ksplit - kb0;
-    const int kb_max = (a.kb + ksplit - 1) / ksplit;     // both CTAs of a pair use one layout
+    const int kb_max = (a.kb + ksplit - 1) / ksplit;     // all CTAs of a cluster use one layout
     const int bar_bytes = ((kb_max * 8 + 127) / 128) * 128;
     uint8_t* blocks = smem + bar_bytes;
     uint8_t* xs = blocks + kb_max * kBlockBytes;
@@ -390,10 +390,10 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         if (__syncthreads_or(failed)) __nanosleep(100000);                 // (but for sums that were on their way when it gave up)
         return;
     }
-    if (ksplit > 1) {
-        // The CTAs of a cluster share the row tile.  Each adds its warps' tiles in warp order; CTA p > 0
-        // puts its 128 * MT sums into slot p - 1 of the first one's shared memory, and after the cluster
-        // barrier the first adds the slots to its own sums in CTA order and writes y.
+    if (GATHER && SPLIT && ksplit > 1) {
+        // The gather form, by plain stores between two cluster barriers: each CTA adds its warps' tiles in warp order; CTA p > 0 puts its
+        // 128 * MT sums into slot p - 1 of the first one's shared memory, and after the cluster barrier the first adds the slots to its
+        // own sums in CTA order and writes y.
         float* tot = reinterpret_cast<float*>(red) + a.warps * MT * 128;       // [MT * 128] own sums
         float* peer = tot + MT * 128;                                          // [ksplit - 1][MT * 128] the others' sums
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
@@ -412,22 +412,6 @@ __device__ __forceinline__ void tile_body(const TileArgs& a, const GatherArgs* g
         }
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (part != 0) return;
-        if (a.act) {
-            for (int e = threadIdx.x; e < MT * 64; e += blockDim.x) {
-                const int mt = e >> 6, rl = (e >> 1) & 31, c = e & 1;
-                const int at = (mt * 32 + rl) * 4 + c;
-                float gate = tot[at], up = tot[at + 2];
-                for (int p = 0; p + 1 < ksplit; ++p) {
-                    gate += peer[p * (MT * 128) + at];
-                    up += peer[p * (MT * 128) + at + 2];
-                }
-                const int rg = rl >> 2, rt = rl & 3;
-                const int m = mt * 8 + 2 * rt + c, n = nt * 16 + rg;
-                if (m < a.m && n + 8 < a.n)
-                    a.y[int64_t(m) * a.ldy + nt * 8 + rg] = silu_mul(finish_output(gate, a.bias, n), finish_output(up, a.bias, n + 8));
-            }
-            return;
-        }
         for (int e = threadIdx.x; e < MT * 128; e += blockDim.x) {
             float sum = tot[e];
             for (int p = 0; p + 1 < ksplit; ++p) sum += peer[p * (MT * 128) + e];
