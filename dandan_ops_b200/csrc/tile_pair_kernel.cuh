@@ -6,9 +6,10 @@
 // bulk copy per 256 columns for the two (neighbouring) native blocks.  As in the tile kernel a unit is half a block, the warps take
 // consecutive units, the first of which each decodes (of its first tile) before the previous kernel has ended, and the warps' sums are
 // added in warp order (the same bits).  The sums' tiles reuse the weights' shared memory.  Bound by the trip of x to every SM (2 us for
-// 128 KB) between the previous kernel's end and the products.  us in a chain of launches at M = 9 / 16, one tile / two per CTA: 4096 x 4096
-// 10.2 / 9.7 -> 7.0 / 7.3, 2560 x 4096 9.5 / 9.5 -> 6.6 / 7.0, 4096 x 2048 4.5 / 4.9 -> 4.4 / 4.6, 2560 x 2048 4.4 / 4.8 -> 4.0 / 4.4.  (Up to 8 rows two
-// CTAs of the tile kernel share an SM and are ahead: 4096 x 4096 at M = 1 / 4 5.1 / 5.4 against 5.4 / 5.5.)
+// 128 KB) between the previous kernel's end and the products.  us in a chain of launches at M = 9 / 16, one tile / two per CTA, on layers
+// that the automatic route leaves to the tile kernel: 4096 x 4096 10.2 / 9.7 -> 7.0 / 7.3, 4096 x 2048 4.5 / 4.9 -> 4.4 / 4.6, 2560 x 2048 4.4 / 4.8 ->
+// 4.0 / 4.4.  (Up to 8 rows two CTAs of the tile kernel share an SM and are ahead: 4096 x 4096 at M = 1 / 4 5.1 / 5.4 against 5.4 / 5.5.)
+// 128 registers; spills of 12 to 24 bytes (stores).
 #pragma once
 #include "tile_kernel.cuh"
 

@@ -39,7 +39,9 @@ extern "C" {
 /* Kernel families selectable through b2_w4a16_linear_route(). */
 #define B2_ROUTE_AUTO 0      /* by size: tile kernel up to 8 rows on layers up to ~10 MB without a long K and up to 16 rows on the
                                 smallest, batch kernel on the others and up to 128 rows (streaming kernel on the widest up to 8
-                                rows and where it does not apply), tensor-memory GEMM above */
+                                rows and where it does not apply), tensor-memory GEMM above.  The choice, and the order in which a
+                                kernel adds its FP32 sums, follow from the arguments of the call (sizes, alignment of x, flags,
+                                workspace) and the device's number of SMs: devices of a kind give the same bits. */
 #define B2_ROUTE_STREAM 1    /* persistent weight-streaming kernel (any M, re-reads the weights every 64 rows) */
 #define B2_ROUTE_TCGEN05 2   /* TMA + tcgen05 GEMM with in-kernel INT4->FP16 converter */
 #define B2_ROUTE_TILE 3      /* one CTA (or a cluster of 2 or 4 CTAs that split K) per 16-row tile, the whole K range
@@ -277,7 +279,7 @@ int b2_w4a16_plan_flags(int64_t m, int64_t n, int64_t k, int flags, int* route, 
  * the process, for tests and tuning.  The single-CTA shapes are rows of x by output columns per
  * CTA; the PAIR shapes run on two SMs per tile (tcgen05 cta_group::2, weights through tensor
  * memory): 256 output columns by 256 or 192 rows of x.  AUTO also has tiles of 128 by 128 of the batch
- * kernel, for layers below 4096 native blocks at up to 1024 rows.  No counterpart in the reference, whose
+ * kernel, for most layers below 4096 native blocks at up to 1024 rows.  No counterpart in the reference, whose
  * route table is fixed offline (dandan_ops/_dispatch.py). */
 #define B2_GEMM_SHAPE_AUTO 0
 #define B2_GEMM_SHAPE_128x128 1
