@@ -255,7 +255,7 @@ class QuantizedLinear(torch.nn.Module):
         return (packed.data_ptr(), scales.data_ptr(), zeros.data_ptr(), packed._version, scales._version, zeros._version)
 
     _slice_flag = 0
-    _image_source = _checked_source = _bias16_source = _Source()
+    _image_source = _bias16_source = _Source()
 
     def serve_as_column_slice(self):
         """This layer is one rank's slice of a column-sharded layer: up to 16 rows of x every call runs the kernels that
@@ -266,21 +266,23 @@ class QuantizedLinear(torch.nn.Module):
     def _set_image(self, image, key, source, found):
         """Adopt an image of the state with this key that is complete in memory (its stream has been synchronized); `found`: its
         QUANT_* bits."""
-        self._image, self._image_key, self._image_source, self._checked_key = image, key, source, None
-        self._image_flags = _native.step_flags(found) | self._slice_flag
+        self._adopt(image, key, source, _native.step_flags(found))
+
+    def _adopt(self, image, key, source, flags):
+        # (in one step, and past Module's attribute hook, which takes about a microsecond per name)
+        self.__dict__.update(_image=image, _image_key=key, _image_source=source, _image_flags=flags | self._slice_flag, _checked_key=None)
 
     def _native_image(self):
         key = self._state_key()
         packed, scales, zeros = self._state()
         of_packed, of_scales, of_zeros = self._image_source.refs
         if self._image is None or self._image_key != key or of_packed() is not packed or of_scales() is not scales or of_zeros() is not zeros:
-            self._image = _native.repack(packed, scales, zeros, self.in_features)
-            self._image_key, self._image_source, self._checked_key = key, _Source(packed, scales, zeros), None
-            self._image_flags = self._layer_flags() | self._slice_flag
+            image = _native.repack(packed, scales, zeros, self.in_features)
+            self._adopt(image, key, _Source(packed, scales, zeros), self._layer_flags(image))
         return self._image
 
-    def _layer_flags(self):
-        """Flags of the C ABI for this layer's image.  FLAG_FP16_STEPS when every step is exactly representable in
+    def _layer_flags(self, image=None):
+        """Flags of the C ABI for an image of this layer (that at hand).  FLAG_FP16_STEPS when every step is exactly representable in
         FP16 (checkpoints with FP16 scales): the decode kernels then use the FP16-only dequantization, which
         is bit-identical for such steps; FLAG_PLAIN_STEPS when none is factored; FLAG_OVERLAP_LAUNCH unless switched off
         (B2_W4A16_OVERLAP=0).  Reads the image's steps once (a host sync), only when an image is (re)built -
@@ -289,7 +291,7 @@ class QuantizedLinear(torch.nn.Module):
             return 0
         # The read synchronizes the stream, so the image is complete in memory from here on: the
         # decode kernel may start under the tail of whatever kernel precedes it (FLAG_OVERLAP_LAUNCH).
-        return _native.step_flags(_native.image_flags(self._image, self.out_features, self.in_features))
+        return _native.step_flags(_native.image_flags(self._image if image is None else image, self.out_features, self.in_features))
 
     def attach_native_image(self, image, factored=True):
         """Use a prebuilt device image of THIS layer's state (e.g. from `checkpoint.ImageCache`)
@@ -298,12 +300,11 @@ class QuantizedLinear(torch.nn.Module):
         if image.dtype != torch.uint8 or image.device != self.packed_weight.device or \
                 image.numel() != _native.native_bytes(self.out_features, self.in_features):
             raise ValueError("not a native image of this layer")
-        self._image = image
-        self._image_key, self._image_source, self._checked_key = self._state_key(), _Source(*self._state()), None
-        self._image_flags = self._slice_flag
+        flags = 0
         if self.scales.is_cuda and not torch.cuda.is_current_stream_capturing():
             fp16 = bool((self.scales.half().float() == self.scales).all())             # (synchronizes, as _layer_flags)
-            self._image_flags |= _native.step_flags((0 if fp16 else _native.QUANT_STEP_NOT_FP16) | (_native.QUANT_FACTORED if factored else 0))
+            flags = _native.step_flags((0 if fp16 else _native.QUANT_STEP_NOT_FP16) | (_native.QUANT_FACTORED if factored else 0))
+        self._adopt(image, self._state_key(), _Source(*self._state()), flags)
 
     def _bias_fp16(self):
         """FP16 copy of the bias for the fused epilogue (derived, rebuilt when the bias changes)."""
@@ -312,8 +313,7 @@ class QuantizedLinear(torch.nn.Module):
             return None
         key = (bias.data_ptr(), bias._version, bias.dtype)
         if self._bias16 is None or self._bias16_key != key or self._bias16_source.refs[0]() is not bias:
-            self._bias16 = bias.detach().to(torch.float16).contiguous()
-            self._bias16_key, self._bias16_source = key, _Source(bias)
+            self.__dict__.update(_bias16=bias.detach().to(torch.float16).contiguous(), _bias16_key=key, _bias16_source=_Source(bias))
         return self._bias16
 
     # -- introspection ---------------------------------------------------------------------
@@ -368,7 +368,7 @@ class QuantizedLinear(torch.nn.Module):
         packed, scales, zeros = self._state()
         bias = self._bias()
         key = self._forward_key(packed, scales, zeros, bias)
-        of_packed, of_scales, of_zeros = self._checked_source.refs
+        of_packed, of_scales, of_zeros = self._image_source.refs       # (a new image takes the checked key back)
         if (key == self._checked_key and of_packed() is packed and of_scales() is scales and of_zeros() is zeros
                 and (bias is None or (self._bias16_key == key[-1] and self._bias16_source.refs[0]() is bias))
                 and type(x) is torch.Tensor and x.dtype is torch.float16 and x.ndim == 2
@@ -379,8 +379,7 @@ class QuantizedLinear(torch.nn.Module):
         if self.backend in ("auto", "cuda", "tensorcore", "naive") and not self.scales.requires_grad \
                 and self._image is not None:
             packed, scales, zeros = self._state()
-            self._checked_key, self._checked_source = self._forward_key(packed, scales, zeros, self._bias()), _Source(packed, scales, zeros)
-            self._checked_device = packed.device
+            self.__dict__.update(_checked_key=self._forward_key(packed, scales, zeros, self._bias()), _checked_device=packed.device)
         return y
 
     def check_input(self, x):

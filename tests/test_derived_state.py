@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import dandan_ops_b200 as ops
+from dandan_ops_b200 import _native
 
 
 class _Memory:
@@ -93,3 +94,25 @@ def test_state_by_value_with_temporary_scales(operator):
 
     once = call(1.0)
     assert torch.equal(call(2.0), once * 2) and torch.equal(call(1.0), once)
+
+
+@pytest.mark.gpu
+def test_what_is_known_of_an_image_comes_with_it(monkeypatch):
+    """A read of the new image's steps that fails leaves no image behind that runs under the old one's flags."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    layer = ops.QuantizedLinear.from_float(torch.randn(64, 128, generator=g, device="cuda").half())
+    x = torch.randn(3, 128, generator=g, device="cuda").half()
+    want, steps = layer(x), layer.scales
+    layer.scales = steps.half().float()
+    layer(x)
+    assert layer._image_flags & _native.FLAG_FP16_STEPS
+    layer.scales = steps
+
+    def fails(*args):
+        raise RuntimeError("read")
+
+    with monkeypatch.context() as patch:
+        patch.setattr(_native, "image_flags", fails)
+        with pytest.raises(RuntimeError, match="read"):
+            layer(x)
+    assert torch.equal(layer(x), want) and not layer._image_flags & _native.FLAG_FP16_STEPS
